@@ -832,15 +832,51 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(rx_conv_desc d, const bf16* 
       }
 }
 
-// dbias[co] += sum_p dy[p][co]
-__global__ void k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy, float* __restrict__ db, int pix_per_block) {
+// dbias[co] += sum_p dy[p][co].  Bound by reading dy once (2 B per pixel
+// and channel).  A thread owns one 16-byte chunk of 8 channels and every
+// `lanes`-th pixel of its block's range, so a warp reads whole pixel rows;
+// the block adds its lanes in shared memory and does one atomic add per
+// channel.  With a thread per channel walking 4096 pixels in series (64
+// blocks at 16 x 128^2 pixels, 32-64 busy threads each, one 2-byte load in
+// flight per thread) the eleven layers of a training step took 3,440 us.
+constexpr int kBiasThreads = 256;
+__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy,
+                                                            float* __restrict__ db, int pix_per_block) {
+  __shared__ float part[kBiasThreads][9];  // 8 channels, padded against bank conflicts
   const long long P = (long long)d.N * d.H * d.W;
-  long long p0 = (long long)blockIdx.x * pix_per_block;
-  long long p1 = P < p0 + pix_per_block ? P : p0 + pix_per_block;
-  for (int co = threadIdx.x; co < d.Cout; co += blockDim.x) {
-    float s = 0.0f;
-    for (long long p = p0; p < p1; ++p) s += __bfloat162float(dy[p * d.y_cstride + d.y_coff + co]);
-    atomicAdd(db + co, s);
+  const long long p0 = (long long)blockIdx.x * pix_per_block;
+  const long long p1 = P < p0 + pix_per_block ? P : p0 + pix_per_block;
+  const int chunks = d.Cout / 8;
+  const int width = chunks < kBiasThreads ? chunks : kBiasThreads;  // chunks handled side by side
+  const int lanes = kBiasThreads / width;
+  const int lane = threadIdx.x / width, col = threadIdx.x - lane * width;
+  for (int c0 = 0; c0 < chunks; c0 += width) {
+    const int ck = c0 + col;
+    float s[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    if (lane < lanes && ck < chunks) {
+      const bf16* src = dy + d.y_coff + ck * 8;
+#pragma unroll 4
+      for (long long p = p0 + lane; p < p1; p += lanes) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + p * d.y_cstride));
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = __bfloat1622float2(h[k]);
+          s[2 * k] += f.x;
+          s[2 * k + 1] += f.y;
+        }
+      }
+    }
+    __syncthreads();  // the previous columns' sums have been read
+#pragma unroll
+    for (int k = 0; k < 8; ++k) part[threadIdx.x][k] = s[k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < width * 8; c += kBiasThreads) {
+      if (c0 + c / 8 >= chunks) continue;
+      float t = 0.0f;
+      for (int l = 0; l < lanes; ++l) t += part[l * width + c / 8][c & 7];
+      atomicAdd(db + c0 * 8 + c, t);
+    }
   }
 }
 
@@ -1313,8 +1349,12 @@ int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void*
   k_conv_wgrad<<<grid, 128, 0, st>>>(*d, static_cast<const bf16*>(dy), static_cast<const bf16*>(x), dw, ppb);
   CUDA_TRY(ctx, cudaGetLastError());
   if (db) {
-    int bppb = 4096;
-    k_bias_grad<<<(unsigned)((P + bppb - 1) / bppb), 128, 0, st>>>(*d, static_cast<const bf16*>(dy), db, bppb);
+    // four blocks per SM, each with at least eight loads per thread
+    const int lanes = kBiasThreads / std::min(d->Cout / 8, kBiasThreads);
+    const long long blocks = std::min<long long>((P + 8LL * lanes - 1) / (8LL * lanes), 4LL * ctx->num_sms);
+    const int bppb = (int)((P + blocks - 1) / blocks);
+    k_bias_grad<<<(unsigned)((P + bppb - 1) / bppb), kBiasThreads, 0, st>>>(*d, static_cast<const bf16*>(dy), db,
+                                                                            bppb);
     CUDA_TRY(ctx, cudaGetLastError());
   }
   return RX_OK;

@@ -258,3 +258,23 @@ def test_training_reduces_the_loss():
     assert np.mean(losses[-10:]) < 0.7 * np.mean(losses[:5]), (losses[:5], losses[-10:])
     out = net.denoise(noisy, alb, nrm, dep)
     assert out.shape == (N, H, W, 3) and bool(torch.isfinite(out).all())
+
+
+@pytest.mark.parametrize("P,Cout,stride,off", [(1, 16, 16, 0), (37, 48, 64, 8), (5000, 32, 32, 0), (263, 2064, 2064, 0),
+                                               (70001, 16, 96, 64)])
+def test_bias_gradient_sums_every_pixel(P, Cout, stride, off):
+    """db over block, lane and chunk remainders.  An fp32 sum of n terms in
+    any order is off by at most (n - 1) 2^-24 sum |term| (n 2^-24 covers the
+    second-order terms here)."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(P)
+    dy = torch.randn((1, 1, P, stride), generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.zeros((1, 1, P, 16), dtype=torch.bfloat16, device="cuda")
+    dw = torch.zeros((Cout, 9, 16), device="cuda")
+    db = torch.ones(Cout, device="cuda")
+    d = nat.ConvDesc(1, 1, P, 16, Cout, 16, 0, stride, off)
+    ctx.check(nat.lib().rx_conv_bf16_bwd_weight(ctx.h, ctypes.byref(d), _p(dy), _p(x), _p(dw), _p(db), _stream()))
+    torch.cuda.synchronize()
+    v = _view(dy, off, Cout).double().reshape(P, Cout)
+    bound = (P + 1) * 2.0 ** -24 * (v.abs().sum(0) + 1.0)
+    assert bool(((db.double() - (v.sum(0) + 1.0)).abs() <= bound).all())
