@@ -12,6 +12,7 @@
 // Tensor-core path: tiles staged in shared memory by cp.async (16-byte
 // copies, zero-filled outside the image), fragments loaded with ldmatrix
 // and multiplied with mma.sync m16n8k16 bf16 -> f32.
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -378,16 +379,6 @@ __global__ void __launch_bounds__(128, 1) k_conv_fwd_tc(rx_conv_desc d, const bf
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
 }
 
-// cp.async.wait_group with a run-time count (0..3; larger waits for 3)
-__device__ __forceinline__ void cp_async_wait_n(int n) {
-  switch (n) {
-    case 0: cp_async_wait<0>(); break;
-    case 1: cp_async_wait<1>(); break;
-    case 2: cp_async_wait<2>(); break;
-    default: cp_async_wait<3>(); break;
-  }
-}
-
 // --------------------------------------- forward conv, warp-specialised
 // Persistent row-strip kernel for layers whose weights fit in shared memory
 // beside a ring of input rows.  The weights are loaded once per CTA.  Each
@@ -398,27 +389,39 @@ __device__ __forceinline__ void cp_async_wait_n(int n) {
 // once per strip instead of three times.  Three jobs run in separate warps
 // that hand work to one another through mbarriers, so that copies, MMAs
 // and epilogues of different rows overlap:
-//   warps 5-6: producers.  Each input row of the strip (130 pixels, zero
-//     outside the image) is copied with coalesced 16-byte cp.async into a
-//     ring slot [kc][130 px x 16 B]; once a row's copies have landed the 64
-//     producers make them visible to the tensor cores (proxy fence) and
-//     arrive on `full[slot]`; a slot is refilled after `empty[slot]`.
-//   warp 4 (one thread): MMA issuer.  Output row y reads the slots of rows
-//     y-1, y, y+1; it accumulates into one of two tensor-memory buffers,
-//     commits to `acc_full[buf]`, and releases row y-1's slot (its last
-//     reader) with a commit to `empty`.
-//   warps 0-3: epilogue.  Warp w reads tensor-memory lanes 32 w .. 32 w + 31
-//     (its 32 pixels), adds the bias, applies ReLU, stores bf16 (and fp32),
-//     then arrives on `acc_empty[buf]`.
+//   warp 10: producer (one elected lane).  Each input row of the strip is one
+//     TMA box of 130 pixels x all channels, read as a 5-d tensor (8
+//     channels, pixel, channel chunk, row, image) so that it lands in its
+//     ring slot as [kc][130 px x 16 B] with zeros outside the image, and
+//     completes on `full[slot]`; a slot is refilled after `empty[slot]`.
+//     These 16-byte rows move at 16 B per cycle and SM (measured, from two
+//     rows in flight on), a row in about 0.7 of its MMAs' time at every
+//     channel count.  128 threads copying 16-byte chunks with cp.async kept
+//     the MMAs waiting instead: a row could only be handed over after a
+//     wait_group, one or two rows late.
+//   warps 8-9: MMA issuers (one elected lane each, alternating rows).  Output
+//     row y reads the slots of rows y-1, y, y+1; it accumulates into one of
+//     four tensor-memory buffers, commits to `acc_full[buf]`, and commits to
+//     `empty` of each slot it read (a slot is free after three commits).
+//   warps 0-7: epilogue.  They load the weights, then warps 0-3 serve the
+//     even rows and 4-7 the odd ones: warp w reads tensor-memory lanes
+//     32 (w % 4) .. + 31 (its 32 pixels), adds the bias, applies ReLU, stores
+//     bf16 (and fp32), then arrives on `acc_empty[buf]`.
 // Output channels may be split into G groups of NG (blockIdx.x % G) when
 // all the weights do not fit in shared memory beside the ring; the G CTAs
 // of a strip run side by side and share its input rows through L2.
 // Every wait is bounded: a wait that runs out (or sees another role give
 // up) raises the shared abort flag, the roles stop, outstanding copies and
 // MMAs are waited for (bounded), the device error flag is set.
+// Bound by the MMAs' A-operand reads (40-48 cycles per M=128, K=16 MMA at
+// N <= 64) in the wide layers, by the row hand-overs in the narrow ones.
+// The eleven layers at 1920x1080, back to back: 984 us (2,157 us with one
+// lane-0 issuer looping over the steps, one epilogue group and cp.async
+// producers); 96 -> 32 channels 167 us, 686 TFLOP/s (472 us, 243).
 namespace tc {
 constexpr int PLANE = HALO_W * 16;  // one 8-channel chunk of one row
-__host__ __device__ constexpr int slot_bytes(int cin) { return (cin / 8) * PLANE; }
+// a row slot, on the 128-byte boundary that a TMA box needs
+__host__ __device__ constexpr int slot_bytes(int cin) { return ((cin / 8) * PLANE + 127) / 128 * 128; }
 __host__ __device__ constexpr int weights_bytes(int cin, int cout) { return 9 * cin * cout * 2; }
 constexpr int kMaxSlots = 8;
 }  // namespace tc
@@ -435,6 +438,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 
 // single-thread bounded wait; gives up when the abort flag is raised
 __device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try(bar, parity)) return true;
   const unsigned long long t0 = clock64();
   for (;;) {
     if (mbar_try(bar, parity)) return true;
@@ -460,23 +464,122 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   }
 }
 
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+
+// One M=128, N=NG, K=16 MMA on K-major, no-swizzle operands (SBO 128 B and
+// descriptor version 1 in the high word); lo words as built by the caller.
+template <int NG>
+__device__ __forceinline__ void mma_k16(uint32_t acc_t, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
+  constexpr uint64_t hi = (uint64_t)((128u >> 4) | (1u << 14)) << 32;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(acc_t),
+      "l"(hi | a_lo), "l"(hi | b_lo), "r"(tc::idesc(NG)), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+}
+
+// The MMAs of one output row: taps in order, KS = Cin / 16 steps each; A
+// moves by one pixel per tap column and two planes per step, B walks
+// [tap][kc][co] in order.  The issuing thread's own instructions set the
+// MMA rate unless the sequence is unrolled with compile-time offsets and
+// issued by an elected lane (descriptors then live in uniform registers):
+// a run-time loop over the steps on `lane == 0` took 140 (KS = 2) and 84
+// (KS = 6) cycles per M=128, N=32 MMA, this takes 40 and 45; the tensor
+// core's own A-operand read is about 40.
+template <int NG, int KS>
+__device__ __forceinline__ void issue_row(uint32_t acc_t, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t b_lo) {
+  uint32_t first = 0u;  // the row's first MMA overwrites the accumulator
+#pragma unroll 1
+  for (int dy = 0; dy < 3; ++dy) {
+    const uint32_t row = dy == 0 ? r0 : dy == 1 ? r1 : r2;
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int k = 0; k < KS; ++k)
+        mma_k16<NG>(acc_t, row + (uint32_t)(dx + k * 2 * (tc::PLANE >> 4)), b_lo + (uint32_t)((dx * KS + k) * 2 * NG),
+                    (dx | k) ? 1u : first);
+    b_lo += 3 * KS * 2 * NG;
+    first = 1u;
+  }
+}
+
+// the same for other channel counts
+template <int NG>
+__device__ __forceinline__ void issue_row_any(int ks, uint32_t acc_t, uint32_t r0, uint32_t r1, uint32_t r2,
+                                              uint32_t b_lo) {
+  uint32_t acc = 0u;
+#pragma unroll 1
+  for (int tap = 0; tap < 9; ++tap) {
+    uint32_t a_lo = (tap < 3 ? r0 : tap < 6 ? r1 : r2) + (uint32_t)(tap % 3);
+#pragma unroll 1
+    for (int k = 0; k < ks; ++k) {
+      mma_k16<NG>(acc_t, a_lo, b_lo, acc);
+      acc = 1u;
+      a_lo += 2 * (tc::PLANE >> 4);
+      b_lo += 2 * NG;
+    }
+  }
+}
+
+constexpr int kWsEpilogue = 256;   // warps 0-7: two groups of four, one per accumulator
+constexpr int kWsMmaWarp = kWsEpilogue / 32;  // the first of two
+constexpr int kWsThreads = kWsEpilogue + 64 + 32;
+constexpr int kWsAcc = 4;          // accumulators
+// resident blocks per SM the registers are kept for (shared memory allows
+// more than one only for the narrow layers)
+constexpr int ws_min_blocks(int ng) { return ng <= 64 ? 2 : 1; }
+
+// N consecutive 32-bit tensor-memory columns of the warp's 32 lanes
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t (&r)[N], uint32_t addr) {
+  static_assert(N == 16 || N == 32, "16 or 32 columns");
+  if constexpr (N == 16)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(addr));
+  else
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(addr));
+}
+
+// 32 bytes (one sector) to a 32-byte aligned address
+__device__ __forceinline__ void st_global_32B(void* p, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
 // acc_in (may be null): fp32 partial sums [pixel][Cout] of the other input
 // channels, added before the bias (a layer split over its input channels,
 // conv_fwd); y (may be null): bf16 output.
 template <int NG>
-__global__ void __launch_bounds__(224, 1) k_conv_fwd_ws(rx_conv_desc d, const bf16* __restrict__ x,
+__global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(const __grid_constant__ CUtensorMap xmap, rx_conv_desc d,
                                                         const bf16* __restrict__ w, const float* __restrict__ bias,
                                                         bf16* __restrict__ y, float* __restrict__ y32,
                                                         const float* __restrict__ acc_in, int relu, int S, int G,
                                                         long long per_cta, int* err) {
-  constexpr int TCOLS = 2 * NG < 32 ? 32 : 2 * NG;  // two accumulators
-  constexpr int kProducers = 64;                     // warps 5 and 6
+  constexpr int TCOLS = kWsAcc * NG;  // a power of two, 64 to 512
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long full[tc::kMaxSlots], empty[tc::kMaxSlots];
-  __shared__ __align__(8) unsigned long long acc_full[2], acc_empty[2], mma_done;
+  __shared__ __align__(8) unsigned long long acc_full[kWsAcc], acc_empty[kWsAcc], w_full, mma_done;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int abort_flag;
-  __shared__ float sbias[NG];
+  __shared__ __align__(16) float sbias[NG];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int KC = d.Cin / 8;
   const int SB = tc::slot_bytes(d.Cin);
@@ -492,14 +595,15 @@ __global__ void __launch_bounds__(224, 1) k_conv_fwd_ws(rx_conv_desc d, const bf
   if (tid == 0) {
     abort_flag = 0;
     for (int s = 0; s < S; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&full[s])), "r"(kProducers));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&empty[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&full[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 3;\n" ::"r"(smem_u32(&empty[s])));
     }
-    for (int b = 0; b < 2; ++b) {
+    for (int b = 0; b < kWsAcc; ++b) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&acc_full[b])));
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" ::"r"(smem_u32(&acc_empty[b])));
     }
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mma_done)));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&w_full)), "r"(kWsEpilogue / 32));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_u32(&mma_done)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   for (int c = tid; c < NG; c += blockDim.x) sbias[c] = bias ? bias[grp * NG + c] : 0.0f;
@@ -508,147 +612,150 @@ __global__ void __launch_bounds__(224, 1) k_conv_fwd_ws(rx_conv_desc d, const bf
                  "r"(TCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
-  // this group's weights, once: chunk ((co * 9 + tap) * KC + kc) -> [tap][kc][co][8]
-  for (int c = tid; c < NG * 9 * KC; c += blockDim.x) {
-    int kc = c % KC, ct = c / KC;
-    int tap = ct % 9, co = ct / 9;
-    const bf16* src = w + ((long long)(grp * NG + co) * 9 + tap) * d.Cin + kc * 8;
-    cp_async16(wsm + ((tap * KC + kc) * NG + co) * 16, src, true);
-  }
-  cp_async_commit();
-  cp_async_wait<0>();
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tmem_base;
 
-  if (warp >= 5) {
-    // ------------------------------------------------ producers (cp.async)
-    // consecutive threads copy consecutive 16-byte chunks of a pixel row,
-    // so each warp request is coalesced; a row is signalled `lag` rows
-    // after it was issued, once its copies have landed
-    const int ptid = tid - 5 * 32;
-    const int lag = S - 3 < 2 ? S - 3 : 2;
-    auto signal = [&](int q) {
-      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&full[q % S])) : "memory");
-    };
-    int k = 0;  // rows issued
-    bool ok = true;
-    for (long long u = u0; u < uend && ok;) {
-      const long long col = u / d.H;
-      const int ylo = (int)(u - col * d.H);
-      const int yhi = (int)((long long)ylo + (uend - u) < d.H ? (long long)ylo + (uend - u) : d.H);
-      const int n = (int)(col / xt), x0 = (int)(col % xt) * tc::TILE;
-      for (int r = ylo - 1; r <= yhi; ++r, ++k) {
-        const int s = (int)(k % S);
-        if (!mbar_wait_warp(smem_u32(&empty[s]), (uint32_t)(((k / S) & 1) ^ 1), &abort_flag)) {
-          ok = false;
-          break;
-        }
-        unsigned char* base = rsm + s * SB;
-        const bool row_ok = r >= 0 && r < d.H;
-        const long long rbase = ((long long)n * d.H + r) * d.W;
-        for (int c = ptid; c < tc::HALO_W * KC; c += kProducers) {
-          const int kc = c % KC, px = c / KC;
-          const int xx = x0 + px - 1;
-          const bool in = row_ok && xx >= 0 && xx < d.W;
-          const bf16* src = in ? x + (rbase + xx) * d.x_cstride + d.x_coff + kc * 8 : x;
-          cp_async16(base + kc * tc::PLANE + px * 16, src, in);
-        }
-        cp_async_commit();
-        if (k >= lag) {
-          cp_async_wait_n(lag);
-          signal(k - lag);
-        }
-      }
-      u += yhi - ylo;
-    }
-    cp_async_wait<0>();
-    if (ok)
-      for (int q = k > lag ? k - lag : 0; q < k; ++q) signal(q);
-  } else if (warp == 4) {
-    // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      const uint32_t rb = smem_u32(rsm), wb = smem_u32(wsm);
-      constexpr uint32_t ID = tc::idesc(NG);
-      // descriptor words (K-major, no swizzle): SBO 128 B and version 1 in
-      // the high word; LBO = one plane (A) or NG x 16 B (B) in the low word
-      constexpr uint32_t desc_hi = (128u >> 4) | (1u << 14);
-      const uint32_t a_lbo = (uint32_t)(tc::PLANE >> 4) << 16;
-      const uint32_t b_lo0 = (wb >> 4) | ((uint32_t)NG << 16);
-      int kb = 0;  // ring index of the segment's first row (ylo - 1)
-      int i = 0;         // output rows issued
+  if (warp > kWsMmaWarp + 1) {
+    // ------------------------------------------------ producer (TMA)
+    if (elect_one()) {
+      const uint32_t rb = smem_u32(rsm), row_bytes = (uint32_t)(KC * tc::PLANE);
+      int k = 0;  // rows issued
       bool ok = true;
       for (long long u = u0; u < uend && ok;) {
         const long long col = u / d.H;
         const int ylo = (int)(u - col * d.H);
         const int yhi = (int)((long long)ylo + (uend - u) < d.H ? (long long)ylo + (uend - u) : d.H);
-        const int nrows = yhi - ylo;
-        for (int yy = ylo; yy < yhi; ++yy, ++i) {
-          const int kr = kb + (yy - ylo);  // ring index of row yy - 1
-          int slot[3];
-          for (int q = 0; q < 3; ++q) {
-            slot[q] = (kr + q) % S;
-            if (ok) ok = mbar_wait_abortable(smem_u32(&full[slot[q]]), (uint32_t)(((kr + q) / S) & 1), &abort_flag);
-          }
-          const int b = i & 1;
-          if (ok) ok = mbar_wait_abortable(smem_u32(&acc_empty[b]), (uint32_t)(((i >> 1) & 1) ^ 1), &abort_flag);
+        const int n = (int)(col / xt), x0 = (int)(col % xt) * tc::TILE;
+        for (int r = ylo - 1; r <= yhi; ++r, ++k) {
+          const int s = k % S;
+          ok = mbar_wait_abortable(smem_u32(&empty[s]), (uint32_t)(((k / S) & 1) ^ 1), &abort_flag);
           if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-          const uint32_t acc_t = tmem + (uint32_t)(b * NG);
-          // The issue loop runs on one thread, so its integer work sets
-          // the MMA rate: descriptors are stepped, not rebuilt.  Low words
-          // hold (address >> 4) | (LBO >> 4) << 16; a byte offset of 16 k
-          // adds k.  A: next chunk pair +2 planes, next tap column +1
-          // pixel; B walks [tap][kc][co] in order, 2 NG x 16 B per step.
-          uint32_t b_lo = b_lo0;
-          uint32_t acc = 0u;
-#pragma unroll 1
-          for (int tap = 0; tap < 9; ++tap) {
-            const int dy = tap / 3, dx = tap % 3;
-            uint32_t a_lo = ((rb + (uint32_t)(slot[dy] * SB)) >> 4) + (uint32_t)dx + a_lbo;
-#pragma unroll 2
-            for (int kc0 = 0; kc0 < KC; kc0 += 2) {
-              const uint64_t ad = ((uint64_t)desc_hi << 32) | a_lo;
-              const uint64_t bd = ((uint64_t)desc_hi << 32) | b_lo;
-              asm volatile(
-                  "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                  "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(acc_t),
-                  "l"(ad), "l"(bd), "r"(ID), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
-              acc = 1u;
-              a_lo += 2 * (tc::PLANE >> 4);
-              b_lo += 2 * NG;
-            }
-          }
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                           smem_u32(&acc_full[b]))
+          const uint32_t bar = smem_u32(&full[s]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(row_bytes)
                        : "memory");
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                           smem_u32(&empty[slot[0]]))
-                       : "memory");
+          asm volatile(
+              "cp.async.bulk.tensor.5d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, "
+              "%5, %6}], [%7];\n" ::"r"(rb + (uint32_t)(s * SB)),
+              "l"(&xmap), "r"(0), "r"(x0 - 1), "r"(0), "r"(r), "r"(n), "r"(bar)
+              : "memory");
         }
-        if (!ok) break;
-        // rows yhi - 1 and yhi have no later reader in this segment
-        for (int q = 0; q < 2; ++q)
-          asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                           smem_u32(&empty[(kb + nrows + q) % S]))
-                       : "memory");
-        kb += nrows + 2;
-        u += nrows;
+        u += yhi - ylo;
+      }
+      // no copy may be in flight when the block ends
+      const unsigned long long t0 = clock64();
+      for (int q = k > S ? k - S : 0; q < k; ++q)
+        while (!mbar_try(smem_u32(&full[q % S]), (uint32_t)((q / S) & 1)) && clock64() - t0 < tc::kSpinCycles) {
+        }
+    }
+    __syncwarp();
+  } else if (warp >= kWsMmaWarp) {
+    // ------------------------------------------------ MMA issuers
+    // One elected lane of each warp walks the rows, warp 0 of the pair taking
+    // the even and warp 1 the odd ones: a row's waits cost several hundred
+    // cycles even when nothing has to be waited for, and the tensor core's
+    // queue is too short to cover them, so the other warp's row does.
+    const int mw = warp - kWsMmaWarp;
+    const uint32_t rb = smem_u32(rsm), wb = smem_u32(wsm);
+    // descriptor low words: (address >> 4) | (LBO >> 4) << 16, LBO = one
+    // plane (A) or NG x 16 B (B)
+    const uint32_t a_lo0 = (rb >> 4) | ((uint32_t)(tc::PLANE >> 4) << 16);
+    const uint32_t b_lo0 = (wb >> 4) | ((uint32_t)NG << 16);
+    const uint32_t slot16 = (uint32_t)SB >> 4;
+    if (elect_one()) {
+      auto advance = [&](int& s, uint32_t& ph) {
+        if (++s == S) {
+          s = 0;
+          ph ^= 1u;
+        }
+      };
+      auto wait = [&](unsigned long long* bar, uint32_t ph) {
+        return mbar_wait_abortable(smem_u32(bar), ph, &abort_flag);
+      };
+      int s2 = 0;        // ring slot of the newest input row read so far
+      uint32_t p2 = 0;   // its phase parity
+      int i = 0;         // output rows so far
+      bool ok = wait(&w_full, 0u);
+      for (long long u = u0; u < uend && ok;) {
+        const long long col = u / d.H;
+        const int ylo = (int)(u - col * d.H);
+        const int yhi = (int)((long long)ylo + (uend - u) < d.H ? (long long)ylo + (uend - u) : d.H);
+        const int nrows = yhi - ylo;
+        // rows yy - 1, yy, yy + 1 sit in slots s0, s1, s2
+        int s0 = s2;
+        uint32_t p0 = p2;
+        int s1 = s0;
+        uint32_t p1 = p0;
+        advance(s1, p1);
+        s2 = s1;
+        p2 = p1;
+        advance(s2, p2);
+        for (int r = 0; r < nrows; ++r, ++i) {
+          if ((i & 1) == mw) {
+            const int b = i % kWsAcc;
+            ok = wait(&full[s0], p0) && wait(&full[s1], p1) && wait(&full[s2], p2) &&
+                 wait(&acc_empty[b], (uint32_t)(((i / kWsAcc) & 1) ^ 1));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t acc_t = tmem + (uint32_t)(b * NG);
+            const uint32_t r0 = a_lo0 + (uint32_t)s0 * slot16, r1 = a_lo0 + (uint32_t)s1 * slot16,
+                           r2 = a_lo0 + (uint32_t)s2 * slot16;
+            switch (KC) {
+              case 2: issue_row<NG, 1>(acc_t, r0, r1, r2, b_lo0); break;
+              case 4: issue_row<NG, 2>(acc_t, r0, r1, r2, b_lo0); break;
+              case 8: issue_row<NG, 4>(acc_t, r0, r1, r2, b_lo0); break;
+              case 12: issue_row<NG, 6>(acc_t, r0, r1, r2, b_lo0); break;
+              default: issue_row_any<NG>(KC / 2, acc_t, r0, r1, r2, b_lo0); break;
+            }
+            tc_commit(smem_u32(&acc_full[b]));
+            // an input row is free once its three output rows have read it;
+            // a segment's first and last rows stand in for the missing ones
+            const int n0 = r == 0 ? 3 : 1, n1 = nrows == 1 ? 3 : (r == 0 || r + 1 == nrows) ? 2 : 1,
+                      n2 = r + 1 == nrows ? 3 : 1;
+            for (int q = 0; q < n0; ++q) tc_commit(smem_u32(&empty[s0]));
+            for (int q = 0; q < n1; ++q) tc_commit(smem_u32(&empty[s1]));
+            for (int q = 0; q < n2; ++q) tc_commit(smem_u32(&empty[s2]));
+          }
+          s0 = s1;
+          p0 = p1;
+          s1 = s2;
+          p1 = p2;
+          advance(s2, p2);
+        }
+        u += nrows;  // s2: the next segment's first row follows this one's last
       }
       // every MMA issued has finished before the tensor memory is released
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                       smem_u32(&mma_done))
-                   : "memory");
+      tc_commit(smem_u32(&mma_done));
       const unsigned long long t0 = clock64();
       while (!mbar_try(smem_u32(&mma_done), 0u) && clock64() - t0 < tc::kSpinCycles) {
       }
     }
+    __syncwarp();
   } else {
-    // ------------------------------------------------ epilogue (warps 0-3)
-    const int qtr = warp;  // tensor-memory lanes 32 qtr .. 32 qtr + 31
+    // ------------------------------------------------ epilogue (warps 0-7)
+    // this group's weights first, while the producers fetch the first rows:
+    // chunk ((co * 9 + tap) * KC + kc) -> [tap][kc][co][8]
+    for (int c = tid; c < NG * 9 * KC; c += kWsEpilogue) {
+      const int kc = c % KC, ct = c / KC;
+      const int tap = ct % 9, co = ct / 9;
+      const bf16* src = w + ((long long)(grp * NG + co) * 9 + tap) * d.Cin + kc * 8;
+      cp_async16(wsm + ((tap * KC + kc) * NG + co) * 16, src, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    __syncwarp();
+    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(&w_full)) : "memory");
+    // warps 0-3 take the even output rows (accumulators 0 and 2), 4-7 the odd ones:
+    // one row's tensor-memory loads, arithmetic and stores take a warp about
+    // 700 cycles per 16 channels, as long as its MMAs in the narrow layers,
+    // so each group gets two rows' time
+    constexpr int CW = NG < 32 ? 16 : 32;  // columns per tensor-memory load
+    const int eg = warp >> 2, qtr = warp & 3;  // group; tensor-memory lanes 32 qtr .. 32 qtr + 31
+    const long long y_off = d.y_coff + grp * NG;
+    // whole-sector stores when every 16-channel run of the view starts on one
+    const bool y_sect = ((uintptr_t)y & 31) == 0 && d.y_cstride % 16 == 0 && d.y_coff % 16 == 0;
     int i = 0;
     bool ok = true;
     for (long long u = u0; u < uend && ok;) {
@@ -656,33 +763,30 @@ __global__ void __launch_bounds__(224, 1) k_conv_fwd_ws(rx_conv_desc d, const bf
       const int ylo = (int)(u - col * d.H);
       const int yhi = (int)((long long)ylo + (uend - u) < d.H ? (long long)ylo + (uend - u) : d.H);
       const int n = (int)(col / xt), x0 = (int)(col % xt) * tc::TILE;
+      const int xx = x0 + qtr * 32 + lane;
       for (int yy = ylo; yy < yhi; ++yy, ++i) {
-        const int b = i & 1;
-        if (!mbar_wait_warp(smem_u32(&acc_full[b]), (uint32_t)((i >> 1) & 1), &abort_flag)) {
+        if ((i & 1) != eg) continue;
+        const int b = i % kWsAcc;
+        const uint32_t acc_t = tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)(b * NG);
+        if (!mbar_wait_warp(smem_u32(&acc_full[b]), (uint32_t)((i / kWsAcc) & 1), &abort_flag)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const int xx = x0 + qtr * 32 + lane;
         const long long m = ((long long)n * d.H + yy) * d.W + xx;
 #pragma unroll 1
-        for (int c0 = 0; c0 < NG; c0 += 16) {
-          uint32_t r[16];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-              "[%16];\n"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)(b * NG + c0)));
+        for (int c0 = 0; c0 < NG; c0 += CW) {
+          uint32_t r[CW];
+          tmem_ld(r, acc_t + (uint32_t)c0);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
           if (xx < d.W) {
-            float v[16];
+            float v[CW];
 #pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
+            for (int k = 0; k < CW; ++k) v[k] = __uint_as_float(r[k]);
             if (acc_in) {
               const float4* a4 = reinterpret_cast<const float4*>(acc_in + m * d.Cout + grp * NG + c0);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
+              for (int k = 0; k < CW / 4; ++k) {
                 const float4 a = a4[k];
                 v[4 * k] += a.x;
                 v[4 * k + 1] += a.y;
@@ -691,27 +795,38 @@ __global__ void __launch_bounds__(224, 1) k_conv_fwd_ws(rx_conv_desc d, const bf
               }
             }
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              v[k] = v[k] + sbias[c0 + k];
-              if (relu) v[k] = fmaxf(v[k], 0.0f);
+            for (int k = 0; k < CW / 4; ++k) {
+              const float4 bb = *reinterpret_cast<const float4*>(sbias + c0 + 4 * k);
+              v[4 * k] += bb.x;
+              v[4 * k + 1] += bb.y;
+              v[4 * k + 2] += bb.z;
+              v[4 * k + 3] += bb.w;
             }
-            const long long o = m * d.y_cstride + d.y_coff + grp * NG + c0;
-            if (y) {
-              uint4 pk[2];
-              uint32_t* pw = reinterpret_cast<uint32_t*>(pk);
+            if (relu) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k) {
+              for (int k = 0; k < CW; ++k) v[k] = fmaxf(v[k], 0.0f);
+            }
+            const long long o = m * d.y_cstride + y_off + c0;
+            if (y) {
+              uint32_t pw[CW / 2];
+#pragma unroll
+              for (int k = 0; k < CW / 2; ++k) {
                 __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
                 pw[k] = *reinterpret_cast<uint32_t*>(&h);
               }
-              uint4* dst = reinterpret_cast<uint4*>(y + o);
-              dst[0] = pk[0];
-              dst[1] = pk[1];
+              if (y_sect) {
+#pragma unroll
+                for (int k = 0; k < CW / 16; ++k) st_global_32B(y + o + 16 * k, pw + 8 * k);
+              } else {
+#pragma unroll
+                for (int k = 0; k < CW / 8; ++k)
+                  reinterpret_cast<uint4*>(y + o)[k] = make_uint4(pw[4 * k], pw[4 * k + 1], pw[4 * k + 2], pw[4 * k + 3]);
+              }
             }
             if (y32) {
               float4* d32 = reinterpret_cast<float4*>(y32 + o);
 #pragma unroll
-              for (int k = 0; k < 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+              for (int k = 0; k < CW / 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
             }
           }
         }
@@ -1138,6 +1253,30 @@ static int launch_tc(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
   return RX_OK;
 }
 
+// The input view of `d` as the 5-d tensor that k_conv_fwd_ws's producer
+// reads: (8 channels, W, channel chunks, H, N).  False when the driver has
+// no tensor maps or cannot describe the view.
+static bool ws_input_map(const rx_conv_desc* d, const bf16* x, CUtensorMap* map) {
+  using Encode = decltype(&cuTensorMapEncodeTiled);
+  static const Encode encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess) {
+      cudaGetLastError();
+      return (Encode)nullptr;
+    }
+    return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(fn) : (Encode)nullptr;
+  }();
+  if (!encode) return false;
+  const cuuint64_t px = (cuuint64_t)d->x_cstride * sizeof(bf16);
+  const cuuint64_t dims[5] = {8, (cuuint64_t)d->W, (cuuint64_t)d->Cin / 8, (cuuint64_t)d->H, (cuuint64_t)d->N};
+  const cuuint64_t strides[4] = {px, 16, px * d->W, px * d->W * d->H};
+  const cuuint32_t box[5] = {8, (cuuint32_t)tc::HALO_W, (cuuint32_t)d->Cin / 8, 1, 1}, step[5] = {1, 1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(x + d->x_coff), dims, strides, box, step,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int NG>
 static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
                         float* y32, const float* acc_in, int relu, int S, int smem, cudaStream_t st, int* rc) {
@@ -1150,23 +1289,25 @@ static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf
     }
     attr_dev = ctx->device;
   }
+  CUtensorMap xmap;
+  if (!ws_input_map(d, x, &xmap)) return 0;
   // resident CTAs per SM from shared memory (dynamic + static + the
-  // per-block reservation), capped so that every resident CTA gets its
-  // tensor memory
+  // per-block reservation), capped by the registers (ws_min_blocks) and so
+  // that every resident CTA gets its tensor memory
   cudaFuncAttributes fa{};
   int smem_sm = 0, reserved = 0;
   cudaFuncGetAttributes(&fa, k_conv_fwd_ws<NG>);
   cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device);
-  constexpr int tcols = 2 * NG < 32 ? 32 : 2 * NG;
+  constexpr int tcols = kWsAcc * NG;
   int per_sm = smem_sm / (smem + (int)fa.sharedSizeBytes + reserved);
-  per_sm = std::max(1, std::min(std::min(per_sm, 512 / tcols), 9));  // 9 x 224 threads
+  per_sm = std::max(1, std::min(std::min(per_sm, 512 / tcols), ws_min_blocks(NG)));
   const int G = d->Cout / NG;
   const long long total = (long long)d->N * d->H * ((d->W + tc::TILE - 1) / tc::TILE);
   const long long strips_want = std::max<long long>(1, (long long)ctx->num_sms * per_sm / G);
   const long long per_cta = (total + std::min(total, strips_want) - 1) / std::min(total, strips_want);
   const long long strips = (total + per_cta - 1) / per_cta;
-  k_conv_fwd_ws<NG><<<(unsigned)(strips * G), 224, smem, st>>>(*d, x, w, bias, y, y32, acc_in, relu, S, G,
+  k_conv_fwd_ws<NG><<<(unsigned)(strips * G), kWsThreads, smem, st>>>(xmap, *d, w, bias, y, y32, acc_in, relu, S, G,
                                                                  per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_fwd: %s", cudaGetErrorString(e)), RX_ERR_CUDA);

@@ -278,3 +278,42 @@ def test_bias_gradient_sums_every_pixel(P, Cout, stride, off):
     v = _view(dy, off, Cout).double().reshape(P, Cout)
     bound = (P + 1) * 2.0 ** -24 * (v.abs().sum(0) + 1.0)
     assert bool(((db.double() - (v.sum(0) + 1.0)).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo,ys,yo,y32", [
+    (1, 1, 1, 16, 16, 16, 0, 16, 0, 1),        # one pixel, one row
+    (3, 2, 127, 32, 32, 40, 8, 40, 8, 0),      # one short tile; views off the 32-byte grid
+    (2, 5, 128, 48, 64, 48, 0, 64, 0, 1),      # a whole tile; a step count outside the unrolled ones
+    (1, 700, 129, 16, 32, 16, 0, 32, 0, 0),    # a second tile of one pixel, strips over several blocks
+    (2, 3, 257, 96, 32, 112, 16, 96, 64, 0),   # six steps per tap
+    (1, 33, 130, 64, 128, 64, 0, 128, 0, 0),   # the widest group
+    (1, 7, 140, 192, 64, 192, 0, 64, 0, 1),    # split over the input channels
+    (1, 4, 300, 160, 16, 160, 0, 16, 0, 0),    # many steps, narrow output
+])
+def test_warp_specialised_conv_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo, y32):
+    """Row strips, tiles and ring phases at their edges against float64.  The
+    sum is fp32 over K = 9 Cin products (each add may truncate: K 2^-22 of
+    the absolute sum), the bf16 output rounds by 2^-8 of the value."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + W)
+    xbuf = torch.randn((N, H, W, xs), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((Cout, 9, Cin), generator=g, device="cuda") / np.sqrt(9 * Cin)).to(torch.bfloat16)
+    bias = torch.randn(Cout, generator=g, device="cuda")
+    ybuf = torch.zeros((N, H, W, ys), dtype=torch.bfloat16, device="cuda")
+    f32 = torch.zeros((N, H, W, ys), device="cuda") if y32 else None
+    d = nat.ConvDesc(N, H, W, Cin, Cout, xs, xo, ys, yo)
+    ctx.check(nat.lib().rx_conv_bf16_fwd(ctx.h, ctypes.byref(d), _p(xbuf), _p(w), _p(bias), _p(ybuf), _p(f32), 0,
+                                         _stream()))
+    ctx.check(nat.lib().rx_ctx_sync(ctx.h))
+    x = _view(xbuf, xo, Cin).double().permute(0, 3, 1, 2)
+    wt = w.double().view(Cout, 3, 3, Cin).permute(0, 3, 1, 2)
+    ref = F.conv2d(x, wt, bias.double(), padding=1).permute(0, 2, 3, 1)
+    mag = F.conv2d(x.abs(), wt.abs(), bias.double().abs(), padding=1).permute(0, 2, 3, 1)
+    tol = 9 * Cin * 2.0 ** -22 * mag
+    got = _view(ybuf, yo, Cout).double()
+    assert bool(((got - ref).abs() <= tol + 2.0 ** -8 * ref.abs()).all())
+    if y32:
+        assert bool(((_view(f32, yo, Cout).double() - ref).abs() <= tol).all())
+    mask = torch.ones(ys, dtype=torch.bool, device="cuda")
+    mask[yo:yo + Cout] = False
+    assert not bool(ybuf[..., mask].any())
