@@ -12,6 +12,7 @@
 // Tensor-core path: tiles staged in shared memory by cp.async (16-byte
 // copies, zero-filled outside the image), fragments loaded with ldmatrix
 // and multiplied with mma.sync m16n8k16 bf16 -> f32.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -949,20 +950,26 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(rx_conv_desc d, const bf16* 
 
 // dbias[co] += sum_p dy[p][co].  Bound by reading dy once (2 B per pixel
 // and channel).  A thread owns one 16-byte chunk of 8 channels and every
-// `lanes`-th pixel of its block's range, so a warp reads whole pixel rows;
-// the block adds its lanes in shared memory and does one atomic add per
-// channel.  With a thread per channel walking 4096 pixels in series (64
-// blocks at 16 x 128^2 pixels, 32-64 busy threads each, one 2-byte load in
-// flight per thread) the eleven layers of a training step took 3,440 us.
-constexpr int kBiasThreads = 256;
-__global__ void __launch_bounds__(kBiasThreads) k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy,
-                                                            float* __restrict__ db, int pix_per_block) {
+// `lanes`-th pixel of its block's range, so a warp reads whole pixel rows.
+// The lanes meet in shared memory, the blocks of a cluster in its first
+// block, both in float64, and one fp32 atomic per channel and cluster adds
+// to db: eight atomics in all (an atomic per block, 592 of them, left db at
+// 4.9e-7 of the float64 sum at 16 x 128^2 pixels, against 1.2e-7).
+// With a thread per channel walking 4096 pixels in series (64 blocks, 32-64
+// busy threads each, one 2-byte load in flight per thread) the eleven layers
+// of a training step took 3,440 us.
+constexpr int kBiasThreads = 1024, kBiasCluster = 8, kBiasBlocks = 64;
+constexpr int kBiasWidth = 128;  // channel chunks handled side by side, at most
+__global__ void __cluster_dims__(kBiasCluster, 1, 1) __launch_bounds__(kBiasThreads)
+    k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy, float* __restrict__ db, int pix_per_block) {
   __shared__ float part[kBiasThreads][9];  // 8 channels, padded against bank conflicts
+  __shared__ double sums[kBiasWidth * 8];
+  auto cluster = cooperative_groups::this_cluster();
   const long long P = (long long)d.N * d.H * d.W;
   const long long p0 = (long long)blockIdx.x * pix_per_block;
-  const long long p1 = P < p0 + pix_per_block ? P : p0 + pix_per_block;
+  const long long p1 = P < p0 + pix_per_block ? P : p0 + pix_per_block;  // may be empty
   const int chunks = d.Cout / 8;
-  const int width = chunks < kBiasThreads ? chunks : kBiasThreads;  // chunks handled side by side
+  const int width = chunks < kBiasWidth ? chunks : kBiasWidth;
   const int lanes = kBiasThreads / width;
   const int lane = threadIdx.x / width, col = threadIdx.x - lane * width;
   for (int c0 = 0; c0 < chunks; c0 += width) {
@@ -982,16 +989,23 @@ __global__ void __launch_bounds__(kBiasThreads) k_bias_grad(rx_conv_desc d, cons
         }
       }
     }
-    __syncthreads();  // the previous columns' sums have been read
 #pragma unroll
     for (int k = 0; k < 8; ++k) part[threadIdx.x][k] = s[k];
     __syncthreads();
     for (int c = threadIdx.x; c < width * 8; c += kBiasThreads) {
-      if (c0 + c / 8 >= chunks) continue;
-      float t = 0.0f;
-      for (int l = 0; l < lanes; ++l) t += part[l * width + c / 8][c & 7];
-      atomicAdd(db + c0 * 8 + c, t);
+      double t = 0.0;
+      for (int l = 0; l < lanes; ++l) t += (double)part[l * width + c / 8][c & 7];
+      sums[c] = t;
     }
+    cluster.sync();
+    if (cluster.block_rank() == 0)
+      for (int c = threadIdx.x; c < width * 8; c += kBiasThreads) {
+        if (c0 + c / 8 >= chunks) continue;
+        double t = 0.0;
+        for (int b = 0; b < kBiasCluster; ++b) t += cluster.map_shared_rank(sums, b)[c];
+        atomicAdd(db + c0 * 8 + c, (float)t);
+      }
+    cluster.sync();  // the sums have been read: next columns, or the end
   }
 }
 
@@ -1490,11 +1504,12 @@ int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void*
   k_conv_wgrad<<<grid, 128, 0, st>>>(*d, static_cast<const bf16*>(dy), static_cast<const bf16*>(x), dw, ppb);
   CUDA_TRY(ctx, cudaGetLastError());
   if (db) {
-    // four blocks per SM, each with at least eight loads per thread
-    const int lanes = kBiasThreads / std::min(d->Cout / 8, kBiasThreads);
-    const long long blocks = std::min<long long>((P + 8LL * lanes - 1) / (8LL * lanes), 4LL * ctx->num_sms);
+    // at least eight loads per thread
+    const int lanes = kBiasThreads / std::min(d->Cout / 8, kBiasWidth);
+    const long long clusters = (P + 8LL * lanes * kBiasCluster - 1) / (8LL * lanes * kBiasCluster);
+    const int blocks = kBiasCluster * (int)std::min<long long>(clusters, kBiasBlocks / kBiasCluster);
     const int bppb = (int)((P + blocks - 1) / blocks);
-    k_bias_grad<<<(unsigned)((P + bppb - 1) / bppb), kBiasThreads, 0, st>>>(*d, static_cast<const bf16*>(dy), db,
+    k_bias_grad<<<(unsigned)blocks, kBiasThreads, 0, st>>>(*d, static_cast<const bf16*>(dy), db,
                                                                             bppb);
     CUDA_TRY(ctx, cudaGetLastError());
   }
