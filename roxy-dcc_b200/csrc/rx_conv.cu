@@ -847,6 +847,242 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TCOLS));
 }
 
+// ------------------------------------------- weight gradient on tcgen05
+// dw[co][tap][ci] += sum_p dy[p][co] x[p + off(tap)][ci] as one GEMM per tap
+// with the pixels as K: M = input channels (up to 128 of them), N = output
+// channels, one tensor-memory accumulator per tap, all of them kept for the
+// whole strip of rows a block walks.  The rows arrive by TMA in the forward
+// kernel's slots [channel chunk][pixel x 16 B], which read as MN-major
+// operands (8 channels contiguous, pixels 16 B apart); a tap is the same x
+// slot moved by one pixel or one row, so x and dy are read once for all
+// taps of a block instead of once per tap.  A block holds T taps of N output
+// channels, T * N <= 512 columns: all nine taps up to N = 32, five (then
+// four) at N = 64, three at N = 128; blockIdx.x % G picks its input-channel
+// group, output-channel group and taps.  At the end the strips' sums meet
+// in dw by fp32 atomics (32 consecutive input channels per warp).
+//   warps 0-3: read the accumulators at the end.  warps 4-5: MMA issuers,
+//   each with half of the block's taps, so that one's waits pass under the
+//   other's MMAs.  warp 6: producer.  Waits are bounded as in k_conv_fwd_ws.
+// Bound by the MMAs' operand reads at N <= 32 (72 MMAs of about 40 cycles
+// per 128 pixels), by TMA's 16 B per cycle at N >= 64.  The eleven layers'
+// weight gradients at 16 x 128^2 pixels, back to back: 1,510 us with
+// k_conv_wgrad (a block per tap, each reading x and dy again), 296 us here;
+// 96 -> 32 channels 390 -> 36 us.  Against float64 the sums are off by
+// 1.3e-6 where k_conv_wgrad's were by 3-7e-6.
+struct WgradArgs {
+  int N, H, W, Cin, Cout;
+  int tw, tiles;     // pixels per row tile (a multiple of 16), tiles per row
+  int cm, mg;        // input channels per group, groups
+  int nc, ng;        // output channels per group, groups
+  int taps, tg;      // taps per group, groups
+  int Sx, Sy;        // ring slots of x and dy rows
+  int xslot, yslot;  // bytes
+  int tcols;         // tensor-memory columns (a power of two)
+};
+constexpr int kWgThreads = 224, kWgSlots = 6;
+
+__global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_constant__ CUtensorMap xmap,
+                                                                 const __grid_constant__ CUtensorMap ymap, WgradArgs A,
+                                                                 float* __restrict__ dw, long long per_cta, int* err) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long xfull[kWgSlots], xempty[kWgSlots], yfull[kWgSlots], yempty[kWgSlots], done;
+  __shared__ uint32_t tmem_base;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t sx = (smem_u32(smem_raw) + 127) & ~127u;
+  const uint32_t sy = sx + (uint32_t)(A.Sx * A.xslot);  // dy rows behind the x rows
+  int g = blockIdx.x % (A.mg * A.ng * A.tg);
+  const long long strip = blockIdx.x / (A.mg * A.ng * A.tg);
+  const int tap0 = (g % A.tg) * A.taps, ntap = min(A.taps, 9 - tap0);
+  g /= A.tg;
+  const int co0 = (g % A.ng) * A.nc, ci0 = (g / A.ng) * A.cm;
+  const long long total = (long long)A.N * A.tiles * A.H;  // row tiles, row fastest
+  const long long u0 = strip * per_cta, uend = min(u0 + per_cta, total);
+
+  if (tid == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < kWgSlots; ++s) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&xfull[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_u32(&xempty[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&yfull[s])));
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_u32(&yempty[s])));
+    }
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_u32(&done)));
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)),
+                 "r"(A.tcols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = tmem_base;
+  auto wait = [&](unsigned long long* bar, uint32_t ph) {
+    return mbar_wait_abortable(smem_u32(bar), ph, &abort_flag);
+  };
+
+  if (warp == 6) {
+    // ------------------------------------------------ producer
+    if (elect_one()) {
+      const uint32_t xbytes = (uint32_t)((A.tw + 2) * 16 * (A.cm / 8)), ybytes = (uint32_t)(A.tw * 16 * (A.nc / 8));
+      auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t bar, uint32_t bytes, int px, int chunk, int row,
+                      int img) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+        asm volatile(
+            "cp.async.bulk.tensor.5d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
+            "%6}], [%7];\n" ::"r"(dst),
+            "l"(map), "r"(0), "r"(px), "r"(chunk), "r"(row), "r"(img), "r"(bar)
+            : "memory");
+      };
+      int kx = 0, ky = 0;  // x and dy rows issued
+      bool ok = true;
+      for (long long u = u0; u < uend && ok;) {
+        const long long col = u / A.H;
+        const int ylo = (int)(u - col * A.H), nrows = (int)min((long long)(A.H - ylo), uend - u);
+        const int n = (int)(col / A.tiles), x0 = (int)(col % A.tiles) * A.tw;
+        for (int r = -1; r <= nrows && ok; ++r) {
+          const int s = kx % A.Sx;
+          ok = wait(&xempty[s], (uint32_t)(((kx / A.Sx) & 1) ^ 1));
+          if (!ok) break;
+          load(&xmap, sx + (uint32_t)(s * A.xslot), smem_u32(&xfull[s]), xbytes, x0 - 1, ci0 / 8, ylo + r, n);
+          ++kx;
+          if (r < 1) continue;
+          // dy row r - 1 goes with x rows r - 2 .. r
+          const int t = ky % A.Sy;
+          ok = wait(&yempty[t], (uint32_t)(((ky / A.Sy) & 1) ^ 1));
+          if (!ok) break;
+          load(&ymap, sy + (uint32_t)(t * A.yslot), smem_u32(&yfull[t]), ybytes, x0, co0 / 8, ylo + r - 1, n);
+          ++ky;
+        }
+        u += nrows;
+      }
+      // no copy may be in flight when the block ends
+      const unsigned long long t0 = clock64();
+      for (int q = kx > A.Sx ? kx - A.Sx : 0; q < kx; ++q)
+        while (!mbar_try(smem_u32(&xfull[q % A.Sx]), (uint32_t)((q / A.Sx) & 1)) && clock64() - t0 < tc::kSpinCycles) {
+        }
+      for (int q = ky > A.Sy ? ky - A.Sy : 0; q < ky; ++q)
+        while (!mbar_try(smem_u32(&yfull[q % A.Sy]), (uint32_t)((q / A.Sy) & 1)) && clock64() - t0 < tc::kSpinCycles) {
+        }
+    }
+    __syncwarp();
+  } else if (warp >= 4) {
+    // ------------------------------------------------ MMA issuers
+    if (elect_one()) {
+      // M = 128, N = nc, FP32 accumulate, BF16, both operands MN-major
+      const uint32_t id = tc::idesc(0) | (1u << 15) | (1u << 16) | ((uint32_t)(A.nc >> 3) << 17);
+      // MN-major, no swizzle: LBO (next 8 pixels) 128 B, SBO (next 8
+      // channels) one plane
+      const uint64_t a_hi = (uint64_t)((uint32_t)(A.tw + 2) | (1u << 14)) << 32;
+      const uint64_t b_hi = (uint64_t)((uint32_t)A.tw | (1u << 14)) << 32;
+      auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t p) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n" ::"r"(d),
+            "l"(ad), "l"(bd), "r"(id), "r"(p), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
+      };
+      const uint32_t a0 = (sx >> 4) | (8u << 16), b0 = (sy >> 4) | (8u << 16);
+      const uint32_t xs16 = (uint32_t)A.xslot >> 4, ys16 = (uint32_t)A.yslot >> 4;
+      // this warp's taps [j0, j1) of the block's
+      const int j0 = warp == 4 ? 0 : (ntap + 1) / 2, j1 = warp == 4 ? (ntap + 1) / 2 : ntap;
+      auto advance = [](int& slot, uint32_t& ph, int n) {
+        if (++slot == n) {
+          slot = 0;
+          ph ^= 1u;
+        }
+      };
+      int xs = 0, ys = 0;          // ring slots of the newest x row, of the dy row
+      uint32_t xph = 0, yph = 0;   // their phase parities
+      bool ok = true;
+      uint32_t acc = 0u;           // the first row overwrites the accumulators
+      for (long long u = u0; u < uend && ok;) {
+        const long long col = u / A.H;
+        const int ylo = (int)(u - col * A.H), nrows = (int)min((long long)(A.H - ylo), uend - u);
+        const int x0 = (int)(col % A.tiles) * A.tw;
+        const int ksteps = (min(A.tw, A.W - x0) + 15) / 16;
+        // x rows yy - 1, yy, yy + 1 of output row yy
+        const int sa = xs;
+        ok = wait(&xfull[xs], xph);
+        advance(xs, xph, A.Sx);
+        const int sb = xs;
+        ok = ok && wait(&xfull[xs], xph);
+        advance(xs, xph, A.Sx);
+        int s0 = sa, s1 = sb;
+        for (int r = 0; r < nrows; ++r) {
+          const int s2 = xs;
+          ok = ok && wait(&xfull[s2], xph) && wait(&yfull[ys], yph);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+          const uint32_t r0 = a0 + (uint32_t)s0 * xs16, r1 = a0 + (uint32_t)s1 * xs16, r2 = a0 + (uint32_t)s2 * xs16;
+          uint32_t b_lo = b0 + (uint32_t)ys * ys16;
+#pragma unroll 1
+          for (int j = j0; j < j1; ++j) {
+            const int tap = tap0 + j;
+            const int dx = tap < 3 ? tap : tap < 6 ? tap - 3 : tap - 6;
+            uint32_t a_lo = (tap < 3 ? r0 : tap < 6 ? r1 : r2) + (uint32_t)dx;
+            const uint32_t d = tmem + (uint32_t)(j * A.nc);
+            if (ksteps == 8) {  // compile-time offsets, as in issue_row
+#pragma unroll
+              for (int k = 0; k < 8; ++k) mma(d, a_hi | (a_lo + 16 * k), b_hi | (b_lo + 16 * k), k ? 1u : acc);
+            } else {
+#pragma unroll 1
+              for (int k = 0; k < ksteps; ++k)  // 16 pixels each
+                mma(d, a_hi | (a_lo + 16 * k), b_hi | (b_lo + 16 * k), k ? 1u : acc);
+            }
+          }
+          acc = 1u;
+          tc_commit(smem_u32(&yempty[ys]));
+          tc_commit(smem_u32(&xempty[s0]));
+          if (r + 1 == nrows) {  // the segment's last two x rows have no later reader
+            tc_commit(smem_u32(&xempty[s1]));
+            tc_commit(smem_u32(&xempty[s2]));
+          }
+          s0 = s1;
+          s1 = s2;
+          advance(xs, xph, A.Sx);
+          advance(ys, yph, A.Sy);
+        }
+        u += nrows;
+      }
+      tc_commit(smem_u32(&done));
+    }
+    __syncwarp();
+  }
+  // every MMA issued has finished (also before the tensor memory is released)
+  {
+    const unsigned long long t0 = clock64();
+    while (!mbar_try(smem_u32(&done), 0u)) {
+      if (clock64() - t0 > tc::kSpinCycles) {
+        abort_flag = 1;
+        break;
+      }
+    }
+  }
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (warp < 4 && !abort_flag && u0 < uend) {
+    const int ci = ci0 + warp * 32 + lane;
+    const bool mine = warp * 32 + lane < A.cm && ci < A.Cin;
+    for (int j = 0; j < ntap; ++j)
+      for (int c = 0; c < A.nc; c += 16) {
+        uint32_t r[16];
+        tmem_ld(r, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * A.nc + c));
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        if (mine) {
+          float* o = dw + ((long long)(co0 + c) * 9 + tap0 + j) * A.Cin + ci;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) atomicAdd(o + (long long)k * 9 * A.Cin, __uint_as_float(r[k]));
+        }
+      }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (tid == 0 && abort_flag) atomicOr(err, ERR_BAD_NODE);
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(A.tcols));
+}
+
 // ------------------------------------------------------- weight gradient
 // dw[co][tap][ci] += sum_p dy[p][co] * x[p + off(tap)][ci]
 // GEMM: M = output channels (64), N = input channels (64), K = pixels
@@ -1267,10 +1503,11 @@ static int launch_tc(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
   return RX_OK;
 }
 
-// The input view of `d` as the 5-d tensor that k_conv_fwd_ws's producer
-// reads: (8 channels, W, channel chunks, H, N).  False when the driver has
-// no tensor maps or cannot describe the view.
-static bool ws_input_map(const rx_conv_desc* d, const bf16* x, CUtensorMap* map) {
+// An NHWC view (`C` channels at `v`, pixel stride `stride` elements) as the
+// 5-d tensor (8 channels, W, channel chunks, H, N) whose boxes -- `px`
+// pixels x `chunks` chunks of one row -- land as [chunk][pixel x 16 B].
+// False when the driver has no tensor maps or cannot describe the view.
+static bool row_map(int N, int H, int W, int C, int stride, const bf16* v, int px_box, int chunks, CUtensorMap* map) {
   using Encode = decltype(&cuTensorMapEncodeTiled);
   static const Encode encode = [] {
     void* fn = nullptr;
@@ -1282,11 +1519,11 @@ static bool ws_input_map(const rx_conv_desc* d, const bf16* x, CUtensorMap* map)
     return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Encode>(fn) : (Encode)nullptr;
   }();
   if (!encode) return false;
-  const cuuint64_t px = (cuuint64_t)d->x_cstride * sizeof(bf16);
-  const cuuint64_t dims[5] = {8, (cuuint64_t)d->W, (cuuint64_t)d->Cin / 8, (cuuint64_t)d->H, (cuuint64_t)d->N};
-  const cuuint64_t strides[4] = {px, 16, px * d->W, px * d->W * d->H};
-  const cuuint32_t box[5] = {8, (cuuint32_t)tc::HALO_W, (cuuint32_t)d->Cin / 8, 1, 1}, step[5] = {1, 1, 1, 1, 1};
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(x + d->x_coff), dims, strides, box, step,
+  const cuuint64_t px = (cuuint64_t)stride * sizeof(bf16);
+  const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)C / 8, (cuuint64_t)H, (cuuint64_t)N};
+  const cuuint64_t strides[4] = {px, 16, px * W, px * W * H};
+  const cuuint32_t box[5] = {8, (cuuint32_t)px_box, (cuuint32_t)chunks, 1, 1}, step[5] = {1, 1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(v), dims, strides, box, step,
                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -1304,7 +1541,7 @@ static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf
     attr_dev = ctx->device;
   }
   CUtensorMap xmap;
-  if (!ws_input_map(d, x, &xmap)) return 0;
+  if (!row_map(d->N, d->H, d->W, d->Cin, d->x_cstride, x + d->x_coff, tc::HALO_W, d->Cin / 8, &xmap)) return 0;
   // resident CTAs per SM from shared memory (dynamic + static + the
   // per-block reservation), capped by the registers (ws_min_blocks) and so
   // that every resident CTA gets its tensor memory
@@ -1492,17 +1729,76 @@ int conv_bwd_data(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* w
   return conv_fwd(ctx, &t, dy, w_rot, nullptr, dx, nullptr, 0, st);
 }
 
+// Weight gradient on k_conv_wgrad_ws.  Returns 1 if it launched, 0 if the
+// shape or the pointers do not suit it.
+static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, const bf16* x, float* dw, cudaStream_t st,
+                           int* rc) {
+  if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15)) return 0;
+  const int limit = 232448 - 1024;  // opt-in shared memory per block, less the static part
+  static int attr_dev = -1;
+  if (attr_dev != ctx->device) {
+    if (cudaFuncSetAttribute(k_conv_wgrad_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    attr_dev = ctx->device;
+  }
+  WgradArgs A{};
+  A.N = d->N, A.H = d->H, A.W = d->W, A.Cin = d->Cin, A.Cout = d->Cout;
+  A.tw = std::min(128, (d->W + 15) / 16 * 16);
+  A.tiles = (d->W + A.tw - 1) / A.tw;
+  A.nc = 128;
+  while (d->Cout % A.nc) A.nc >>= 1;  // 16 divides Cout
+  A.ng = d->Cout / A.nc;
+  A.taps = A.nc <= 32 ? 9 : A.nc == 64 ? 5 : 3;
+  A.tg = (9 + A.taps - 1) / A.taps;
+  A.mg = (d->Cin + 127) / 128;
+  A.cm = (d->Cin / 8 + A.mg - 1) / A.mg * 8;
+  A.tcols = 32;
+  while (A.tcols < A.taps * A.nc) A.tcols <<= 1;
+  const int plane = (A.tw + 2) * 16;
+  A.xslot = (A.cm / 8 * plane + 127) / 128 * 128;
+  A.yslot = (A.nc / 8 * A.tw * 16 + 127) / 128 * 128;
+  // M = 128 reads sixteen planes from any x slot: room behind the last one
+  // (the dy slots count; rows past the group's channels are not stored)
+  const int tail = 16 * plane;
+  A.Sy = 3, A.Sx = kWgSlots;
+  auto bytes = [&] { return std::max(A.Sx * A.xslot + A.Sy * A.yslot, (A.Sx - 1) * A.xslot + tail) + 128; };
+  while (bytes() > limit && A.Sx > 4) --A.Sx;
+  while (bytes() > limit && A.Sy > 2) --A.Sy;
+  if (bytes() > limit) return 0;
+  CUtensorMap xmap, ymap;
+  if (!row_map(d->N, d->H, d->W, d->Cin, d->x_cstride, x + d->x_coff, A.tw + 2, A.cm / 8, &xmap) ||
+      !row_map(d->N, d->H, d->W, d->Cout, d->y_cstride, dy + d->y_coff, A.tw, A.nc / 8, &ymap))
+    return 0;
+  // one block per SM (its accumulators take most of the tensor memory)
+  const int G = A.mg * A.ng * A.tg;
+  const long long total = (long long)d->N * d->H * A.tiles;
+  const long long want = std::min(total, std::max<long long>(1, ctx->num_sms / G));
+  const long long per_cta = (total + want - 1) / want, strips = (total + per_cta - 1) / per_cta;
+  k_conv_wgrad_ws<<<(unsigned)(strips * G), kWgThreads, bytes(), st>>>(xmap, ymap, A, dw, per_cta, ctx->d_err);
+  cudaError_t e = cudaGetLastError();
+  *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_bwd_weight: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
+  return 1;
+}
+
 int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* x, float* dw, float* db,
                     cudaStream_t st) {
   if (!conv_ok(d) || !dy || !x || !dw) return set_error(ctx, "conv_bf16_bwd_weight: bad arguments"), RX_ERR_ARG;
   long long P = (long long)d->N * d->H * d->W;
+  int rc = RX_OK;
+  const bool ws = ctx->conv_impl == 0 && launch_wgrad_ws(ctx, d, static_cast<const bf16*>(dy),
+                                                         static_cast<const bf16*>(x), dw, st, &rc);
+  if (rc) return rc;
   // enough pixel chunks to fill the GPU with every (tap, channel block)
   int cb = ((d->Cout + 63) / 64) * ((d->Cin + 63) / 64);
   long long want = (long long)ctx->num_sms * 4 / std::max(1, 9 * cb) + 1;
   int ppb = (int)std::max<long long>(256, ((P + want - 1) / want + 31) / 32 * 32);
-  dim3 grid((unsigned)((P + ppb - 1) / ppb), (unsigned)cb, 9);
-  k_conv_wgrad<<<grid, 128, 0, st>>>(*d, static_cast<const bf16*>(dy), static_cast<const bf16*>(x), dw, ppb);
-  CUDA_TRY(ctx, cudaGetLastError());
+  if (!ws) {
+    dim3 grid((unsigned)((P + ppb - 1) / ppb), (unsigned)cb, 9);
+    k_conv_wgrad<<<grid, 128, 0, st>>>(*d, static_cast<const bf16*>(dy), static_cast<const bf16*>(x), dw, ppb);
+    CUDA_TRY(ctx, cudaGetLastError());
+  }
   if (db) {
     // at least eight loads per thread
     const int lanes = kBiasThreads / std::min(d->Cout / 8, kBiasWidth);

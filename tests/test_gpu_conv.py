@@ -317,3 +317,33 @@ def test_warp_specialised_conv_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo, y3
     mask = torch.ones(ys, dtype=torch.bool, device="cuda")
     mask[yo:yo + Cout] = False
     assert not bool(ybuf[..., mask].any())
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo,ys,yo", [
+    (1, 1, 1, 16, 16, 16, 0, 16, 0),          # one pixel: every tap but the centre reads zeros
+    (2, 3, 17, 32, 32, 40, 8, 48, 16),        # a 32-pixel tile with 15 of them past the image
+    (1, 2, 129, 96, 32, 96, 0, 32, 0),        # a second tile of one pixel
+    (3, 90, 130, 16, 48, 16, 0, 48, 0),       # strips over several blocks and images, three output groups
+    (1, 5, 300, 64, 64, 64, 0, 64, 0),        # nine taps in two groups
+    (2, 9, 33, 128, 128, 128, 0, 192, 64),    # nine taps in three groups, four x slots
+    (1, 6, 40, 272, 96, 272, 0, 96, 0),       # three input groups, the last one short
+    (1, 4, 20, 144, 256, 144, 0, 256, 0),     # two input and two output groups
+])
+def test_weight_gradient_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo):
+    """dw += the float64 gradient, over tiles, strips and channel groups.  An
+    fp32 sum of N H W products whose adds may truncate is off by at most
+    2^-22 N H W of the absolute sum."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + W)
+    x = torch.randn((N, H, W, xs), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randn((N, H, W, ys), generator=g, device="cuda").to(torch.bfloat16)
+    dw = torch.ones((Cout, 9, Cin), device="cuda")
+    d = nat.ConvDesc(N, H, W, Cin, Cout, xs, xo, ys, yo)
+    ctx.check(nat.lib().rx_conv_bf16_bwd_weight(ctx.h, ctypes.byref(d), _p(dy), _p(x), _p(dw), None, _stream()))
+    ctx.check(nat.lib().rx_ctx_sync(ctx.h))
+    xv = F.pad(_view(x, xo, Cin).double(), (0, 0, 1, 1, 1, 1))
+    dv = _view(dy, yo, Cout).double().reshape(-1, Cout)
+    for tap in range(9):
+        cols = xv[:, tap // 3:tap // 3 + H, tap % 3:tap % 3 + W].reshape(-1, Cin)
+        ref, mag = dv.t() @ cols, dv.abs().t() @ cols.abs()
+        assert bool(((dw[:, tap].double() - 1.0 - ref).abs() <= (N * H * W + 2) * 2.0 ** -22 * (mag + 1.0)).all()), tap
