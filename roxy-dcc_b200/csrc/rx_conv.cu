@@ -866,9 +866,8 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
 // Bound by the MMAs' operand reads at N <= 32 (72 MMAs of about 40 cycles
 // per 128 pixels), by TMA's 16 B per cycle at N >= 64.  The eleven layers'
 // weight gradients at 16 x 128^2 pixels, back to back: 1,510 us with
-// k_conv_wgrad (a block per tap, each reading x and dy again), 296 us here;
-// 96 -> 32 channels 390 -> 36 us.  Against float64 the sums are off by
-// 1.3e-6 where k_conv_wgrad's were by 3-7e-6.
+// k_conv_wgrad (a block per tap, each reading x and dy again), 371 us here;
+// 96 -> 32 channels 390 -> 68 us.
 struct WgradArgs {
   int N, H, W, Cin, Cout;
   int tw, tiles;     // pixels per row tile (a multiple of 16), tiles per row
@@ -1729,6 +1728,15 @@ int conv_bwd_data(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* w
   return conv_fwd(ctx, &t, dy, w_rot, nullptr, dx, nullptr, 0, st);
 }
 
+// Pixels per partial sum of the weight gradient: enough of them to fill the
+// GPU with every (tap, 64 x 64 channel block) of k_conv_wgrad.
+static int wgrad_chain(Ctx* ctx, const rx_conv_desc* d) {
+  const long long P = (long long)d->N * d->H * d->W;
+  const int cb = ((d->Cout + 63) / 64) * ((d->Cin + 63) / 64);
+  const long long want = (long long)ctx->num_sms * 4 / std::max(1, 9 * cb) + 1;
+  return (int)std::max<long long>(256, ((P + want - 1) / want + 31) / 32 * 32);
+}
+
 // Weight gradient on k_conv_wgrad_ws.  Returns 1 if it launched, 0 if the
 // shape or the pointers do not suit it.
 static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, const bf16* x, float* dw, cudaStream_t st,
@@ -1745,15 +1753,37 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   }
   WgradArgs A{};
   A.N = d->N, A.H = d->H, A.W = d->W, A.Cin = d->Cin, A.Cout = d->Cout;
-  A.tw = std::min(128, (d->W + 15) / 16 * 16);
-  A.tiles = (d->W + A.tw - 1) / A.tw;
+  // equal tiles of up to 128 pixels: every strip then sums about as many
+  A.tiles = (d->W + 127) / 128;
+  A.tw = ((d->W + A.tiles - 1) / A.tiles + 15) / 16 * 16;
   A.nc = 128;
   while (d->Cout % A.nc) A.nc >>= 1;  // 16 divides Cout
   A.ng = d->Cout / A.nc;
-  A.taps = A.nc <= 32 ? 9 : A.nc == 64 ? 5 : 3;
-  A.tg = (9 + A.taps - 1) / A.taps;
-  A.mg = (d->Cin + 127) / 128;
-  A.cm = (d->Cin / 8 + A.mg - 1) / A.mg * 8;
+  // Pixels one accumulator sums before it meets the others in dw: the split
+  // k_conv_wgrad makes.  The tensor core truncates as it accumulates, so a
+  // sum's distance from the exact one grows with this length (1e-6 of it per
+  // 1,300 pixels); with k_conv_wgrad's split the two kernels agree to a few
+  // 1e-7, where one block per SM (1,772 pixels at 16 x 128^2, against 7,944)
+  // left 96 -> 32 channels 1.7e-5 apart.
+  const int chain = wgrad_chain(ctx, d);
+  const long long total = (long long)d->N * d->H * A.tiles;
+  const long long per_cta = std::max<long long>(1, (long long)chain * A.tiles / d->W);
+  const long long strips = (total + per_cta - 1) / per_cta;
+  // Blocks beyond the strips come from splitting the input channels and the
+  // taps; both read rows again.  The cheapest split by the cycles of a row
+  // (MMAs: about 40 each up to N = 32, N / 2 above; TMA: 16 B per cycle),
+  // the rows of a block and the rounds of blocks.
+  const int mg_min = (d->Cin + 127) / 128, mma = A.nc <= 32 ? 40 : A.nc == 64 ? 48 : 64;
+  double best = 0.0;
+  for (int mg = mg_min; mg <= 4 * mg_min && (mg == mg_min || d->Cin / mg >= 16); ++mg)
+    for (int tg = 1; tg <= 9; ++tg) {
+      const int taps = (9 + tg - 1) / tg, cm = (d->Cin / 8 + mg - 1) / mg * 8;
+      if (taps * A.nc > 512 || (tg - 1) * taps >= 9) continue;
+      const double row = std::max<double>(taps * (A.tw / 16) * mma, (double)((A.tw + 2) * cm + A.tw * A.nc) * 2 / 16);
+      const long long rounds = (strips * mg * A.ng * tg + ctx->num_sms - 1) / ctx->num_sms;
+      const double cost = (double)rounds * ((double)per_cta * row + 8000.0);  // 8,000: a block's start and end
+      if (best == 0.0 || cost < best) best = cost, A.mg = mg, A.cm = cm, A.tg = tg, A.taps = taps;
+    }
   A.tcols = 32;
   while (A.tcols < A.taps * A.nc) A.tcols <<= 1;
   const int plane = (A.tw + 2) * 16;
@@ -1771,11 +1801,7 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   if (!row_map(d->N, d->H, d->W, d->Cin, d->x_cstride, x + d->x_coff, A.tw + 2, A.cm / 8, &xmap) ||
       !row_map(d->N, d->H, d->W, d->Cout, d->y_cstride, dy + d->y_coff, A.tw, A.nc / 8, &ymap))
     return 0;
-  // one block per SM (its accumulators take most of the tensor memory)
   const int G = A.mg * A.ng * A.tg;
-  const long long total = (long long)d->N * d->H * A.tiles;
-  const long long want = std::min(total, std::max<long long>(1, ctx->num_sms / G));
-  const long long per_cta = (total + want - 1) / want, strips = (total + per_cta - 1) / per_cta;
   k_conv_wgrad_ws<<<(unsigned)(strips * G), kWgThreads, bytes(), st>>>(xmap, ymap, A, dw, per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_bwd_weight: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
@@ -1790,11 +1816,8 @@ int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void*
   const bool ws = ctx->conv_impl == 0 && launch_wgrad_ws(ctx, d, static_cast<const bf16*>(dy),
                                                          static_cast<const bf16*>(x), dw, st, &rc);
   if (rc) return rc;
-  // enough pixel chunks to fill the GPU with every (tap, channel block)
-  int cb = ((d->Cout + 63) / 64) * ((d->Cin + 63) / 64);
-  long long want = (long long)ctx->num_sms * 4 / std::max(1, 9 * cb) + 1;
-  int ppb = (int)std::max<long long>(256, ((P + want - 1) / want + 31) / 32 * 32);
   if (!ws) {
+    const int ppb = wgrad_chain(ctx, d), cb = ((d->Cout + 63) / 64) * ((d->Cin + 63) / 64);
     dim3 grid((unsigned)((P + ppb - 1) / ppb), (unsigned)cb, 9);
     k_conv_wgrad<<<grid, 128, 0, st>>>(*d, static_cast<const bf16*>(dy), static_cast<const bf16*>(x), dw, ppb);
     CUDA_TRY(ctx, cudaGetLastError());
