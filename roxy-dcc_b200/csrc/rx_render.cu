@@ -1510,16 +1510,24 @@ int render(Scene* sc, Accum* a, const rx_render_params* p, int frames) {
   // power of two from 32 M to 128 M paths whose state (path SoA, queues,
   // hit and shadow records: ~120 B + 48 B per shadow record slot) fits in a
   // quarter of the free device memory; 128 M paths hold ~22 GB.
+  // The free memory is asked for only when it can matter -- more than 32 M
+  // paths, and a wave buffer that does not hold them yet: the question takes
+  // 70 us, and tens of milliseconds while another process of the machine
+  // holds the driver.
   long long target = p->wave_paths;
   if (target <= 0) {
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
-      cudaGetLastError();
-      free_b = 0;
-    }
-    const long long per_path = 120 + 48LL * (p->direct_light_mode == 1 ? std::max(sc->n_lights, 1) : 1);
+    const int per_shadow = p->direct_light_mode == 1 ? std::max(sc->n_lights, 1) : 1;
     target = 1LL << 27;
-    while (target > (1LL << 25) && (long long)(free_b / 4) < target * per_path) target >>= 1;
+    const long long want = std::min((long long)frames * a->P, target);
+    if (want > (1LL << 25) && (a->cap < want || a->shadow_cap < want * per_shadow)) {
+      size_t free_b = 0, total_b = 0;
+      if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        free_b = 0;
+      }
+      const long long per_path = 120 + 48LL * per_shadow;
+      while (target > (1LL << 25) && (long long)(free_b / 4) < target * per_path) target >>= 1;
+    }
   }
   int spf = (int)std::max<long long>(1, std::min<long long>(frames, target / std::max<long long>(a->P, 1)));
   long long cap = (long long)spf * a->P;
