@@ -440,7 +440,7 @@ __global__ void k_gather_prims(int n, const int* __restrict__ order, int n_tris,
                                float4* __restrict__ prims, float4* __restrict__ shade) {
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     int i = order[k];
-    float4* P = prims + 3 * (size_t)k;
+    float4* P = prims + kPrimQuads * (size_t)k;
     float4* S = shade + 3 * (size_t)k;
     if (i < n_tris) {
       float3 a = f3(v0[3 * i], v0[3 * i + 1], v0[3 * i + 2]);
@@ -448,8 +448,8 @@ __global__ void k_gather_prims(int n, const int* __restrict__ order, int n_tris,
       float3 c = f3(v2[3 * i], v2[3 * i + 1], v2[3 * i + 2]);
       float3 e1 = b - a, e2 = c - a;
       P[0] = make_float4(a.x, a.y, a.z, __int_as_float(PRIM_TRI));
-      P[1] = make_float4(e1.x, e1.y, e1.z, 0.0f);
-      P[2] = make_float4(e2.x, e2.y, e2.z, 0.0f);
+      P[1] = make_float4(e1.x, e1.y, e1.z, e2.x);
+      P[2] = make_float4(e2.y, e2.z, 0.0f, 0.0f);
       S[0] = make_float4(n0[3 * i], n0[3 * i + 1], n0[3 * i + 2], __int_as_float(tri_mat ? tri_mat[i] : 0));
       S[1] = make_float4(n1[3 * i], n1[3 * i + 1], n1[3 * i + 2], __int_as_float(i));
       S[2] = make_float4(n2[3 * i], n2[3 * i + 1], n2[3 * i + 2], 0.0f);
@@ -655,7 +655,8 @@ __global__ void k_lbvh_layout_level(const int* __restrict__ cur, int* __restrict
 // taking both grandchildren (6-8 % fewer visits per ray on the displaced
 // icosphere).  Leaf children stay leaves; internal children that remain
 // become 4-wide nodes of the next level.  Empty binary slots (count 0
-// leaves) are dropped; unused slots get a box at 1e30 and count 0.
+// leaves) are dropped; unused slots get a centre of 1e30, half extent 0 and count
+// 0.
 __global__ void k_bvh4_level(const int* __restrict__ cur, int* __restrict__ next, int* __restrict__ lv,
                              const float4* __restrict__ bin, int n_bin, float4* __restrict__ out4, int* err) {
   const int ncur = lv[LV_NCUR], out_base = lv[LV_BASE];
@@ -738,19 +739,27 @@ __global__ void k_bvh4_level(const int* __restrict__ cur, int* __restrict__ next
         wd[i] = pack_leaf(0, 0);
       }
     }
+    // min, max -> centre, half extent; the half extent is rounded up and
+    // widened by 2^-22 of the box's distance from the origin, so that
+    // [c - h, c + h] holds [min, max] after the slab test's roundings too
+    for (int i = 0; i < k; ++i)
+      for (int a = 0; a < 3; ++a) {
+        const float lo = mn[i][a], hi = mx[i][a], c = 0.5f * lo + 0.5f * hi;
+        const float h = fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo));
+        mn[i][a] = c;
+        mx[i][a] = __fadd_ru(h, 0x1p-22f * fmaxf(fabsf(lo), fabsf(hi)));
+      }
     for (; k < 4; ++k) {
       mn[k][0] = mn[k][1] = mn[k][2] = 1e30f;
-      mx[k][0] = mx[k][1] = mx[k][2] = 1e30f;
+      mx[k][0] = mx[k][1] = mx[k][2] = 0.0f;
       wd[k] = pack_leaf(0, 0);
       ct[k] = 0;
     }
     float4* o = out4 + 8 * (size_t)(out_base + q);
-    o[0] = make_float4(mn[0][0], mn[1][0], mn[2][0], mn[3][0]);
-    o[1] = make_float4(mx[0][0], mx[1][0], mx[2][0], mx[3][0]);
-    o[2] = make_float4(mn[0][1], mn[1][1], mn[2][1], mn[3][1]);
-    o[3] = make_float4(mx[0][1], mx[1][1], mx[2][1], mx[3][1]);
-    o[4] = make_float4(mn[0][2], mn[1][2], mn[2][2], mn[3][2]);
-    o[5] = make_float4(mx[0][2], mx[1][2], mx[2][2], mx[3][2]);
+    for (int a = 0; a < 3; ++a) {
+      o[2 * a] = make_float4(mn[0][a], mn[1][a], mn[2][a], mn[3][a]);
+      o[2 * a + 1] = make_float4(mx[0][a], mx[1][a], mx[2][a], mx[3][a]);
+    }
     o[6] = make_float4(__int_as_float(wd[0]), __int_as_float(wd[1]), __int_as_float(wd[2]), __int_as_float(wd[3]));
     o[7] = make_float4(__int_as_float(ct[0]), __int_as_float(ct[1]), __int_as_float(ct[2]), __int_as_float(ct[3]));
   }
@@ -839,7 +848,7 @@ int build_reference(Ctx* ctx, Scene* sc, int leaf) {
   k_ref_bounds<<<grid_for(ctx, n_nodes), 256, 0, st>>>(n_nodes, left.p, right.p, tstart.p, tcount.p, parent.p,
                                                         order.p, pmin.p, pmax.p, nmin.p, nmax.p, flags.p);
   sc->d_nodes.alloc(ctx, (size_t)4 * n_nodes);
-  sc->d_prims.alloc(ctx, (size_t)3 * n);
+  sc->d_prims.alloc(ctx, (size_t)kPrimQuads * n);
   sc->d_shade.alloc(ctx, (size_t)3 * n);
   if (!all_ok(sc->d_nodes, sc->d_prims, sc->d_shade)) {
     sc->clear_bvh();
@@ -883,7 +892,7 @@ int set_reference_nodes(Ctx* ctx, Scene* sc, int n_nodes, const float* node_min,
   DevBuf<int> l(ctx, n_nodes), r(ctx, n_nodes), s(ctx, n_nodes), c(ctx, n_nodes), ord(ctx, n);
   DevBuf<float3> nmin(ctx, n_nodes), nmax(ctx, n_nodes);
   sc->d_nodes.alloc(ctx, (size_t)4 * n_nodes);
-  sc->d_prims.alloc(ctx, (size_t)3 * n);
+  sc->d_prims.alloc(ctx, (size_t)kPrimQuads * n);
   sc->d_shade.alloc(ctx, (size_t)3 * n);
   if (!all_ok(l, r, s, c, ord, nmin, nmax, sc->d_nodes, sc->d_prims, sc->d_shade)) {
     sc->clear_bvh();
@@ -1017,7 +1026,7 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
   DevBuf<float3> pmin(ctx, n), pmax(ctx, n);
   DevBuf<int> order(ctx, n);
   if (int rc = front_end(ctx, sc, n_obj, d_oa.p, d_ob.p, 1, pmin, pmax, order)) return rc;
-  sc->d_prims.alloc(ctx, (size_t)3 * n);
+  sc->d_prims.alloc(ctx, (size_t)kPrimQuads * n);
   sc->d_shade.alloc(ctx, (size_t)3 * n);
   DevBuf<float3> rb(ctx, 2);
   if (!all_ok(sc->d_prims, sc->d_shade, rb)) {

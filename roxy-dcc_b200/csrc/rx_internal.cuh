@@ -59,11 +59,18 @@ struct Node4 {
   float4 a, b, c, d;
 };
 
-// Primitives in leaf order, three float4 each (48 B):
-//   triangle: a = (v0, kind = 0), b = (v1 - v0, 0), c = (v2 - v0, 0)
+// Primitives in leaf order, one 64-byte record each (kPrimQuads float4, the
+// last unused):
+//   triangle: a = (v0, kind = 0), b = (e1, e2.x), c = (e2.y, e2.z, 0, 0)
+//             with e1 = v1 - v0, e2 = v2 - v0
 //   sphere:   a = (centre, kind = 1), b = (radius, 0, 0, 0), c = 0
 //   cube:     a = (centre, kind = 2), b = (half extents, 0), c = 0
+// Divergent rays pay one pass of the L1 data pipe per lane and load whatever
+// its width, so a record is read as one 32-byte load (a, b) and, for a
+// triangle, one 8-byte load (load_prim); the record keeps both inside one
+// cache line.
 enum PrimKind { PRIM_TRI = 0, PRIM_SPHERE = 1, PRIM_CUBE = 2 };
+constexpr int kPrimQuads = 4;
 
 // Shading record per primitive in leaf order (three float4):
 //   s0 = (n0, material index bits), s1 = (n1, source id bits), s2 = (n2, 0)
@@ -222,14 +229,13 @@ __device__ __forceinline__ float3 make_inv_dir(float3 d) {
 // Moller-Trumbore with the reference's operation order and thresholds
 // (rendering/taichi/intersect.py:57-78).  v0 and the two edges are stored
 // precomputed; e = v - v0 rounds exactly as the reference computes it.
-__device__ __forceinline__ bool tri_hit(float3 o, float3 d, float4 a, float4 b, float4 c, float tmax, float& t,
+__device__ __forceinline__ bool tri_hit(float3 o, float3 d, float3 v0, float3 e1, float3 e2, float tmax, float& t,
                                         float& u, float& v) {
-  float3 e1 = xyz(b), e2 = xyz(c);
   float3 h = cross(d, e2);
   float det = dot(e1, h);
   if (!(fabsf(det) > 1e-8f)) return false;
   float f = 1.0f / det;
-  float3 s = o - xyz(a);
+  float3 s = o - v0;
   float uu = f * dot(s, h);
   if (!(uu >= 0.0f && uu <= 1.0f)) return false;
   float3 q = cross(s, e1);
@@ -317,10 +323,7 @@ __device__ __forceinline__ float objs_closest(const DevScene& S, float3 o, float
     else if (ob.type == 2) t = cube_t(o, d, ob.center, ob.extra);
     else if (ob.type == 4) {
       float uu, vv, tt;
-      float4 a = make_float4(ob.v0.x, ob.v0.y, ob.v0.z, 0.0f);
-      float4 b = make_float4(ob.v1.x - ob.v0.x, ob.v1.y - ob.v0.y, ob.v1.z - ob.v0.z, 0.0f);
-      float4 c = make_float4(ob.v2.x - ob.v0.x, ob.v2.y - ob.v0.y, ob.v2.z - ob.v0.z, 0.0f);
-      if (tri_hit(o, d, a, b, c, 3.0e38f, tt, uu, vv)) t = tt;
+      if (tri_hit(o, d, ob.v0, ob.v1 - ob.v0, ob.v2 - ob.v0, 3.0e38f, tt, uu, vv)) t = tt;
     }
     if (t > 0.001f && t < best) {
       best = t;
@@ -339,10 +342,7 @@ __device__ __forceinline__ bool objs_any(const DevScene& S, float3 o, float3 d, 
     else if (ob.type == 2) t = cube_t(o, d, ob.center, ob.extra);
     else if (ob.type == 4) {
       float uu, vv, tt;
-      float4 a = make_float4(ob.v0.x, ob.v0.y, ob.v0.z, 0.0f);
-      float4 b = make_float4(ob.v1.x - ob.v0.x, ob.v1.y - ob.v0.y, ob.v1.z - ob.v0.z, 0.0f);
-      float4 c = make_float4(ob.v2.x - ob.v0.x, ob.v2.y - ob.v0.y, ob.v2.z - ob.v0.z, 0.0f);
-      if (tri_hit(o, d, a, b, c, 3.0e38f, tt, uu, vv)) t = tt;
+      if (tri_hit(o, d, ob.v0, ob.v1 - ob.v0, ob.v2 - ob.v0, 3.0e38f, tt, uu, vv)) t = tt;
     }
     if (0.001f < t && t < max_t) return true;
   }
@@ -419,107 +419,49 @@ __host__ __device__ __forceinline__ int pack_leaf(int first, int count) { return
 __device__ __forceinline__ int leaf_first(int w) { return (~w) >> kLeafBits; }
 __device__ __forceinline__ int leaf_count(int w) { return (~w) & kMaxLeafPrims; }
 
-// Closest hit over the BVH (intersect.py:81-152 semantics): nearer child
-// first, ties to the right child, leaves tested in depth-first order, a hit
-// replaces the current one only when strictly closer.  The loop is the
-// while-while form with postponed leaves (Aila & Laine, "Understanding the
-// efficiency of ray traversal on GPUs", HPG 2009): a lane that reaches a leaf
-// parks it and keeps descending until every lane of the warp holds a leaf,
-// so leaf tests run together.  Leaves still execute in DFS order, so the
-// first hit found among equally distant ones is the reference's.
-// tmax in: current best distance (the linear scan's), out: closest hit.
-// Returns the leaf-order primitive index or -1.
-template <bool EXACT>
-__device__ __forceinline__ int bvh_closest_ww(const DevScene& S, float3 o, float3 d, float& tmax, float& hu,
-                                              float& hv, int* err) {
-  int stack[kStack];
-  int sp = 0;
-  stack[0] = kSentinel;
-  float3 inv = make_inv_dir(d);
-  float3 oinv = o * inv;
-  int hit = -1;
-  float te;
-  if (S.n_nodes <= 0 || !slab1(S.root_min, S.root_max, o, inv, tmax, te)) return -1;
-  int node = 0, leaf = 0;  // leaf >= 0: no leaf parked
-  // each record is visited at most once per ray; the guard turns a
-  // malformed tree into an error flag instead of an endless loop
-  int guard = 4 * S.n_nodes + 64;
-  while (node != kSentinel) {
-    while ((unsigned)node < (unsigned)kSentinel) {
-      if (--guard < 0 || node >= S.n_nodes) {
-        if (err) atomicOr(err, ERR_BAD_NODE);
-        return hit;
-      }
-      const float4* np = S.nodes + 4 * (size_t)node;
-      float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
-      bool hl, hr;
-      float tl, tr;
-      slab2<EXACT>(n0, n1, n2, o, inv, oinv, tmax, hl, hr, tl, tr);
-      int lw = __float_as_int(n3.x), rw = __float_as_int(n3.y);
-      if (!hl && !hr) {
-        node = stack[sp--];
-      } else {
-        bool left_first = hl && (!hr || tl < tr);
-        node = left_first ? lw : rw;
-        if (hl && hr) {
-          if (sp + 1 < kStack) {
-            stack[++sp] = left_first ? rw : lw;
-          } else if (err) {
-            atomicOr(err, ERR_STACK_OVERFLOW);
-          }
-        }
-      }
-      if (node < 0 && leaf >= 0) {
-        leaf = node;
-        node = stack[sp--];
-      }
-      if (!__any_sync(__activemask(), leaf >= 0)) break;
-    }
-    while (leaf < 0) {
-      int first = leaf_first(leaf), cnt = leaf_count(leaf);
-      if (first + cnt > S.n_prims) {
-        if (err) atomicOr(err, ERR_BAD_NODE);
-        return hit;
-      }
-      for (int k = first; k < first + cnt; ++k) {
-        const float4* pp = S.prims + 3 * (size_t)k;
-        float4 a = __ldg(pp);
-        float t, u, v;
-        if (__float_as_int(a.w) == PRIM_TRI) {
-          float4 b = __ldg(pp + 1), c = __ldg(pp + 2);
-          if (tri_hit(o, d, a, b, c, tmax, t, u, v)) {
-            tmax = t; hu = u; hv = v; hit = k;
-          }
-        } else {
-          float4 b = __ldg(pp + 1);
-          t = analytic_t(o, d, a, b);
-          if (t > 0.001f && t < tmax) {
-            tmax = t; hu = 0.0f; hv = 0.0f; hit = k;
-          }
-        }
-      }
-      leaf = node;
-      if (node < 0) node = stack[sp--];
-    }
-  }
-  return hit;
+// 32 bytes from a 32-byte aligned address (sm_100: one 256-bit load)
+__device__ __forceinline__ void ldg256(const void* p, float (&v)[8]) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
 }
 
+// A primitive record: a = (v0 or centre, kind), b as stored, and for a
+// triangle e1, e2 from b and c.
+struct Prim {
+  float4 a, b;
+  float2 c;  // triangles only
+  __device__ __forceinline__ bool tri() const { return __float_as_int(a.w) == PRIM_TRI; }
+  __device__ __forceinline__ float3 e1() const { return f3(b.x, b.y, b.z); }
+  __device__ __forceinline__ float3 e2() const { return f3(b.w, c.x, c.y); }
+};
+__device__ __forceinline__ Prim load_prim(const float4* prims, int k) {
+  const float4* p = prims + kPrimQuads * (size_t)k;
+  float v[8];
+  ldg256(p, v);
+  Prim r;
+  r.a = make_float4(v[0], v[1], v[2], v[3]);
+  r.b = make_float4(v[4], v[5], v[6], v[7]);
+  r.c = __ldg(reinterpret_cast<const float2*>(p + 2));
+  return r;
+}
+
+// Closest hit over the BVH (intersect.py:81-152 semantics): nearer child
+// first, ties to the right child, a hit replaces the current one only when
+// strictly closer.  tmax in: current best distance (the linear scan's), out:
+// closest hit.  The traversals return the leaf-order primitive index or -1.
 // Leaf test shared by the closest-hit loops.
 __device__ __forceinline__ void leaf_closest(const DevScene& S, float3 o, float3 d, int first, int cnt, float& tmax,
                                              float& hu, float& hv, int& hit) {
   for (int k = first; k < first + cnt; ++k) {
-    const float4* pp = S.prims + 3 * (size_t)k;
-    float4 a = __ldg(pp);
+    const Prim p = load_prim(S.prims, k);
     float t, u, v;
-    if (__float_as_int(a.w) == PRIM_TRI) {
-      float4 b = __ldg(pp + 1), c = __ldg(pp + 2);
-      if (tri_hit(o, d, a, b, c, tmax, t, u, v)) {
+    if (p.tri()) {
+      if (tri_hit(o, d, xyz(p.a), p.e1(), p.e2(), tmax, t, u, v)) {
         tmax = t; hu = u; hv = v; hit = k;
       }
     } else {
-      float4 b = __ldg(pp + 1);
-      t = analytic_t(o, d, a, b);
+      t = analytic_t(o, d, p.a, p.b);
       if (t > 0.001f && t < tmax) {
         tmax = t; hu = 0.0f; hv = 0.0f; hit = k;
       }
@@ -588,88 +530,21 @@ __device__ __forceinline__ int bvh_closest_ii(const DevScene& S, float3 o, float
   return hit;
 }
 
-// While-while form with postponed leaves and pop culling.
-template <bool EXACT>
-__device__ __forceinline__ int bvh_closest_wwt(const DevScene& S, float3 o, float3 d, float& tmax, float& hu,
-                                               float& hv, int* err) {
-  int stk_w[kStack];
-  float stk_t[kStack];
-  int sp = 0;
-  stk_w[0] = kSentinel;
-  stk_t[0] = -INFINITY;
-  float3 inv = make_inv_dir(d);
-  float3 oinv = o * inv;
-  int hit = -1;
-  float te;
-  if (S.n_nodes <= 0 || !slab1(S.root_min, S.root_max, o, inv, tmax, te)) return -1;
-  int node = 0, leaf = 0;
-  int guard = 4 * S.n_nodes + 64;
-  auto pop = [&]() {
-    int w;
-    float t;
-    do {
-      w = stk_w[sp];
-      t = stk_t[sp];
-      --sp;
-    } while (t > tmax);
-    return w;
-  };
-  while (node != kSentinel) {
-    while ((unsigned)node < (unsigned)kSentinel) {
-      if (--guard < 0 || node >= S.n_nodes) {
-        if (err) atomicOr(err, ERR_BAD_NODE);
-        return hit;
-      }
-      const float4* np = S.nodes + 4 * (size_t)node;
-      float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
-      bool hl, hr;
-      float tl, tr;
-      slab2<EXACT>(n0, n1, n2, o, inv, oinv, tmax, hl, hr, tl, tr);
-      int lw = __float_as_int(n3.x), rw = __float_as_int(n3.y);
-      if (!hl && !hr) {
-        node = pop();
-      } else {
-        bool left_first = hl && (!hr || tl < tr);
-        node = left_first ? lw : rw;
-        if (hl && hr) {
-          if (sp + 1 < kStack) {
-            ++sp;
-            stk_w[sp] = left_first ? rw : lw;
-            stk_t[sp] = left_first ? tr : tl;
-          } else if (err) {
-            atomicOr(err, ERR_STACK_OVERFLOW);
-          }
-        }
-      }
-      if (node < 0 && leaf >= 0) {
-        leaf = node;
-        node = pop();
-      }
-      if (!__any_sync(__activemask(), leaf >= 0)) break;
-    }
-    while (leaf < 0) {
-      int first = leaf_first(leaf), cnt = leaf_count(leaf);
-      if (first + cnt > S.n_prims) {
-        if (err) atomicOr(err, ERR_BAD_NODE);
-        return hit;
-      }
-      leaf_closest(S, o, d, first, cnt, tmax, hu, hv, hit);
-      leaf = node;
-      if (node < 0) node = pop();
-    }
-  }
-  return hit;
-}
-
 // ------------------------------------------------------------ 4-wide BVH
-// Node of 8 float4 (128 B, two cache lines): the children's boxes as
-// (min x, max x, min y, max y, min z, max z) each over the four children,
-// then the child words (>= 0: 4-wide node, < 0: packed leaf) and the
-// children's primitive counts.  An empty slot has a box at 1e30 (never
-// entered) and count 0.  The 4-wide tree is built from the LBVH: a node
-// starts from its binary children and, while it has fewer than four, opens
-// the internal child of largest surface area (leaves stay leaves), so
-// traversal needs about half the dependent node fetches.
+// Node of 8 float4 (128 B): the children's boxes as (centre x, half extent
+// x, centre y, half extent y, centre z, half extent z), each over the four
+// children, then the child words (>= 0: 4-wide node, < 0: packed leaf) and
+// the children's primitive counts.  An empty slot has its centre at 1e30,
+// half extent 0 (never entered) and count 0.  The 4-wide tree is built from
+// the LBVH: a node starts from its binary children and, while it has fewer
+// than four, opens the internal child of largest surface area (leaves stay
+// leaves), so traversal needs about half the dependent node fetches.
+// Divergent rays are bound by the L1 data pipe (73 % of its passes taken on
+// incoherent rays with 16-byte loads): a lane's load is a pass of its own
+// whatever its width, so a node is read with four 32-byte loads instead of
+// seven of 16.  Centre and half extent give the near and far distance by
+// two FMAs without choosing between planes by the direction's sign, which
+// 16-byte loads did by address.
 
 // Three-input min / max (PTX ISA 8.8, sm_100): one instruction each.
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -684,31 +559,26 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
 }
 
 // Entry distances of a 4-wide node's children (INFINITY where the ray
-// misses a child box before tmax) and their child words.  Each axis's near
-// and far planes are chosen once per ray: for a direction component >= 0
-// (inv > 0) the children's minima are the near planes, else their maxima;
-// `sx`, `sy`, `sz` (1 where inv < 0) select the float4 of each.  For a fixed
-// inv the rounded fma(plane, inv, -o*inv) is monotonic in the plane, so the
-// near plane's distance equals min(t_min_plane, t_max_plane) exactly and the
-// test gives the entry and exit distances of the two-sided slab test bit
-// for bit, at 6 FMA and 5 min/max/compare per child instead of 6 FMA and 13
-// (on the 1080p benchmark frame `k_extend` 25.3 -> 24.5 ms).
-__device__ __forceinline__ void slab4_oct(const float4* np, int sx, int sy, int sz, float3 inv, float3 oinv,
-                                          float tmax, float (&t)[4], int (&w)[4]) {
-  const float4 nx4 = __ldg(np + sx), fx4 = __ldg(np + (sx ^ 1));
-  const float4 ny4 = __ldg(np + 2 + sy), fy4 = __ldg(np + 2 + (sy ^ 1));
-  const float4 nz4 = __ldg(np + 4 + sz), fz4 = __ldg(np + 4 + (sz ^ 1));
+// misses a child box before tmax) and their child words.  Per axis the
+// centre's distance tc = c * inv - o * inv, then tc -/+ h |inv|; the boxes
+// are padded by 1e-4 and the stored half extents rounded up (k_bvh4_level),
+// which covers the roundings.
+__device__ __forceinline__ void slab4(const float4* np, float3 inv, float3 oinv, float tmax, float (&t)[4],
+                                      int (&w)[4]) {
+  float x[8], y[8], z[8];
+  ldg256(np, x);
+  ldg256(np + 2, y);
+  ldg256(np + 4, z);
   const float4 wd4 = __ldg(np + 6);
-  const float nx[4] = {nx4.x, nx4.y, nx4.z, nx4.w}, fx[4] = {fx4.x, fx4.y, fx4.z, fx4.w};
-  const float ny[4] = {ny4.x, ny4.y, ny4.z, ny4.w}, fy[4] = {fy4.x, fy4.y, fy4.z, fy4.w};
-  const float nz[4] = {nz4.x, nz4.y, nz4.z, nz4.w}, fz[4] = {fz4.x, fz4.y, fz4.z, fz4.w};
   const int wd[4] = {__float_as_int(wd4.x), __float_as_int(wd4.y), __float_as_int(wd4.z), __float_as_int(wd4.w)};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float te = max3f(__fmaf_rn(nx[i], inv.x, -oinv.x), __fmaf_rn(ny[i], inv.y, -oinv.y),
-                           __fmaf_rn(nz[i], inv.z, -oinv.z));
-    const float tx = min3f(__fmaf_rn(fx[i], inv.x, -oinv.x), __fmaf_rn(fy[i], inv.y, -oinv.y),
-                           fminf(__fmaf_rn(fz[i], inv.z, -oinv.z), tmax));
+    const float cx = __fmaf_rn(x[i], inv.x, -oinv.x), cy = __fmaf_rn(y[i], inv.y, -oinv.y),
+                cz = __fmaf_rn(z[i], inv.z, -oinv.z);
+    const float te = max3f(__fmaf_rn(-x[4 + i], fabsf(inv.x), cx), __fmaf_rn(-y[4 + i], fabsf(inv.y), cy),
+                           __fmaf_rn(-z[4 + i], fabsf(inv.z), cz));
+    const float tx = min3f(__fmaf_rn(x[4 + i], fabsf(inv.x), cx), __fmaf_rn(y[4 + i], fabsf(inv.y), cy),
+                           fminf(__fmaf_rn(z[4 + i], fabsf(inv.z), cz), tmax));
     t[i] = fmaxf(te, 0.001f) <= tx ? te : INFINITY;
     w[i] = wd[i];
   }
@@ -737,7 +607,6 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
   int sp = 0;
   const float3 inv = make_inv_dir(d);
   const float3 oinv = o * inv;
-  const int sx = inv.x < 0.0f, sy = inv.y < 0.0f, sz = inv.z < 0.0f;
   int hit = -1;
   float te;
   if (S.n_nodes4 <= 0 || !slab1(S.root_min, S.root_max, o, inv, tmax, te)) return -1;
@@ -754,7 +623,7 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
         const float4* np = S.nodes4 + 8 * (size_t)word;
         float t[4];
         int w[4];
-        slab4_oct(np, sx, sy, sz, inv, oinv, tmax, t, w);
+        slab4(np, inv, oinv, tmax, t, w);
         cswap(t, w, 0, 1);
         cswap(t, w, 2, 3);
         cswap(t, w, 0, 2);
@@ -793,23 +662,13 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
   return hit;
 }
 
-#ifndef RX_TRAV
-#define RX_TRAV 0
-#endif
-
 template <bool EXACT>
 __device__ __forceinline__ int bvh_closest(const DevScene& S, float3 o, float3 d, float& tmax, float& hu, float& hv,
                                            int* err) {
   if constexpr (!EXACT) {
     if (S.nodes4) return bvh4_closest(S, o, d, tmax, hu, hv, err);
   }
-#if RX_TRAV == 1
-  return bvh_closest_ww<EXACT>(S, o, d, tmax, hu, hv, err);
-#elif RX_TRAV == 2
-  return bvh_closest_wwt<EXACT>(S, o, d, tmax, hu, hv, err);
-#else
   return bvh_closest_ii<EXACT>(S, o, d, tmax, hu, hv, err);
-#endif
 }
 
 // Any hit before max_t on the 4-wide tree: every entered child is visited
@@ -819,7 +678,6 @@ __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, 
   int sp = 0;
   const float3 inv = make_inv_dir(d);
   const float3 oinv = o * inv;
-  const int sx = inv.x < 0.0f, sy = inv.y < 0.0f, sz = inv.z < 0.0f;
   float te;
   if (S.n_nodes4 <= 0 || !slab1(S.root_min, S.root_max, o, inv, max_t, te)) return false;
   int word = 0;
@@ -833,7 +691,7 @@ __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, 
       const float4* np = S.nodes4 + 8 * (size_t)word;
       float t[4];
       int w[4];
-      slab4_oct(np, sx, sy, sz, inv, oinv, max_t, t, w);
+      slab4(np, inv, oinv, max_t, t, w);
       cswap(t, w, 0, 1);
       cswap(t, w, 2, 3);
       cswap(t, w, 0, 2);
@@ -863,15 +721,12 @@ __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, 
         return false;
       }
       for (int k = first; k < first + cnt; ++k) {
-        const float4* pp = S.prims + 3 * (size_t)k;
-        float4 a = __ldg(pp);
+        const Prim p = load_prim(S.prims, k);
         float t, u, v;
-        if (__float_as_int(a.w) == PRIM_TRI) {
-          float4 b = __ldg(pp + 1), c = __ldg(pp + 2);
-          if (tri_hit(o, d, a, b, c, max_t, t, u, v)) return true;
+        if (p.tri()) {
+          if (tri_hit(o, d, xyz(p.a), p.e1(), p.e2(), max_t, t, u, v)) return true;
         } else {
-          float4 b = __ldg(pp + 1);
-          t = analytic_t(o, d, a, b);
+          t = analytic_t(o, d, p.a, p.b);
           if (0.001f < t && t < max_t) return true;
         }
       }
@@ -927,15 +782,12 @@ __device__ __forceinline__ bool bvh_any(const DevScene& S, float3 o, float3 d, f
         return false;
       }
       for (int k = first; k < first + cnt; ++k) {
-        const float4* pp = S.prims + 3 * (size_t)k;
-        float4 a = __ldg(pp);
+        const Prim p = load_prim(S.prims, k);
         float t, u, v;
-        if (__float_as_int(a.w) == PRIM_TRI) {
-          float4 b = __ldg(pp + 1), c = __ldg(pp + 2);
-          if (tri_hit(o, d, a, b, c, max_t, t, u, v)) return true;
+        if (p.tri()) {
+          if (tri_hit(o, d, xyz(p.a), p.e1(), p.e2(), max_t, t, u, v)) return true;
         } else {
-          float4 b = __ldg(pp + 1);
-          t = analytic_t(o, d, a, b);
+          t = analytic_t(o, d, p.a, p.b);
           if (0.001f < t && t < max_t) return true;
         }
       }

@@ -664,7 +664,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene& S, const RenderK& K
   bool listed;
   if (code >= 0) {
     const float4* sp = S.shade + 3 * (size_t)code;
-    float4 pa = __ldg(S.prims + 3 * (size_t)code);
+    float4 pa = __ldg(S.prims + kPrimQuads * (size_t)code);
     float4 s0 = __ldg(sp);
     m = __float_as_int(s0.w);
     if (__float_as_int(pa.w) == PRIM_TRI) {
@@ -673,7 +673,7 @@ __device__ __forceinline__ void shade_vertex(const DevScene& S, const RenderK& K
       src_tri = __float_as_int(s1.w);
       nn = normalized((xyz(s0) * w + xyz(s1) * h.z) + xyz(__ldg(sp + 2)) * h.w);
     } else {
-      nn = analytic_normal(o + d * t, pa, __ldg(S.prims + 3 * (size_t)code + 1));
+      nn = analytic_normal(o + d * t, pa, __ldg(S.prims + kPrimQuads * (size_t)code + 1));
     }
     // triangles and spheres can be lights; cubes are not in the light list
     listed = __float_as_int(pa.w) != PRIM_CUBE;

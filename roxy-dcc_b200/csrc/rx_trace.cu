@@ -20,7 +20,7 @@ __global__ void k_trace_closest(DevScene S, long n, const float* __restrict__ ro
     int p = bvh_closest<EXACT>(S, o, d, t, u, v, err);
     int id = -1;
     if (p >= 0) {
-      float4 a = __ldg(S.prims + 3 * (size_t)p);
+      float4 a = __ldg(S.prims + kPrimQuads * (size_t)p);
       int src = __float_as_int(__ldg(S.shade + 3 * (size_t)p + 1).w);
       id = __float_as_int(a.w) == PRIM_TRI ? src : -(src + 2);
     }
@@ -43,13 +43,13 @@ __global__ void k_trace_any(DevScene S, long n, const float* __restrict__ ro, co
 __device__ __forceinline__ float3 hit_normal(const DevScene& S, float3 o, float3 d, const SceneHit& h) {
   if (h.prim >= 0) {
     const float4* sp = S.shade + 3 * (size_t)h.prim;
-    float4 a = __ldg(S.prims + 3 * (size_t)h.prim);
+    float4 a = __ldg(S.prims + kPrimQuads * (size_t)h.prim);
     if (__float_as_int(a.w) == PRIM_TRI) {
       float w = 1.0f - h.u - h.v;
       float3 n0 = xyz(__ldg(sp)), n1 = xyz(__ldg(sp + 1)), n2 = xyz(__ldg(sp + 2));
       return normalized((n0 * w + n1 * h.u) + n2 * h.v);
     }
-    return analytic_normal(o + d * h.t, a, __ldg(S.prims + 3 * (size_t)h.prim + 1));
+    return analytic_normal(o + d * h.t, a, __ldg(S.prims + kPrimQuads * (size_t)h.prim + 1));
   }
   if (h.slot >= 0) {
     const ObjSlot& ob = S.objs[h.slot];
@@ -71,7 +71,7 @@ __global__ void k_scene_query(DevScene S, long n, const float* __restrict__ ro, 
     SceneHit h = scene_closest<EXACT>(S, o, d, err);
     int kind = 0, id = -1;
     if (h.prim >= 0) {
-      float4 a = __ldg(S.prims + 3 * (size_t)h.prim);
+      float4 a = __ldg(S.prims + kPrimQuads * (size_t)h.prim);
       id = __float_as_int(__ldg(S.shade + 3 * (size_t)h.prim + 1).w);
       kind = __float_as_int(a.w) == PRIM_TRI ? 1 : 2;
     } else if (h.slot >= 0) {

@@ -210,3 +210,30 @@ def test_benchmark_scene_hit_ids_match_reference_traversal():
     assert r["hits"] > 0.3 * r["rays"] and r["object_hits"] > 1000
     assert r["excluded_edge"] + r["excluded_ties"] < 0.001 * r["rays"]
     assert r["t_bit_exact"]
+
+
+@pytest.mark.parametrize("n,scale,offset", [(1, 1.0, 0.0), (2, 0.01, 0.0), (5, 1.0, 50.0), (33, 100.0, 0.0),
+                                            (3000, 1.0, 0.0), (3000, 0.05, 20.0), (3000, 100.0, 50.0)])
+def test_wide_nodes_find_what_the_reference_tree_finds(n, scale, offset):
+    """The 4-wide traversal's centre / half-extent boxes against the binary
+    tree with the reference's slab test: the same t bit for bit on every ray
+    (the triangle test is the same; a box may only cost a visit), over scene
+    sizes, positions and axis-parallel directions."""
+    rng = np.random.default_rng(n + int(scale * 100) + int(offset))
+    ctr = rng.uniform(-1, 1, (n, 1, 3))
+    tri = ((ctr + rng.normal(0, 0.1, (n, 3, 3))) * scale + offset).astype(np.float32)
+    m = 20000
+    aim = tri[rng.integers(0, n, m)].mean(axis=1) + rng.normal(0, 0.05 * scale, (m, 3))
+    rd = rng.normal(size=(m, 3))
+    axis = rng.integers(0, 3, m // 4)
+    rd[:m // 4] = 0.0
+    rd[np.arange(m // 4), axis] = rng.choice([-1.0, 1.0], m // 4)
+    rd = (rd / np.linalg.norm(rd, axis=1, keepdims=True)).astype(np.float32)
+    ro = (aim - rd * rng.uniform(0.0, 3.0 * scale, (m, 1))).astype(np.float32)
+    wide = _scene(tri[:, 0], tri[:, 1], tri[:, 2], nat.RX_BVH_LBVH_SAH, 4)
+    ref = _scene(tri[:, 0], tri[:, 1], tri[:, 2], nat.RX_BVH_REFERENCE, 4)
+    t0, t1 = wide.trace_closest(ro, rd)[0], ref.trace_closest(ro, rd)[0]
+    assert (t1 < 1e9).sum() > m // 50
+    np.testing.assert_array_equal(t0.view(np.uint32), t1.view(np.uint32))
+    tmax = rng.uniform(0.0, 3.0 * scale, m).astype(np.float32)
+    np.testing.assert_array_equal(wide.trace_any(ro, rd, tmax), ref.trace_any(ro, rd, tmax))
