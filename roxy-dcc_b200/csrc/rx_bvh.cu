@@ -655,8 +655,7 @@ __global__ void k_lbvh_layout_level(const int* __restrict__ cur, int* __restrict
 // taking both grandchildren (6-8 % fewer visits per ray on the displaced
 // icosphere).  Leaf children stay leaves; internal children that remain
 // become 4-wide nodes of the next level.  Empty binary slots (count 0
-// leaves) are dropped; unused slots get a centre of 1e30, half extent 0 and count
-// 0.
+// leaves) are dropped; unused slots get a box at 1e30 and count 0.
 __global__ void k_bvh4_level(const int* __restrict__ cur, int* __restrict__ next, int* __restrict__ lv,
                              const float4* __restrict__ bin, int n_bin, float4* __restrict__ out4, int* err) {
   const int ncur = lv[LV_NCUR], out_base = lv[LV_BASE];
@@ -739,27 +738,19 @@ __global__ void k_bvh4_level(const int* __restrict__ cur, int* __restrict__ next
         wd[i] = pack_leaf(0, 0);
       }
     }
-    // min, max -> centre, half extent; the half extent is rounded up and
-    // widened by 2^-22 of the box's distance from the origin, so that
-    // [c - h, c + h] holds [min, max] after the slab test's roundings too
-    for (int i = 0; i < k; ++i)
-      for (int a = 0; a < 3; ++a) {
-        const float lo = mn[i][a], hi = mx[i][a], c = 0.5f * lo + 0.5f * hi;
-        const float h = fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo));
-        mn[i][a] = c;
-        mx[i][a] = __fadd_ru(h, 0x1p-22f * fmaxf(fabsf(lo), fabsf(hi)));
-      }
     for (; k < 4; ++k) {
       mn[k][0] = mn[k][1] = mn[k][2] = 1e30f;
-      mx[k][0] = mx[k][1] = mx[k][2] = 0.0f;
+      mx[k][0] = mx[k][1] = mx[k][2] = 1e30f;
       wd[k] = pack_leaf(0, 0);
       ct[k] = 0;
     }
     float4* o = out4 + 8 * (size_t)(out_base + q);
-    for (int a = 0; a < 3; ++a) {
-      o[2 * a] = make_float4(mn[0][a], mn[1][a], mn[2][a], mn[3][a]);
-      o[2 * a + 1] = make_float4(mx[0][a], mx[1][a], mx[2][a], mx[3][a]);
-    }
+    o[0] = make_float4(mn[0][0], mn[1][0], mn[2][0], mn[3][0]);
+    o[1] = make_float4(mx[0][0], mx[1][0], mx[2][0], mx[3][0]);
+    o[2] = make_float4(mn[0][1], mn[1][1], mn[2][1], mn[3][1]);
+    o[3] = make_float4(mx[0][1], mx[1][1], mx[2][1], mx[3][1]);
+    o[4] = make_float4(mn[0][2], mn[1][2], mn[2][2], mn[3][2]);
+    o[5] = make_float4(mx[0][2], mx[1][2], mx[2][2], mx[3][2]);
     o[6] = make_float4(__int_as_float(wd[0]), __int_as_float(wd[1]), __int_as_float(wd[2]), __int_as_float(wd[3]));
     o[7] = make_float4(__int_as_float(ct[0]), __int_as_float(ct[1]), __int_as_float(ct[2]), __int_as_float(ct[3]));
   }

@@ -531,20 +531,14 @@ __device__ __forceinline__ int bvh_closest_ii(const DevScene& S, float3 o, float
 }
 
 // ------------------------------------------------------------ 4-wide BVH
-// Node of 8 float4 (128 B): the children's boxes as (centre x, half extent
-// x, centre y, half extent y, centre z, half extent z), each over the four
-// children, then the child words (>= 0: 4-wide node, < 0: packed leaf) and
-// the children's primitive counts.  An empty slot has its centre at 1e30,
-// half extent 0 (never entered) and count 0.  The 4-wide tree is built from
-// the LBVH: a node starts from its binary children and, while it has fewer
-// than four, opens the internal child of largest surface area (leaves stay
-// leaves), so traversal needs about half the dependent node fetches.
-// Divergent rays are bound by the L1 data pipe (73 % of its passes taken on
-// incoherent rays with 16-byte loads): a lane's load is a pass of its own
-// whatever its width, so a node is read with four 32-byte loads instead of
-// seven of 16.  Centre and half extent give the near and far distance by
-// two FMAs without choosing between planes by the direction's sign, which
-// 16-byte loads did by address.
+// Node of 8 float4 (128 B, two cache lines): the children's boxes as
+// (min x, max x, min y, max y, min z, max z) each over the four children,
+// then the child words (>= 0: 4-wide node, < 0: packed leaf) and the
+// children's primitive counts.  An empty slot has a box at 1e30 (never
+// entered) and count 0.  The 4-wide tree is built from the LBVH: a node
+// starts from its binary children and, while it has fewer than four, opens
+// the internal child of largest surface area (leaves stay leaves), so
+// traversal needs about half the dependent node fetches.
 
 // Three-input min / max (PTX ISA 8.8, sm_100): one instruction each.
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -558,27 +552,74 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
   return r;
 }
 
+// Two float32 multiply-adds in one instruction (sm_100), each rounded as
+// __fmaf_rn rounds.
+__device__ __forceinline__ unsigned long long dup2(float x) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long a, unsigned long long b, unsigned long long c, float& x,
+                                     float& y) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
+}
+
+// Distances of one axis's near and far planes of the four children.  For a
+// direction component >= 0 (inv > 0) the children's minima are the near
+// planes, else their maxima; for a fixed inv the rounded fma(plane, inv,
+// -o*inv) is monotonic in the plane, so taking the planes by the direction's
+// sign and taking the smaller and larger distance give the same bits.
+//   PICK  by sign: `off` is the byte offset of the near planes (the node is
+//         128-byte aligned, so an OR and an XOR form both addresses), two
+//         16-byte loads.  Fewest instructions: the render kernels, which are
+//         bound by issue (1080p frame: extend 18.65 ms; planes picked with
+//         64-bit adds and scalar FMAs 19.71, without PICK 19.18).
+//   else  one 32-byte load of both, then min and max.  Fewest requests: ray
+//         queries in no order, bound by the L1 data pipe and latency (two
+//         million: 950 us against 977).
+template <bool PICK>
+__device__ __forceinline__ void slab_axis(const float4* np, unsigned off, float inv, float oinv, float (&n)[4],
+                                          float (&f)[4]) {
+  const unsigned long long I = dup2(inv), O = dup2(-oinv);
+  const size_t a = reinterpret_cast<size_t>(np) | off;
+  unsigned long long p, q, r, s;
+  if constexpr (PICK) {
+    asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(p), "=l"(q) : "l"(a));
+    asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(r), "=l"(s) : "l"(a ^ 16u));
+    fma2(p, I, O, n[0], n[1]);
+    fma2(q, I, O, n[2], n[3]);
+    fma2(r, I, O, f[0], f[1]);
+    fma2(s, I, O, f[2], f[3]);
+  } else {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(p), "=l"(q), "=l"(r), "=l"(s) : "l"(a));
+    float lo[4], hi[4];
+    fma2(p, I, O, lo[0], lo[1]);
+    fma2(q, I, O, lo[2], lo[3]);
+    fma2(r, I, O, hi[0], hi[1]);
+    fma2(s, I, O, hi[2], hi[3]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) n[i] = fminf(lo[i], hi[i]), f[i] = fmaxf(lo[i], hi[i]);
+  }
+}
+
 // Entry distances of a 4-wide node's children (INFINITY where the ray
-// misses a child box before tmax) and their child words.  Per axis the
-// centre's distance tc = c * inv - o * inv, then tc -/+ h |inv|; the boxes
-// are padded by 1e-4 and the stored half extents rounded up (k_bvh4_level),
-// which covers the roundings.
-__device__ __forceinline__ void slab4(const float4* np, float3 inv, float3 oinv, float tmax, float (&t)[4],
-                                      int (&w)[4]) {
-  float x[8], y[8], z[8];
-  ldg256(np, x);
-  ldg256(np + 2, y);
-  ldg256(np + 4, z);
+// misses a child box before tmax) and their child words.  sx, sy, sz: 16
+// where the direction component is negative, else 0 (PICK only).
+template <bool PICK>
+__device__ __forceinline__ void slab4(const float4* np, unsigned sx, unsigned sy, unsigned sz, float3 inv, float3 oinv,
+                                      float tmax, float (&t)[4], int (&w)[4]) {
+  float nx[4], fx[4], ny[4], fy[4], nz[4], fz[4];
+  slab_axis<PICK>(np, PICK ? sx : 0u, inv.x, oinv.x, nx, fx);
+  slab_axis<PICK>(np, 32u + (PICK ? sy : 0u), inv.y, oinv.y, ny, fy);
+  slab_axis<PICK>(np, 64u + (PICK ? sz : 0u), inv.z, oinv.z, nz, fz);
   const float4 wd4 = __ldg(np + 6);
   const int wd[4] = {__float_as_int(wd4.x), __float_as_int(wd4.y), __float_as_int(wd4.z), __float_as_int(wd4.w)};
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float cx = __fmaf_rn(x[i], inv.x, -oinv.x), cy = __fmaf_rn(y[i], inv.y, -oinv.y),
-                cz = __fmaf_rn(z[i], inv.z, -oinv.z);
-    const float te = max3f(__fmaf_rn(-x[4 + i], fabsf(inv.x), cx), __fmaf_rn(-y[4 + i], fabsf(inv.y), cy),
-                           __fmaf_rn(-z[4 + i], fabsf(inv.z), cz));
-    const float tx = min3f(__fmaf_rn(x[4 + i], fabsf(inv.x), cx), __fmaf_rn(y[4 + i], fabsf(inv.y), cy),
-                           fminf(__fmaf_rn(z[4 + i], fabsf(inv.z), cz), tmax));
+    const float te = max3f(nx[i], ny[i], nz[i]);
+    const float tx = min3f(fx[i], fy[i], fminf(fz[i], tmax));
     t[i] = fmaxf(te, 0.001f) <= tx ? te : INFINITY;
     w[i] = wd[i];
   }
@@ -600,6 +641,7 @@ __device__ __forceinline__ void cswap(float (&t)[4], int (&w)[4], int a, int b) 
 // skipped on pop once the current hit is closer.  Returns the same closest
 // primitive as the binary traversal (up to the order among exactly equal
 // hit distances).
+template <bool PICK = true>
 __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 d, float& tmax, float& hu, float& hv,
                                             int* err) {
   int stk_w[kStack];
@@ -609,6 +651,7 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
   const float3 oinv = o * inv;
   int hit = -1;
   float te;
+  const unsigned sx = inv.x < 0.0f ? 16u : 0u, sy = inv.y < 0.0f ? 16u : 0u, sz = inv.z < 0.0f ? 16u : 0u;
   if (S.n_nodes4 <= 0 || !slab1(S.root_min, S.root_max, o, inv, tmax, te)) return -1;
   int word = 0;
   float wt = te;
@@ -623,7 +666,7 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
         const float4* np = S.nodes4 + 8 * (size_t)word;
         float t[4];
         int w[4];
-        slab4(np, inv, oinv, tmax, t, w);
+        slab4<PICK>(np, sx, sy, sz, inv, oinv, tmax, t, w);
         cswap(t, w, 0, 1);
         cswap(t, w, 2, 3);
         cswap(t, w, 0, 2);
@@ -662,23 +705,25 @@ __device__ __forceinline__ int bvh4_closest(const DevScene& S, float3 o, float3 
   return hit;
 }
 
-template <bool EXACT>
+template <bool EXACT, bool PICK = true>
 __device__ __forceinline__ int bvh_closest(const DevScene& S, float3 o, float3 d, float& tmax, float& hu, float& hv,
                                            int* err) {
   if constexpr (!EXACT) {
-    if (S.nodes4) return bvh4_closest(S, o, d, tmax, hu, hv, err);
+    if (S.nodes4) return bvh4_closest<PICK>(S, o, d, tmax, hu, hv, err);
   }
   return bvh_closest_ii<EXACT>(S, o, d, tmax, hu, hv, err);
 }
 
 // Any hit before max_t on the 4-wide tree: every entered child is visited
 // (nearest first, the rest stacked) until the first primitive hit.
+template <bool PICK = true>
 __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, float max_t, int* err) {
   int stack[kStack];
   int sp = 0;
   const float3 inv = make_inv_dir(d);
   const float3 oinv = o * inv;
   float te;
+  const unsigned sx = inv.x < 0.0f ? 16u : 0u, sy = inv.y < 0.0f ? 16u : 0u, sz = inv.z < 0.0f ? 16u : 0u;
   if (S.n_nodes4 <= 0 || !slab1(S.root_min, S.root_max, o, inv, max_t, te)) return false;
   int word = 0;
   int guard = 4 * S.n_nodes4 + 64;
@@ -691,7 +736,7 @@ __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, 
       const float4* np = S.nodes4 + 8 * (size_t)word;
       float t[4];
       int w[4];
-      slab4(np, inv, oinv, max_t, t, w);
+      slab4<PICK>(np, sx, sy, sz, inv, oinv, max_t, t, w);
       cswap(t, w, 0, 1);
       cswap(t, w, 2, 3);
       cswap(t, w, 0, 2);
@@ -737,10 +782,10 @@ __device__ __forceinline__ bool bvh4_any(const DevScene& S, float3 o, float3 d, 
 }
 
 // Any hit before max_t (intersect.py:155-219): stops at the first hit.
-template <bool EXACT>
+template <bool EXACT, bool PICK = true>
 __device__ __forceinline__ bool bvh_any(const DevScene& S, float3 o, float3 d, float max_t, int* err) {
   if constexpr (!EXACT) {
-    if (S.nodes4) return bvh4_any(S, o, d, max_t, err);
+    if (S.nodes4) return bvh4_any<PICK>(S, o, d, max_t, err);
   }
   int stack[kStack];
   int sp = 0;
@@ -809,7 +854,7 @@ struct SceneHit {
 
 // WIDE: the caller guarantees a 4-wide tree (only that traversal is
 // compiled in, which keeps the batch kernels within their registers).
-template <bool EXACT, bool WIDE = false>
+template <bool EXACT, bool WIDE = false, bool PICK = true>
 __device__ __forceinline__ SceneHit scene_closest(const DevScene& S, float3 o, float3 d, int* err) {
   SceneHit h;
   int slot;
@@ -819,7 +864,7 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene& S, float3 o, f
   h.u = 0.0f;
   h.v = 0.0f;
   float u = 0.0f, v = 0.0f;
-  int p = WIDE ? bvh4_closest(S, o, d, t, u, v, err) : bvh_closest<EXACT>(S, o, d, t, u, v, err);
+  int p = WIDE ? bvh4_closest<PICK>(S, o, d, t, u, v, err) : bvh_closest<EXACT, PICK>(S, o, d, t, u, v, err);
   if (p >= 0) {
     h.prim = p;
     h.slot = -1;
@@ -830,10 +875,10 @@ __device__ __forceinline__ SceneHit scene_closest(const DevScene& S, float3 o, f
   return h;
 }
 
-template <bool EXACT, bool WIDE = false>
+template <bool EXACT, bool WIDE = false, bool PICK = true>
 __device__ __forceinline__ bool scene_any(const DevScene& S, float3 o, float3 d, float max_t, int* err) {
   if (objs_any(S, o, d, max_t)) return true;
-  return WIDE ? bvh4_any(S, o, d, max_t, err) : bvh_any<EXACT>(S, o, d, max_t, err);
+  return WIDE ? bvh4_any<PICK>(S, o, d, max_t, err) : bvh_any<EXACT, PICK>(S, o, d, max_t, err);
 }
 
 }  // namespace rx

@@ -17,7 +17,7 @@ __global__ void k_trace_closest(DevScene S, long n, const float* __restrict__ ro
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     float3 o = ld3f(ro, i), d = ld3f(rd, i);
     float t = 1e9f, u = 0.0f, v = 0.0f;
-    int p = bvh_closest<EXACT>(S, o, d, t, u, v, err);
+    int p = bvh_closest<EXACT, false>(S, o, d, t, u, v, err);
     int id = -1;
     if (p >= 0) {
       float4 a = __ldg(S.prims + kPrimQuads * (size_t)p);
@@ -35,7 +35,7 @@ template <bool EXACT>
 __global__ void k_trace_any(DevScene S, long n, const float* __restrict__ ro, const float* __restrict__ rd,
                             const float* __restrict__ tmax, int* __restrict__ out, int* err) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    out[i] = scene_any<EXACT>(S, ld3f(ro, i), ld3f(rd, i), tmax[i], err) ? 1 : 0;
+    out[i] = scene_any<EXACT, false, false>(S, ld3f(ro, i), ld3f(rd, i), tmax[i], err) ? 1 : 0;
   }
 }
 
@@ -68,7 +68,7 @@ __global__ void k_scene_query(DevScene S, long n, const float* __restrict__ ro, 
                               float* __restrict__ out_n, int* err) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     float3 o = ld3f(ro, i), d = ld3f(rd, i);
-    SceneHit h = scene_closest<EXACT>(S, o, d, err);
+    SceneHit h = scene_closest<EXACT, false, false>(S, o, d, err);
     int kind = 0, id = -1;
     if (h.prim >= 0) {
       float4 a = __ldg(S.prims + kPrimQuads * (size_t)h.prim);

@@ -215,10 +215,10 @@ def test_benchmark_scene_hit_ids_match_reference_traversal():
 @pytest.mark.parametrize("n,scale,offset", [(1, 1.0, 0.0), (2, 0.01, 0.0), (5, 1.0, 50.0), (33, 100.0, 0.0),
                                             (3000, 1.0, 0.0), (3000, 0.05, 20.0), (3000, 100.0, 50.0)])
 def test_wide_nodes_find_what_the_reference_tree_finds(n, scale, offset):
-    """The 4-wide traversal's centre / half-extent boxes against the binary
-    tree with the reference's slab test: the same t bit for bit on every ray
-    (the triangle test is the same; a box may only cost a visit), over scene
-    sizes, positions and axis-parallel directions."""
+    """The 4-wide traversal of ray queries (both planes of an axis in one
+    load) against the binary tree with the reference's slab test: the same t
+    bit for bit on every ray (the triangle test is the same; a box may only
+    cost a visit), over scene sizes, positions and axis-parallel directions."""
     rng = np.random.default_rng(n + int(scale * 100) + int(offset))
     ctr = rng.uniform(-1, 1, (n, 1, 3))
     tri = ((ctr + rng.normal(0, 0.1, (n, 3, 3))) * scale + offset).astype(np.float32)
