@@ -39,9 +39,27 @@ enum { C_Q = 0, C_FE = 64, C_FS = 128, C_S = 192, C_TAIL = 256, C_FT = 257, C_N 
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kTwoPi = 6.283185307179586f;
 
+// n / d for n < 2^31 as a multiplication and a shift (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", PLDI
+// 1994): with 2^s >= d the quotient is (umulhi(m, n) + n) >> s.
+struct FastDiv {
+  uint32_t m = 1, d = 1;
+  int s = 0;
+  FastDiv() {}
+  explicit FastDiv(uint32_t d_) : d(d_) {
+    while ((1ull << s) < d) ++s;
+    m = (uint32_t)((((1ull << s) - d) << 32) / d + 1);
+  }
+  __device__ __forceinline__ uint32_t div(uint32_t n) const { return (__umulhi(m, n) + n) >> s; }
+};
+
 struct RenderK {
   int W, H;
   long long P;
+  float rW, rH;      // RN(1 / W), RN(1 / H)
+  FastDiv strip;     // pixels of a whole strip
+  int cam_log2;      // log2 of the samples of a pixel on consecutive camera items
+  FastDiv span;      // camera items of a group of 2^cam_log2 frames
   int spf;
   float fov_tan, aspect;
   float3 cam_pos, cam_fwd, cam_right, cam_up;
@@ -61,14 +79,18 @@ __device__ __forceinline__ float fractf_(float x) { return x - floorf(x); }
 
 // camera.py:23-30 with a counter-based per-pixel phase in place of the
 // sin-hash: jitter = fract(phase + (frame + 1) * R2).
-__device__ __forceinline__ float3 camera_dir(const RenderK& K, int px, int py, int frame) {
+__device__ __forceinline__ float2 camera_phase(const RenderK& K, int px, int py) {
   uint32_t ph[4];
   philox((uint32_t)((long long)py * K.W + px), 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, K.seed, kKeyHi, ph);
+  return make_float2(u01(ph[0]), u01(ph[1]));
+}
+__device__ __forceinline__ float3 camera_dir(const RenderK& K, int px, int py, int frame, float2 phase) {
   float i = (float)(frame + 1);
-  float jx = fractf_(u01(ph[0]) + i * 0.7548776662466927f);
-  float jy = fractf_(u01(ph[1]) + i * 0.5698402909980532f);
-  float u = ((float)px + jx) / (float)K.W * 2.0f - 1.0f;
-  float v = 1.0f - ((float)py + jy) / (float)K.H * 2.0f;
+  float jx = fractf_(phase.x + i * 0.7548776662466927f);
+  float jy = fractf_(phase.y + i * 0.5698402909980532f);
+  // each quotient is the float the division gives (div_by)
+  float u = div_by((float)px + jx, (float)K.W, K.rW) * 2.0f - 1.0f;
+  float v = 1.0f - div_by((float)py + jy, (float)K.H, K.rH) * 2.0f;
   float ndx = u * K.aspect * K.fov_tan;
   float ndy = v * K.fov_tan;
   return normalized((K.cam_fwd + K.cam_right * ndx) + K.cam_up * ndy);
@@ -262,7 +284,7 @@ struct JobAcc {
 constexpr int kStripRows = 2;  // a power of two (2: 6,316 against 6,262 Mrays/s with 4 on the 1080p benchmark)
 __device__ __forceinline__ void strip_pixel(const RenderK& K, long long s, int& px, int& py) {
   const int si = (int)s, ws = kStripRows * K.W;
-  const int strip = si / ws, r = si - strip * ws;
+  const int strip = (int)K.strip.div((uint32_t)si), r = si - strip * ws;
   const int hs = min(kStripRows, K.H - kStripRows * strip);
   if (hs == kStripRows) {  // every strip but a short last one
     px = r / kStripRows;
@@ -283,23 +305,23 @@ __device__ __forceinline__ void strip_pixel(const RenderK& K, long long s, int& 
 // as eight runs of 4 consecutive paths.  Any order gives the same image: a
 // path's random numbers depend on its pixel, sample and bounce.
 constexpr int kCamFrames = 8;
-// the largest power of two up to kCamFrames that divides `frames`
-__device__ __forceinline__ int group_of(int frames) {
-  int g = kCamFrames;
-  while (frames % g) g >>= 1;
-  return g;
+// log2 of the largest power of two up to kCamFrames that divides `frames`
+__host__ __device__ __forceinline__ int group_log2(int frames) {
+  int l = 0;
+  while ((2 << l) <= kCamFrames && frames % (2 << l) == 0) ++l;
+  return l;
 }
-__device__ __forceinline__ int camera_group(const RenderK& K) { return group_of(K.spf); }
-__device__ __forceinline__ long long camera_path(const RenderK& K, long long t, int& px, int& py, int& f) {
-  const int g = camera_group(K);
-  const long long span = (long long)g * K.P;
-  const long long c = t / span;
-  const int r = (int)(t - c * span);
-  const int s = r / g;
-  f = (int)(c * g) + (r - s * g);
-  strip_pixel(K, s, px, py);
-  return (long long)f * K.P + s;
+// frame f and strip index s of camera item t (t < 2^31); returns its path
+__device__ __forceinline__ int camera_path(const RenderK& K, uint32_t t, int& s, int& f) {
+  const uint32_t c = K.span.div(t), r = t - c * K.span.d;
+  s = (int)(r >> K.cam_log2);
+  f = (int)((c << K.cam_log2) + (r & ((1u << K.cam_log2) - 1u)));
+  return (int)((uint32_t)f * (uint32_t)K.P) + s;
 }
+// Camera phases of a wave's pixels, by strip index.  A pixel's phase is a
+// Philox block that each of its samples needs in k_extend and, on a hit, in
+// k_shade; from kPhaseFrames frames on it is computed once per pixel.
+constexpr int kPhaseFrames = 8;
 
 struct SingleSrc {
   static constexpr bool kBatch = false;
@@ -322,17 +344,25 @@ struct SingleSrc {
     return b == 0 && K.camera0 ? (long long)K.spf * K.P : 0;
   }
   __device__ __forceinline__ int frame0() const { return *fbase; }
-  // camera ray of item t; pix / smp: its pixel (row major) and sample
-  __device__ __forceinline__ int camera_ray(long long t, int fb, float3& o, float3& d, uint32_t& pix,
-                                            uint32_t& smp) const {
-    int px, py, f;
-    const long long p = camera_path(K, t, px, py, f);
-    o = K.cam_pos;
-    d = camera_dir(K, px, py, fb + f);
-    pix = (uint32_t)(py * K.W + px);
-    smp = (uint32_t)(fb + f);
-    return (int)p;
+  const float2* phase = nullptr;  // camera phases by strip index, or null
+  // camera item t: its path, pixel and sample
+  struct CamItem {
+    int p, s, px, py;
+    uint32_t smp;
+  };
+  __device__ __forceinline__ CamItem camera_item(long long t, int fb) const {
+    CamItem c;
+    int f;
+    c.p = camera_path(K, (uint32_t)t, c.s, f);
+    strip_pixel(K, c.s, c.px, c.py);
+    c.smp = (uint32_t)(fb + f);
+    return c;
   }
+  __device__ __forceinline__ uint32_t pixel(const CamItem& c) const { return (uint32_t)(c.py * K.W + c.px); }
+  __device__ __forceinline__ float3 camera_ray(const CamItem& c) const {
+    return camera_dir(K, c.px, c.py, (int)c.smp, phase ? __ldg(phase + c.s) : camera_phase(K, c.px, c.py));
+  }
+  __device__ __forceinline__ float3 camera_pos() const { return K.cam_pos; }
 };
 
 struct BatchSrc {
@@ -361,9 +391,14 @@ struct BatchSrc {
   // batches keep k_generate_batch's queue and path state at bounce 0
   __device__ __forceinline__ long long camera_items(int) const { return 0; }
   __device__ __forceinline__ int frame0() const { return 0; }
-  __device__ __forceinline__ int camera_ray(long long, int, float3&, float3&, uint32_t&, uint32_t&) const {
-    return 0;
-  }
+  struct CamItem {
+    int p;
+    uint32_t smp;
+  };
+  __device__ __forceinline__ CamItem camera_item(long long, int) const { return CamItem{0, 0u}; }
+  __device__ __forceinline__ uint32_t pixel(const CamItem&) const { return 0u; }
+  __device__ __forceinline__ float3 camera_ray(const CamItem&) const { return f3(0.0f, 0.0f, 0.0f); }
+  __device__ __forceinline__ float3 camera_pos() const { return f3(0.0f, 0.0f, 0.0f); }
 };
 
 // A batch whose scenes all have a 4-wide tree (LBVH builds): extend traverses
@@ -374,32 +409,67 @@ struct BatchSrc4 : BatchSrc {
 };
 
 // -------------------------------------------------------------------- kernels
-// Camera ray and empty path state of path p (pixel px, py; sample `frame`).
-__device__ __forceinline__ void init_path(const RenderK& K, int px, int py, int frame, long long p,
-                                          float4* __restrict__ ray_o, float4* __restrict__ ray_d,
-                                          float4* __restrict__ thr, float4* __restrict__ rad,
-                                          float4* __restrict__ gn, float4* __restrict__ ga) {
-  float3 d = camera_dir(K, px, py, frame);
-  ray_o[p] = make_float4(K.cam_pos.x, K.cam_pos.y, K.cam_pos.z, 1.0f);
-  ray_d[p] = make_float4(d.x, d.y, d.z, 0.0f);
-  thr[p] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float((uint32_t)(py * K.W + px)));  // w: the pixel
-  rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  gn[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  ga[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+// Two float4 of one path kept side by side -- the ray (origin + ior,
+// direction + NEE weight) and the first-hit guides (normal + depth, albedo)
+// -- as one 32-byte sector, loaded and stored whole.  Paths that go on or
+// hit something are scattered among those that do not, so arrays of their
+// own gave half-written sectors: the 1080p frame's k_shade then took 5.5 to
+// 7.4 ms from one placement of the arrays to another.
+__device__ __forceinline__ void store_pair(float4* a, long long p, float4 x, float4 y) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(a + 2 * p), "f"(x.x), "f"(x.y), "f"(x.z),
+               "f"(x.w), "f"(y.x), "f"(y.y), "f"(y.z), "f"(y.w)
+               : "memory");
+}
+// the same, streaming
+__device__ __forceinline__ void load_pair_cs(const float4* a, long long p, float4& x, float4& y) {
+  asm volatile("ld.global.cs.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
+               : "l"(a + 2 * p)
+               : "memory");
+}
+__device__ __forceinline__ void load_pair(const float4* a, long long p, float4& x, float4& y) {
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(x.w), "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
+               : "l"(a + 2 * p)
+               : "memory");
 }
 
-__global__ void k_generate(RenderK K, const int* __restrict__ frame_base, float4* __restrict__ ray_o,
-                           float4* __restrict__ ray_d, float4* __restrict__ thr, float4* __restrict__ rad,
-                           float4* __restrict__ gn, float4* __restrict__ ga, int* __restrict__ q0,
-                           int* __restrict__ counters) {
+// Camera ray and empty path state of path p (pixel px, py; sample `frame`).
+// rad.w says whether the path's first ray hit a surface: only then do its
+// guides (gd) hold anything, and only then does the accumulation read
+// them -- three quarters of the 1080p benchmark's paths miss, and writing
+// and reading their zeros was 64 B each.
+__device__ __forceinline__ void init_path(const RenderK& K, int px, int py, int frame, long long p,
+                                          float4* __restrict__ ray, float4* __restrict__ thr,
+                                          float4* __restrict__ rad) {
+  float3 d = camera_dir(K, px, py, frame, camera_phase(K, px, py));
+  store_pair(ray, p, make_float4(K.cam_pos.x, K.cam_pos.y, K.cam_pos.z, 1.0f), make_float4(d.x, d.y, d.z, 0.0f));
+  thr[p] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float((uint32_t)(py * K.W + px)));  // w: the pixel
+  rad[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
+// Camera phases by strip index (see kPhaseFrames).
+__global__ void k_phase(RenderK K, float2* __restrict__ phase) {
+  for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < K.P;
+       s += (long long)gridDim.x * blockDim.x) {
+    int px, py;
+    strip_pixel(K, s, px, py);
+    phase[s] = camera_phase(K, px, py);
+  }
+}
+
+__global__ void k_generate(RenderK K, const int* __restrict__ frame_base, float4* __restrict__ ray,
+                           float4* __restrict__ thr, float4* __restrict__ rad,
+                           int* __restrict__ q0, int* __restrict__ counters) {
   long long total = (long long)K.spf * K.P;
   int fb = *frame_base;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += stride) {
-    int px, py, f;
-    const long long p = camera_path(K, t, px, py, f);
-    init_path(K, px, py, fb + f, p, ray_o, ray_d, thr, rad, gn, ga);
-    q0[t] = (int)p;
+    int px, py, s, f;
+    const int p = camera_path(K, (uint32_t)t, s, f);
+    strip_pixel(K, s, px, py);
+    init_path(K, px, py, fb + f, p, ray, thr, rad);
+    q0[t] = p;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) counters[C_Q + 0] = (int)total;
 }
@@ -417,10 +487,9 @@ __device__ __forceinline__ int find_seg(const WaveSeg* __restrict__ segs, int n_
   return lo;
 }
 
-__global__ void k_generate_batch(BatchSrc src, int n_segs, long long total, float4* __restrict__ ray_o,
-                                 float4* __restrict__ ray_d, float4* __restrict__ thr, float4* __restrict__ rad,
-                                 float4* __restrict__ gn, float4* __restrict__ ga, int* __restrict__ q0,
-                                 int* __restrict__ pseg, int* __restrict__ counters) {
+__global__ void k_generate_batch(BatchSrc src, int n_segs, long long total, float4* __restrict__ ray,
+                                 float4* __restrict__ thr, float4* __restrict__ rad,
+                                 int* __restrict__ q0, int* __restrict__ pseg, int* __restrict__ counters) {
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += stride) {
     int si = find_seg<false>(src.segs, n_segs, t);
@@ -430,16 +499,15 @@ __global__ void k_generate_batch(BatchSrc src, int n_segs, long long total, floa
     // the single-render order and layout per segment: samples of a pixel
     // on consecutive items, path state at path0 + f * P + strip index
     const long long l = t - g.path0;
-    const int gs = group_of(g.frames);
-    const long long span = (long long)gs * g.P;
-    const long long c = l / span;
-    const int r = (int)(l - c * span);
-    const int si2 = r / gs;
-    const int f = (int)(c * gs) + (r - si2 * gs);
+    const int gl = group_log2(g.frames);
+    const uint32_t span = (uint32_t)g.P << gl;  // a wave holds fewer than 2^31 paths
+    const uint32_t c = (uint32_t)l / span, r = (uint32_t)l - c * span;
+    const int si2 = (int)(r >> gl);
+    const int f = (int)((c << gl) + (r & ((1u << gl) - 1u)));
     int px, py;
     strip_pixel(K, si2, px, py);
     long long p = g.path0 + (long long)f * g.P + si2;
-    init_path(K, px, py, fb + f, p, ray_o, ray_d, thr, rad, gn, ga);
+    init_path(K, px, py, fb + f, p, ray, thr, rad);
     pseg[p] = si;
     q0[t] = (int)p;
   }
@@ -484,8 +552,8 @@ __device__ __forceinline__ int shadow_item(const Src& src, const float4* __restr
 // rays); the other launches are compiled without that code.
 template <bool EXACT, class Src, int BS, bool CAM = false>
 __global__ void __launch_bounds__(BS, 1024 / BS)
-    k_extend(Src src, int b, const int* __restrict__ qin, int* counters, const float4* __restrict__ ray_o,
-             const float4* __restrict__ ray_d, float4* __restrict__ hits, int sb, const float4* __restrict__ shadow,
+    k_extend(Src src, int b, const int* __restrict__ qin, int* counters, const float4* __restrict__ ray,
+             float4* __restrict__ hits, int sb, const float4* __restrict__ shadow,
              float4* __restrict__ rad, long long shadow_cap, int* err) {
   // Items [0, n): closest hit of bounce b's queue.  Items [n, n + ns): the
   // shadow rays bounce sb (the previous one) emitted, traced any-hit here so
@@ -514,12 +582,16 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
       float3 o, d;
       int p;
       if (cam_n) {
-        uint32_t pix_unused, smp_unused;
-        p = src.camera_ray(i, fb, o, d, pix_unused, smp_unused);
+        const auto c = src.camera_item(i, fb);
+        p = c.p;
+        o = src.camera_pos();
+        d = src.camera_ray(c);
       } else {
         p = qin[i];
-        o = xyz(ray_o[p]);
-        d = xyz(ray_d[p]);
+        float4 o4, d4;
+        load_pair(ray, p, o4, d4);
+        o = xyz(o4);
+        d = xyz(d4);
       }
       const int si = src.seg(p);
       const DevScene S = src.scene(si);
@@ -788,22 +860,16 @@ __device__ __forceinline__ void shade_vertex(const DevScene& S, const RenderK& K
 // k_shade's vertex output: guides of bounce 0 and the next ray go to the
 // path's state at once
 struct PathStateOut {
-  float4* gn;
-  float4* ga;
-  float4* ray_o;
-  float4* ray_d;
+  float4* gd;
+  float4* ray;
   float4* thr;
   int p, b;
   uint32_t pix;  // the path's pixel, kept in thr.w for the later bounces
   __device__ __forceinline__ void guides(float4 n, float4 a) {
-    if (b == 0) {
-      gn[p] = n;
-      ga[p] = a;
-    }
+    if (b == 0) store_pair(gd, p, n, a);
   }
   __device__ __forceinline__ void next(float3 o, float ior, float3 d, float w, float3 t) {
-    ray_o[p] = make_float4(o.x, o.y, o.z, ior);
-    ray_d[p] = make_float4(d.x, d.y, d.z, w);
+    store_pair(ray, p, make_float4(o.x, o.y, o.z, ior), make_float4(d.x, d.y, d.z, w));
     thr[p] = make_float4(t.x, t.y, t.z, __uint_as_float(pix));
   }
 };
@@ -811,10 +877,9 @@ struct PathStateOut {
 template <class Src>
 __global__ void __launch_bounds__(128, Src::kBatch ? 5 : 1) k_shade(Src src, int b, const int* __restrict__ qin,
                                                int* __restrict__ qout, int* counters,
-                                               const int* __restrict__ frame_base, float4* __restrict__ ray_o,
-                                               float4* __restrict__ ray_d, float4* __restrict__ thr_b,
-                                               float4* __restrict__ rad_b, float4* __restrict__ gn,
-                                               float4* __restrict__ ga, const float4* __restrict__ hits,
+                                               const int* __restrict__ frame_base, float4* __restrict__ ray,
+                                               float4* __restrict__ thr_b, float4* __restrict__ rad_b,
+                                               float4* __restrict__ gd, const float4* __restrict__ hits,
                                                float4* __restrict__ shadow, int* err) {
   // camera items: bounce 0 without k_generate (see k_extend); the path's
   // state is the camera ray, unit throughput and no radiance yet.  Nothing
@@ -847,29 +912,29 @@ __global__ void __launch_bounds__(128, Src::kBatch ? 5 : 1) k_shade(Src src, int
     if (valid) {
       float4 o4, d4, t4;
       uint32_t pix_id, smp;
+      const float4 h = hits[i];
       if (cam_n) {
-        float3 co, cd;
-        p = src.camera_ray(i, fb, co, cd, pix_id, smp);
+        const auto c = src.camera_item(i, fb);
+        p = c.p;
+        pix_id = src.pixel(c);
+        smp = c.smp;
+        // made for misses too, whose direction only the sky needs: waiting
+        // for the hit record first took the frame's shade 5.8 -> 7.7 ms
+        const float3 co = src.camera_pos(), cd = src.camera_ray(c);
         o4 = make_float4(co.x, co.y, co.z, 1.0f);
         d4 = make_float4(cd.x, cd.y, cd.z, 0.0f);
         t4 = make_float4(1.0f, 1.0f, 1.0f, 0.0f);
       } else {
         p = qin[i];
-        o4 = ray_o[p];
-        d4 = ray_d[p];
+        load_pair(ray, p, o4, d4);
         t4 = thr_b[p];
         pix_id = __float_as_uint(t4.w);
         smp = src.sample(si, p, fb);
       }
-      const float4 h = hits[i];
       rng.init(pix_id, smp, (uint32_t)b, K.seed);
       Vertex v;
-      PathStateOut out{gn, ga, ray_o, ray_d, thr_b, p, b, pix_id};
+      PathStateOut out{gd, ray, thr_b, p, b, pix_id};
       shade_vertex(S, K, mis, b, last_bounce, xyz(o4), xyz(d4), xyz(t4), o4.w, d4.w, h, rng, v, out);
-      if (!v.hit && cam_n) {  // no first hit: empty guides
-        gn[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        ga[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
       alive = v.alive;
       do_nee = v.do_nee;
       nee_scale = v.nee_scale;
@@ -878,10 +943,12 @@ __global__ void __launch_bounds__(128, Src::kBatch ? 5 : 1) k_shade(Src src, int
       alb = v.alb;
       thr_nee = v.thr_nee;
       if (cam_n) {
-        rad_b[p] = make_float4(v.add.x, v.add.y, v.add.z, 0.0f);  // the path's first radiance
-      } else if (v.has_add) {
+        rad_b[p] = make_float4(v.add.x, v.add.y, v.add.z, v.hit ? 1.0f : 0.0f);  // the path's first radiance
+      } else if (v.has_add || (b == 0 && v.hit)) {
         float4 r = rad_b[p];
-        rad_b[p] = make_float4(r.x + v.add.x, r.y + v.add.y, r.z + v.add.z, 0.0f);
+        if (v.has_add) r = make_float4(r.x + v.add.x, r.y + v.add.y, r.z + v.add.z, r.w);
+        if (b == 0 && v.hit) r.w = 1.0f;
+        rad_b[p] = r;
       }
     }
     // next-event estimation: shadow records for connect.  The default
@@ -998,7 +1065,7 @@ struct RegisterOut {
 template <bool EXACT, class Src>
 __global__ void __launch_bounds__(128) k_tail(Src src, int b, const int* __restrict__ qin, int* counters,
                                               int max_paths, const int* __restrict__ frame_base,
-                                              const float4* __restrict__ ray_o, const float4* __restrict__ ray_d,
+                                              const float4* __restrict__ ray,
                                               const float4* __restrict__ thr_b, float4* __restrict__ rad_b,
                                               const float4* __restrict__ hits, int* err) {
   const int taken = *(volatile int*)&counters[C_TAIL];
@@ -1026,7 +1093,9 @@ __global__ void __launch_bounds__(128) k_tail(Src src, int b, const int* __restr
       if constexpr (Src::kBatch) job = src.segs[si].job;
       const int closest0 = n_closest, shadow0 = n_shadow;
       const bool mis = K.mis && S.light_of_lin != nullptr;
-      const float4 o4 = ray_o[p], d4 = ray_d[p], t4 = thr_b[p];
+      float4 o4, d4;
+      load_pair(ray, p, o4, d4);
+      const float4 t4 = thr_b[p];
       float3 o = xyz(o4), d = xyz(d4), thr = xyz(t4);
       float ior = o4.w, w = d4.w;
       float4 h = hits[i];
@@ -1038,7 +1107,7 @@ __global__ void __launch_bounds__(128) k_tail(Src src, int b, const int* __restr
         Vertex v;
         RegisterOut out;
         shade_vertex(S, K, mis, bb, (bb + 1) >= K.max_depth, o, d, thr, ior, w, h, rng, v, out);
-        if (v.has_add) r = make_float4(r.x + v.add.x, r.y + v.add.y, r.z + v.add.z, 0.0f);
+        if (v.has_add) r = make_float4(r.x + v.add.x, r.y + v.add.y, r.z + v.add.z, r.w);
         if (v.do_nee) {
           // the shadow rays this vertex would have written as records, traced
           // in record order and summed as the next extend launch sums them
@@ -1105,8 +1174,7 @@ __global__ void __launch_bounds__(128) k_tail(Src src, int b, const int* __restr
 // pix: its accumulator index.
 __device__ __forceinline__ void accumulate_pixel(float clamp, int spf, int fb, long long P, long long path0,
                                                  long long src, long long pix, const float4* __restrict__ rad,
-                                                 const float4* __restrict__ gn, const float4* __restrict__ ga,
-                                                 const JobAcc& A) {
+                                                 const float4* __restrict__ gd, const JobAcc& A) {
   float4 a = A.acc_r[pix], an = A.acc_n[pix], aa = A.acc_a[pix];
   double sx = 0.0, sy = 0.0, sz = 0.0;
   const bool f64 = A.acc64 != nullptr;
@@ -1134,24 +1202,30 @@ __device__ __forceinline__ void accumulate_pixel(float clamp, int spf, int fb, l
     }
   };
   // the wave's samples are read once: streaming loads, kU frames in flight
-  // per thread ahead of the (sequential) running-mean updates
+  // per thread ahead of the (sequential) running-mean updates; the guides of
+  // the samples whose first ray hit something (rad.w) follow
   constexpr int kU = 4;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   int f = 0;
   for (; f + kU <= spf; f += kU) {
+    const long long p = path0 + (long long)f * P + src;
     float4 s[kU], g[kU], al[kU];
 #pragma unroll
+    for (int u = 0; u < kU; ++u) s[u] = __ldcs(rad + p + u * P);
+#pragma unroll
     for (int u = 0; u < kU; ++u) {
-      const long long p = path0 + (long long)(f + u) * P + src;
-      s[u] = __ldcs(rad + p);
-      g[u] = __ldcs(gn + p);
-      al[u] = __ldcs(ga + p);
+      g[u] = al[u] = zero;
+      if (s[u].w != 0.0f) load_pair_cs(gd, p + u * P, g[u], al[u]);
     }
 #pragma unroll
     for (int u = 0; u < kU; ++u) fold(s[u], g[u], al[u], fb + f + u);
   }
   for (; f < spf; ++f) {
     const long long p = path0 + (long long)f * P + src;
-    fold(__ldcs(rad + p), __ldcs(gn + p), __ldcs(ga + p), fb + f);
+    const float4 s = __ldcs(rad + p);
+    float4 g = zero, al = zero;
+    if (s.w != 0.0f) load_pair_cs(gd, p, g, al);
+    fold(s, g, al, fb + f);
   }
   A.acc_r[pix] = a;
   A.acc_n[pix] = an;
@@ -1165,20 +1239,19 @@ __device__ __forceinline__ void accumulate_pixel(float clamp, int spf, int fb, l
   A.pixels[pix] = make_float4(sqrtf(fminf(a.x, 1.0f)), sqrtf(fminf(a.y, 1.0f)), sqrtf(fminf(a.z, 1.0f)), 0.0f);
 }
 
-__global__ void k_accumulate(RenderK K, JobAcc A, const float4* __restrict__ rad, const float4* __restrict__ gn,
-                             const float4* __restrict__ ga) {
+__global__ void k_accumulate(RenderK K, JobAcc A, const float4* __restrict__ rad, const float4* __restrict__ gd) {
   int fb = *A.frame_base;
   // pixels in strip order: a frame's samples are read contiguously
   for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < K.P;
        s += (long long)gridDim.x * blockDim.x) {
     int px, py;
     strip_pixel(K, s, px, py);
-    accumulate_pixel(K.clamp, K.spf, fb, K.P, 0, s, (long long)py * K.W + px, rad, gn, ga, A);
+    accumulate_pixel(K.clamp, K.spf, fb, K.P, 0, s, (long long)py * K.W + px, rad, gd, A);
   }
 }
 
 __global__ void k_accumulate_batch(BatchSrc src, int n_segs, long long total, const float4* __restrict__ rad,
-                                   const float4* __restrict__ gn, const float4* __restrict__ ga) {
+                                   const float4* __restrict__ gd) {
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     int si = find_seg<true>(src.segs, n_segs, t);
@@ -1188,8 +1261,8 @@ __global__ void k_accumulate_batch(BatchSrc src, int n_segs, long long total, co
     const RenderK& K = src.ks[g.job];
     int px, py;
     strip_pixel(K, t - g.acc0, px, py);
-    accumulate_pixel(K.clamp, g.frames, *A.frame_base, g.P, g.path0, t - g.acc0, (long long)py * K.W + px, rad, gn,
-                     ga, A);
+    accumulate_pixel(K.clamp, g.frames, *A.frame_base, g.P, g.path0, t - g.acc0, (long long)py * K.W + px, rad, gd,
+                     A);
   }
 }
 
@@ -1239,8 +1312,9 @@ struct Accum {
   int frames = 0;
   // wavefront state
   long long cap = 0, shadow_cap = 0;
-  DevBuf<float4> ray_o, ray_d, thr, rad, gn, ga, hits, shadow;
+  DevBuf<float4> ray, thr, rad, gd, hits, shadow;  // ray, gd: two per path
   DevBuf<int> q0, q1, counters;
+  DevBuf<float2> phase;  // camera phases of the wave's pixels (k_phase)
   // graph cache
   cudaGraphExec_t gexec = nullptr;
   bool g_timed = false;
@@ -1322,6 +1396,11 @@ static RenderK make_k(const rx_render_params* p, const Accum* a, int spf, long l
   K.W = p->width;
   K.H = p->height;
   K.P = (long long)p->width * p->height;
+  K.rW = 1.0f / (float)std::max(p->width, 1);
+  K.rH = 1.0f / (float)std::max(p->height, 1);
+  K.strip = FastDiv((uint32_t)std::max<long long>(1, (long long)kStripRows * p->width));
+  K.cam_log2 = group_log2(std::max(spf, 1));
+  K.span = FastDiv((uint32_t)std::max<long long>(1, K.P << K.cam_log2));
   K.spf = spf;
   K.fov_tan = p->fov_tan;
   K.aspect = p->aspect;
@@ -1353,11 +1432,16 @@ static int blocks_for(Ctx* ctx, const void* fn, int block) {
   return per_sm * ctx->num_sms;
 }
 
+// the phases k_phase computes for this wave, or null
+static const float2* wave_phase(const Accum* a, const RenderK& K) {
+  return K.camera0 && K.spf >= kPhaseFrames ? a->phase.p : nullptr;
+}
+
 static void launch_extend(Accum* a, const DevScene& S, const RenderK& K, int b, const int* qin, int sb) {
   Ctx* ctx = a->ctx;
-  SingleSrc src{S, K, a->frame_base.p};
+  SingleSrc src{S, K, a->frame_base.p, wave_phase(a, K)};
   auto go = [&](auto kernel) {
-    kernel<<<a->occ_ext, 128, 0, ctx->stream>>>(src, b, qin, a->counters.p, a->ray_o.p, a->ray_d.p, a->hits.p, sb,
+    kernel<<<a->occ_ext, 128, 0, ctx->stream>>>(src, b, qin, a->counters.p, a->ray.p, a->hits.p, sb,
                                                  a->shadow.p, a->rad.p, K.shadow_cap, ctx->d_err);
   };
   const bool cam = b == 0 && K.camera0;
@@ -1372,10 +1456,10 @@ static void launch_extend(Accum* a, const DevScene& S, const RenderK& K, int b, 
 
 static void launch_tail(Accum* a, const DevScene& S, const RenderK& K, int b, const int* qin) {
   Ctx* ctx = a->ctx;
-  SingleSrc src{S, K, a->frame_base.p};
+  SingleSrc src{S, K, a->frame_base.p, wave_phase(a, K)};
   auto go = [&](auto kernel) {
     kernel<<<a->occ_tail, 128, 0, ctx->stream>>>(src, b, qin, a->counters.p, a->tail_paths, a->frame_base.p,
-                                                  a->ray_o.p, a->ray_d.p, a->thr.p, a->rad.p, a->hits.p, ctx->d_err);
+                                                  a->ray.p, a->thr.p, a->rad.p, a->hits.p, ctx->d_err);
   };
   if (S.exact_slab) go(k_tail<true, SingleSrc>);
   else go(k_tail<false, SingleSrc>);
@@ -1402,8 +1486,12 @@ static void enqueue_wave(Accum* a, Scene* sc, const RenderK& K, bool timed, int*
   if (!K.camera0) {
     long long total = (long long)K.spf * K.P;
     int gblocks = (int)std::min<long long>((total + 255) / 256, (long long)ctx->num_sms * 16);
-    k_generate<<<std::max(gblocks, 1), 256, 0, st>>>(K, a->frame_base.p, a->ray_o.p, a->ray_d.p, a->thr.p,
-                                                      a->rad.p, a->gn.p, a->ga.p, a->q0.p, a->counters.p);
+    k_generate<<<std::max(gblocks, 1), 256, 0, st>>>(K, a->frame_base.p, a->ray.p, a->thr.p,
+                                                      a->rad.p, a->q0.p, a->counters.p);
+    ++launches;
+  } else if (wave_phase(a, K)) {
+    const int pblocks = (int)std::min<long long>((K.P + 255) / 256, (long long)ctx->num_sms * 8);
+    k_phase<<<std::max(pblocks, 1), 256, 0, st>>>(K, a->phase.p);
     ++launches;
   }
   mark(K_OTHER);
@@ -1422,9 +1510,9 @@ static void enqueue_wave(Accum* a, Scene* sc, const RenderK& K, bool timed, int*
       ++launches;
       mark(K_EXTEND);
     }
-    k_shade<SingleSrc><<<a->occ_shade, 128, 0, st>>>(SingleSrc{S, K, a->frame_base.p}, b, qin, qout, a->counters.p,
-                                                      a->frame_base.p, a->ray_o.p, a->ray_d.p, a->thr.p, a->rad.p,
-                                                      a->gn.p, a->ga.p, a->hits.p, a->shadow.p, ctx->d_err);
+    k_shade<SingleSrc><<<a->occ_shade, 128, 0, st>>>(SingleSrc{S, K, a->frame_base.p, wave_phase(a, K)}, b, qin, qout, a->counters.p,
+                                                      a->frame_base.p, a->ray.p, a->thr.p, a->rad.p,
+                                                      a->gd.p, a->hits.p, a->shadow.p, ctx->d_err);
     ++launches;
     mark(K_SHADE);
   }
@@ -1436,7 +1524,7 @@ static void enqueue_wave(Accum* a, Scene* sc, const RenderK& K, bool timed, int*
   }
   int ablocks = (int)std::min<long long>((K.P + 255) / 256, (long long)ctx->num_sms * 16);
   JobAcc A{a->acc_r.p, a->acc_n.p, a->acc_a.p, a->pixels.p, a->acc64.p, a->frame_base.p, a->rays.p};
-  k_accumulate<<<std::max(ablocks, 1), 256, 0, st>>>(K, A, a->rad.p, a->gn.p, a->ga.p);
+  k_accumulate<<<std::max(ablocks, 1), 256, 0, st>>>(K, A, a->rad.p, a->gd.p);
   mark(K_ACCUM);
   k_finish<<<1, 1, 0, st>>>(a->counters.p, K.max_depth, a->frame_base.p, a->rays.p, K.spf);
   launches += 2;
@@ -1445,12 +1533,16 @@ static void enqueue_wave(Accum* a, Scene* sc, const RenderK& K, bool timed, int*
   *n_events = ev_i;
 }
 
-static int ensure_wave_buffers(Accum* a, long long cap, long long shadow_cap) {
+static int ensure_wave_buffers(Accum* a, long long cap, long long shadow_cap, bool phases) {
   Ctx* ctx = a->ctx;
+  if (phases && !a->phase.p) {
+    a->drop_graph();
+    if (!a->phase.alloc(ctx, a->P)) return set_error(ctx, "out of device memory for camera phases"), RX_ERR_CAPACITY;
+  }
   if (cap > a->cap) {
     a->drop_graph();
-    bool ok = a->ray_o.alloc(ctx, cap) && a->ray_d.alloc(ctx, cap) && a->thr.alloc(ctx, cap) &&
-              a->rad.alloc(ctx, cap) && a->gn.alloc(ctx, cap) && a->ga.alloc(ctx, cap) &&
+    bool ok = a->ray.alloc(ctx, 2 * cap) && a->thr.alloc(ctx, cap) &&
+              a->rad.alloc(ctx, cap) && a->gd.alloc(ctx, 2 * cap) &&
               a->hits.alloc(ctx, cap) && a->q0.alloc(ctx, cap) && a->q1.alloc(ctx, cap);
     if (!ok) {
       a->cap = 0;
@@ -1534,7 +1626,7 @@ int render(Scene* sc, Accum* a, const rx_render_params* p, int frames) {
   if (cap >= (1LL << 31)) return set_error(ctx, "render: wavefront of %lld paths is too large", cap), RX_ERR_CAPACITY;
   int nl = sc->n_lights;
   long long shadow_cap = cap * (p->direct_light_mode == 1 ? std::max(nl, 1) : 1);
-  rc = ensure_wave_buffers(a, cap, shadow_cap);
+  rc = ensure_wave_buffers(a, cap, shadow_cap, spf >= kPhaseFrames && p->max_depth > 0);
   if (rc) return rc;
   if (p->max_depth == 0) {
     // no bounce: every sample is black (the reference's loop never runs)
@@ -1766,7 +1858,7 @@ struct Batch {
   int tail_paths = kTailPaths;  // k_tail's threshold (0: never)
   bool use_graph = true;
   long long cap = 0, shadow_cap = 0;
-  DevBuf<float4> ray_o, ray_d, thr, rad, gn, ga, hits, shadow;
+  DevBuf<float4> ray, thr, rad, gd, hits, shadow;  // ray, gd: two per path
   DevBuf<int> q0, q1, counters, pseg;
   DevBuf<DevScene> d_scenes;
   DevBuf<RenderK> d_ks;
@@ -1880,7 +1972,7 @@ static std::vector<PlannedWave> plan_waves(const Batch* b, std::vector<WaveSeg>&
 template <int BS>
 static void launch_extend_batch(Batch* B, const BatchSrc& src, bool wide, int occ, int b, const int* qin, int sb) {
   auto go = [&](auto kernel, const auto& s) {
-    kernel<<<occ, BS, 0, B->ctx->stream>>>(s, b, qin, B->counters.p, B->ray_o.p, B->ray_d.p, B->hits.p, sb,
+    kernel<<<occ, BS, 0, B->ctx->stream>>>(s, b, qin, B->counters.p, B->ray.p, B->hits.p, sb,
                                            B->shadow.p, B->rad.p, B->shadow_cap, B->ctx->d_err);
   };
   if (wide) go(k_extend<false, BatchSrc4, BS>, BatchSrc4{src});
@@ -1913,9 +2005,8 @@ static void enqueue_batch(Batch* B, const std::vector<PlannedWave>& waves, int* 
     BatchSrc src{B->pseg.p, B->d_segs.p + w.seg0, B->d_scenes.p, B->d_ks.p, B->d_accs.p, B->d_job_rays.p};
     cudaMemsetAsync(B->counters.p, 0, sizeof(int) * C_N, st);
     int gblocks = (int)std::min<long long>((w.paths + 255) / 256, (long long)ctx->num_sms * 16);
-    k_generate_batch<<<std::max(gblocks, 1), 256, 0, st>>>(src, w.nseg, w.paths, B->ray_o.p, B->ray_d.p, B->thr.p,
-                                                            B->rad.p, B->gn.p, B->ga.p, B->q0.p, B->pseg.p,
-                                                            B->counters.p);
+    k_generate_batch<<<std::max(gblocks, 1), 256, 0, st>>>(src, w.nseg, w.paths, B->ray.p, B->thr.p,
+                                                            B->rad.p, B->q0.p, B->pseg.p, B->counters.p);
     ++launches;
     auto ext = [&](int b, const int* qin, int sb) {
       if (B->ext_block == 64) launch_extend_batch<64>(B, src, wide, occ_ext, b, qin, sb);
@@ -1929,22 +2020,20 @@ static void enqueue_batch(Batch* B, const std::vector<PlannedWave>& waves, int* 
       ext(b, qin, b >= 1 ? b - 1 : -1);
       if (b >= 1 && B->tail_paths > 0) {
         auto tail = [&](auto kernel, const auto& s) {
-          kernel<<<occ_tail, 128, 0, st>>>(s, b, qin, B->counters.p, B->tail_paths, nullptr, B->ray_o.p, B->ray_d.p,
+          kernel<<<occ_tail, 128, 0, st>>>(s, b, qin, B->counters.p, B->tail_paths, nullptr, B->ray.p,
                                            B->thr.p, B->rad.p, B->hits.p, ctx->d_err);
         };
         if (wide) tail(k_tail<false, BatchSrc4>, BatchSrc4{src});
         else tail(k_tail<false, BatchSrc>, src);
         ++launches;
       }
-      k_shade<BatchSrc><<<occ_shade, 128, 0, st>>>(src, b, qin, qout, B->counters.p, nullptr, B->ray_o.p,
-                                                    B->ray_d.p, B->thr.p, B->rad.p, B->gn.p, B->ga.p, B->hits.p,
+      k_shade<BatchSrc><<<occ_shade, 128, 0, st>>>(src, b, qin, qout, B->counters.p, nullptr, B->ray.p, B->thr.p, B->rad.p, B->gd.p, B->hits.p,
                                                     B->shadow.p, ctx->d_err);
       ++launches;
     }
     if (w.max_depth > 0) ext(-1, nullptr, w.max_depth - 1);
     int ablocks = (int)std::min<long long>((w.acc_threads + 255) / 256, (long long)ctx->num_sms * 16);
-    k_accumulate_batch<<<std::max(ablocks, 1), 256, 0, st>>>(src, w.nseg, w.acc_threads, B->rad.p, B->gn.p,
-                                                              B->ga.p);
+    k_accumulate_batch<<<std::max(ablocks, 1), 256, 0, st>>>(src, w.nseg, w.acc_threads, B->rad.p, B->gd.p);
     k_finish_batch<<<(w.nseg + 127) / 128, 128, 0, st>>>(src, w.nseg);
     launches += 2;
   }
@@ -1978,8 +2067,8 @@ int batch_render(Batch* B) {
   // wave buffers
   if (cap > B->cap) {
     B->drop_graph();
-    bool ok = B->ray_o.alloc(ctx, cap) && B->ray_d.alloc(ctx, cap) && B->thr.alloc(ctx, cap) &&
-              B->rad.alloc(ctx, cap) && B->gn.alloc(ctx, cap) && B->ga.alloc(ctx, cap) && B->hits.alloc(ctx, cap) &&
+    bool ok = B->ray.alloc(ctx, 2 * cap) && B->thr.alloc(ctx, cap) &&
+              B->rad.alloc(ctx, cap) && B->gd.alloc(ctx, 2 * cap) && B->hits.alloc(ctx, cap) &&
               B->q0.alloc(ctx, cap) && B->q1.alloc(ctx, cap) && B->pseg.alloc(ctx, cap);
     if (!ok) {
       B->cap = 0;
@@ -2076,8 +2165,8 @@ int batch_reserve(Batch* B, long long cap) {
   Ctx* ctx = B->ctx;
   if (cap > B->cap) {
     B->drop_graph();
-    bool ok = B->ray_o.alloc(ctx, cap) && B->ray_d.alloc(ctx, cap) && B->thr.alloc(ctx, cap) &&
-              B->rad.alloc(ctx, cap) && B->gn.alloc(ctx, cap) && B->ga.alloc(ctx, cap) && B->hits.alloc(ctx, cap) &&
+    bool ok = B->ray.alloc(ctx, 2 * cap) && B->thr.alloc(ctx, cap) &&
+              B->rad.alloc(ctx, cap) && B->gd.alloc(ctx, 2 * cap) && B->hits.alloc(ctx, cap) &&
               B->q0.alloc(ctx, cap) && B->q1.alloc(ctx, cap) && B->pseg.alloc(ctx, cap);
     if (!ok) {
       B->cap = 0;
@@ -2106,13 +2195,13 @@ void batch_use_graph(Batch* B, bool on) {
 
 size_t accum_bytes(const Accum* a) {
   return a->acc_r.bytes() + a->acc_n.bytes() + a->acc_a.bytes() + a->pixels.bytes() + a->acc64.bytes() +
-         a->ray_o.bytes() + a->ray_d.bytes() + a->thr.bytes() + a->rad.bytes() + a->gn.bytes() + a->ga.bytes() +
-         a->hits.bytes() + a->shadow.bytes() + a->q0.bytes() + a->q1.bytes() + a->dn0.bytes() + a->dn1.bytes() +
+         a->ray.bytes() + a->thr.bytes() + a->rad.bytes() + a->gd.bytes() +
+         a->hits.bytes() + a->shadow.bytes() + a->q0.bytes() + a->q1.bytes() + a->phase.bytes() + a->dn0.bytes() + a->dn1.bytes() +
          a->dn_out.bytes() + 64;
 }
 
 size_t batch_bytes(const Batch* B) {
-  return B->ray_o.bytes() + B->ray_d.bytes() + B->thr.bytes() + B->rad.bytes() + B->gn.bytes() + B->ga.bytes() +
+  return B->ray.bytes() + B->thr.bytes() + B->rad.bytes() + B->gd.bytes() +
          B->hits.bytes() + B->shadow.bytes() + B->q0.bytes() + B->q1.bytes() + B->pseg.bytes();
 }
 
