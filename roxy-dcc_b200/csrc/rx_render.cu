@@ -34,7 +34,11 @@ constexpr int kMaxBounce = 64;
 constexpr int kTailPaths = 1 << 16;
 // counters, 64 per kind (one per bounce): queue lengths, extend fetch,
 // shade fetch, shadow record counts; then the bounce + 1 at which k_tail
-// took the wave over (0: not taken) and k_tail's fetch counter
+// took the wave over (0: not taken) and k_tail's fetch counter.  Atomics on
+// one address pass at about one per clock, and counters may share an L2
+// slice: with a fetch per warp and 32 items k_shade took 5.8 ms of a 133 M
+// path frame, or 8.4 where the counters happened to lie so; with larger
+// fetches for long queues (shade_chunk) it takes 4.7 wherever they lie.
 enum { C_Q = 0, C_FE = 64, C_FS = 128, C_S = 192, C_TAIL = 256, C_FT = 257, C_N = 260 };
 constexpr float kPi = 3.14159265358979323846f;
 constexpr float kTwoPi = 6.283185307179586f;
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
   const int total = n + (int)ns;
   int* fetch = &counters[C_FE + (b >= 0 ? b : kMaxBounce - 1)];
   const int lane = threadIdx.x & 31;
+  int run_job = -1, run_rays = 0;  // batches: rays of this warp's current job, not yet added to its count
   for (;;) {
     int base = 0;
     if (lane == 0) base = atomicAdd(fetch, 32);
@@ -607,12 +612,24 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
       if constexpr (!CAM) rays_here = shadow_item<EXACT>(src, shadow, i - n, ns, rad, err, job);
     }
     if constexpr (Src::kBatch) {
-      // rays traced, counted per job (lanes of a warp mostly share one)
-      unsigned m = __match_any_sync(0xffffffffu, job);
-      int tot = __reduce_add_sync(m, rays_here);
-      if (job >= 0 && lane == __ffs(m) - 1) atomicAdd(src.job_rays + job, (unsigned long long)tot);
+      // rays traced, counted per job: lanes of a warp mostly share one, and
+      // consecutive items of a warp too
+      const unsigned m = __match_any_sync(0xffffffffu, job);
+      const int tot = __reduce_add_sync(m, rays_here);
+      if (__all_sync(0xffffffffu, m == 0xffffffffu)) {
+        if (job != run_job) {
+          if (run_rays && lane == 0) atomicAdd(src.job_rays + run_job, (unsigned long long)run_rays);
+          run_job = job;
+          run_rays = 0;
+        }
+        run_rays += tot;
+      } else if (job >= 0 && lane == __ffs(m) - 1) {
+        atomicAdd(src.job_rays + job, (unsigned long long)tot);
+      }
     }
   }
+  if constexpr (Src::kBatch)
+    if (run_rays && lane == 0) atomicAdd(src.job_rays + run_job, (unsigned long long)run_rays);
 }
 
 // warp-aggregated append: one atomic per warp, ranks by ballot / popc
@@ -874,6 +891,15 @@ struct PathStateOut {
   }
 };
 
+// Items a warp of k_shade fetches at once: 32, and up to 128 for queues long
+// enough that the fetches' atomics on one address take a good part of the
+// launch.  Larger fetches spread the warps over a longer stretch of the
+// queue, and the next queue inherits that order: on the 1080p frame (133 M,
+// 33 M, ... paths) fetches of 64 / 128 / 256 / 512 items everywhere gave
+// extend 18.73 / 18.75 / 18.79 / 18.87 ms (18.66 with 32) and shade 4.84 /
+// 4.73 / 4.75 / 4.84 (5.8-8.4); the batched scenes (10 M paths) lost 1-4 %.
+__device__ __forceinline__ unsigned shade_chunk(unsigned n) { return 32u * min(4u, max(1u, n >> 24)); }
+
 template <class Src>
 __global__ void __launch_bounds__(128, Src::kBatch ? 5 : 1) k_shade(Src src, int b, const int* __restrict__ qin,
                                                int* __restrict__ qout, int* counters,
@@ -889,13 +915,17 @@ __global__ void __launch_bounds__(128, Src::kBatch ? 5 : 1) k_shade(Src src, int
   const int n = cam_n ? (int)cam_n : *(volatile int*)&counters[C_Q + b];
   const int fb = frame_base ? *frame_base : 0;
   const int lane = threadIdx.x & 31;
-  for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&counters[C_FS + b], 32);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
-    int i = base + lane;
-    bool valid = i < n;
+  const unsigned chunk = shade_chunk((unsigned)n);
+  unsigned at = 0, end = 0;
+  for (;; at += 32) {
+    if (at >= end) {
+      if (lane == 0) at = (unsigned)atomicAdd(&counters[C_FS + b], (int)chunk);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (at >= (unsigned)n) break;
+      end = min(at + chunk, (unsigned)n);
+    }
+    const int base = (int)at, i = base + lane;
+    const bool valid = (unsigned)i < (unsigned)n;
     // lanes past the end take the first item's job (they write nothing)
     const int si = src.seg(cam_n ? 0 : qin[valid ? i : base]);
     const DevScene S = src.scene(si);
@@ -1078,12 +1108,14 @@ __global__ void __launch_bounds__(128) k_tail(Src src, int b, const int* __restr
   const int fb = frame_base ? *frame_base : 0;
   const int lane = threadIdx.x & 31;
   int n_closest = 0, n_shadow = 0;  // rays traced here, counted as the one-bounce launches count them
+  const unsigned first = (blockIdx.x * 128u + threadIdx.x) & ~31u;
   for (;;) {
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&counters[C_FT], 32);
+    if (first >= (unsigned)n) break;  // no items can reach this warp
+    unsigned base = 0;
+    if (lane == 0) base = (unsigned)atomicAdd(&counters[C_FT], 32);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
-    const int i = base + lane;
+    if (base >= (unsigned)n) break;
+    const int i = (int)base + lane;
     int job = -1, rays_here = 0;  // batches: the rays this lane traced, counted for its job
     if (i < n) {
       const int p = qin[i];
