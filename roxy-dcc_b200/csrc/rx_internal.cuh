@@ -65,10 +65,10 @@ struct Node4 {
 //             with e1 = v1 - v0, e2 = v2 - v0
 //   sphere:   a = (centre, kind = 1), b = (radius, 0, 0, 0), c = 0
 //   cube:     a = (centre, kind = 2), b = (half extents, 0), c = 0
-// Divergent rays pay one pass of the L1 data pipe per lane and load whatever
-// its width, so a record is read as one 32-byte load (a, b) and, for a
-// triangle, one 8-byte load (load_prim); the record keeps both inside one
-// cache line.
+// A record is read as one 32-byte load (a, b) and, for a triangle, one 8-byte
+// load (load_prim), both inside one cache line: two requests instead of three.
+// A 32-byte load of divergent lanes still takes two passes of the L1 data
+// pipe, so it saves instructions and requests, not passes.
 enum PrimKind { PRIM_TRI = 0, PRIM_SPHERE = 1, PRIM_CUBE = 2 };
 constexpr int kPrimQuads = 4;
 

@@ -100,6 +100,20 @@ def test_cornell_same_randoms_and_wavefront_sizes():
         assert abs(g["rays"] - o["rays"]) <= 0.005 * o["rays"]
 
 
+def test_large_waves_equal_small_waves():
+    """37 M paths in one wave (long-queue fetches, camera phases once per
+    pixel) and waves of 5 and 9 frames (phases only in the second) add the
+    same samples in the same order: every plane bit for bit."""
+    W, H, spp = 1917, 1081, 18
+    world = workloads.cornell_box(W, H)
+    ref = _gpu_render(world, W, H, spp, 3, seed=7, wave_paths=5 * W * H)
+    for wp in (9 * W * H, 18 * W * H):
+        out = _gpu_render(world, W, H, spp, 3, seed=7, wave_paths=wp)
+        for k in ("radiance", "normal", "albedo", "depth", "pixels"):
+            assert np.array_equal(ref[k].view(np.uint32), out[k].view(np.uint32)), (k, wp)
+        assert ref["rays"] == out["rays"]
+
+
 def _batch_means(world, W, H, batches, per, compat, seed0, dlmd=8, max_depth=8, mis=False, mode=0):
     ds = build_device_scene(world, method="lbvh")
     ds.use_lights(compat)
