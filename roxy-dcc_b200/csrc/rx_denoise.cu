@@ -14,6 +14,7 @@
 // guide float4 (rgb, -) — the accumulators' own layout, so the renderer
 // filters its resident buffers without a copy.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <mutex>
 
@@ -82,6 +83,43 @@ __device__ __forceinline__ float tap_weight(const AtrousArgs& A, float sw, float
   }
   if (A.use_d) {
     float gd = g.w - cn.w;
+    e = __fmaf_rn(gd * gd, A.r2d, e);
+  }
+  return sw * __expf(-e);
+}
+
+// Weight of a pair of pixels as tap_weight's, without branches, so that the
+// pairs of a row interleave; guides that are not in use are zeros (a term of
+// exactly 1, or nothing added to the exponent).
+//
+// EXACT forms div_by's quotient without its range test, which the
+// exponential makes needless for 2 sigma^2 in [2^-30, 2^30]: below 2^-96 any
+// quotient is under 2^-66 and the term is 1; beyond 2^90 it is over 2^60 and
+// the term is 0, also when x is infinite (min keeps a NaN).
+template <bool EXACT, bool GUIDES>
+__device__ __forceinline__ float pair_weight(const AtrousArgs& A, float sw, float4 nb, float4 cc, float4 g, float4 cn,
+                                             float4 al, float4 ca) {
+  const float ex = nb.x - cc.x, ey = nb.y - cc.y, ez = nb.z - cc.z;
+  const float gx = g.x - cn.x, gy = g.y - cn.y, gz = g.z - cn.z, gd = g.w - cn.w;
+  const float hx = al.x - ca.x, hy = al.y - ca.y, hz = al.z - ca.z;
+  if (EXACT) {
+    auto term = [](float x, float s2, float r2) {
+      asm("min.NaN.f32 %0, %0, 0f6C800000;" : "+f"(x));  // 2^90
+      const float q = x * r2;
+      return expf(-__fmaf_rn(__fmaf_rn(-q, s2, x), r2, q));
+    };
+    float w = sw * term((ex * ex + ey * ey) + ez * ez, A.s2c, A.r2c);
+    if (GUIDES) {
+      w = w * term((gx * gx + gy * gy) + gz * gz, A.s2n, A.r2n);
+      w = w * term((hx * hx + hy * hy) + hz * hz, A.s2a, A.r2a);
+      w = w * term(gd * gd, A.s2d, A.r2d);
+    }
+    return w;
+  }
+  float e = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, ex * ex)) * A.r2c;
+  if (GUIDES) {
+    e = __fmaf_rn(__fmaf_rn(gz, gz, __fmaf_rn(gy, gy, gx * gx)), A.r2n, e);
+    e = __fmaf_rn(__fmaf_rn(hz, hz, __fmaf_rn(hy, hy, hx * hx)), A.r2a, e);
     e = __fmaf_rn(gd * gd, A.r2d, e);
   }
   return sw * __expf(-e);
@@ -205,101 +243,150 @@ __global__ void __launch_bounds__(kAtThreads) k_atrous_tiled(AtrousArgs A, int t
 
 // Radius 1 (the renderer's default): a tap's weight is symmetric in its two
 // pixels, bit for bit even in pass 0 ((a - b)^2 equals (b - a)^2 exactly
-// and the spatial weight depends on |dx|, |dy|), so each pair of
-// neighbours is weighed once.  A block loads a 32-column x 16-row grid of
-// the sub-lattice (tiles of outputs plus their one-pixel halo), every grid
-// pixel of rows 0-14 weighs its four forward neighbours (right, down-left,
-// down, down-right) into shared memory, and each output then gathers its
-// nine weights -- the centre's is 1 -- and sums its taps in the reference's
-// order: 4.6 weight evaluations per output instead of 9.
-// P = 1 (pass 0, step 1): one 30 x 14 output tile, lane = grid column.
-// P = 2 (step >= 2): two adjacent x residues side by side, grid column c
-// of residue plane k stored at c * 2 + k, so two neighbouring lanes read
-// and write two adjacent pixels and every 32-byte sector a warp touches is
-// used whole (one residue per block would use half of each); 2 x 14 x 14
-// outputs.
-constexpr int kA1H = 14, kA1GW = 32, kA1GH = 16, kA1Src = (kA1H + 1) * kA1GW;
+// and the spatial weight depends on |dx|, |dy|), so each pair of neighbours
+// is weighed once, and nothing but registers holds it.  A warp owns a strip
+// of the sub-lattice, one lane per column, and walks down its rows: a lane
+// keeps its own pixel and its right neighbour's of the row above and of this
+// row, which is all that the four pairs right, down, down-right and the
+// crossing diagonal need.  The right neighbour's ten channels, the left
+// one's colour and three weights come by shuffles (16 per pixel); the sum of
+// a row is opened with the taps above it and closed one row later, in the
+// reference's tap order.
+// P = 1 (step 1): 30 outputs and two halo lanes.  P = 2 (step >= 2): two
+// adjacent x residues interleaved, lane = column * 2 + residue, so that
+// every 32-byte sector is used whole; 2 x 14 outputs.
+// GUIDES: any guide in use; guides that are not are zeros (pair_weight).
+// Bound by issue: 264 warp instructions per row of 28 outputs in the later
+// passes (16.5 -> 9.8 M at 1280x720 against shared-memory tiles of weights),
+// 71 % of the issue slots of the active cycles.  Five passes at 1280x720
+// with all guides 158 -> 88 us (pass 0 alone 35 -> 24), without guides 102
+// -> 56; 640x360 60 -> 35; 64x48 33 -> 18, where the passes' starts overlap
+// (launch_pass).
+template <bool GUIDES>
+struct AtRow {
+  float4 c, g, a;     // own pixel: colour, normal / depth, albedo
+  float4 rc, rg, ra;  // the right neighbour's
+  float lx, ly, lz;   // the left neighbour's colour
+};
 
-template <bool EXACT, int P>
-__global__ void __launch_bounds__(kAtThreads) k_atrous_r1(AtrousArgs A, int tiles_x, const float4* __restrict__ in,
-                                                          const float4* __restrict__ src,
-                                                          const float4* __restrict__ gn,
-                                                          const float4* __restrict__ ga, float4* __restrict__ out) {
-  constexpr int PW = kA1GW / P, OW = PW - 2, NOUT = P * OW * kA1H;
-  __shared__ float4 s_c[kA1GW * kA1GH], s_g[kA1GW * kA1GH], s_a[kA1GW * kA1GH];
-  __shared__ float s_w[4][kA1Src];  // forward weights: right, down-left, down, down-right
+constexpr int kA1Warps = 4;     // warps (strips) per block
+constexpr int kA1MaxRows = 32;  // longest strip
+// Blocks per SM: 96 registers with pass 0's exponentials, 80 in the later
+// passes, 54 to 60 without guides; fewer registers spill and lose 3-10 %.
+constexpr int a1_blocks(bool exact, bool guides) { return guides ? (exact ? 5 : 6) : 8; }
+
+template <bool EXACT, int P, bool GUIDES>
+__global__ void __launch_bounds__(kA1Warps * 32, a1_blocks(EXACT, GUIDES))
+    k_atrous_r1(AtrousArgs A, int tiles_x, int rows, long long strips, const float4* in,
+                const float4* __restrict__ src, const float4* __restrict__ gn, const float4* __restrict__ ga,
+                float4* out) {
+  constexpr int OW = 32 / P - 2;
+  constexpr unsigned kAll = 0xffffffffu;
   const int step = A.step;
-  const bool need_g = A.use_n || A.use_d;
   const int xres = step / P;  // x residue groups
-  long long b = blockIdx.x;
+  long long b = blockIdx.x * (long long)kA1Warps + (threadIdx.x >> 5);
+  if (b >= strips) return;
   const int rx0 = (int)(b % xres) * P;
   b /= xres;
   const int ry = (int)(b % step);
   b /= step;
   const int tx0 = (int)(b % tiles_x) * OW;
-  const int ty0 = (int)(b / tiles_x) * kA1H;
+  const int ty0 = (int)(b / tiles_x) * rows;
+  const int y0 = ry + step * ty0;  // first output row
+  if (rx0 >= A.W || y0 >= A.H) return;
   const int lane = threadIdx.x & 31;
-  {
-    const int col = lane / P, plane = lane % P;
-    const int gx = reflect_idx(rx0 + plane + step * (tx0 + col - 1), A.W);
-    for (int sy = threadIdx.x >> 5; sy < kA1GH; sy += kAtThreads / 32) {
-      const int gy = reflect_idx(ry + step * (ty0 + sy - 1), A.H);
-      const long long q = (long long)gy * A.W + gx;
-      const int i = sy * kA1GW + lane;
-      s_c[i] = __ldg(in + q);
-      if (need_g) s_g[i] = __ldg(gn + q);
-      if (A.use_a) s_a[i] = __ldg(ga + q);
-    }
-  }
-  __syncthreads();
+  const int col = lane / P, plane = lane % P;
+  const int x = rx0 + plane + step * (tx0 + col - 1);
+  const int gx = reflect_idx(x, A.W);
+  const bool writes = col >= 1 && col <= OW && x < A.W;
+  const int n_out = min(rows, (A.H - 1 - y0) / step + 1);
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  for (int i = threadIdx.x; i < kA1Src; i += kAtThreads) {
-    const int c = (i & 31) / P;
-    const float4 oc = s_c[i], og = need_g ? s_g[i] : zero, oa = A.use_a ? s_a[i] : zero;
-    // right (dx 1), down-left (dx -1, dy 1), down (dy 1), down-right (1, 1)
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int dx = k == 0 ? 1 : k - 2, dy = k == 0 ? 0 : 1;
-      const int tc = c + dx;
-      float w = 0.0f;
-      if (tc >= 0 && tc < PW) {
-        const int t = i + dy * kA1GW + dx * P;
-        w = tap_weight<EXACT>(A, spatial_weight(dx, dy), s_c[t], oc, need_g ? s_g[t] : zero, og,
-                              A.use_a ? s_a[t] : zero, oa);
-      }
-      s_w[k][i] = w;
+  using Row = AtRow<GUIDES>;
+  auto load = [&](Row& w, int y) {
+    const long long q = (long long)reflect_idx(y, A.H) * A.W + gx;
+    w.c = __ldca(in + q);  // written by the pass before: not a read-only load
+    w.g = w.a = zero;
+    if (GUIDES) {
+      if (A.use_n || A.use_d) w.g = __ldg(gn + q);
+      if (A.use_a) w.a = __ldg(ga + q);
     }
-  }
-  __syncthreads();
-  for (int j = threadIdx.x; j < NOUT; j += kAtThreads) {
-    const int oy = j / (P * OW), rem = j - oy * (P * OW);
-    const int plane = rem % P, ox = rem / P;
-    const int x = rx0 + plane + step * (tx0 + ox), y = ry + step * (ty0 + oy);
-    if (x >= A.W || y >= A.H) continue;
-    const int p = (oy + 1) * kA1GW + (ox + 1) * P + plane;
-    constexpr int U = kA1GW, L = P;  // one grid row up, one grid column left
-    // taps in the reference's order: dy -1..1 outer, dx -1..1 inner
-    const int tq[9] = {p - U - L, p - U, p - U + L, p - L, p, p + L, p + U - L, p + U, p + U + L};
-    const float tw[9] = {s_w[3][p - U - L], s_w[2][p - U], s_w[1][p - U + L], s_w[0][p - L], 1.0f,
-                         s_w[0][p], s_w[1][p], s_w[2][p], s_w[3][p]};
-    float ax = 0.0f, ay = 0.0f, az = 0.0f, ws = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float4 nb = s_c[tq[k]];
-      const float w = tw[k];
-      if (EXACT) {
-        ax = ax + nb.x * w;
-        ay = ay + nb.y * w;
-        az = az + nb.z * w;
-      } else {
-        ax = __fmaf_rn(nb.x, w, ax);
-        ay = __fmaf_rn(nb.y, w, ay);
-        az = __fmaf_rn(nb.z, w, az);
-      }
-      ws = ws + w;
+  };
+  // the neighbours' values of a row that has arrived (its first use: no load
+  // is waited for before)
+  auto spread = [&](Row& w) {
+    if (GUIDES && !A.use_n) w.g.x = w.g.y = w.g.z = 0.0f;
+    if (GUIDES && !A.use_d) w.g.w = 0.0f;
+    w.rg = w.ra = zero;
+    w.rc = make_float4(__shfl_down_sync(kAll, w.c.x, P), __shfl_down_sync(kAll, w.c.y, P),
+                       __shfl_down_sync(kAll, w.c.z, P), 0.0f);
+    w.lx = __shfl_up_sync(kAll, w.c.x, P);
+    w.ly = __shfl_up_sync(kAll, w.c.y, P);
+    w.lz = __shfl_up_sync(kAll, w.c.z, P);
+    if (GUIDES) {
+      w.rg = make_float4(__shfl_down_sync(kAll, w.g.x, P), __shfl_down_sync(kAll, w.g.y, P),
+                         __shfl_down_sync(kAll, w.g.z, P), __shfl_down_sync(kAll, w.g.w, P));
+      w.ra = make_float4(__shfl_down_sync(kAll, w.a.x, P), __shfl_down_sync(kAll, w.a.y, P),
+                         __shfl_down_sync(kAll, w.a.z, P), 0.0f);
     }
-    const long long c = (long long)y * A.W + x;
-    out[c] = finish_pixel<EXACT>(A, ax, ay, az, ws, src, c);
+  };
+  float ax, ay, az, ws;
+  auto tap = [&](float cx, float cy, float cz, float w) {
+    if (EXACT) {
+      ax = ax + cx * w;
+      ay = ay + cy * w;
+      az = az + cz * w;
+    } else {
+      ax = __fmaf_rn(cx, w, ax);
+      ay = __fmaf_rn(cy, w, ay);
+      az = __fmaf_rn(cz, w, az);
+    }
+    ws = ws + w;
+  };
+  const float swd = spatial_weight(1, 1), sws = spatial_weight(1, 0);
+  // u: row k - 1, v: row k (own pixels loaded), n: takes row k + 1
+  auto step_row = [&](int k, Row& u, Row& v, Row& n) {
+    if (k < n_out) load(n, y0 + step * (k + 1));
+    spread(v);
+    const float w_dn = pair_weight<EXACT, GUIDES>(A, sws, v.c, u.c, v.g, u.g, v.a, u.a);
+    const float w_dr = pair_weight<EXACT, GUIDES>(A, swd, v.rc, u.c, v.rg, u.g, v.ra, u.a);
+    const float w_ad = pair_weight<EXACT, GUIDES>(A, swd, v.c, u.rc, v.g, u.rg, v.a, u.ra);
+    const float wl_dr = __shfl_up_sync(kAll, w_dr, P), wl_ad = __shfl_up_sync(kAll, w_ad, P);
+    if (k > 0) {  // the taps below row k - 1 close it
+      tap(v.lx, v.ly, v.lz, wl_ad);
+      tap(v.c.x, v.c.y, v.c.z, w_dn);
+      tap(v.rc.x, v.rc.y, v.rc.z, w_dr);
+      if (writes) {
+        const long long c = (long long)(y0 + step * (k - 1)) * A.W + x;
+        out[c] = finish_pixel<EXACT>(A, ax, ay, az, ws, src, c);
+      }
+    }
+    if (k == n_out) return;
+    const float w_rt = pair_weight<EXACT, GUIDES>(A, sws, v.rc, v.c, v.rg, v.g, v.ra, v.a);
+    const float wl_rt = __shfl_up_sync(kAll, w_rt, P);
+    ax = ay = az = ws = 0.0f;
+    tap(u.lx, u.ly, u.lz, wl_dr);
+    tap(u.c.x, u.c.y, u.c.z, w_dn);
+    tap(u.rc.x, u.rc.y, u.rc.z, w_ad);
+    tap(v.lx, v.ly, v.lz, wl_rt);
+    tap(v.c.x, v.c.y, v.c.z, 1.0f);
+    tap(v.rc.x, v.rc.y, v.rc.z, w_rt);
+  };
+  // launched while the pass before still runs (launch_pass): wait for its
+  // results, then let the next one come
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // three row buffers in turn, so that no row is moved between registers
+  Row r0, r1, r2;
+  load(r0, y0 - step);
+  load(r1, y0);
+  spread(r0);
+  for (int k = 0;; k += 3) {
+    step_row(k, r0, r1, r2);
+    if (k == n_out) break;
+    step_row(k + 1, r1, r2, r0);
+    if (k + 1 == n_out) break;
+    step_row(k + 2, r2, r0, r1);
+    if (k + 2 == n_out) break;
   }
 }
 
@@ -358,6 +445,22 @@ static size_t atrous_smem(const AtrousArgs& A) {
   return px * sizeof(float4) * (1 + ((A.use_n || A.use_d) ? 1 : 0) + (A.use_a ? 1 : 0));
 }
 
+// One radius-1 pass; from the second on it may start its blocks before the
+// pass it follows has ended, and waits for that inside.
+template <typename... Args>
+static cudaError_t launch_pass(cudaStream_t st, bool follows, unsigned blocks, void (*kern)(Args...), Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(kA1Warps * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = follows ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // Enqueues `passes` a-trous passes on `st`: pass i reads `in` (the colour for
 // i = 0) and writes scratch half (i & 1), the last pass writes `out` (and
 // reads `color` again for the blend).  A is filled except step / last.
@@ -372,24 +475,40 @@ static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, cons
     A.last = i == passes - 1;
     const bool exact = i == 0;
     float4* o = A.last ? out : ((i & 1) ? s1 : s0);
-    if (A.r == 1) {
-      const int P = A.step >= 2 ? 2 : 1, ow = kA1GW / P - 2;
+    if (A.r == 1 && (A.quot || !exact)) {
+      const int P = exact ? 1 : 2, ow = 32 / P - 2;
       const long long sub_w = (A.W + A.step - 1) / A.step, sub_h = (A.H + A.step - 1) / A.step;
-      const long long tiles_x = (sub_w + ow - 1) / ow, tiles_y = (sub_h + kA1H - 1) / kA1H;
-      const long long blocks = tiles_x * tiles_y * (A.step / P) * A.step;
-      if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-      auto kern = P == 1 ? (exact ? k_atrous_r1<true, 1> : k_atrous_r1<false, 1>)
-                         : (exact ? k_atrous_r1<true, 2> : k_atrous_r1<false, 2>);
-      kern<<<(unsigned)blocks, kAtThreads, 0, st>>>(A, (int)tiles_x, in, color, gn, ga, o);
+      const long long tiles_x = (sub_w + ow - 1) / ow, per_row = tiles_x * (A.step / P) * A.step;
+      const bool guides = A.use_n || A.use_a || A.use_d;
+      // Output rows of a strip.  A strip of r rows loads r + 2, and a strip
+      // more than the device holds at once waits for a whole one, so the
+      // cost is waves x (r + 2).  1280x720, later passes, us for all five:
+      // 3 rows 113, 4 104, 6 98, 8 111, 12 97, 16 107 by this rule's
+      // 20, 18, 16, 20, 14, 18; 640x360: 2 rows 43, 3 35, 4 41.
+      const long long cap = 148LL * kA1Warps * a1_blocks(exact, guides);
+      long long rows = 1, best = LLONG_MAX;
+      for (long long r = 1; r <= kA1MaxRows && r <= sub_h; ++r) {
+        const long long n = per_row * ((sub_h + r - 1) / r), cost = (n + cap - 1) / cap * (r + 2);
+        if (cost < best) best = cost, rows = r;
+      }
+      const long long tiles_y = (sub_h + rows - 1) / rows;
+      rows = (sub_h + tiles_y - 1) / tiles_y;  // the same in every strip of a column
+      const long long strips = per_row * tiles_y, blocks = (strips + kA1Warps - 1) / kA1Warps;
+      if (strips > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+      // pass 0 is the one with step 1
+      auto kern = exact ? (guides ? k_atrous_r1<true, 1, true> : k_atrous_r1<true, 1, false>)
+                        : (guides ? k_atrous_r1<false, 2, true> : k_atrous_r1<false, 2, false>);
+      cudaError_t e = launch_pass(st, i > 0, (unsigned)blocks, kern, A, (int)tiles_x, (int)rows, strips, in, color,
+                                  gn, ga, o);
+      if (e != cudaSuccess) return e;
     } else if (A.r <= kAtMaxTiledR) {
       const long long sub_w = (A.W + A.step - 1) / A.step, sub_h = (A.H + A.step - 1) / A.step;
       const long long tiles_x = (sub_w + kAtTW - 1) / kAtTW, tiles_y = (sub_h + kAtTH - 1) / kAtTH;
       const long long blocks = tiles_x * tiles_y * A.step * A.step;
       const size_t smem = atrous_smem(A);
       if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-      auto kern = A.r == 1   ? (exact ? k_atrous_tiled<true, 1> : k_atrous_tiled<false, 1>)
-                  : A.r == 2 ? (exact ? k_atrous_tiled<true, 2> : k_atrous_tiled<false, 2>)
-                             : (exact ? k_atrous_tiled<true, 0> : k_atrous_tiled<false, 0>);
+      auto kern = A.r == 2 ? (exact ? k_atrous_tiled<true, 2> : k_atrous_tiled<false, 2>)
+                           : (exact ? k_atrous_tiled<true, 0> : k_atrous_tiled<false, 0>);
       if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

@@ -119,6 +119,31 @@ def test_atrous_five_passes_against_numpy():
     np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("W,H", [(27, 9), (28, 33), (31, 2), (59, 65), (61, 130), (257, 47)])
+@pytest.mark.parametrize("guides,sc", [("nad", 0.08), ("", 0.08), ("n", 0.08), ("d", 0.08), ("ad", 0.08),
+                                       ("nad", 4e4)])
+def test_atrous_strip_edges(W, H, guides, sc):
+    """Radius-1 passes at sizes around a strip's 28 and 30 columns and its
+    rows, with each kind of guide set and a sigma beyond the quotients' range
+    (pass 0 by the tiled kernel), and one pixel whose colour distance is
+    infinite in float32 (weight 0).  An element's error is that of five
+    passes' float32 sums and exponents: exponents reach ~80 with a relative
+    error of a few 2^-24, so weights are good to ~2e-5."""
+    rng = np.random.default_rng(W * 1000 + H)
+    src = rng.random((H, W, 3)).astype(np.float32)
+    src[H // 2, W // 2] = 1e25
+    nrm = rng.normal(size=(H, W, 3)).astype(np.float32)
+    nrm /= np.linalg.norm(nrm, axis=2, keepdims=True)
+    alb = rng.random((H, W, 3)).astype(np.float32)
+    dep = (rng.random((H, W)) * 3 + 1).astype(np.float32)
+    pick = lambda k, v: v if k in guides else None
+    flat = lambda k, v: v if k in guides else np.zeros_like(v)
+    got = edge_aware_denoise(src, 1, sc, 0.8, normal=pick("n", nrm), albedo=pick("a", alb), depth=pick("d", dep),
+                             passes=5)
+    ref = _atrous_numpy(src, flat("n", nrm), flat("a", alb), flat("d", dep), 5, sc=sc)
+    np.testing.assert_allclose(got, ref, rtol=1e-4, atol=1e-5)
+
+
 def test_denoise_edge_sizes():
     for H, W in ((1, 1), (1, 7), (6, 1), (2, 2), (17, 3)):
         px = np.random.default_rng(H * 31 + W).random((H, W, 3), dtype=np.float32)
