@@ -1256,6 +1256,24 @@ __global__ void k_rot_weights(int Cout, int Cin, const bf16* __restrict__ w, bf1
   }
 }
 
+// The same with eight output channels per item: lanes read eight weights
+// each along ci and write one 16-byte chunk (Cout is a multiple of 16).  The
+// scalar form's 64-bit divisions and 2-byte stores took 39 us for the ten
+// layers of a training step, this 31 (a launch each).
+__global__ void k_rot_weights_v8(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
+  const unsigned n = (unsigned)(Cout / 8) * 9u * (unsigned)Cin;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned t = i / (unsigned)Cin, ci = i - t * (unsigned)Cin;
+    const unsigned co8 = t / 9u, tap = t - co8 * 9u;
+    const bf16* s = w + ((size_t)co8 * 72 + (8 - tap)) * Cin + ci;
+    uint4 v;
+    bf16* e = reinterpret_cast<bf16*>(&v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e[k] = s[(size_t)k * 9 * Cin];
+    *reinterpret_cast<uint4*>(wr + ((size_t)ci * 9 + tap) * Cout + co8 * 8) = v;
+  }
+}
+
 // ------------------------------------------------------------ element-wise
 // Every element-wise kernel walks (pixel, channel) of an NHWC view
 // (stride, offset) with a grid-stride loop.
@@ -1285,6 +1303,43 @@ __global__ void k_relu_mask(long long P, int C, const bf16* __restrict__ yv, int
   }
 }
 
+// The same on 8-channel chunks (views whose channel count, stride and offset
+// are multiples of 8): the gradient is read and written only where some
+// output is not positive.  Bound by memory; the ten masks of a 16x128x128
+// training step 203 -> 89 us.
+__global__ void k_relu_mask_v8(long long P, int C, const bf16* __restrict__ yv, int y_stride, int y_off,
+                               bf16* __restrict__ g, int g_stride, int g_off) {
+  const int CK = C >> 3;
+  const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+  RX_EW_LOOP(P * CK) {
+    long long p;
+    int ck;
+    if (i <= 0xffffffffLL) {
+      const unsigned q = (unsigned)i / (unsigned)CK;
+      p = q;
+      ck = (int)((unsigned)i - q * (unsigned)CK);
+    } else {
+      p = i / CK;
+      ck = (int)(i - p * CK);
+    }
+    const uint4 y = *reinterpret_cast<const uint4*>(yv + p * y_stride + y_off + ck * 8);
+    const unsigned* ye = reinterpret_cast<const unsigned*>(&y);
+    unsigned keep[4], all = 0xffffffffu;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      __nv_bfloat162 v;
+      *reinterpret_cast<unsigned*>(&v) = ye[k];
+      keep[k] = __hgt2_mask(v, zero);  // a NaN is not positive
+      all &= keep[k];
+    }
+    if (all == 0xffffffffu) continue;
+    uint4* d = reinterpret_cast<uint4*>(g + p * g_stride + g_off + ck * 8);
+    uint4 v = *d;
+    v.x &= keep[0], v.y &= keep[1], v.z &= keep[2], v.w &= keep[3];
+    *d = v;
+  }
+}
+
 // 2x2 average pool (H, W even): out (N, H/2, W/2, C)
 __global__ void k_pool2(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                         bf16* __restrict__ y, int y_stride, int y_off) {
@@ -1307,6 +1362,14 @@ __global__ void k_pool2(int N, int H, int W, int C, const bf16* __restrict__ x, 
 // of an input pixel (upsample: one load, four stores) or of an output pixel
 // (pool: four loads, one store); same float32 sum order as above.
 __device__ __forceinline__ void chunk_index(long long i, int CK, int W, int H, int& ck, int& x, int& y, long long& n) {
+  if (i <= 0xffffffffLL) {  // 32-bit divisions, a quarter of the instructions
+    const unsigned u = (unsigned)i, a = u / (unsigned)CK, b = a / (unsigned)W, c = b / (unsigned)H;
+    ck = (int)(u - a * (unsigned)CK);
+    x = (int)(a - b * (unsigned)W);
+    y = (int)(b - c * (unsigned)H);
+    n = c;
+    return;
+  }
   ck = (int)(i % CK);
   long long q = i / CK;
   x = (int)(q % W);
@@ -1374,6 +1437,71 @@ __global__ void k_pool2_bwd(int N, int H, int W, int C, const bf16* __restrict__
   }
 }
 
+// The two gradients on 8-channel chunks, one item per chunk of a pooled
+// (small) pixel: the pool's reads its gradient once for four input pixels,
+// the upsample's sums four; float32 sums in the order of the scalar forms.
+// Bound by memory; in a 16x128x128 training step the two pools' gradients
+// 86 -> 15 us, the two upsamples' 52 -> 16.
+__global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
+                               bf16* __restrict__ dx, int dx_stride, int dx_off, int accumulate) {
+  const int CK = C >> 3, h2 = H / 2, w2 = W / 2;
+  RX_EW_LOOP((long long)N * h2 * w2 * CK) {
+    int ck, xo, yo;
+    long long n;
+    chunk_index(i, CK, w2, h2, ck, xo, yo, n);
+    const uint4 q = *reinterpret_cast<const uint4*>(dy + ((n * h2 + yo) * w2 + xo) * dy_stride + dy_off + ck * 8);
+    const bf16* e = reinterpret_cast<const bf16*>(&q);
+    const long long b = (n * H + 2 * yo) * W + 2 * xo;
+    bf16* d = dx + dx_off + ck * 8;
+    uint4* o[4] = {reinterpret_cast<uint4*>(d + b * dx_stride), reinterpret_cast<uint4*>(d + (b + 1) * dx_stride),
+                   reinterpret_cast<uint4*>(d + (b + W) * dx_stride),
+                   reinterpret_cast<uint4*>(d + (b + W + 1) * dx_stride)};
+    uint4 old[4];
+    if (accumulate) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) old[j] = *o[j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint4 out;
+      bf16* r = reinterpret_cast<bf16*>(&out);
+      const bf16* oe = reinterpret_cast<const bf16*>(&old[j]);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float v = 0.25f * __bfloat162float(e[k]);
+        if (accumulate) v += __bfloat162float(oe[k]);
+        r[k] = __float2bfloat16_rn(v);
+      }
+      *o[j] = out;
+    }
+  }
+}
+
+__global__ void k_up2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
+                             bf16* __restrict__ dx, int dx_stride, int dx_off) {
+  const int CK = C >> 3;
+  RX_EW_LOOP((long long)N * H * W * CK) {
+    int ck, xx, yy;
+    long long n;
+    chunk_index(i, CK, W, H, ck, xx, yy, n);
+    const long long b = (n * 2 * H + 2 * yy) * 2LL * W + 2 * xx, w2 = 2LL * W;
+    const bf16* s = dy + dy_off + ck * 8;
+    const uint4 q[4] = {*reinterpret_cast<const uint4*>(s + b * dy_stride),
+                        *reinterpret_cast<const uint4*>(s + (b + 1) * dy_stride),
+                        *reinterpret_cast<const uint4*>(s + (b + w2) * dy_stride),
+                        *reinterpret_cast<const uint4*>(s + (b + w2 + 1) * dy_stride)};
+    const bf16* e[4] = {reinterpret_cast<const bf16*>(&q[0]), reinterpret_cast<const bf16*>(&q[1]),
+                        reinterpret_cast<const bf16*>(&q[2]), reinterpret_cast<const bf16*>(&q[3])};
+    uint4 out;
+    bf16* o = reinterpret_cast<bf16*>(&out);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      o[k] = __float2bfloat16_rn(__bfloat162float(e[0][k]) + __bfloat162float(e[1][k]) + __bfloat162float(e[2][k]) +
+                                 __bfloat162float(e[3][k]));
+    *reinterpret_cast<uint4*>(dx + ((n * H + yy) * W + xx) * dx_stride + dx_off + ck * 8) = out;
+  }
+}
+
 // nearest 2x upsample: out (N, 2H, 2W, C) from x (N, H, W, C)
 __global__ void k_up2(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                       bf16* __restrict__ y, int y_stride, int y_off) {
@@ -1407,43 +1535,99 @@ __global__ void k_up2_bwd(int N, int H, int W, int C, const bf16* __restrict__ d
 // Network input: 16 channels (log1p radiance, albedo, normal, depth/(1+depth),
 // six zeros) from float32 (P, 3) planes; base (optional) receives the
 // float32 log1p radiance the network's output is added to.
+__device__ __forceinline__ void feature_pixel(const float* rad, const float* alb, const float* nrm, float dep,
+                                              float* base, unsigned* o) {
+  float f[10];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    f[k] = log1pf(fmaxf(rad[k], 0.0f));
+    f[3 + k] = alb[k];
+    f[6 + k] = nrm[k];
+    base[k] = f[k];
+  }
+  const float dd = fmaxf(dep, 0.0f);
+  f[9] = dd / (1.0f + dd);
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+    o[k] = *reinterpret_cast<const unsigned*>(&v);
+  }
+  o[5] = o[6] = o[7] = 0;
+}
+
 __global__ void k_features(long long P, const float* __restrict__ rad, const float* __restrict__ alb,
                            const float* __restrict__ nrm, const float* __restrict__ dep, bf16* __restrict__ out,
                            float* __restrict__ base) {
   RX_EW_LOOP(P) {
-    float f[16];
+    unsigned o[8];
+    float l[3];
+    feature_pixel(rad + 3 * i, alb + 3 * i, nrm + 3 * i, dep[i], l, o);
+    if (base)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      f[k] = log1pf(fmaxf(rad[3 * i + k], 0.0f));
-      f[3 + k] = alb[3 * i + k];
-      f[6 + k] = nrm[3 * i + k];
-      if (base) base[3 * i + k] = f[k];
+      for (int k = 0; k < 3; ++k) base[3 * i + k] = l[k];
+    unsigned* d = reinterpret_cast<unsigned*>(out + 16 * i);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) d[k] = o[k];
+  }
+}
+
+// Four pixels per item (P a multiple of 4, 16-byte aligned planes): the
+// three-float pixels of a plane are three 16-byte loads, a pixel's features
+// two 16-byte stores.  1920x1080: 51 -> 37 us (174 MB).
+__global__ void k_features_v4(long long P4, const float4* __restrict__ rad, const float4* __restrict__ alb,
+                              const float4* __restrict__ nrm, const float4* __restrict__ dep, uint4* __restrict__ out,
+                              float4* __restrict__ base) {
+  RX_EW_LOOP(P4) {
+    float4 r[3], a[3], n[3], l[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] = rad[3 * i + k], a[k] = alb[3 * i + k], n[k] = nrm[3 * i + k];
+    const float4 d = dep[i];
+    const float dd[4] = {d.x, d.y, d.z, d.w};
+    const float *rf = reinterpret_cast<const float*>(r), *af = reinterpret_cast<const float*>(a),
+                *nf = reinterpret_cast<const float*>(n);
+    float* lf = reinterpret_cast<float*>(l);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      unsigned o[8];
+      feature_pixel(rf + 3 * p, af + 3 * p, nf + 3 * p, dd[p], lf + 3 * p, o);
+      out[8 * i + 2 * p] = make_uint4(o[0], o[1], o[2], o[3]);
+      out[8 * i + 2 * p + 1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
-    float dd = fmaxf(dep[i], 0.0f);
-    f[9] = dd / (1.0f + dd);
+    if (base)
 #pragma unroll
-    for (int k = 10; k < 16; ++k) f[k] = 0.0f;
-    __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(out + 16 * i);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = __floats2bfloat162_rn(f[2 * k], f[2 * k + 1]);
+      for (int k = 0; k < 3; ++k) base[3 * i + k] = l[k];
   }
 }
 
 // L1 loss in log1p space of y + base (base optional) against target t
 // (P, 3): sum |y + base - t| into *loss, gradient sign(.) * scale into g
 // (bf16, channel stride gs; pad channels 3..gs-1 zero)
+// CHUNKS: gs is a multiple of 8 and g 16-byte aligned, so the pixel's
+// channels are stored 16 bytes at a time (16x128x128, gs 16: 28 -> 18 us).
+template <bool CHUNKS>
 __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
                           const float* __restrict__ t, float scale, bf16* __restrict__ g, int gs,
                           float* __restrict__ loss) {
   float s = 0.0f;
   RX_EW_LOOP(P) {
+    alignas(4) bf16 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __float2bfloat16_rn(0.0f);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       float dlt = (y32[i * y_stride + k] + (base ? base[3 * i + k] : 0.0f)) - t[3 * i + k];
       s += fabsf(dlt);
-      g[i * gs + k] = __float2bfloat16_rn(dlt > 0.0f ? scale : (dlt < 0.0f ? -scale : 0.0f));
+      v[k] = __float2bfloat16_rn(dlt > 0.0f ? scale : (dlt < 0.0f ? -scale : 0.0f));
     }
-    for (int k = 3; k < gs; ++k) g[i * gs + k] = __float2bfloat16_rn(0.0f);
+    if (CHUNKS) {
+      uint4* d = reinterpret_cast<uint4*>(g + i * gs);
+      const unsigned* w = reinterpret_cast<const unsigned*>(v);
+      d[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      for (int k = 1; k < gs / 8; ++k) d[k] = make_uint4(0, 0, 0, 0);
+    } else {
+      for (int k = 0; k < 3; ++k) g[i * gs + k] = v[k];
+      for (int k = 3; k < gs; ++k) g[i * gs + k] = v[7];
+    }
   }
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
@@ -1714,8 +1898,13 @@ int conv_bwd_data(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* w
                   cudaStream_t st) {
   if (!conv_ok(d) || !dy || !w || !w_rot || !dx) return set_error(ctx, "conv_bf16_bwd_data: bad arguments"), RX_ERR_ARG;
   long long nw = (long long)d->Cout * 9 * d->Cin;
-  k_rot_weights<<<ew_blocks(ctx, nw), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
-                                                   static_cast<bf16*>(w_rot));
+  // whole 16-byte chunks where the buffer allows them and 32 bits count them
+  if (((uintptr_t)w_rot & 15) == 0 && nw / 8 <= 0x7fffffffLL)
+    k_rot_weights_v8<<<ew_blocks(ctx, nw / 8), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
+                                                            static_cast<bf16*>(w_rot));
+  else
+    k_rot_weights<<<ew_blocks(ctx, nw), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
+                                                     static_cast<bf16*>(w_rot));
   CUDA_TRY(ctx, cudaGetLastError());
   // dx = conv(dy, w_rot): input channels Cout (read from the y view), output Cin (the x view)
   rx_conv_desc t = *d;
@@ -1849,8 +2038,12 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
                                                          o->flag);
       break;
     case RX_DN_RELU_MASK:
-      k_relu_mask<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(P, o->C, a, o->a_stride, o->a_off, b, o->b_stride,
-                                                           o->b_off);
+      if (v8)
+        k_relu_mask_v8<<<ew_blocks(ctx, P * (o->C / 8)), 256, 0, st>>>(P, o->C, a, o->a_stride, o->a_off, b,
+                                                                      o->b_stride, o->b_off);
+      else
+        k_relu_mask<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(P, o->C, a, o->a_stride, o->a_off, b, o->b_stride,
+                                                             o->b_off);
       break;
     case RX_DN_POOL:
       if (o->H % 2 || o->W % 2) return set_error(ctx, "dn_op: pool needs even H and W"), RX_ERR_ARG;
@@ -1863,8 +2056,12 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
       break;
     case RX_DN_POOL_BWD:
       if (o->H % 2 || o->W % 2) return set_error(ctx, "dn_op: pool needs even H and W"), RX_ERR_ARG;
-      k_pool2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
-                                                           o->b_stride, o->b_off, o->flag);
+      if (v8)
+        k_pool2_bwd_v8<<<ew_blocks(ctx, P / 4 * (o->C / 8)), 256, 0, st>>>(
+            o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b, o->b_stride, o->b_off, o->flag);
+      else
+        k_pool2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
+                                                             o->b_stride, o->b_off, o->flag);
       break;
     case RX_DN_UP:
       if (v8)
@@ -1875,8 +2072,12 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
                                                            o->b_stride, o->b_off);
       break;
     case RX_DN_UP_BWD:
-      k_up2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
-                                                         o->b_stride, o->b_off);
+      if (v8)
+        k_up2_bwd_v8<<<ew_blocks(ctx, P * (o->C / 8)), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off,
+                                                                    b, o->b_stride, o->b_off);
+      else
+        k_up2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
+                                                           o->b_stride, o->b_off);
       break;
     default:
       return set_error(ctx, "dn_op: unknown kind %d", o->kind), RX_ERR_ARG;
@@ -1888,7 +2089,15 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
 int dn_features(Ctx* ctx, long long P, const float* rad, const float* alb, const float* nrm, const float* dep,
                 void* out, float* base, cudaStream_t st) {
   if (P <= 0 || !rad || !alb || !nrm || !dep || !out) return set_error(ctx, "dn_features: bad arguments"), RX_ERR_ARG;
-  k_features<<<ew_blocks(ctx, P), 256, 0, st>>>(P, rad, alb, nrm, dep, static_cast<bf16*>(out), base);
+  const uintptr_t all = (uintptr_t)rad | (uintptr_t)alb | (uintptr_t)nrm | (uintptr_t)dep | (uintptr_t)out |
+                        (uintptr_t)base;
+  if (P % 4 == 0 && all % 16 == 0) {
+    auto f4 = [](const float* p) { return reinterpret_cast<const float4*>(p); };
+    k_features_v4<<<ew_blocks(ctx, P / 4), 256, 0, st>>>(P / 4, f4(rad), f4(alb), f4(nrm), f4(dep),
+                                                         static_cast<uint4*>(out), reinterpret_cast<float4*>(base));
+  } else {
+    k_features<<<ew_blocks(ctx, P), 256, 0, st>>>(P, rad, alb, nrm, dep, static_cast<bf16*>(out), base);
+  }
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }
@@ -1897,8 +2106,9 @@ int dn_l1_loss(Ctx* ctx, long long P, const float* y32, int y_stride, const floa
                float scale, void* grad, int grad_stride, float* loss, cudaStream_t st) {
   if (P <= 0 || !y32 || !target || !grad || !loss || y_stride < 3 || grad_stride < 3)
     return set_error(ctx, "dn_l1_loss: bad arguments"), RX_ERR_ARG;
-  k_l1_loss<<<ew_blocks(ctx, P), 256, 0, st>>>(P, y32, y_stride, base, target, scale, static_cast<bf16*>(grad),
-                                               grad_stride, loss);
+  auto kern = grad_stride % 8 == 0 && (uintptr_t)grad % 16 == 0 ? k_l1_loss<true> : k_l1_loss<false>;
+  kern<<<ew_blocks(ctx, P), 256, 0, st>>>(P, y32, y_stride, base, target, scale, static_cast<bf16*>(grad), grad_stride,
+                                          loss);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }

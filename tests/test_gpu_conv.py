@@ -188,6 +188,66 @@ def _torch_net(net, x16, base, target):
     return float(loss.detach()), {k: (v[0].grad, v[1].grad) for k, v in params.items()}
 
 
+@pytest.mark.parametrize("N,H,W,C,stride,off", [(1, 2, 2, 8, 8, 0), (2, 6, 10, 24, 48, 16), (3, 2, 34, 32, 40, 8),
+                                                (1, 66, 130, 128, 192, 64)])
+def test_chunked_layer_gradients_equal_the_element_kernels(N, H, W, C, stride, off):
+    """ReLU mask, pool and upsample gradients on 8-channel chunks give the
+    bits of the element kernels (reached by a stride that is no multiple of
+    8) and leave the other channels alone."""
+    ctx, L = _ctx(), nat.lib()
+    g = torch.Generator(device="cuda").manual_seed(N * 100 + C)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g).to(torch.bfloat16)  # noqa: E731
+    y, big, small = rnd(N, H, W, C), rnd(N, H, W, C), rnd(N, H // 2, W // 2, C)
+    y.view(-1)[::7] = 0.0
+    y.view(-1)[3::11] = float("nan")
+
+    def run(kind, n, h, w, a, b, flag, st, of):
+        wide = lambda t: F.pad(t, (of, st - of - C), value=3.0).contiguous()  # noqa: E731
+        aw, bw = wide(a), wide(b)
+        ctx.check(L.rx_dn_layer(ctx.h, ctypes.byref(nat.DnOp(kind, n, h, w, C, _p(aw), st, of, _p(bw), st, of, flag)),
+                                _stream()))
+        torch.cuda.synchronize()
+        assert bool((bw[..., :of] == 3.0).all()) and bool((bw[..., of + C:] == 3.0).all())
+        return bw[..., of:of + C].contiguous().view(torch.int16)
+
+    for kind, n, h, w, a, b, flag in ((nat.RX_DN_RELU_MASK, N, H, W, y, big, 0),
+                                      (nat.RX_DN_POOL_BWD, N, H, W, small, big, 0),
+                                      (nat.RX_DN_POOL_BWD, N, H, W, small, big, 1),
+                                      (nat.RX_DN_UP_BWD, N, H // 2, W // 2, big, small, 0)):
+        assert torch.equal(run(kind, n, h, w, a, b, flag, stride, off),
+                           run(kind, n, h, w, a, b, flag, stride + 4, off + 2)), kind
+
+
+@pytest.mark.parametrize("P", [1, 4, 6, 1028])
+def test_features_and_loss_chunks_equal_the_element_kernels(P):
+    """Four pixels per item (P a multiple of 4, aligned planes) against the
+    same pixels one by one (planes shifted by one pixel), and the loss
+    gradient in 16-byte stores against stride 12."""
+    ctx, L = _ctx(), nat.lib()
+    g = torch.Generator(device="cuda").manual_seed(P)
+    planes = [torch.rand((P + 1, k), device="cuda", generator=g) * 4 - 1 for k in (3, 3, 3, 1)]
+
+    def feats(ts):
+        out, base = (torch.empty((P, k), dtype=d, device="cuda") for k, d in ((16, torch.bfloat16), (3, torch.float32)))
+        ctx.check(L.rx_dn_features(ctx.h, P, *[_p(t) for t in ts], _p(out), _p(base), _stream()))
+        torch.cuda.synchronize()
+        return out.view(torch.int16), base
+
+    a, b = feats([t[1:].contiguous() for t in planes]), feats([t[1:] for t in planes])
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
+    y32, t = torch.randn((P, 16), device="cuda", generator=g), torch.rand((P, 3), device="cuda", generator=g)
+    grads = []
+    for gs in (16, 12):
+        gr = torch.full((P, gs), 5.0, dtype=torch.bfloat16, device="cuda")
+        loss = torch.zeros(1, device="cuda")
+        ctx.check(L.rx_dn_l1_loss(ctx.h, P, _p(y32), 16, _p(a[1]), _p(t), ctypes.c_float(0.5), _p(gr), gs, _p(loss),
+                                  _stream()))
+        torch.cuda.synchronize()
+        assert not gr[:, 3:].any()
+        grads.append(gr[:, :3].clone())
+    assert torch.equal(*grads)
+
+
 def test_tcgen05_and_mma_sync_convolutions_agree():
     """The forward kernels on the same operands (persistent and streaming
     tcgen05, then mma.sync): same values up to the order of their float32
