@@ -14,10 +14,11 @@
 //    construction of BVHs, octrees, and k-d trees", HPG 2012) over the same
 //    codes, a bottom-up pass computing bounds and SAH costs, and an SAH
 //    collapse of subtrees into leaves of up to `max_leaf` primitives, laid
-//    out breadth-first so the top levels are contiguous.
+//    out in Morton order (the root first), and a 4-wide copy.
 //
 // Both emit the traversal layout described in rx_internal.cuh.
 #include <algorithm>
+#include <climits>
 #include <cstdio>
 #include <vector>
 
@@ -173,103 +174,125 @@ __global__ void k_morton(int n, const float3* __restrict__ cen, const float3* __
 
 // ----------------------------------------------------------------------------
 // stable LSD radix sort, 8-bit digits, (key, value) pairs
-// tile = 8 warps x 16 chunks x 32 keys = 4096 keys per block
+// tile = 8 warps x CHUNKS x 32 keys per block: 1,024 keys (CHUNKS 4) up to
+// 2^20 keys, which fills the device at 150 k keys, else 4,096 with a quarter
+// of the histogram.  Four passes over 327 k keys 200 -> 82 us: scatter 22 ->
+// 11 us with smaller tiles and all loads ahead of the ranking, the counters'
+// scan 21 -> 4 with a block per digit.
 // ----------------------------------------------------------------------------
 constexpr int kSortWarps = 8;
-constexpr int kSortChunks = 16;
-constexpr int kSortTile = kSortWarps * kSortChunks * 32;
+__host__ __device__ constexpr int sort_tile(int chunks) { return kSortWarps * chunks * 32; }
 
-__global__ void k_sort_hist(int n, const uint32_t* __restrict__ keys, int shift, uint32_t* __restrict__ hist,
+__global__ void k_sort_hist(int n, const uint32_t* __restrict__ keys, int shift, int tile, uint32_t* __restrict__ hist,
                             int nblocks) {
   __shared__ uint32_t h[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
   __syncthreads();
-  int base = blockIdx.x * kSortTile;
-  int end = min(base + kSortTile, n);
+  int base = blockIdx.x * tile;
+  int end = min(base + tile, n);
   for (int i = base + threadIdx.x; i < end; i += blockDim.x) atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
   __syncthreads();
   for (int d = threadIdx.x; d < 256; d += blockDim.x) hist[d * nblocks + blockIdx.x] = h[d];
 }
 
-// exclusive scan of hist[256 * nblocks] (digit-major), one block of 1024
-__global__ void k_sort_scan(uint32_t* __restrict__ hist, int total) {
-  __shared__ uint32_t warp_sums[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int base = 0; base < total; base += blockDim.x) {
-    int i = base + threadIdx.x;
-    uint32_t v = i < total ? hist[i] : 0u;
-    uint32_t x = v;
+// Exclusive sums of 256 values, one per thread of a 256-thread block;
+// *total: their sum.  Ends with a barrier.
+__device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t x = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sums[wid] = x;
-    __syncthreads();
-    if (wid == 0) {
-      uint32_t w = warp_sums[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      warp_sums[lane] = w;
-    }
-    __syncthreads();
-    uint32_t prefix = (wid > 0 ? warp_sums[wid - 1] : 0u) + carry;
-    if (i < total) hist[i] = prefix + x - v;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = prefix + x;
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
+  if (lane == 31) warp_sums[wid] = x;
+  __syncthreads();
+  uint32_t before = 0, all = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const uint32_t y = warp_sums[w];
+    if (w < wid) before += y;
+    all += y;
+  }
+  *total = all;
+  __syncthreads();
+  return before + x - v;
 }
 
+// Exclusive sums along each digit's row of hist[256][nblocks] and the rows'
+// totals, one block per digit.  (One block over all 256 x nblocks counters
+// took 21 us per pass at 80 blocks; a row each takes 3.)
+__global__ void __launch_bounds__(256) k_sort_rows(uint32_t* __restrict__ hist, uint32_t* __restrict__ totals,
+                                                   int nblocks) {
+  __shared__ uint32_t warp_sums[8];
+  uint32_t* row = hist + (size_t)blockIdx.x * nblocks;
+  uint32_t carry = 0;
+  for (int base = 0; base < nblocks; base += 256) {
+    const int i = base + threadIdx.x;
+    const uint32_t v = i < nblocks ? row[i] : 0u;
+    uint32_t total;
+    const uint32_t e = block_exclusive_256(v, warp_sums, &total);
+    if (i < nblocks) row[i] = carry + e;
+    carry += total;
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
+template <int CHUNKS>
 __global__ void __launch_bounds__(kSortWarps * 32)
     k_sort_scatter(int n, const uint32_t* __restrict__ keys_in, const int* __restrict__ vals_in,
                    uint32_t* __restrict__ keys_out, int* __restrict__ vals_out, int shift,
-                   const uint32_t* __restrict__ hist, int nblocks) {
+                   const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, int nblocks) {
+  static_assert(kSortWarps * 32 == 256, "one thread per digit");
   __shared__ uint32_t wcount[kSortWarps][256];
+  __shared__ uint32_t warp_sums[8];
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int wbase = blockIdx.x * sort_tile(CHUNKS) + w * CHUNKS * 32 + lane;
+  // every load in flight before the first use
+  uint32_t key[CHUNKS];
+  int val[CHUNKS];
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    const int i = wbase + c * 32;
+    key[c] = i < n ? keys_in[i] : 0u;
+    val[c] = i < n ? vals_in[i] : 0;
+  }
+  const uint32_t row = hist[threadIdx.x * nblocks + blockIdx.x];
   for (int i = threadIdx.x; i < kSortWarps * 256; i += blockDim.x) (&wcount[0][0])[i] = 0;
-  __syncthreads();
-  int wbase = blockIdx.x * kSortTile + w * kSortChunks * 32;
+  uint32_t all;
+  const uint32_t start = block_exclusive_256(totals[threadIdx.x], warp_sums, &all) + row;
   // pass 1: per-warp digit counts
-  for (int c = 0; c < kSortChunks; ++c) {
-    int i = wbase + c * 32 + lane;
-    bool ok = i < n;
-    uint32_t dgt = ok ? (keys_in[i] >> shift) & 255u : 256u;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    bool ok = wbase + c * 32 < n;
+    uint32_t dgt = ok ? (key[c] >> shift) & 255u : 256u;
     unsigned peers = __match_any_sync(0xffffffffu, dgt);
     int leader = __ffs(peers) - 1;
     if (ok && lane == leader) wcount[w][dgt] += __popc(peers);
     __syncwarp();
   }
   __syncthreads();
-  // per-warp starting offsets (block offset from the scanned histogram)
-  for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-    uint32_t run = hist[d * nblocks + blockIdx.x];
-    for (int ww = 0; ww < kSortWarps; ++ww) {
-      uint32_t c = wcount[ww][d];
-      wcount[ww][d] = run;
-      run += c;
-    }
+  // per-warp starting offsets: the digit's start, the earlier blocks', the
+  // earlier warps'
+  uint32_t run = start;
+  for (int ww = 0; ww < kSortWarps; ++ww) {
+    uint32_t c = wcount[ww][threadIdx.x];
+    wcount[ww][threadIdx.x] = run;
+    run += c;
   }
   __syncthreads();
   // pass 2: stable scatter in key order
   unsigned lt = (1u << lane) - 1u;
-  for (int c = 0; c < kSortChunks; ++c) {
-    int i = wbase + c * 32 + lane;
-    bool ok = i < n;
-    uint32_t key = ok ? keys_in[i] : 0u;
-    uint32_t dgt = ok ? (key >> shift) & 255u : 256u;
+#pragma unroll
+  for (int c = 0; c < CHUNKS; ++c) {
+    bool ok = wbase + c * 32 < n;
+    uint32_t dgt = ok ? (key[c] >> shift) & 255u : 256u;
     unsigned peers = __match_any_sync(0xffffffffu, dgt);
     int leader = __ffs(peers) - 1;
     if (ok) {
       uint32_t pos = wcount[w][dgt] + __popc(peers & lt);
-      keys_out[pos] = key;
-      vals_out[pos] = vals_in[i];
+      keys_out[pos] = key[c];
+      vals_out[pos] = val[c];
     }
     __syncwarp();
     if (ok && lane == leader) wcount[w][dgt] += __popc(peers);
@@ -281,10 +304,11 @@ __global__ void __launch_bounds__(kSortWarps * 32)
 static int radix_sort(Ctx* ctx, int n, uint32_t* keys, int* vals, int bits) {
   if (n <= 1) return RX_OK;
   cudaStream_t st = ctx->stream;
-  int nblocks = (n + kSortTile - 1) / kSortTile;
-  DevBuf<uint32_t> k2(ctx, n), hist(ctx, (size_t)256 * nblocks);
+  const int chunks = n <= (1 << 20) ? 4 : 16, tile = sort_tile(chunks);
+  int nblocks = (n + tile - 1) / tile;
+  DevBuf<uint32_t> k2(ctx, n), hist(ctx, (size_t)256 * nblocks), totals(ctx, 256);
   DevBuf<int> v2(ctx, n);
-  if (!all_ok(k2, hist, v2)) return set_error(ctx, "BVH sort: out of device memory"), RX_ERR_CAPACITY;
+  if (!all_ok(k2, hist, totals, v2)) return set_error(ctx, "BVH sort: out of device memory"), RX_ERR_CAPACITY;
   uint32_t* ka = keys;
   uint32_t* kb = k2.p;
   int* va = vals;
@@ -292,9 +316,10 @@ static int radix_sort(Ctx* ctx, int n, uint32_t* keys, int* vals, int bits) {
   int passes = (bits + 7) / 8;
   for (int p = 0; p < passes; ++p) {
     int shift = 8 * p;
-    k_sort_hist<<<nblocks, 256, 0, st>>>(n, ka, shift, hist.p, nblocks);
-    k_sort_scan<<<1, 1024, 0, st>>>(hist.p, 256 * nblocks);
-    k_sort_scatter<<<nblocks, kSortWarps * 32, 0, st>>>(n, ka, va, kb, vb, shift, hist.p, nblocks);
+    k_sort_hist<<<nblocks, 256, 0, st>>>(n, ka, shift, tile, hist.p, nblocks);
+    k_sort_rows<<<256, 256, 0, st>>>(hist.p, totals.p, nblocks);
+    auto scatter = chunks == 4 ? k_sort_scatter<4> : k_sort_scatter<16>;
+    scatter<<<nblocks, kSortWarps * 32, 0, st>>>(n, ka, va, kb, vb, shift, hist.p, totals.p, nblocks);
     std::swap(ka, kb);
     std::swap(va, vb);
   }
@@ -302,7 +327,7 @@ static int radix_sort(Ctx* ctx, int n, uint32_t* keys, int* vals, int bits) {
     cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(vals, va, sizeof(int) * n, cudaMemcpyDeviceToDevice, st);
   }
-  // k2, v2, hist are released after the stream drains (DevBuf defers frees)
+  // k2, v2, hist, totals are released after the stream drains (DevBuf defers frees)
   return RX_OK;
 }
 
@@ -475,11 +500,14 @@ __device__ __forceinline__ int lcp(const uint32_t* codes, int n, int i, int j) {
   return __clz(a ^ b);
 }
 
-// Internal node i of n - 1.  Children are encoded as c >= 0 internal, c < 0
-// leaf ~prim (sorted position).
-__global__ void k_karras(int n, const uint32_t* __restrict__ codes, int* __restrict__ kl, int* __restrict__ kr,
-                         int* __restrict__ first, int* __restrict__ last, int* __restrict__ parent_int,
-                         int* __restrict__ parent_leaf) {
+// Children are encoded as c >= 0 internal, c < 0 leaf ~prim (sorted position).
+__device__ __forceinline__ int left_child(int lo, int gamma) { return lo == gamma ? ~gamma : gamma; }
+__device__ __forceinline__ int right_child(int hi, int gamma) { return hi == gamma + 1 ? ~(gamma + 1) : gamma + 1; }
+
+// Internal node i of n - 1 covers the sorted positions [lo, hi], split after
+// gamma: record (lo, hi, gamma, -).
+__global__ void k_karras(int n, const uint32_t* __restrict__ codes, int4* __restrict__ range,
+                         int* __restrict__ parent_int, int* __restrict__ parent_leaf) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
     int d = (lcp(codes, n, i, i + 1) - lcp(codes, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = lcp(codes, n, i, i - d);
@@ -498,12 +526,8 @@ __global__ void k_karras(int n, const uint32_t* __restrict__ codes, int* __restr
     } while (t > 1);
     int gamma = i + s * d + min(d, 0);
     int lo = min(i, j), hi = max(i, j);
-    int lc = (lo == gamma) ? ~gamma : gamma;
-    int rc = (hi == gamma + 1) ? ~(gamma + 1) : gamma + 1;
-    kl[i] = lc;
-    kr[i] = rc;
-    first[i] = lo;
-    last[i] = hi;
+    range[i] = make_int4(lo, hi, gamma, 0);
+    const int lc = left_child(lo, gamma), rc = right_child(hi, gamma);
     if (lc >= 0) parent_int[lc] = i; else parent_leaf[~lc] = i;
     if (rc >= 0) parent_int[rc] = i; else parent_leaf[~rc] = i;
   }
@@ -515,246 +539,374 @@ __device__ __forceinline__ float half_area(float3 lo, float3 hi) {
 }
 
 // Bottom-up bounds and SAH cost.  cost(node) = min(C_i * count (if count <=
-// max_leaf), C_t + (A_l cost_l + A_r cost_r) / A); collapse[] records which
-// choice won.
-__global__ void k_lbvh_bottom_up(int n, const int* __restrict__ order, const int* __restrict__ kl,
-                                 const int* __restrict__ kr, const int* __restrict__ parent_int,
-                                 const int* __restrict__ parent_leaf, const float3* __restrict__ pmin,
-                                 const float3* __restrict__ pmax, float3* __restrict__ imin,
-                                 float3* __restrict__ imax, float* __restrict__ icost, int* __restrict__ icount,
-                                 int* __restrict__ collapse, int* __restrict__ flags, int max_leaf, float c_t,
-                                 float c_i) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    int node = parent_leaf[k];
-    while (node >= 0) {
-      __threadfence();
-      if (atomicAdd(&flags[node], 1) == 0) break;
-      __threadfence();
-      int l = kl[node], r = kr[node];
-      float3 l0, l1, r0, r1;
-      float lcost, rcost;
-      int lcnt, rcnt;
-      if (l < 0) {
-        int p = order[~l];
-        l0 = pmin[p]; l1 = pmax[p]; lcost = c_i; lcnt = 1;
-      } else {
-        l0 = ldcg3(imin + l); l1 = ldcg3(imax + l);
-        lcost = __ldcg(icost + l); lcnt = __ldcg(icount + l);
-      }
-      if (r < 0) {
-        int p = order[~r];
-        r0 = pmin[p]; r1 = pmax[p]; rcost = c_i; rcnt = 1;
-      } else {
-        r0 = ldcg3(imin + r); r1 = ldcg3(imax + r);
-        rcost = __ldcg(icost + r); rcnt = __ldcg(icount + r);
-      }
-      float3 lo = vmin(l0, r0), hi = vmax(l1, r1);
-      float a = fmaxf(half_area(lo, hi), 1e-30f);
-      float split = c_t + (half_area(l0, l1) * lcost + half_area(r0, r1) * rcost) / a;
-      int cnt = lcnt + rcnt;
-      float leafc = c_i * (float)cnt;
-      int col = (cnt <= max_leaf && leafc <= split) ? 1 : 0;
-      imin[node] = lo;
-      imax[node] = hi;
-      icost[node] = col ? leafc : split;
-      icount[node] = cnt;
-      collapse[node] = col;
-      node = parent_int[node];
-    }
-  }
+// max_leaf), C_t + (A_l cost_l + A_r cost_r) / A).  Node record: a = (min,
+// cost), b = (max, height bits), height = levels of the tree under the node,
+// 0 where it collapses into a leaf.
+//
+// The second thread to reach a node computes it.  A block owns kUpLeaves
+// consecutive sorted positions: a node that covers none outside them (9 of
+// ~20 levels, all but some thousand nodes of a 327 k mesh) is counted and
+// its record handed on in shared memory, the rest by device-scope fences and
+// atomics; that chain of ~2 us per level was the pass's time.
+constexpr int kUpLeaves = 512;
+
+struct UpBox {
+  float3 lo, hi;
+  float cost;
+  int height;
+};
+
+__device__ __forceinline__ UpBox up_box(float4 a, float4 b) {
+  return {f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), a.w, __float_as_int(b.w)};
 }
 
-// Breadth-first level walks run without a host round trip per level: the
-// walk's state lives on the device -- lv[0] nodes of the level being laid
-// out, lv[1] output index of its first node, lv[2] nodes queued for the next
-// level, lv[3] blocks of the current launch that have finished, lv[4] levels
-// laid out, lv[5] set when a level would overflow the tree -- and the last
-// block of each level launch advances it for the
-// next launch.  Every block reads lv[0] and lv[1] before it counts itself
-// finished, so the advance never races with a reader.  A launch that finds
-// lv[0] == 0 (the walk is over) returns at once; the host enqueues levels in
-// batches and reads lv back once per batch.
-enum { LV_NCUR = 0, LV_BASE = 1, LV_NEXT = 2, LV_DONE = 3, LV_LEVELS = 4, LV_OVERFLOW = 5, LV_N = 8 };
-
-__device__ __forceinline__ void level_advance(int* lv) {
+__global__ void __launch_bounds__(kUpLeaves)
+    k_lbvh_bottom_up(int n, const int* __restrict__ order, const int4* __restrict__ range,
+                     const int* __restrict__ parent_int, const int* __restrict__ parent_leaf,
+                     const float3* __restrict__ pmin, const float3* __restrict__ pmax, float4* __restrict__ rec,
+                     int* __restrict__ flags, int max_leaf, float c_t, float c_i) {
+  __shared__ float4 s_a[kUpLeaves], s_b[kUpLeaves];  // records of this block's nodes, by node - base
+  __shared__ float3 s_lo[kUpLeaves], s_hi[kUpLeaves];
+  __shared__ int4 s_range[kUpLeaves];  // (lo, hi, gamma, parent)
+  __shared__ int s_flag[kUpLeaves];
+  const int base = blockIdx.x * kUpLeaves, end = min(base + kUpLeaves, n), k = base + threadIdx.x;
+  int node = -1;
+  s_flag[threadIdx.x] = 0;
+  if (k < end) {
+    const int p = order[k];
+    node = parent_leaf[k];
+    s_lo[threadIdx.x] = pmin[p];
+    s_hi[threadIdx.x] = pmax[p];
+    if (k < n - 1) {
+      int4 q = range[k];
+      q.w = parent_int[k];
+      s_range[threadIdx.x] = q;
+    }
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (k >= end) return;
+  // a node's index lies inside its range, so one that is not here is no
+  // block's own
+  auto node_range = [&](int i) {
+    if (i >= base && i < end) return s_range[i - base];
+    int4 q = range[i];
+    q.w = parent_int[i];
+    return q;
+  };
+  auto compute = [&](const int4 q, const UpBox& l, const UpBox& r, float4& a, float4& b) {
+    const float3 lo = vmin(l.lo, r.lo), hi = vmax(l.hi, r.hi);
+    const float area = fmaxf(half_area(lo, hi), 1e-30f);
+    const float split = c_t + (half_area(l.lo, l.hi) * l.cost + half_area(r.lo, r.hi) * r.cost) / area;
+    const int cnt = q.y - q.x + 1;
+    const float leafc = c_i * (float)cnt;
+    const bool col = cnt <= max_leaf && leafc <= split;
+    a = make_float4(lo.x, lo.y, lo.z, col ? leafc : split);
+    b = make_float4(hi.x, hi.y, hi.z, __int_as_float(col ? 0 : 1 + max(l.height, r.height)));
+  };
+  int4 q = node_range(node);
+  while (q.x >= base && q.y < end) {
+    __threadfence_block();
+    if (atomicAdd(&s_flag[node - base], 1) == 0) return;
+    __threadfence_block();
+    auto child = [&](int c) {
+      if (c < 0) return UpBox{s_lo[~c - base], s_hi[~c - base], c_i, 0};
+      return up_box(s_a[c - base], s_b[c - base]);
+    };
+    float4 a, b;
+    compute(q, child(left_child(q.x, q.z)), child(right_child(q.y, q.z)), a, b);
+    s_a[node - base] = a;
+    s_b[node - base] = b;
+    rec[2 * (size_t)node] = a;
+    rec[2 * (size_t)node + 1] = b;
+    if (q.w < 0) return;
+    node = q.w;
+    q = node_range(node);
+  }
+  while (true) {
     __threadfence();
-    if (atomicAdd(&lv[LV_DONE], 1) == (int)gridDim.x - 1) {
-      const int ncur = lv[LV_NCUR];
-      lv[LV_BASE] += ncur;
-      lv[LV_NCUR] = atomicAdd(&lv[LV_NEXT], 0);
-      lv[LV_NEXT] = 0;
-      lv[LV_DONE] = 0;
-      lv[LV_LEVELS] += 1;
-      __threadfence();
-    }
+    if (atomicAdd(&flags[node], 1) == 0) return;
+    const int4 up = q.w < 0 ? q : node_range(q.w);  // in flight with the children's records
+    __threadfence();
+    auto child = [&](int c) {
+      if (c >= 0) return up_box(__ldcg(rec + 2 * (size_t)c), __ldcg(rec + 2 * (size_t)c + 1));
+      const int p = order[~c];
+      return UpBox{pmin[p], pmax[p], c_i, 0};
+    };
+    float4 a, b;
+    compute(q, child(left_child(q.x, q.z)), child(right_child(q.y, q.z)), a, b);
+    rec[2 * (size_t)node] = a;
+    rec[2 * (size_t)node + 1] = b;
+    if (q.w < 0) return;
+    node = q.w;
+    q = up;
   }
 }
 
-// One breadth-first level of the collapsed tree.  `cur` holds Karras node
-// ids; their output indices are base + position.  Kept internal children
-// are appended to `next` and receive indices in the following level.
-__global__ void k_lbvh_layout_level(const int* __restrict__ cur, int* __restrict__ next, int* __restrict__ lv,
-                                    int n_total, const int* __restrict__ kl,
-                                    const int* __restrict__ kr, const int* __restrict__ first,
-                                    const int* __restrict__ last, const int* __restrict__ collapse,
-                                    const int* __restrict__ order, const float3* __restrict__ pmin,
-                                    const float3* __restrict__ pmax, const float3* __restrict__ imin,
-                                    const float3* __restrict__ imax, float4* __restrict__ out) {
-  const int ncur = lv[LV_NCUR], out_base = lv[LV_BASE];
-  if (ncur <= 0) return;
-  if (out_base + ncur > n_total) {  // cannot happen for a tree of n_total nodes
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      lv[LV_OVERFLOW] = 1;
-      lv[LV_NCUR] = 0;
-    }
-    return;
+// Compaction of marked nodes: a bit mask, the marked nodes per kRankWords
+// mask words (added up while marking), and the rank of every mask word.
+constexpr int kRankWords = 256;
+
+struct NodeMask {
+  uint32_t* mask;  // a multiple of kRankWords words
+  int* rank;       // marked nodes before each word
+  int* counts;     // marked nodes per kRankWords words; zero before marking
+  __device__ __forceinline__ int index(int i) const {
+    return rank[i >> 5] + __popc(mask[i >> 5] & ((1u << (i & 31)) - 1u));
   }
-  const int next_base = out_base + ncur, next_cap = n_total - next_base;
-  int* next_count = &lv[LV_NEXT];
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ncur; q += gridDim.x * blockDim.x) {
-    int node = cur[q];
+  __device__ __forceinline__ bool has(int i) const { return mask[i >> 5] >> (i & 31) & 1u; }
+  // one word per warp, called by whole warps
+  __device__ __forceinline__ void mark(int i, bool keep) const {
+    const unsigned m = __ballot_sync(0xffffffffu, keep);
+    if ((i & 31) == 0) {
+      mask[i >> 5] = m;
+      if (m) atomicAdd(counts + (i >> 5) / kRankWords, __popc(m));
+    }
+  }
+};
+
+// One block per kRankWords words; the last one writes *total.
+__global__ void __launch_bounds__(kRankWords) k_rank(NodeMask m, int* __restrict__ total) {
+  __shared__ uint32_t warp_sums[8];
+  uint32_t before = 0, part = 0, here = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += kRankWords) part += m.counts[b];
+  block_exclusive_256(part, warp_sums, &before);
+  const int w = blockIdx.x * kRankWords + threadIdx.x;
+  const uint32_t e = block_exclusive_256(__popc(m.mask[w]), warp_sums, &here);
+  m.rank[w] = (int)(before + e);
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = (int)(before + here);
+}
+
+// Layout of the collapsed tree: a node stays when neither it nor an ancestor
+// collapses, and its index is the number of nodes before it that stay (the
+// root is node 0).  Only nodes of up to max_leaf primitives have ancestors
+// that can collapse.  (One launch per level, breadth first, was 26 to 32
+// launches of 3-12 us, 265 us for the 327 k mesh; these three take 34.)
+__device__ __forceinline__ int rec_height(const float4* rec, int node) {
+  return __float_as_int(rec[2 * (size_t)node + 1].w);
+}
+
+__global__ void __launch_bounds__(256)
+    k_lbvh_keep(int n_int, const int4* __restrict__ range, const int* __restrict__ parent_int,
+                const float4* __restrict__ rec, int max_leaf, NodeMask m, int* __restrict__ levels) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  bool keep = i < n_int && rec_height(rec, i) > 0;
+  for (int p = i; keep;) {
+    const int4 q = range[p];
+    if (q.y - q.x + 1 > max_leaf) break;
+    p = parent_int[p];
+    if (p < 0) break;
+    keep = rec_height(rec, p) > 0;
+  }
+  m.mark(i, keep);
+  if (i == 0) *levels = rec_height(rec, 0);
+}
+
+// at_lo: first sorted position under each laid-out node.
+__global__ void k_lbvh_layout(int n_int, const int4* __restrict__ range, const int* __restrict__ order,
+                              const float3* __restrict__ pmin, const float3* __restrict__ pmax,
+                              const float4* __restrict__ rec, NodeMask m, float4* __restrict__ out,
+                              int* __restrict__ at_lo) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_int; i += gridDim.x * blockDim.x) {
+    if (!m.has(i)) continue;
+    const int4 q = range[i];
+    const int ch[2] = {left_child(q.x, q.z), right_child(q.y, q.z)};
     int words[2], counts[2];
     float3 b0[2], b1[2];
-    int ch[2] = {kl[node], kr[node]};
     for (int s = 0; s < 2; ++s) {
-      int c = ch[s];
+      const int c = ch[s];
       if (c < 0) {
-        int p = order[~c];
-        b0[s] = pmin[p]; b1[s] = pmax[p];
+        const int p = order[~c];
+        b0[s] = pmin[p];
+        b1[s] = pmax[p];
         words[s] = pack_leaf(~c, 1);  // one primitive at sorted position ~c
         counts[s] = 1;
-      } else if (collapse[c]) {
-        b0[s] = imin[c]; b1[s] = imax[c];
-        words[s] = pack_leaf(first[c], last[c] - first[c] + 1);
-        counts[s] = last[c] - first[c] + 1;
+        continue;
+      }
+      const UpBox u = up_box(rec[2 * (size_t)c], rec[2 * (size_t)c + 1]);
+      b0[s] = u.lo;
+      b1[s] = u.hi;
+      if (u.height == 0) {  // the left child covers [lo, gamma], the right one [gamma + 1, hi]
+        const int lo = s ? q.z + 1 : q.x, hi = s ? q.y : q.z;
+        words[s] = pack_leaf(lo, hi - lo + 1);
+        counts[s] = hi - lo + 1;
       } else {
-        b0[s] = imin[c]; b1[s] = imax[c];
-        int o = atomicAdd(next_count, 1);
-        if (o < next_cap) next[o] = c;
-        words[s] = next_base + o;
+        words[s] = m.index(c);
         counts[s] = 0;
       }
     }
-    float4* o = out + 4 * (size_t)(out_base + q);
+    const size_t at = m.index(i);
+    at_lo[at] = q.x;
+    float4* o = out + 4 * at;
     o[0] = make_float4(b0[0].x, b1[0].x, b0[0].y, b1[0].y);
     o[1] = make_float4(b0[0].z, b1[0].z, b0[1].x, b1[1].x);
     o[2] = make_float4(b0[1].y, b1[1].y, b0[1].z, b1[1].z);
     o[3] = make_float4(__int_as_float(words[0]), __int_as_float(words[1]), __int_as_float(counts[0]),
                        __int_as_float(counts[1]));
   }
-  level_advance(lv);
 }
 
-// 4-wide nodes from the laid-out binary tree, one level per launch.  The
-// 4-wide node of binary node b starts from b's two children and, while it
-// has fewer than four, opens the internal child of largest surface area
-// (replacing it by its own two children): the children that the most rays
-// enter are expanded first, which removes more node visits than always
-// taking both grandchildren (6-8 % fewer visits per ray on the displaced
-// icosphere).  Leaf children stay leaves; internal children that remain
-// become 4-wide nodes of the next level.  Empty binary slots (count 0
-// leaves) are dropped; unused slots get a box at 1e30 and count 0.
-__global__ void k_bvh4_level(const int* __restrict__ cur, int* __restrict__ next, int* __restrict__ lv,
-                             const float4* __restrict__ bin, int n_bin, float4* __restrict__ out4, int* err) {
-  const int ncur = lv[LV_NCUR], out_base = lv[LV_BASE];
-  if (ncur <= 0) return;
-  if (out_base + ncur > n_bin) {  // a 4-wide tree has at most as many nodes as the binary one
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      lv[LV_OVERFLOW] = 1;
-      lv[LV_NCUR] = 0;
-    }
+// 4-wide nodes from the laid-out binary tree.  The 4-wide node of binary
+// node b starts from b's two children and, while it has fewer than four,
+// opens the internal child of largest surface area (replacing it by its own
+// two children): the children that the most rays enter are expanded first,
+// which removes more node visits than always taking both grandchildren
+// (6-8 % fewer visits per ray on the displaced icosphere).  Leaf children
+// stay leaves; internal children that remain are 4-wide nodes themselves.
+// Empty binary slots (count 0 leaves) are dropped; unused slots get a box at
+// 1e30 and count 0.
+//
+// Which children b would have depends on b's subtree alone, so every binary
+// node works them out at once (k_wide_kids); a node then follows those lists
+// from the root towards itself to see whether it is reached (k_wide_roots),
+// and the reached ones write their records (k_wide_write).  Four short
+// launches, whatever the depth: 150 -> 45 us for the 327 k mesh against a
+// launch per level of the 4-wide tree (and 184 us with one cooperative
+// launch and a grid barrier per level).
+struct WideNode {
+  float mn[4][3], mx[4][3];
+  int wd[4], ct[4];
+  int k;
+};
+
+// All slots are registers: every index below is a constant after unrolling.
+__device__ __forceinline__ void wide_add(WideNode& v, const float4* __restrict__ nb, bool second, int* err) {
+  const float4 n0 = nb[0], n1 = nb[1], n2 = nb[2], n3 = nb[3];
+  const int w = __float_as_int(second ? n3.y : n3.x), c = __float_as_int(second ? n3.w : n3.z);
+  if (w < 0 && c == 0) return;  // empty slot
+  if (v.k >= 4) {               // cannot happen: a node is opened only while k < 4
+    atomicOr(err, ERR_BAD_NODE);
     return;
   }
-  const int next_base = out_base + ncur, next_cap = n_bin - next_base;
-  int* next_count = &lv[LV_NEXT];
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < ncur; q += gridDim.x * blockDim.x) {
-    float mn[4][3], mx[4][3];
-    int wd[4], ct[4];
-    int k = 0;
-    // appends child `side` of the binary record nb (nothing for an empty slot)
-    auto add = [&](const float4* nb, int side) {
-      const float4 n0 = nb[0], n1 = nb[1], n2 = nb[2], n3 = nb[3];
-      const int w = __float_as_int(side ? n3.y : n3.x), c = __float_as_int(side ? n3.w : n3.z);
-      if (w < 0 && c == 0) return;  // empty slot
-      if (k >= 4) {                 // cannot happen: a node is opened only while k < 4
-        atomicOr(err, ERR_BAD_NODE);
-        return;
-      }
-      if (side == 0) {
-        mn[k][0] = n0.x, mx[k][0] = n0.y, mn[k][1] = n0.z, mx[k][1] = n0.w, mn[k][2] = n1.x, mx[k][2] = n1.y;
-      } else {
-        mn[k][0] = n1.z, mx[k][0] = n1.w, mn[k][1] = n2.x, mx[k][1] = n2.y, mn[k][2] = n2.z, mx[k][2] = n2.w;
-      }
-      wd[k] = w;
-      ct[k] = w >= 0 ? 0 : c;
-      ++k;
-    };
-    const int b = cur[q];
-    const float4* nb = bin + 4 * (size_t)b;
-    add(nb, 0);
-    add(nb, 1);
-    while (k < 4) {
-      int bi = -1;
-      float ba = -1.0f;
-      for (int i = 0; i < k; ++i) {
-        if (wd[i] < 0) continue;
-        if (wd[i] >= n_bin) {  // never entered: flagged and turned into an empty leaf
-          atomicOr(err, ERR_BAD_NODE);
-          wd[i] = pack_leaf(0, 0);
-          ct[i] = 0;
-          continue;
-        }
-        const float ex = mx[i][0] - mn[i][0], ey = mx[i][1] - mn[i][1], ez = mx[i][2] - mn[i][2];
-        const float a = ex * ey + ey * ez + ez * ex;
-        if (a > ba) {
-          ba = a;
-          bi = i;
-        }
-      }
-      if (bi < 0) break;
-      const float4* cb = bin + 4 * (size_t)wd[bi];
-      // remove entry bi (the last entry moves into its place), then append
-      // its two children
-      --k;
-      if (bi != k) {
-        for (int a = 0; a < 3; ++a) mn[bi][a] = mn[k][a], mx[bi][a] = mx[k][a];
-        wd[bi] = wd[k];
-        ct[bi] = ct[k];
-      }
-      add(cb, 0);
-      add(cb, 1);
-    }
-    for (int i = 0; i < k; ++i) {
-      if (wd[i] < 0) continue;
-      // an internal binary node becomes a 4-wide node of the next level
-      const int o = atomicAdd(next_count, 1);
-      if (o < next_cap) {
-        next[o] = wd[i];
-        wd[i] = next_base + o;
-      } else {
-        atomicOr(err, ERR_BAD_NODE);
-        wd[i] = pack_leaf(0, 0);
-      }
-    }
-    for (; k < 4; ++k) {
-      mn[k][0] = mn[k][1] = mn[k][2] = 1e30f;
-      mx[k][0] = mx[k][1] = mx[k][2] = 1e30f;
-      wd[k] = pack_leaf(0, 0);
-      ct[k] = 0;
-    }
-    float4* o = out4 + 8 * (size_t)(out_base + q);
-    o[0] = make_float4(mn[0][0], mn[1][0], mn[2][0], mn[3][0]);
-    o[1] = make_float4(mx[0][0], mx[1][0], mx[2][0], mx[3][0]);
-    o[2] = make_float4(mn[0][1], mn[1][1], mn[2][1], mn[3][1]);
-    o[3] = make_float4(mx[0][1], mx[1][1], mx[2][1], mx[3][1]);
-    o[4] = make_float4(mn[0][2], mn[1][2], mn[2][2], mn[3][2]);
-    o[5] = make_float4(mx[0][2], mx[1][2], mx[2][2], mx[3][2]);
-    o[6] = make_float4(__int_as_float(wd[0]), __int_as_float(wd[1]), __int_as_float(wd[2]), __int_as_float(wd[3]));
-    o[7] = make_float4(__int_as_float(ct[0]), __int_as_float(ct[1]), __int_as_float(ct[2]), __int_as_float(ct[3]));
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (i != v.k) continue;
+    v.mn[i][0] = second ? n1.z : n0.x, v.mx[i][0] = second ? n1.w : n0.y;
+    v.mn[i][1] = second ? n2.x : n0.z, v.mx[i][1] = second ? n2.y : n0.w;
+    v.mn[i][2] = second ? n2.z : n1.x, v.mx[i][2] = second ? n2.w : n1.y;
+    v.wd[i] = w;
+    v.ct[i] = w >= 0 ? 0 : c;
   }
-  level_advance(lv);
+  ++v.k;
+}
+
+__device__ __forceinline__ void wide_open(WideNode& v, const float4* __restrict__ bin, int n_bin, int b, int* err) {
+  v.k = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v.mn[i][0] = v.mn[i][1] = v.mn[i][2] = 1e30f;
+    v.mx[i][0] = v.mx[i][1] = v.mx[i][2] = 1e30f;
+    v.wd[i] = pack_leaf(0, 0);
+    v.ct[i] = 0;
+  }
+  wide_add(v, bin + 4 * (size_t)b, false, err);
+  wide_add(v, bin + 4 * (size_t)b, true, err);
+  while (v.k < 4) {
+    int bi = -1, open = 0;
+    float ba = -1.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i >= v.k || v.wd[i] < 0) continue;
+      if (v.wd[i] >= n_bin) {  // never entered: flagged and turned into an empty leaf
+        atomicOr(err, ERR_BAD_NODE);
+        v.wd[i] = pack_leaf(0, 0);
+        v.ct[i] = 0;
+        continue;
+      }
+      const float ex = v.mx[i][0] - v.mn[i][0], ey = v.mx[i][1] - v.mn[i][1], ez = v.mx[i][2] - v.mn[i][2];
+      const float a = ex * ey + ey * ez + ez * ex;
+      if (a > ba) {
+        ba = a;
+        bi = i;
+        open = v.wd[i];
+      }
+    }
+    if (bi < 0) break;
+    // remove entry bi (the last entry moves into its place), then append its
+    // two children
+    --v.k;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+#pragma unroll
+      for (int j = i + 1; j < 4; ++j) {
+        if (i != bi || j != v.k) continue;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) v.mn[i][a] = v.mn[j][a], v.mx[i][a] = v.mx[j][a];
+        v.wd[i] = v.wd[j];
+        v.ct[i] = v.ct[j];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i != v.k) continue;  // the freed slot, should both children be empty
+      v.mn[i][0] = v.mn[i][1] = v.mn[i][2] = 1e30f;
+      v.mx[i][0] = v.mx[i][1] = v.mx[i][2] = 1e30f;
+      v.wd[i] = pack_leaf(0, 0);
+      v.ct[i] = 0;
+    }
+    wide_add(v, bin + 4 * (size_t)open, false, err);
+    wide_add(v, bin + 4 * (size_t)open, true, err);
+  }
+}
+
+// kids[2b]: the internal children of b's 4-wide node (-1: none), kids[2b + 1]:
+// the first sorted position under each.
+__global__ void __launch_bounds__(128) k_wide_kids(const float4* __restrict__ bin, int n_bin,
+                                                   const int* __restrict__ at_lo, int4* __restrict__ kids, int* err) {
+  const int b = blockIdx.x * 128 + threadIdx.x;
+  if (b >= n_bin) return;
+  WideNode v;
+  wide_open(v, bin, n_bin, b, err);
+  int id[4], lo[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const bool in = v.wd[i] >= 0 && v.wd[i] < n_bin;
+    id[i] = in ? v.wd[i] : -1;
+    lo[i] = in ? at_lo[v.wd[i]] : INT_MAX;
+  }
+  kids[2 * (size_t)b] = make_int4(id[0], id[1], id[2], id[3]);
+  kids[2 * (size_t)b + 1] = make_int4(lo[0], lo[1], lo[2], lo[3]);
+}
+
+// Marks the binary nodes that are 4-wide nodes: from the root, the child
+// that holds b's first position is the one of largest first position not
+// beyond it.  A node that an ancestor opened is passed by and the walk ends
+// below it.
+__global__ void __launch_bounds__(256) k_wide_roots(int n_bin, const int4* __restrict__ kids,
+                                                    const int* __restrict__ at_lo, NodeMask m) {
+  const int b = blockIdx.x * 256 + threadIdx.x;
+  int cur = b < n_bin ? 0 : -1;
+  const int p = b < n_bin ? at_lo[b] : 0;
+  for (int s = 0; s < 64 && cur >= 0 && cur != b; ++s) {  // a tree of 62-bit keys has fewer levels
+    const int4 id = kids[2 * (size_t)cur], lo = kids[2 * (size_t)cur + 1];
+    int best = -1;
+    cur = -1;
+    if (lo.x <= p && lo.x > best) best = lo.x, cur = id.x;
+    if (lo.y <= p && lo.y > best) best = lo.y, cur = id.y;
+    if (lo.z <= p && lo.z > best) best = lo.z, cur = id.z;
+    if (lo.w <= p && lo.w > best) best = lo.w, cur = id.w;
+  }
+  m.mark(b, b < n_bin && cur == b);
+}
+
+__global__ void __launch_bounds__(128) k_wide_write(const float4* __restrict__ bin, int n_bin, NodeMask m,
+                                                    float4* __restrict__ out4, int* err) {
+  const int b = blockIdx.x * 128 + threadIdx.x;
+  if (b >= n_bin || !m.has(b)) return;
+  WideNode v;
+  wide_open(v, bin, n_bin, b, err);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (v.wd[i] >= 0 && v.wd[i] < n_bin) v.wd[i] = m.index(v.wd[i]);
+  float4* o = out4 + 8 * (size_t)m.index(b);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    o[2 * a] = make_float4(v.mn[0][a], v.mn[1][a], v.mn[2][a], v.mn[3][a]);
+    o[2 * a + 1] = make_float4(v.mx[0][a], v.mx[1][a], v.mx[2][a], v.mx[3][a]);
+  }
+  o[6] = make_float4(__int_as_float(v.wd[0]), __int_as_float(v.wd[1]), __int_as_float(v.wd[2]),
+                     __int_as_float(v.wd[3]));
+  o[7] = make_float4(__int_as_float(v.ct[0]), __int_as_float(v.ct[1]), __int_as_float(v.ct[2]),
+                     __int_as_float(v.ct[3]));
 }
 
 // Root record for a tree that is a single leaf of `cnt` primitives.
@@ -920,59 +1072,46 @@ int set_reference_nodes(Ctx* ctx, Scene* sc, int n_nodes, const float* node_min,
   return RX_OK;
 }
 
-// Runs a device-driven level walk: `launch(level, cur, next, lv)` enqueues
-// one level (cur / next alternate between a and b); levels are enqueued in
-// batches of kLevelBatch and the state is read back once per batch.  The
-// root (node 0) is the only node of level 0.  Returns the total nodes laid
-// out through *n_out and the number of levels through *levels.
-constexpr int kLevelBatch = 16, kMaxLevels = 1024;
-template <class F>
-static int level_walk(Ctx* ctx, int* a, int* b, int* lv, int* n_out, int* levels, F launch) {
-  cudaStream_t st = ctx->stream;
-  const int init[LV_N] = {1, 0, 0, 0, 0, 0, 0, 0};
-  CUDA_TRY(ctx, cudaMemsetAsync(a, 0, sizeof(int), st));
-  CUDA_TRY(ctx, cudaMemcpyAsync(lv, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  int h[LV_N] = {0};
-  for (int level = 0;;) {
-    for (int k = 0; k < kLevelBatch; ++k, ++level) launch(level, (level & 1) ? b : a, (level & 1) ? a : b, lv);
-    CUDA_TRY(ctx, cudaGetLastError());
-    CUDA_TRY(ctx, cudaMemcpyAsync(h, lv, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (h[LV_OVERFLOW]) return set_error(ctx, "BVH level walk: a level overflowed the tree"), RX_ERR_DEVICE;
-    if (h[LV_NCUR] == 0) break;
-    if (level >= kMaxLevels) return set_error(ctx, "BVH level walk did not terminate"), RX_ERR_DEVICE;
+// Mask, ranks and counts for n nodes, the counts cleared on the stream.
+struct MaskBuf {
+  int blocks;
+  DevBuf<uint32_t> mask;
+  DevBuf<int> rank, counts;
+  MaskBuf(Ctx* ctx, int n)
+      : blocks((n + 32 * kRankWords - 1) / (32 * kRankWords)),
+        mask(ctx, (size_t)blocks * kRankWords),
+        rank(ctx, (size_t)blocks * kRankWords),
+        counts(ctx, blocks) {}
+  cudaError_t clear(cudaStream_t st) {
+    // words beyond the last marked node are never written: they must be zero
+    cudaError_t e = cudaMemsetAsync(mask.p, 0, sizeof(uint32_t) * (size_t)blocks * kRankWords, st);
+    return e != cudaSuccess ? e : cudaMemsetAsync(counts.p, 0, sizeof(int) * (size_t)blocks, st);
   }
-  *n_out = h[LV_BASE];
-  *levels = h[LV_LEVELS];
-  return RX_OK;
-}
+  NodeMask view() const { return {mask.p, rank.p, counts.p}; }
+};
 
-// Blocks for level `level` of a tree whose nodes have up to `fan` children:
-// at most fan^level nodes, and never more than the whole tree's n.
-static int level_grid(Ctx* ctx, int level, int fan_log2, long long n) {
-  const long long bound = level * fan_log2 >= 40 ? n : std::min<long long>(n, 1LL << (level * fan_log2));
-  long long g = (bound + 255) / 256;
-  const long long cap = (long long)ctx->num_sms * 32;
-  return (int)std::max<long long>(1, std::min(g, cap));
-}
-
-// The 4-wide copy of the laid-out binary tree (k_bvh4_level, level by
-// level from the root, breadth first).
-static int build_wide(Ctx* ctx, Scene* sc) {
+// The 4-wide copy of the laid-out binary tree; at_lo: the first sorted
+// position under each of its nodes.
+static int build_wide(Ctx* ctx, Scene* sc, const int* at_lo) {
   cudaStream_t st = ctx->stream;
   const int nb = sc->n_nodes;
   sc->n_nodes4 = 0;
   if (nb <= 0) return RX_OK;
   if (!sc->d_nodes4.alloc(ctx, (size_t)8 * nb)) return set_error(ctx, "out of device memory for the 4-wide BVH"), RX_ERR_CAPACITY;
-  DevBuf<int> la(ctx, nb), lb(ctx, nb), lv(ctx, LV_N);
-  if (!all_ok(la, lb, lv)) return set_error(ctx, "out of device memory"), RX_ERR_CAPACITY;
-  int base = 0, levels = 0;
-  int rc = level_walk(ctx, la.p, lb.p, lv.p, &base, &levels, [&](int level, int* cur, int* nxt, int* st_lv) {
-    k_bvh4_level<<<level_grid(ctx, level, 2, nb), 256, 0, st>>>(cur, nxt, st_lv, sc->d_nodes.p, nb, sc->d_nodes4.p,
-                                                              ctx->d_err);
-  });
-  if (rc) return rc;
-  sc->n_nodes4 = base;
+  MaskBuf m(ctx, nb);
+  DevBuf<int4> kids(ctx, (size_t)2 * nb);
+  DevBuf<int> total(ctx, 1);
+  if (!all_ok(m.mask, m.rank, m.counts, kids, total)) return set_error(ctx, "out of device memory"), RX_ERR_CAPACITY;
+  CUDA_TRY(ctx, m.clear(st));
+  k_wide_kids<<<(nb + 127) / 128, 128, 0, st>>>(sc->d_nodes.p, nb, at_lo, kids.p, ctx->d_err);
+  k_wide_roots<<<(nb + 255) / 256, 256, 0, st>>>(nb, kids.p, at_lo, m.view());
+  k_rank<<<m.blocks, kRankWords, 0, st>>>(m.view(), total.p);
+  k_wide_write<<<(nb + 127) / 128, 128, 0, st>>>(sc->d_nodes.p, nb, m.view(), sc->d_nodes4.p, ctx->d_err);
+  CUDA_TRY(ctx, cudaGetLastError());
+  int n4 = 0;
+  CUDA_TRY(ctx, cudaMemcpyAsync(&n4, total.p, sizeof(n4), cudaMemcpyDeviceToHost, st));
+  CUDA_TRY(ctx, cudaStreamSynchronize(st));
+  sc->n_nodes4 = n4;
   return RX_OK;
 }
 
@@ -1042,63 +1181,50 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
   float3 hb[2];
   cudaMemcpyAsync(hb, rb.p, sizeof(hb), cudaMemcpyDeviceToHost, st);
   int n_int = n - 1;
+  DevBuf<int> at_lo;  // first sorted position under each laid-out node
   if (n == 1) {
-    if (!sc->d_nodes.alloc(ctx, 4)) {
+    if (!sc->d_nodes.alloc(ctx, 4) || !at_lo.alloc(ctx, 1)) {
       sc->clear_bvh();
       return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
     }
     k_single_leaf_root<<<1, 1, 0, st>>>(rb.p, rb.p + 1, 1, sc->d_nodes.p);
     sc->n_nodes = 1;
   } else {
-    DevBuf<int> kl(ctx, n_int), kr(ctx, n_int), first(ctx, n_int), last(ctx, n_int);
-    DevBuf<int> par_int(ctx, n_int), par_leaf(ctx, n), flags(ctx, n_int), icount(ctx, n_int), collapse(ctx, n_int);
-    DevBuf<float3> imin(ctx, n_int), imax(ctx, n_int);
-    DevBuf<float> icost(ctx, n_int);
-    if (!all_ok(kl, kr, first, last, par_int, par_leaf, flags, icount, collapse, imin, imax, icost)) {
+    DevBuf<int4> range(ctx, n_int);
+    DevBuf<int> par_int(ctx, n_int), par_leaf(ctx, n), flags(ctx, n_int);
+    DevBuf<float4> rec(ctx, (size_t)2 * n_int);
+    MaskBuf m(ctx, n_int);
+    DevBuf<int> info(ctx, 2);  // nodes laid out, levels
+    sc->d_nodes.alloc(ctx, (size_t)4 * n_int);
+    at_lo.alloc(ctx, n_int);
+    if (!all_ok(sc->d_nodes, at_lo, range, par_int, par_leaf, flags, rec, m.mask, m.rank, m.counts, info)) {
       sc->clear_bvh();
       return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
     }
     cudaMemsetAsync(par_int.p, 0xff, sizeof(int) * n_int, st);
-    k_karras<<<grid_for(ctx, n_int), 256, 0, st>>>(n, sc->tmp_codes.p, kl.p, kr.p, first.p, last.p, par_int.p,
-                                                    par_leaf.p);
+    k_karras<<<grid_for(ctx, n_int), 256, 0, st>>>(n, sc->tmp_codes.p, range.p, par_int.p, par_leaf.p);
     cudaMemsetAsync(flags.p, 0, sizeof(int) * n_int, st);
-    k_lbvh_bottom_up<<<grid_for(ctx, n), 256, 0, st>>>(n, order.p, kl.p, kr.p, par_int.p, par_leaf.p, pmin.p,
-                                                        pmax.p, imin.p, imax.p, icost.p, icount.p, collapse.p,
-                                                        flags.p, max_leaf, c_t, c_i);
-    int root_col = 0;
-    cudaMemcpyAsync(&root_col, collapse.p, sizeof(int), cudaMemcpyDeviceToHost, st);
+    k_lbvh_bottom_up<<<(n + kUpLeaves - 1) / kUpLeaves, kUpLeaves, 0, st>>>(
+        n, order.p, range.p, par_int.p, par_leaf.p, pmin.p, pmax.p, rec.p, flags.p, max_leaf, c_t, c_i);
+    CUDA_TRY(ctx, m.clear(st));
+    k_lbvh_keep<<<(n_int + 255) / 256, 256, 0, st>>>(n_int, range.p, par_int.p, rec.p, max_leaf, m.view(), info.p + 1);
+    k_rank<<<m.blocks, kRankWords, 0, st>>>(m.view(), info.p);
+    k_lbvh_layout<<<grid_for(ctx, n_int), 256, 0, st>>>(n_int, range.p, order.p, pmin.p, pmax.p, rec.p, m.view(),
+                                                         sc->d_nodes.p, at_lo.p);
+    CUDA_TRY(ctx, cudaGetLastError());
+    int h_info[2] = {0, 0};
+    CUDA_TRY(ctx, cudaMemcpyAsync(h_info, info.p, sizeof(h_info), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    if (root_col) {
-      if (!sc->d_nodes.alloc(ctx, 4)) {
-        sc->clear_bvh();
-        return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
-      }
+    sc->n_nodes = h_info[0];
+    sc->depth = h_info[1];
+    if (sc->n_nodes == 0) {  // the whole tree is one leaf
       k_single_leaf_root<<<1, 1, 0, st>>>(rb.p, rb.p + 1, n, sc->d_nodes.p);
       sc->n_nodes = 1;
-    } else {
-      sc->d_nodes.alloc(ctx, (size_t)4 * n_int);
-      DevBuf<int> la(ctx, n_int), lb(ctx, n_int), lv(ctx, LV_N);
-      if (!all_ok(sc->d_nodes, la, lb, lv)) {
-        sc->clear_bvh();
-        return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
-      }
-      int base = 0, levels = 0;
-      int rc = level_walk(ctx, la.p, lb.p, lv.p, &base, &levels, [&](int level, int* cur, int* nxt, int* st_lv) {
-        k_lbvh_layout_level<<<level_grid(ctx, level, 1, n_int), 256, 0, st>>>(
-            cur, nxt, st_lv, n_int, kl.p, kr.p, first.p, last.p, collapse.p, order.p, pmin.p, pmax.p,
-            imin.p, imax.p, sc->d_nodes.p);
-      });
-      if (rc) {
-        sc->clear_bvh();
-        return rc;
-      }
-      sc->depth = levels;
-      sc->n_nodes = base;
     }
   }
   sc->order.swap(order);
   CUDA_TRY(ctx, cudaStreamSynchronize(st));
-  if (int rc = build_wide(ctx, sc)) {
+  if (int rc = build_wide(ctx, sc, at_lo.p)) {
     sc->clear_bvh();
     return rc;
   }

@@ -142,6 +142,52 @@ def test_lbvh_structure(n, leaf):
     _check_layout(nodes, order, n, st.min(1) - 1e-4, st.max(1) + 1e-4)
 
 
+@pytest.mark.parametrize("n,leaf,spread", [(511, 4, 1.0), (512, 4, 1.0), (513, 1, 1.0), (1025, 8, 0.0), (8192, 4, 1.0),
+                                           (8194, 4, 1e-3), (40000, 2, 1e-2)])
+def test_lbvh_block_edges(n, leaf, spread):
+    """Tree builds around the blocks of the bottom-up pass (512 leaves) and of
+    the layout (8,192 nodes), with triangles spread out, in one dense cluster
+    beside a few far ones, and all in one place (equal codes): every
+    primitive once, every box holds its primitives, and the 4-wide copy finds
+    the t of the reference's tree on every ray."""
+    v = np.stack(gs.soup_triangles(n, 7 * n + leaf), 1)
+    v[5:] = v[5:] * spread + (1.0 - spread) * v[5:6].mean(axis=(0, 1), keepdims=True)
+    v0, v1, v2 = (np.ascontiguousarray(v[:, k], np.float32) for k in range(3))
+    scenes = []
+    for method in (nat.RX_BVH_LBVH_SAH, nat.RX_BVH_REFERENCE):
+        sc = nat.NativeScene()
+        sc.set_triangles(v0, v1, v2)
+        sc.set_materials([0], [[0.5, 0.5, 0.5]], [0.0], [1.0], [0.0])
+        sc.build_bvh(method, leaf, True)
+        scenes.append(sc)
+    nodes, order = scenes[0].export_layout()
+    st = np.stack([v0, v1, v2], 1)
+    _check_layout(nodes, order, n, st.min(1) - 1e-4, st.max(1) + 1e-4)
+    rng = np.random.default_rng(n)
+    at = st.mean(1)[rng.integers(0, n, 4000)]
+    ro = (at + rng.normal(size=at.shape)).astype(np.float32)
+    rd = (at - ro).astype(np.float32)
+    rd /= np.linalg.norm(rd, axis=1, keepdims=True)
+    a, b = (sc.trace_closest(ro, rd)[0] for sc in scenes)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("n", [1, 31, 1023, 1025, 4097, 262_145, (1 << 20) + 1])
+def test_sort_order_matches_oracle(n):
+    """Both tile sizes of the radix sort (1,024 keys up to 2^20 of them, then
+    4,096), at tile edges: the oracle's stable Morton order."""
+    v0, v1, v2 = gs.soup_triangles(n, 3)
+    v0[n // 2:] = v0[:n - n // 2]
+    v1[n // 2:] = v1[:n - n // 2]
+    v2[n // 2:] = v2[:n - n // 2]  # every code twice: stability shows
+    sc = nat.NativeScene()
+    sc.set_triangles(v0, v1, v2)
+    sc.set_materials([0], [[0.5, 0.5, 0.5]], [0.0], [1.0], [0.0])
+    sc.build_bvh(nat.RX_BVH_REFERENCE, 8)
+    _, order = sc.export_layout()
+    np.testing.assert_array_equal(order, oracle.bvh_build_morton(v0, v1, v2, 8)["order"])
+
+
 def test_lbvh_with_spheres_in_tree():
     v0, v1, v2 = gs.soup_triangles(500, 7)
     sc = nat.NativeScene()
