@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "rx_internal.cuh"
 #include "rx_runtime.h"
@@ -42,6 +43,11 @@ __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(smem_u32(p)));
+}
+__device__ __forceinline__ void ldsm_x4_at(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(saddr));
 }
 __device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], const void* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -179,6 +185,158 @@ __global__ void __launch_bounds__(128) k_conv_fwd(rx_conv_desc d, const bf16* __
           y32[m * d.y_cstride + d.y_coff + co + 1] = v1;
         }
       }
+}
+
+// The same convolution for few input channels (KS 16-channel steps per tap)
+// and many output channels -- the gradients of the layers after a concat,
+// 32 -> 96 and 64 -> 192, which the tcgen05 path's groups do not cover.  The
+// products of an output are added in k_conv_fwd's order (taps outer, steps
+// inner), so the results are its bits.
+//
+// k_conv_fwd copies every tap's pixels and weights to shared memory again
+// (121 and 97 us for 14.5 GFLOP each at 16x128x128).  Here a block keeps all
+// nine taps' weights of its BN channels, and a tile's pixels are copied once
+// with their halo (two buffers: the next tile's copies run under this tile's
+// products); a tap is an offset of the ldmatrix addresses.  Tiles are
+// 128 pixels of 128 >> cl rows by 1 << cl columns.  Pixel and weight rows are
+// padded to an odd number of 16-byte chunks: no bank conflicts.  121 -> 65 and
+// 97 -> 56 us; mma.sync keeps the tensor pipe 45-53 % busy with the two warps
+// per scheduler that the weights leave room for (its floor is 29 us).
+template <int BN, int KS>
+struct ResShape {
+  static constexpr int CIN = 16 * KS, PX = CIN + 8, WROW = 9 * CIN + 8;  // elements
+  static constexpr int W_BYTES = BN * WROW * 2;
+  static int halo(int cl) { return ((128 >> cl) + 2) * ((1 << cl) + 2) * PX * 2; }
+  static size_t smem(int cl) { return (size_t)W_BYTES + 2 * (size_t)halo(cl); }
+};
+
+template <int BN, int KS>
+__global__ void __launch_bounds__(256, 1)
+    k_conv_fwd_res(rx_conv_desc d, const bf16* __restrict__ x, const bf16* __restrict__ w,
+                   const float* __restrict__ bias, bf16* __restrict__ y, float* __restrict__ y32, int relu, int cl,
+                   int tiles_x, int tiles_y, int halo_bytes) {
+  using S = ResShape<BN, KS>;
+  constexpr int NT = BN / 16, KC = 2 * KS, LOADERS = 256 / KC;  // n8 tiles per warp, chunks per pixel
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  const uint32_t sw = smem_u32(res_smem), sx = sw + S::W_BYTES;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = warp & 3, wn = warp >> 2;
+  const int n0 = blockIdx.y * BN;
+  const int HC = (1 << cl) + 2, HR = (128 >> cl) + 2;  // halo columns and rows
+  const int tiles = d.N * tiles_y * tiles_x;           // fits: launch_res
+
+  auto tile_at = [&](int t, int& n, int& y0, int& x0) {
+    const int r = t / tiles_x;
+    x0 = (t - r * tiles_x) << cl;
+    n = r / tiles_y;
+    y0 = (r - n * tiles_y) * (128 >> cl);
+  };
+  auto load = [&](int t, int buf) {
+    int n, y0, x0;
+    tile_at(t, n, y0, x0);
+    const int kc = tid % KC;
+    int hc = tid / KC, hr = 0;
+    unsigned char* dst = res_smem + S::W_BYTES + buf * halo_bytes + kc * 16;
+    const bf16* img = x + (long long)n * d.H * d.W * d.x_cstride + d.x_coff + kc * 8;
+    while (true) {
+      while (hc >= HC) hc -= HC, ++hr;
+      if (hr >= HR) break;
+      const int yy = y0 + hr - 1, xx = x0 + hc - 1;
+      const bool ok = (unsigned)yy < (unsigned)d.H && (unsigned)xx < (unsigned)d.W;
+      cp_async16(dst + (hr * HC + hc) * (S::PX * 2), ok ? img + ((long long)yy * d.W + xx) * d.x_cstride : x, ok);
+      hc += LOADERS;
+    }
+  };
+
+  for (int c = tid; c < BN * 9 * KC; c += 256) {
+    const int row = c / (9 * KC), k = c - row * (9 * KC);
+    const bool ok = n0 + row < d.Cout;
+    cp_async16(res_smem + row * (S::WROW * 2) + k * 16, ok ? w + (long long)(n0 + row) * 9 * S::CIN + k * 8 : w, ok);
+  }
+  int t = blockIdx.x, buf = 0;
+  if (t < tiles) load(t, 0);
+  cp_async_commit();
+
+  // this lane's ldmatrix rows: two m16 tiles of pixels, BN / 32 n16 tiles of weights
+  uint32_t a_at[2];
+#pragma unroll
+  for (int mi = 0; mi < 2; ++mi) {
+    const int m = wm * 32 + mi * 16 + (lane & 15);
+    a_at[mi] = ((m >> cl) * HC + (m & ((1 << cl) - 1))) * (S::PX * 2) + (lane >> 4) * 16;
+  }
+  const uint32_t b_at =
+      sw + (wn * (BN / 2) + (lane & 7) + (lane >> 4) * 8) * (S::WROW * 2) + ((lane >> 3) & 1) * 16;
+
+  for (; t < tiles; t += gridDim.x, buf ^= 1) {
+    // one barrier a tile: this tile's copies have landed for every thread, and
+    // every warp has left the other buffer, which the next tile's copies take
+    cp_async_wait<0>();
+    __syncthreads();
+    if (t + (int)gridDim.x < tiles) load(t + gridDim.x, buf ^ 1);
+    cp_async_commit();
+    float acc[2][NT][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.0f;
+    const uint32_t xb = sx + buf * halo_bytes;
+    for (int ty = 0; ty < 3; ++ty) {
+#pragma unroll
+      for (int tx = 0; tx < 3; ++tx) {
+        const uint32_t xo = xb + (ty * HC + tx) * (S::PX * 2), wo = b_at + (ty * 3 + tx) * (S::CIN * 2);
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks) {
+          uint32_t af[2][4];
+#pragma unroll
+          for (int mi = 0; mi < 2; ++mi) ldsm_x4_at(af[mi], xo + a_at[mi] + ks * 32);
+#pragma unroll
+          for (int nj = 0; nj < NT / 2; ++nj) {
+            uint32_t bfr[4];
+            ldsm_x4_at(bfr, wo + nj * 16 * (S::WROW * 2) + ks * 32);
+#pragma unroll
+            for (int mi = 0; mi < 2; ++mi) {
+              mma_bf16(acc[mi][2 * nj], af[mi], bfr[0], bfr[1]);
+              mma_bf16(acc[mi][2 * nj + 1], af[mi], bfr[2], bfr[3]);
+            }
+          }
+        }
+      }
+    }
+    int n, y0, x0;
+    tile_at(t, n, y0, x0);
+    const int g = lane >> 2, q = lane & 3;
+#pragma unroll
+    for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int m = wm * 32 + mi * 16 + g + h * 8;
+        const int yy = y0 + (m >> cl), xx = x0 + (m & ((1 << cl) - 1));
+        if (yy >= d.H || xx >= d.W) continue;
+        const long long at = (((long long)n * d.H + yy) * d.W + xx) * d.y_cstride + d.y_coff;
+#pragma unroll
+        for (int ni = 0; ni < NT; ++ni) {
+          const int co = n0 + wn * (BN / 2) + ni * 8 + 2 * q;
+          if (co >= d.Cout) continue;
+          float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
+          if (bias) {
+            v0 += bias[co];
+            v1 += bias[co + 1];
+          }
+          if (relu) {
+            v0 = fmaxf(v0, 0.0f);
+            v1 = fmaxf(v1, 0.0f);
+          }
+          *reinterpret_cast<__nv_bfloat162*>(y + at + co) = __floats2bfloat162_rn(v0, v1);
+          if (y32) {
+            y32[at + co] = v0;
+            y32[at + co + 1] = v1;
+          }
+        }
+      }
+  }
+  cp_async_wait<0>();
 }
 
 // ------------------------------------------- forward conv on tcgen05 (UMMA)
@@ -1848,6 +2006,56 @@ static int launch_ws_split(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const
   return 1;
 }
 
+template <int BN, int KS>
+static int launch_res_as(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
+                         float* y32, int relu, cudaStream_t st, int* rc) {
+  using S = ResShape<BN, KS>;
+  // the tile shape that covers the image with the fewest tiles; wider ones
+  // first (longer rows, less halo)
+  int cl = 7;
+  long long best = LLONG_MAX, tx = 0, ty = 0;
+  for (int c = 7; c >= 3; --c) {
+    const long long nx = (d->W + (1 << c) - 1) >> c, ny = (d->H + (128 >> c) - 1) / (128 >> c);
+    if (nx * ny < best) best = nx * ny, cl = c, tx = nx, ty = ny;
+  }
+  if (best * d->N > 0x3fffffffLL || S::smem(cl) > 232448) return 0;  // opt-in shared memory per block
+  auto kern = k_conv_fwd_res<BN, KS>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem(cl));
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  const int ny = (d->Cout + BN - 1) / BN;
+  const int nx = (int)std::max<long long>(1, std::min<long long>(best * d->N, ctx->num_sms / ny));
+  kern<<<dim3(nx, ny), 256, S::smem(cl), st>>>(*d, x, w, bias, y, y32, relu, cl, (int)tx, (int)ty, S::halo(cl));
+  e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_error(ctx, "conv_bf16_fwd: %s", cudaGetErrorString(e));
+    *rc = RX_ERR_CUDA;
+  }
+  return 1;
+}
+
+// k_conv_fwd_res for 16, 32 or 64 input and more than 32 output channels, in
+// blocks of 96 or 64 output channels, whichever computes fewer.  0: not for it.
+static int launch_res(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
+                      float* y32, int relu, cudaStream_t st, int* rc) {
+  if (d->Cout <= 32 || d->Cout > 64 * 65535) return 0;
+  const bool wide = (d->Cout + 95) / 96 * 96 <= (d->Cout + 63) / 64 * 64;
+  switch (d->Cin) {
+    case 16:
+      return wide ? launch_res_as<96, 1>(ctx, d, x, w, bias, y, y32, relu, st, rc)
+                  : launch_res_as<64, 1>(ctx, d, x, w, bias, y, y32, relu, st, rc);
+    case 32:
+      return wide ? launch_res_as<96, 2>(ctx, d, x, w, bias, y, y32, relu, st, rc)
+                  : launch_res_as<64, 2>(ctx, d, x, w, bias, y, y32, relu, st, rc);
+    case 64:
+      return wide ? launch_res_as<96, 4>(ctx, d, x, w, bias, y, y32, relu, st, rc)
+                  : launch_res_as<64, 4>(ctx, d, x, w, bias, y, y32, relu, st, rc);
+    default: return 0;
+  }
+}
+
 int conv_fwd(Ctx* ctx, const rx_conv_desc* d, const void* x, const void* w, const float* bias, void* y, float* y32,
              int relu, cudaStream_t st) {
   if (!conv_ok(d) || !x || !w || !y)
@@ -1870,6 +2078,12 @@ int conv_fwd(Ctx* ctx, const rx_conv_desc* d, const void* x, const void* w, cons
       case 128: return launch_tc<128>(ctx, d, xb, wb, bias, yb, y32, relu, st);
       default: break;
     }
+  }
+  {
+    int rc = RX_OK;
+    if (launch_res(ctx, d, static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, static_cast<bf16*>(y), y32,
+                   relu, st, &rc))
+      return rc;
   }
   long long P = (long long)d->N * d->H * d->W;
   dim3 grid((unsigned)((P + 63) / 64), 1);

@@ -341,6 +341,20 @@ def test_bias_gradient_sums_every_pixel(P, Cout, stride, off):
 
 
 @pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo,ys,yo,y32", [
+    (1, 1, 1, 16, 48, 16, 0, 48, 0, 1),        # one pixel; a group partly out of range
+    (2, 3, 8, 32, 96, 40, 8, 104, 8, 0),       # narrow images: 16 rows of 8 pixels
+    (3, 17, 33, 64, 192, 64, 0, 192, 0, 1),    # two groups of 96, ragged tiles
+    (1, 5, 129, 32, 160, 32, 0, 160, 0, 0),    # one pixel beyond a tile
+    (2, 128, 128, 32, 96, 32, 0, 96, 0, 0),    # more tiles than blocks
+    (1, 40, 70, 16, 224, 16, 0, 224, 0, 0),    # groups of 64 and of 96 tie
+])
+def test_resident_weight_conv_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo, y32):
+    """The kernel that keeps a group's weights in shared memory, at its tiles'
+    and groups' edges: bounds as for the warp-specialised kernel below."""
+    test_warp_specialised_conv_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo, y32)
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo,ys,yo,y32", [
     (1, 1, 1, 16, 16, 16, 0, 16, 0, 1),        # one pixel, one row
     (3, 2, 127, 32, 32, 40, 8, 40, 8, 0),      # one short tile; views off the 32-byte grid
     (2, 5, 128, 48, 64, 48, 0, 64, 0, 1),      # a whole tile; a step count outside the unrolled ones
