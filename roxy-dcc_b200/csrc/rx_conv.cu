@@ -248,6 +248,8 @@ __global__ void __launch_bounds__(256, 1)
     }
   };
 
+  chain_wait();
+  chain_go();
   for (int c = tid; c < BN * 9 * KC; c += 256) {
     const int row = c / (9 * KC), k = c - row * (9 * KC);
     const bool ok = n0 + row < d.Cout;
@@ -765,12 +767,16 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;\n" ::"r"(smem_u32(&mma_done)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  for (int c = tid; c < NG; c += blockDim.x) sbias[c] = bias ? bias[grp * NG + c] : 0.0f;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)),
                  "r"(TCOLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
+  // no chain_go: the next kernel's blocks, let in while this one works, took
+  // more than they hid (a 1080p inference 1,255 us with it, 1,160 without,
+  // 1,225 unchained)
+  chain_wait();
+  for (int c = tid; c < NG; c += blockDim.x) sbias[c] = bias ? bias[grp * NG + c] : 0.0f;
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -979,7 +985,8 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
               } else {
 #pragma unroll
                 for (int k = 0; k < CW / 8; ++k)
-                  reinterpret_cast<uint4*>(y + o)[k] = make_uint4(pw[4 * k], pw[4 * k + 1], pw[4 * k + 2], pw[4 * k + 3]);
+                  reinterpret_cast<uint4*>(y + o)[k] = make_uint4(pw[4 * k], pw[4 * k + 1], pw[4 * k + 2],
+                  pw[4 * k + 3]);
               }
             }
             if (y32) {
@@ -1072,9 +1079,11 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
                  "r"(A.tcols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
+  chain_wait();
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  chain_go();
   const uint32_t tmem = tmem_base;
   auto wait = [&](unsigned long long* bar, uint32_t ph) {
     return mbar_wait_abortable(smem_u32(bar), ph, &abort_flag);
@@ -1357,6 +1366,8 @@ __global__ void __cluster_dims__(kBiasCluster, 1, 1) __launch_bounds__(kBiasThre
     k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy, float* __restrict__ db, int pix_per_block) {
   __shared__ float part[kBiasThreads][9];  // 8 channels, padded against bank conflicts
   __shared__ double sums[kBiasWidth * 8];
+  chain_wait();
+  chain_go();
   auto cluster = cooperative_groups::this_cluster();
   const long long P = (long long)d.N * d.H * d.W;
   const long long p0 = (long long)blockIdx.x * pix_per_block;
@@ -1419,6 +1430,8 @@ __global__ void k_rot_weights(int Cout, int Cin, const bf16* __restrict__ w, bf1
 // scalar form's 64-bit divisions and 2-byte stores took 39 us for the ten
 // layers of a training step, this 31 (a launch each).
 __global__ void k_rot_weights_v8(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
+  chain_wait();
+  chain_go();
   const unsigned n = (unsigned)(Cout / 8) * 9u * (unsigned)Cin;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const unsigned t = i / (unsigned)Cin, ci = i - t * (unsigned)Cin;
@@ -1467,6 +1480,8 @@ __global__ void k_relu_mask(long long P, int C, const bf16* __restrict__ yv, int
 // training step 203 -> 89 us.
 __global__ void k_relu_mask_v8(long long P, int C, const bf16* __restrict__ yv, int y_stride, int y_off,
                                bf16* __restrict__ g, int g_stride, int g_off) {
+  chain_wait();
+  chain_go();
   const int CK = C >> 3;
   const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
   RX_EW_LOOP(P * CK) {
@@ -1538,6 +1553,8 @@ __device__ __forceinline__ void chunk_index(long long i, int CK, int W, int H, i
 
 __global__ void k_up2_v8(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                          bf16* __restrict__ y, int y_stride, int y_off) {
+  chain_wait();
+  chain_go();
   const int CK = C >> 3;
   RX_EW_LOOP((long long)N * H * W * CK) {
     int ck, xx, yy;
@@ -1555,6 +1572,8 @@ __global__ void k_up2_v8(int N, int H, int W, int C, const bf16* __restrict__ x,
 
 __global__ void k_pool2_v8(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                            bf16* __restrict__ y, int y_stride, int y_off) {
+  chain_wait();
+  chain_go();
   const int CK = C >> 3, h2 = H / 2, w2 = W / 2;
   RX_EW_LOOP((long long)N * h2 * w2 * CK) {
     int ck, xo, yo;
@@ -1602,6 +1621,8 @@ __global__ void k_pool2_bwd(int N, int H, int W, int C, const bf16* __restrict__
 // 86 -> 15 us, the two upsamples' 52 -> 16.
 __global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
                                bf16* __restrict__ dx, int dx_stride, int dx_off, int accumulate) {
+  chain_wait();
+  chain_go();
   const int CK = C >> 3, h2 = H / 2, w2 = W / 2;
   RX_EW_LOOP((long long)N * h2 * w2 * CK) {
     int ck, xo, yo;
@@ -1637,6 +1658,8 @@ __global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restric
 
 __global__ void k_up2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
                              bf16* __restrict__ dx, int dx_stride, int dx_off) {
+  chain_wait();
+  chain_go();
   const int CK = C >> 3;
   RX_EW_LOOP((long long)N * H * W * CK) {
     int ck, xx, yy;
@@ -1735,6 +1758,8 @@ __global__ void k_features(long long P, const float* __restrict__ rad, const flo
 __global__ void k_features_v4(long long P4, const float4* __restrict__ rad, const float4* __restrict__ alb,
                               const float4* __restrict__ nrm, const float4* __restrict__ dep, uint4* __restrict__ out,
                               float4* __restrict__ base) {
+  chain_wait();
+  chain_go();
   RX_EW_LOOP(P4) {
     float4 r[3], a[3], n[3], l[3];
 #pragma unroll
@@ -1766,6 +1791,8 @@ template <bool CHUNKS>
 __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
                           const float* __restrict__ t, float scale, bf16* __restrict__ g, int gs,
                           float* __restrict__ loss) {
+  chain_wait();
+  chain_go();
   float s = 0.0f;
   RX_EW_LOOP(P) {
     alignas(4) bf16 v[8];
@@ -1794,6 +1821,8 @@ __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stri
 // radiance = max(expm1(y + base), 0) from the head's first three channels
 __global__ void k_output(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
                          float* __restrict__ out) {
+  chain_wait();
+  chain_go();
   RX_EW_LOOP(P) {
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -1869,6 +1898,15 @@ static bool row_map(int N, int H, int W, int C, int stride, const bf16* v, int p
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Dynamic shared memory of a launch with at most one block per SM: enough
+// that a second block does not fit.  Blocks that come up while the kernel
+// before drains would otherwise pair up on the SMs that are free first and
+// leave others idle (and a pair may want all the tensor memory twice): a
+// 16x256x256 training step took 4,050 instead of 3,100 us.
+static int sole_block_smem(Ctx* ctx, long long blocks, int smem) {
+  return blocks <= ctx->num_sms ? std::max(smem, 233472 / 2) : smem;
+}
+
 template <int NG>
 static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
                         float* y32, const float* acc_in, int relu, int S, int smem, cudaStream_t st, int* rc) {
@@ -1899,8 +1937,8 @@ static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf
   const long long strips_want = std::max<long long>(1, (long long)ctx->num_sms * per_sm / G);
   const long long per_cta = (total + std::min(total, strips_want) - 1) / std::min(total, strips_want);
   const long long strips = (total + per_cta - 1) / per_cta;
-  k_conv_fwd_ws<NG><<<(unsigned)(strips * G), kWsThreads, smem, st>>>(xmap, *d, w, bias, y, y32, acc_in, relu, S, G,
-                                                                 per_cta, ctx->d_err);
+  launch_chained(st, true, dim3((unsigned)(strips * G)), kWsThreads, sole_block_smem(ctx, strips * G, smem),
+                 k_conv_fwd_ws<NG>, xmap, *d, w, bias, y, y32, acc_in, relu, S, G, per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_fwd: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
   return 1;
@@ -1948,6 +1986,8 @@ static int launch_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
 // Input channels [p * cp, (p + 1) * cp) of weights [Cout][9][Cin] as
 // contiguous [Cout][9][cp], for p = 0, 1 (16-byte chunks).
 __global__ void k_weight_halves(int Cout, int Cin, const uint4* __restrict__ w, uint4* __restrict__ out) {
+  chain_wait();
+  chain_go();
   const int cp8 = Cin / 16, c8 = Cin / 8;  // chunks per half row, per row
   const long long n = (long long)Cout * 9 * c8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -1983,8 +2023,9 @@ static int launch_ws_split(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const
     return 0;
   }
   const long long chunks = (long long)d->Cout * 9 * (d->Cin / 8);
-  k_weight_halves<<<(int)std::min<long long>((chunks + 255) / 256, (long long)ctx->num_sms * 8), 256, 0, st>>>(
-      d->Cout, d->Cin, reinterpret_cast<const uint4*>(w), static_cast<uint4*>(halves));
+  launch_chained(st, true,
+                 dim3((int)std::min<long long>((chunks + 255) / 256, (long long)ctx->num_sms * 8)), 256, 0,
+                 k_weight_halves, d->Cout, d->Cin, reinterpret_cast<const uint4*>(w), static_cast<uint4*>(halves));
   const bf16* w0 = static_cast<const bf16*>(halves);
   const bf16* w1 = w0 + (size_t)d->Cout * 9 * cp;
   rx_conv_desc d0 = *d, d1 = *d;
@@ -2020,14 +2061,16 @@ static int launch_res_as(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const b
   }
   if (best * d->N > 0x3fffffffLL || S::smem(cl) > 232448) return 0;  // opt-in shared memory per block
   auto kern = k_conv_fwd_res<BN, KS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem(cl));
+  const int smem = sole_block_smem(ctx, 0, (int)S::smem(cl));
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
   }
   const int ny = (d->Cout + BN - 1) / BN;
   const int nx = (int)std::max<long long>(1, std::min<long long>(best * d->N, ctx->num_sms / ny));
-  kern<<<dim3(nx, ny), 256, S::smem(cl), st>>>(*d, x, w, bias, y, y32, relu, cl, (int)tx, (int)ty, S::halo(cl));
+  launch_chained(st, true, dim3(nx, ny), 256, smem, kern, *d, x, w, bias, y, y32, relu, cl, (int)tx, (int)ty,
+                 S::halo(cl));
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error(ctx, "conv_bf16_fwd: %s", cudaGetErrorString(e));
@@ -2114,8 +2157,8 @@ int conv_bwd_data(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* w
   long long nw = (long long)d->Cout * 9 * d->Cin;
   // whole 16-byte chunks where the buffer allows them and 32 bits count them
   if (((uintptr_t)w_rot & 15) == 0 && nw / 8 <= 0x7fffffffLL)
-    k_rot_weights_v8<<<ew_blocks(ctx, nw / 8), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
-                                                            static_cast<bf16*>(w_rot));
+    launch_chained(st, true, dim3(ew_blocks(ctx, nw / 8)), 256, 0, k_rot_weights_v8,
+                   d->Cout, d->Cin, static_cast<const bf16*>(w), static_cast<bf16*>(w_rot));
   else
     k_rot_weights<<<ew_blocks(ctx, nw), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
                                                      static_cast<bf16*>(w_rot));
@@ -2205,7 +2248,8 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
       !row_map(d->N, d->H, d->W, d->Cout, d->y_cstride, dy + d->y_coff, A.tw, A.nc / 8, &ymap))
     return 0;
   const int G = A.mg * A.ng * A.tg;
-  k_conv_wgrad_ws<<<(unsigned)(strips * G), kWgThreads, bytes(), st>>>(xmap, ymap, A, dw, per_cta, ctx->d_err);
+  launch_chained(st, true, dim3((unsigned)(strips * G)), kWgThreads, sole_block_smem(ctx, strips * G, bytes()),
+                 k_conv_wgrad_ws, xmap, ymap, A, dw, per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_bwd_weight: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
   return 1;
@@ -2231,8 +2275,8 @@ int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void*
     const long long clusters = (P + 8LL * lanes * kBiasCluster - 1) / (8LL * lanes * kBiasCluster);
     const int blocks = kBiasCluster * (int)std::min<long long>(clusters, kBiasBlocks / kBiasCluster);
     const int bppb = (int)((P + blocks - 1) / blocks);
-    k_bias_grad<<<(unsigned)blocks, kBiasThreads, 0, st>>>(*d, static_cast<const bf16*>(dy), db,
-                                                                            bppb);
+    launch_chained(st, true, dim3((unsigned)blocks), kBiasThreads, 0, k_bias_grad, *d, static_cast<const bf16*>(dy),
+                   db, bppb);
     CUDA_TRY(ctx, cudaGetLastError());
   }
   return RX_OK;
@@ -2253,8 +2297,9 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
       break;
     case RX_DN_RELU_MASK:
       if (v8)
-        k_relu_mask_v8<<<ew_blocks(ctx, P * (o->C / 8)), 256, 0, st>>>(P, o->C, a, o->a_stride, o->a_off, b,
-                                                                      o->b_stride, o->b_off);
+        launch_chained(st, true,
+                       dim3(ew_blocks(ctx, P * (o->C / 8))), 256, 0, k_relu_mask_v8, P, o->C, a, o->a_stride,
+                       o->a_off, b, o->b_stride, o->b_off);
       else
         k_relu_mask<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(P, o->C, a, o->a_stride, o->a_off, b, o->b_stride,
                                                              o->b_off);
@@ -2262,8 +2307,9 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
     case RX_DN_POOL:
       if (o->H % 2 || o->W % 2) return set_error(ctx, "dn_op: pool needs even H and W"), RX_ERR_ARG;
       if (v8)
-        k_pool2_v8<<<ew_blocks(ctx, P / 4 * (o->C / 8)), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride,
-                                                                      o->a_off, b, o->b_stride, o->b_off);
+        launch_chained(st, true,
+                       dim3(ew_blocks(ctx, P / 4 * (o->C / 8))), 256, 0, k_pool2_v8, o->N, o->H, o->W, o->C, a,
+                       o->a_stride, o->a_off, b, o->b_stride, o->b_off);
       else
         k_pool2<<<ew_blocks(ctx, P / 4 * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
                                                              o->b_stride, o->b_off);
@@ -2271,24 +2317,27 @@ int dn_op(Ctx* ctx, const rx_dn_op* o, cudaStream_t st) {
     case RX_DN_POOL_BWD:
       if (o->H % 2 || o->W % 2) return set_error(ctx, "dn_op: pool needs even H and W"), RX_ERR_ARG;
       if (v8)
-        k_pool2_bwd_v8<<<ew_blocks(ctx, P / 4 * (o->C / 8)), 256, 0, st>>>(
-            o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b, o->b_stride, o->b_off, o->flag);
+        launch_chained(st, true,
+                       dim3(ew_blocks(ctx, P / 4 * (o->C / 8))), 256, 0, k_pool2_bwd_v8, o->N, o->H, o->W, o->C, a,
+                       o->a_stride, o->a_off, b, o->b_stride, o->b_off, o->flag);
       else
         k_pool2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
                                                              o->b_stride, o->b_off, o->flag);
       break;
     case RX_DN_UP:
       if (v8)
-        k_up2_v8<<<ew_blocks(ctx, P * (o->C / 8)), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
-                                                                o->b_stride, o->b_off);
+        launch_chained(st, true,
+                       dim3(ew_blocks(ctx, P * (o->C / 8))), 256, 0, k_up2_v8, o->N, o->H, o->W, o->C, a, o->a_stride,
+                       o->a_off, b, o->b_stride, o->b_off);
       else
         k_up2<<<ew_blocks(ctx, 4 * P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
                                                            o->b_stride, o->b_off);
       break;
     case RX_DN_UP_BWD:
       if (v8)
-        k_up2_bwd_v8<<<ew_blocks(ctx, P * (o->C / 8)), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off,
-                                                                    b, o->b_stride, o->b_off);
+        launch_chained(st, true,
+                       dim3(ew_blocks(ctx, P * (o->C / 8))), 256, 0, k_up2_bwd_v8, o->N, o->H, o->W, o->C, a,
+                       o->a_stride, o->a_off, b, o->b_stride, o->b_off);
       else
         k_up2_bwd<<<ew_blocks(ctx, P * o->C), 256, 0, st>>>(o->N, o->H, o->W, o->C, a, o->a_stride, o->a_off, b,
                                                            o->b_stride, o->b_off);
@@ -2307,8 +2356,8 @@ int dn_features(Ctx* ctx, long long P, const float* rad, const float* alb, const
                         (uintptr_t)base;
   if (P % 4 == 0 && all % 16 == 0) {
     auto f4 = [](const float* p) { return reinterpret_cast<const float4*>(p); };
-    k_features_v4<<<ew_blocks(ctx, P / 4), 256, 0, st>>>(P / 4, f4(rad), f4(alb), f4(nrm), f4(dep),
-                                                         static_cast<uint4*>(out), reinterpret_cast<float4*>(base));
+    launch_chained(st, true, dim3(ew_blocks(ctx, P / 4)), 256, 0, k_features_v4, P / 4, f4(rad), f4(alb), f4(nrm),
+                   f4(dep), static_cast<uint4*>(out), reinterpret_cast<float4*>(base));
   } else {
     k_features<<<ew_blocks(ctx, P), 256, 0, st>>>(P, rad, alb, nrm, dep, static_cast<bf16*>(out), base);
   }
@@ -2321,8 +2370,8 @@ int dn_l1_loss(Ctx* ctx, long long P, const float* y32, int y_stride, const floa
   if (P <= 0 || !y32 || !target || !grad || !loss || y_stride < 3 || grad_stride < 3)
     return set_error(ctx, "dn_l1_loss: bad arguments"), RX_ERR_ARG;
   auto kern = grad_stride % 8 == 0 && (uintptr_t)grad % 16 == 0 ? k_l1_loss<true> : k_l1_loss<false>;
-  kern<<<ew_blocks(ctx, P), 256, 0, st>>>(P, y32, y_stride, base, target, scale, static_cast<bf16*>(grad), grad_stride,
-                                          loss);
+  launch_chained(st, true, dim3(ew_blocks(ctx, P)), 256, 0, kern, P, y32, y_stride, base, target, scale,
+                 static_cast<bf16*>(grad), grad_stride, loss);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }
@@ -2330,7 +2379,7 @@ int dn_l1_loss(Ctx* ctx, long long P, const float* y32, int y_stride, const floa
 int dn_output(Ctx* ctx, long long P, const float* y32, int y_stride, const float* base, float* out,
               cudaStream_t st) {
   if (P <= 0 || !y32 || !out || y_stride < 3) return set_error(ctx, "dn_output: bad arguments"), RX_ERR_ARG;
-  k_output<<<ew_blocks(ctx, P), 256, 0, st>>>(P, y32, y_stride, base, out);
+  launch_chained(st, true, dim3(ew_blocks(ctx, P)), 256, 0, k_output, P, y32, y_stride, base, out);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }

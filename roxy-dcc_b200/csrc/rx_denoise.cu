@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kAtThreads) k_atrous_tiled(AtrousArgs A, int t
 // 71 % of the issue slots of the active cycles.  Five passes at 1280x720
 // with all guides 158 -> 88 us (pass 0 alone 35 -> 24), without guides 102
 // -> 56; 640x360 60 -> 35; 64x48 33 -> 18, where the passes' starts overlap
-// (launch_pass).
+// (launch_chained).
 template <bool GUIDES>
 struct AtRow {
   float4 c, g, a;     // own pixel: colour, normal / depth, albedo
@@ -371,10 +371,10 @@ __global__ void __launch_bounds__(kA1Warps * 32, a1_blocks(EXACT, GUIDES))
     tap(v.c.x, v.c.y, v.c.z, 1.0f);
     tap(v.rc.x, v.rc.y, v.rc.z, w_rt);
   };
-  // launched while the pass before still runs (launch_pass): wait for its
-  // results, then let the next one come
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // launched while the pass before still runs: wait for its results, then let
+  // the next one come
+  chain_wait();
+  chain_go();
   // three row buffers in turn, so that no row is moved between registers
   Row r0, r1, r2;
   load(r0, y0 - step);
@@ -445,22 +445,6 @@ static size_t atrous_smem(const AtrousArgs& A) {
   return px * sizeof(float4) * (1 + ((A.use_n || A.use_d) ? 1 : 0) + (A.use_a ? 1 : 0));
 }
 
-// One radius-1 pass; from the second on it may start its blocks before the
-// pass it follows has ended, and waits for that inside.
-template <typename... Args>
-static cudaError_t launch_pass(cudaStream_t st, bool follows, unsigned blocks, void (*kern)(Args...), Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(kA1Warps * 32);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1] = {};
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = follows ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 // Enqueues `passes` a-trous passes on `st`: pass i reads `in` (the colour for
 // i = 0) and writes scratch half (i & 1), the last pass writes `out` (and
 // reads `color` again for the blend).  A is filled except step / last.
@@ -498,8 +482,8 @@ static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, cons
       // pass 0 is the one with step 1
       auto kern = exact ? (guides ? k_atrous_r1<true, 1, true> : k_atrous_r1<true, 1, false>)
                         : (guides ? k_atrous_r1<false, 2, true> : k_atrous_r1<false, 2, false>);
-      cudaError_t e = launch_pass(st, i > 0, (unsigned)blocks, kern, A, (int)tiles_x, (int)rows, strips, in, color,
-                                  gn, ga, o);
+      cudaError_t e = launch_chained(st, i > 0, dim3((unsigned)blocks), kA1Warps * 32, 0, kern, A, (int)tiles_x,
+                                     (int)rows, strips, in, color, gn, ga, o);
       if (e != cudaSuccess) return e;
     } else if (A.r <= kAtMaxTiledR) {
       const long long sub_w = (A.W + A.step - 1) / A.step, sub_h = (A.H + A.step - 1) / A.step;

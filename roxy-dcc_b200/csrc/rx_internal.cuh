@@ -408,6 +408,14 @@ __device__ __forceinline__ float div_by(float x, float d, float r) {
   return res == 0.0f ? q : __fmaf_rn(res, r, q);
 }
 
+// A kernel launched with launch_chained may start its blocks while the kernel
+// before it in the stream still runs: everything before chain_wait must leave
+// global memory alone; chain_go lets the next kernel's blocks come (after any
+// allocation of tensor memory, so that a waiting block cannot hold what an
+// unstarted one needs).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Packed child word: >= 0 internal node index; < 0 leaf with
 // ~word = (first primitive << kLeafBits) | primitive count.
 constexpr int kLeafBits = 5;

@@ -34,6 +34,25 @@ struct Ctx {
 
 void set_error(Ctx* ctx, const char* fmt, ...);
 
+// Launch on `st`; follows: the kernel (chain_wait first) may come up while the
+// one before it in the stream drains.  Errors are also left for
+// cudaGetLastError, as by <<<>>>.
+template <typename... P, typename... Args>
+inline cudaError_t launch_chained(cudaStream_t st, bool follows, dim3 grid, unsigned block, size_t smem,
+                                  void (*kern)(P...), Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1] = {};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = follows ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // One host array and its device destination (upload) or source (download).
 struct HostPiece {
   void* dev;
