@@ -696,7 +696,7 @@ constexpr int kWsThreads = kWsEpilogue + 64 + 32;
 constexpr int kWsAcc = 4;          // accumulators
 // resident blocks per SM the registers are kept for (shared memory allows
 // more than one only for the narrow layers)
-constexpr int ws_min_blocks(int ng) { return ng <= 64 ? 2 : 1; }
+constexpr int ws_min_blocks(int ng, bool add) { return ng <= 64 && !add ? 2 : 1; }
 
 // N consecutive 32-bit tensor-memory columns of the warp's 32 lanes
 template <int N>
@@ -720,6 +720,18 @@ __device__ __forceinline__ void tmem_ld(uint32_t (&r)[N], uint32_t addr) {
 }
 
 // 32 bytes (one sector) to a 32-byte aligned address
+// CW floats from a 32-byte aligned address (not through the read-only path:
+// the kernel before wrote them)
+template <int CW>
+__device__ __forceinline__ void ld_global_floats(float (&v)[CW], const float* p) {
+#pragma unroll
+  for (int k = 0; k < CW; k += 8)
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[k]), "=f"(v[k + 1]), "=f"(v[k + 2]), "=f"(v[k + 3]), "=f"(v[k + 4]), "=f"(v[k + 5]),
+                   "=f"(v[k + 6]), "=f"(v[k + 7])
+                 : "l"(p + k));
+}
+
 __device__ __forceinline__ void st_global_32B(void* p, const uint32_t* v) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -728,8 +740,10 @@ __device__ __forceinline__ void st_global_32B(void* p, const uint32_t* v) {
 // acc_in (may be null): fp32 partial sums [pixel][Cout] of the other input
 // channels, added before the bias (a layer split over its input channels,
 // conv_fwd); y (may be null): bf16 output.
-template <int NG>
-__global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(const __grid_constant__ CUtensorMap xmap, rx_conv_desc d,
+// ADD: acc_in is there; its loads take registers for one block per SM, which
+// is all that fits beside a split layer's weights.
+template <int NG, bool ADD>
+__global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG, ADD)) k_conv_fwd_ws(const __grid_constant__ CUtensorMap xmap, rx_conv_desc d,
                                                         const bf16* __restrict__ w, const float* __restrict__ bias,
                                                         bf16* __restrict__ y, float* __restrict__ y32,
                                                         const float* __restrict__ acc_in, int relu, int S, int G,
@@ -921,6 +935,7 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
     const long long y_off = d.y_coff + grp * NG;
     // whole-sector stores when every 16-channel run of the view starts on one
     const bool y_sect = ((uintptr_t)y & 31) == 0 && d.y_cstride % 16 == 0 && d.y_coff % 16 == 0;
+    const bool f_sect = ((uintptr_t)y32 & 31) == 0 && d.y_cstride % 8 == 0 && d.y_coff % 8 == 0;
     int i = 0;
     bool ok = true;
     for (long long u = u0; u < uend && ok;) {
@@ -933,31 +948,30 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
         if ((i & 1) != eg) continue;
         const int b = i % kWsAcc;
         const uint32_t acc_t = tmem + ((uint32_t)(qtr * 32) << 16) + (uint32_t)(b * NG);
+        const long long m = ((long long)n * d.H + yy) * d.W + xx;
+        // the other half's sums (launch_ws_split) do not wait for this row's
+        float part[CW];
+        const float* part_at = acc_in + m * d.Cout + grp * NG;
+        const bool add = ADD && xx < d.W;
+        if (add) ld_global_floats(part, part_at);
         if (!mbar_wait_warp(smem_u32(&acc_full[b]), (uint32_t)((i / kWsAcc) & 1), &abort_flag)) {
           ok = false;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        const long long m = ((long long)n * d.H + yy) * d.W + xx;
 #pragma unroll 1
         for (int c0 = 0; c0 < NG; c0 += CW) {
           uint32_t r[CW];
+          if (add && c0) ld_global_floats(part, part_at + c0);
           tmem_ld(r, acc_t + (uint32_t)c0);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
           if (xx < d.W) {
             float v[CW];
 #pragma unroll
             for (int k = 0; k < CW; ++k) v[k] = __uint_as_float(r[k]);
-            if (acc_in) {
-              const float4* a4 = reinterpret_cast<const float4*>(acc_in + m * d.Cout + grp * NG + c0);
+            if (ADD) {
 #pragma unroll
-              for (int k = 0; k < CW / 4; ++k) {
-                const float4 a = a4[k];
-                v[4 * k] += a.x;
-                v[4 * k + 1] += a.y;
-                v[4 * k + 2] += a.z;
-                v[4 * k + 3] += a.w;
-              }
+              for (int k = 0; k < CW; ++k) v[k] += part[k];
             }
 #pragma unroll
             for (int k = 0; k < CW / 4; ++k) {
@@ -990,9 +1004,16 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG)) k_conv_fwd_ws(c
               }
             }
             if (y32) {
-              float4* d32 = reinterpret_cast<float4*>(y32 + o);
+              if (f_sect) {
 #pragma unroll
-              for (int k = 0; k < CW / 4; ++k) d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                for (int k = 0; k < CW / 8; ++k)
+                  st_global_32B(y32 + o + 8 * k, reinterpret_cast<const uint32_t*>(v) + 8 * k);
+              } else {
+                float4* d32 = reinterpret_cast<float4*>(y32 + o);
+#pragma unroll
+                for (int k = 0; k < CW / 4; ++k)
+                  d32[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+              }
             }
           }
         }
@@ -1907,13 +1928,13 @@ static int sole_block_smem(Ctx* ctx, long long blocks, int smem) {
   return blocks <= ctx->num_sms ? std::max(smem, 233472 / 2) : smem;
 }
 
-template <int NG>
+template <int NG, bool ADD>
 static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
                         float* y32, const float* acc_in, int relu, int S, int smem, cudaStream_t st, int* rc) {
   const int limit = 232448 - 1024;  // opt-in shared memory per block, less the static part
   static int attr_dev = -1;
   if (attr_dev != ctx->device) {
-    if (cudaFuncSetAttribute(k_conv_fwd_ws<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_conv_fwd_ws<NG, ADD>, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
       cudaGetLastError();
       return 0;
     }
@@ -1926,19 +1947,19 @@ static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf
   // that every resident CTA gets its tensor memory
   cudaFuncAttributes fa{};
   int smem_sm = 0, reserved = 0;
-  cudaFuncGetAttributes(&fa, k_conv_fwd_ws<NG>);
+  cudaFuncGetAttributes(&fa, k_conv_fwd_ws<NG, ADD>);
   cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, ctx->device);
   cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, ctx->device);
   constexpr int tcols = kWsAcc * NG;
   int per_sm = smem_sm / (smem + (int)fa.sharedSizeBytes + reserved);
-  per_sm = std::max(1, std::min(std::min(per_sm, 512 / tcols), ws_min_blocks(NG)));
+  per_sm = std::max(1, std::min(std::min(per_sm, 512 / tcols), ws_min_blocks(NG, ADD)));
   const int G = d->Cout / NG;
   const long long total = (long long)d->N * d->H * ((d->W + tc::TILE - 1) / tc::TILE);
   const long long strips_want = std::max<long long>(1, (long long)ctx->num_sms * per_sm / G);
   const long long per_cta = (total + std::min(total, strips_want) - 1) / std::min(total, strips_want);
   const long long strips = (total + per_cta - 1) / per_cta;
   launch_chained(st, true, dim3((unsigned)(strips * G)), kWsThreads, sole_block_smem(ctx, strips * G, smem),
-                 k_conv_fwd_ws<NG>, xmap, *d, w, bias, y, y32, acc_in, relu, S, G, per_cta, ctx->d_err);
+                 k_conv_fwd_ws<NG, ADD>, xmap, *d, w, bias, y, y32, acc_in, relu, S, G, per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_fwd: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
   return 1;
@@ -1975,10 +1996,18 @@ static int launch_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
   int S = 0, smem = 0;
   const int NG = ws_group(d->Cin, d->Cout, &S, &smem);
   switch (NG) {
-    case 128: return launch_ws_ng<128>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc);
-    case 64: return launch_ws_ng<64>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc);
-    case 32: return launch_ws_ng<32>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc);
-    case 16: return launch_ws_ng<16>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc);
+    case 128:
+      return acc_in ? launch_ws_ng<128, true>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc)
+                    : launch_ws_ng<128, false>(ctx, d, x, w, bias, y, y32, nullptr, relu, S, smem, st, rc);
+    case 64:
+      return acc_in ? launch_ws_ng<64, true>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc)
+                    : launch_ws_ng<64, false>(ctx, d, x, w, bias, y, y32, nullptr, relu, S, smem, st, rc);
+    case 32:
+      return acc_in ? launch_ws_ng<32, true>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc)
+                    : launch_ws_ng<32, false>(ctx, d, x, w, bias, y, y32, nullptr, relu, S, smem, st, rc);
+    case 16:
+      return acc_in ? launch_ws_ng<16, true>(ctx, d, x, w, bias, y, y32, acc_in, relu, S, smem, st, rc)
+                    : launch_ws_ng<16, false>(ctx, d, x, w, bias, y, y32, nullptr, relu, S, smem, st, rc);
     default: return 0;
   }
 }
