@@ -914,12 +914,12 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG, ADD)) k_conv_fwd
   } else {
     // ------------------------------------------------ epilogue (warps 0-7)
     // this group's weights first, while the producers fetch the first rows:
-    // chunk ((co * 9 + tap) * KC + kc) -> [tap][kc][co][8]
+    // [co][tap][kc] -> [tap][kc][co][8], neighbouring threads on neighbouring
+    // channels: 16-byte pieces side by side in shared memory (along kc they
+    // would all meet in the same banks)
     for (int c = tid; c < NG * 9 * KC; c += kWsEpilogue) {
-      const int kc = c % KC, ct = c / KC;
-      const int tap = ct % 9, co = ct / 9;
-      const bf16* src = w + ((long long)(grp * NG + co) * 9 + tap) * d.Cin + kc * 8;
-      cp_async16(wsm + ((tap * KC + kc) * NG + co) * 16, src, true);
+      const int co = c % NG, tk = c / NG;  // tk = tap * KC + kc: also the source's order
+      cp_async16(wsm + c * 16, w + (long long)(grp * NG + co) * 9 * d.Cin + tk * 8, true);
     }
     cp_async_commit();
     cp_async_wait<0>();
