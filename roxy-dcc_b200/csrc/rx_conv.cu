@@ -1158,8 +1158,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
   } else if (warp >= 4) {
     // ------------------------------------------------ MMA issuers
     if (elect_one()) {
-      // M = 128, N = nc, FP32 accumulate, BF16, both operands MN-major
-      const uint32_t id = tc::idesc(0) | (1u << 15) | (1u << 16) | ((uint32_t)(A.nc >> 3) << 17);
+      // M = 64 (up to 64 channels) or 128, N = nc, FP32 accumulate, BF16, both
+      // operands MN-major
+      const uint32_t id = tc::idesc(0) - (A.cm <= 64 ? 4u << 24 : 0u) + (1u << 15) + (1u << 16) +
+                          ((uint32_t)(A.nc >> 3) << 17);
       // MN-major, no swizzle: LBO (next 8 pixels) 128 B, SBO (next 8
       // channels) one plane
       const uint64_t a_hi = (uint64_t)((uint32_t)(A.tw + 2) | (1u << 14)) << 32;
@@ -1250,8 +1252,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   if (warp < 4 && !abort_flag && u0 < uend) {
-    const int ci = ci0 + warp * 32 + lane;
-    const bool mine = warp * 32 + lane < A.cm && ci < A.Cin;
+    // an M = 64 accumulator has 16 rows in each quarter of the lanes
+    const int rows = A.cm <= 64 ? 16 : 32, ci = ci0 + warp * rows + lane;
+    const bool mine = lane < rows && warp * rows + lane < A.cm && ci < A.Cin;
     for (int j = 0; j < ntap; ++j)
       for (int c = 0; c < A.nc; c += 16) {
         uint32_t r[16];
@@ -2246,14 +2249,17 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   const long long strips = (total + per_cta - 1) / per_cta;
   // Blocks beyond the strips come from splitting the input channels and the
   // taps; both read rows again.  The cheapest split by the cycles of a row
-  // (MMAs: about 40 each up to N = 32, N / 2 above; TMA: 16 B per cycle),
-  // the rows of a block and the rounds of blocks.
-  const int mg_min = (d->Cin + 127) / 128, mma = A.nc <= 32 ? 40 : A.nc == 64 ? 48 : 64;
+  // (MMAs: about 40 each up to N = 32, N / 2 above, and 28 and 44 for N = 32
+  // and 64 with M = 64, half the channels to read; TMA: 16 B per cycle), the
+  // rows of a block and the rounds of blocks.  M = 64 for up to 64 channels
+  // took the eleven layers of a 16x128x128 step from 346 to 296 us.
+  const int mg_min = (d->Cin + 127) / 128;
   double best = 0.0;
   for (int mg = mg_min; mg <= 4 * mg_min && (mg == mg_min || d->Cin / mg >= 16); ++mg)
     for (int tg = 1; tg <= 9; ++tg) {
       const int taps = (9 + tg - 1) / tg, cm = (d->Cin / 8 + mg - 1) / mg * 8;
       if (taps * A.nc > 512 || (tg - 1) * taps >= 9) continue;
+      const int mma = A.nc > 64 ? 64 : cm <= 64 ? (A.nc <= 32 ? 28 : 44) : (A.nc <= 32 ? 40 : 48);
       const double row = std::max<double>(taps * (A.tw / 16) * mma, (double)((A.tw + 2) * cm + A.tw * A.nc) * 2 / 16);
       const long long rounds = (strips * mg * A.ng * tg + ctx->num_sms - 1) / ctx->num_sms;
       const double cost = (double)rounds * ((double)per_cta * row + 8000.0);  // 8,000: a block's start and end
