@@ -72,6 +72,8 @@ __global__ void k_prim_bounds(int n_tris, const float* __restrict__ v0, const fl
 // Two-stage exact min/max reduction of the centroids.
 __global__ void k_reduce_bounds(int n, const float3* __restrict__ p, float3* __restrict__ part_min,
                                 float3* __restrict__ part_max) {
+  chain_wait();
+  chain_go();
   __shared__ float smin[3][256], smax[3][256];
   float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -105,6 +107,8 @@ constexpr int kBoundsThreads = 1024;
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds_final(int parts, const float3* __restrict__ mins,
                                                                  const float3* __restrict__ maxs,
                                                                  float3* __restrict__ out) {
+  chain_wait();
+  chain_go();
   __shared__ float3 slo[kBoundsThreads], shi[kBoundsThreads];
   float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
   for (int k = threadIdx.x; k < parts; k += kBoundsThreads) {
@@ -145,6 +149,8 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
 // `bounds`: the centroid bounds (k_bounds_final).
 __global__ void k_morton(int n, const float3* __restrict__ cen, const float3* __restrict__ bounds, int cubic,
                          uint32_t* __restrict__ codes, int* __restrict__ idx) {
+  chain_wait();
+  chain_go();
   __shared__ float3 s_lo, s_ext;
   if (threadIdx.x == 0) {
     const float3 lo = bounds[0], hi = bounds[1];
@@ -185,6 +191,8 @@ __host__ __device__ constexpr int sort_tile(int chunks) { return kSortWarps * ch
 
 __global__ void k_sort_hist(int n, const uint32_t* __restrict__ keys, int shift, int tile, uint32_t* __restrict__ hist,
                             int nblocks) {
+  chain_wait();
+  chain_go();
   __shared__ uint32_t h[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
   __syncthreads();
@@ -224,6 +232,8 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* wa
 // took 21 us per pass at 80 blocks; a row each takes 3.)
 __global__ void __launch_bounds__(256) k_sort_rows(uint32_t* __restrict__ hist, uint32_t* __restrict__ totals,
                                                    int nblocks) {
+  chain_wait();
+  chain_go();
   __shared__ uint32_t warp_sums[8];
   uint32_t* row = hist + (size_t)blockIdx.x * nblocks;
   uint32_t carry = 0;
@@ -243,6 +253,8 @@ __global__ void __launch_bounds__(kSortWarps * 32)
     k_sort_scatter(int n, const uint32_t* __restrict__ keys_in, const int* __restrict__ vals_in,
                    uint32_t* __restrict__ keys_out, int* __restrict__ vals_out, int shift,
                    const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, int nblocks) {
+  chain_wait();
+  chain_go();
   static_assert(kSortWarps * 32 == 256, "one thread per digit");
   __shared__ uint32_t wcount[kSortWarps][256];
   __shared__ uint32_t warp_sums[8];
@@ -316,10 +328,11 @@ static int radix_sort(Ctx* ctx, int n, uint32_t* keys, int* vals, int bits) {
   int passes = (bits + 7) / 8;
   for (int p = 0; p < passes; ++p) {
     int shift = 8 * p;
-    k_sort_hist<<<nblocks, 256, 0, st>>>(n, ka, shift, tile, hist.p, nblocks);
-    k_sort_rows<<<256, 256, 0, st>>>(hist.p, totals.p, nblocks);
+    launch_chained(st, true, dim3(nblocks), 256, 0, k_sort_hist, n, ka, shift, tile, hist.p, nblocks);
+    launch_chained(st, true, dim3(256), 256, 0, k_sort_rows, hist.p, totals.p, nblocks);
     auto scatter = chunks == 4 ? k_sort_scatter<4> : k_sort_scatter<16>;
-    scatter<<<nblocks, kSortWarps * 32, 0, st>>>(n, ka, va, kb, vb, shift, hist.p, totals.p, nblocks);
+    launch_chained(st, true, dim3(nblocks), kSortWarps * 32, 0, scatter, n, ka, va, kb, vb, shift, hist.p, totals.p,
+                   nblocks);
     std::swap(ka, kb);
     std::swap(va, vb);
   }
@@ -463,6 +476,8 @@ __global__ void k_gather_prims(int n, const int* __restrict__ order, int n_tris,
                                const float4* __restrict__ obj_a, const float4* __restrict__ obj_b,
                                const int* __restrict__ obj_mat, const int* __restrict__ obj_slot,
                                float4* __restrict__ prims, float4* __restrict__ shade) {
+  chain_wait();
+  chain_go();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     int i = order[k];
     float4* P = prims + kPrimQuads * (size_t)k;
@@ -505,9 +520,13 @@ __device__ __forceinline__ int left_child(int lo, int gamma) { return lo == gamm
 __device__ __forceinline__ int right_child(int hi, int gamma) { return hi == gamma + 1 ? ~(gamma + 1) : gamma + 1; }
 
 // Internal node i of n - 1 covers the sorted positions [lo, hi], split after
-// gamma: record (lo, hi, gamma, -).
+// gamma: record (lo, hi, gamma, -).  Also clears the bottom-up flags and the
+// mask counts of the passes that follow.
 __global__ void k_karras(int n, const uint32_t* __restrict__ codes, int4* __restrict__ range,
-                         int* __restrict__ parent_int, int* __restrict__ parent_leaf) {
+                         int* __restrict__ parent_int, int* __restrict__ parent_leaf, int* __restrict__ flags,
+                         int* __restrict__ counts, int n_counts) {
+  chain_wait();
+  chain_go();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
     int d = (lcp(codes, n, i, i + 1) - lcp(codes, n, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = lcp(codes, n, i, i - d);
@@ -527,6 +546,9 @@ __global__ void k_karras(int n, const uint32_t* __restrict__ codes, int4* __rest
     int gamma = i + s * d + min(d, 0);
     int lo = min(i, j), hi = max(i, j);
     range[i] = make_int4(lo, hi, gamma, 0);
+    flags[i] = 0;
+    if (i < n_counts) counts[i] = 0;
+    if (i == 0) parent_int[0] = -1;  // the root; every other node has a parent that writes it
     const int lc = left_child(lo, gamma), rc = right_child(hi, gamma);
     if (lc >= 0) parent_int[lc] = i; else parent_leaf[~lc] = i;
     if (rc >= 0) parent_int[rc] = i; else parent_leaf[~rc] = i;
@@ -550,6 +572,23 @@ __device__ __forceinline__ float half_area(float3 lo, float3 hi) {
 // atomics; that chain of ~2 us per level was the pass's time.
 constexpr int kUpLeaves = 512;
 
+// Adds 1 to a node's counter; what the other thread wrote before its own call
+// is visible to the second caller.  (An atomicAdd between two __threadfence,
+// which order more: 76 us for the pass, 69 with this.)
+__device__ __forceinline__ int arrive(int* flag) {
+  int old;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(flag) : "memory");
+  return old;
+}
+__device__ __forceinline__ int arrive_shared(int* flag) {
+  int old;
+  asm volatile("atom.acq_rel.cta.shared.add.s32 %0, [%1], 1;"
+               : "=r"(old)
+               : "r"((uint32_t)__cvta_generic_to_shared(flag))
+               : "memory");
+  return old;
+}
+
 struct UpBox {
   float3 lo, hi;
   float cost;
@@ -565,6 +604,8 @@ __global__ void __launch_bounds__(kUpLeaves)
                      const int* __restrict__ parent_int, const int* __restrict__ parent_leaf,
                      const float3* __restrict__ pmin, const float3* __restrict__ pmax, float4* __restrict__ rec,
                      int* __restrict__ flags, int max_leaf, float c_t, float c_i) {
+  chain_wait();
+  chain_go();
   __shared__ float4 s_a[kUpLeaves], s_b[kUpLeaves];  // records of this block's nodes, by node - base
   __shared__ float3 s_lo[kUpLeaves], s_hi[kUpLeaves];
   __shared__ int4 s_range[kUpLeaves];  // (lo, hi, gamma, parent)
@@ -605,9 +646,7 @@ __global__ void __launch_bounds__(kUpLeaves)
   };
   int4 q = node_range(node);
   while (q.x >= base && q.y < end) {
-    __threadfence_block();
-    if (atomicAdd(&s_flag[node - base], 1) == 0) return;
-    __threadfence_block();
+    if (arrive_shared(&s_flag[node - base]) == 0) return;
     auto child = [&](int c) {
       if (c < 0) return UpBox{s_lo[~c - base], s_hi[~c - base], c_i, 0};
       return up_box(s_a[c - base], s_b[c - base]);
@@ -623,10 +662,8 @@ __global__ void __launch_bounds__(kUpLeaves)
     q = node_range(node);
   }
   while (true) {
-    __threadfence();
-    if (atomicAdd(&flags[node], 1) == 0) return;
+    if (arrive(flags + node) == 0) return;
     const int4 up = q.w < 0 ? q : node_range(q.w);  // in flight with the children's records
-    __threadfence();
     auto child = [&](int c) {
       if (c >= 0) return up_box(__ldcg(rec + 2 * (size_t)c), __ldcg(rec + 2 * (size_t)c + 1));
       const int p = order[~c];
@@ -665,13 +702,16 @@ struct NodeMask {
 };
 
 // One block per kRankWords words; the last one writes *total.
-__global__ void __launch_bounds__(kRankWords) k_rank(NodeMask m, int* __restrict__ total) {
+__global__ void __launch_bounds__(kRankWords) k_rank(NodeMask m, int n, int* __restrict__ total) {
+  chain_wait();
+  chain_go();
   __shared__ uint32_t warp_sums[8];
   uint32_t before = 0, part = 0, here = 0;
   for (int b = threadIdx.x; b < (int)blockIdx.x; b += kRankWords) part += m.counts[b];
   block_exclusive_256(part, warp_sums, &before);
   const int w = blockIdx.x * kRankWords + threadIdx.x;
-  const uint32_t e = block_exclusive_256(__popc(m.mask[w]), warp_sums, &here);
+  // words beyond the last node are never written
+  const uint32_t e = block_exclusive_256(w * 32LL < n ? __popc(m.mask[w]) : 0, warp_sums, &here);
   m.rank[w] = (int)(before + e);
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = (int)(before + here);
 }
@@ -688,6 +728,8 @@ __device__ __forceinline__ int rec_height(const float4* rec, int node) {
 __global__ void __launch_bounds__(256)
     k_lbvh_keep(int n_int, const int4* __restrict__ range, const int* __restrict__ parent_int,
                 const float4* __restrict__ rec, int max_leaf, NodeMask m, int* __restrict__ levels) {
+  chain_wait();
+  chain_go();
   const int i = blockIdx.x * 256 + threadIdx.x;
   bool keep = i < n_int && rec_height(rec, i) > 0;
   for (int p = i; keep;) {
@@ -706,6 +748,8 @@ __global__ void k_lbvh_layout(int n_int, const int4* __restrict__ range, const i
                               const float3* __restrict__ pmin, const float3* __restrict__ pmax,
                               const float4* __restrict__ rec, NodeMask m, float4* __restrict__ out,
                               int* __restrict__ at_lo) {
+  chain_wait();
+  chain_go();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_int; i += gridDim.x * blockDim.x) {
     if (!m.has(i)) continue;
     const int4 q = range[i];
@@ -849,11 +893,15 @@ __device__ __forceinline__ void wide_open(WideNode& v, const float4* __restrict_
 }
 
 // kids[2b]: the internal children of b's 4-wide node (-1: none), kids[2b + 1]:
-// the first sorted position under each.
+// the first sorted position under each.  Also clears the mask counts.
 __global__ void __launch_bounds__(128) k_wide_kids(const float4* __restrict__ bin, int n_bin,
-                                                   const int* __restrict__ at_lo, int4* __restrict__ kids, int* err) {
+                                                   const int* __restrict__ at_lo, int4* __restrict__ kids,
+                                                   int* __restrict__ counts, int n_counts, int* err) {
+  chain_wait();
+  chain_go();
   const int b = blockIdx.x * 128 + threadIdx.x;
   if (b >= n_bin) return;
+  if (b < n_counts) counts[b] = 0;
   WideNode v;
   wide_open(v, bin, n_bin, b, err);
   int id[4], lo[4];
@@ -873,6 +921,8 @@ __global__ void __launch_bounds__(128) k_wide_kids(const float4* __restrict__ bi
 // below it.
 __global__ void __launch_bounds__(256) k_wide_roots(int n_bin, const int4* __restrict__ kids,
                                                     const int* __restrict__ at_lo, NodeMask m) {
+  chain_wait();
+  chain_go();
   const int b = blockIdx.x * 256 + threadIdx.x;
   int cur = b < n_bin ? 0 : -1;
   const int p = b < n_bin ? at_lo[b] : 0;
@@ -890,6 +940,8 @@ __global__ void __launch_bounds__(256) k_wide_roots(int n_bin, const int4* __res
 
 __global__ void __launch_bounds__(128) k_wide_write(const float4* __restrict__ bin, int n_bin, NodeMask m,
                                                     float4* __restrict__ out4, int* err) {
+  chain_wait();
+  chain_go();
   const int b = blockIdx.x * 128 + threadIdx.x;
   if (b >= n_bin || !m.has(b)) return;
   WideNode v;
@@ -917,7 +969,8 @@ __global__ void k_single_leaf_root(const float3* __restrict__ bmin, const float3
   out[0] = make_float4(l0.x, l1.x, l0.y, l1.y);
   out[1] = make_float4(l0.z, l1.z, r0.x, r0.x);
   out[2] = make_float4(r0.y, r0.y, r0.z, r0.z);
-  out[3] = make_float4(__int_as_float(pack_leaf(0, cnt)), __int_as_float(pack_leaf(0, 0)), __int_as_float(cnt), __int_as_float(0));
+  out[3] = make_float4(__int_as_float(pack_leaf(0, cnt)), __int_as_float(pack_leaf(0, 0)), __int_as_float(cnt),
+  __int_as_float(0));
 }
 
 static int grid_for(Ctx* ctx, long long n, int block = 256) {
@@ -944,9 +997,9 @@ static int front_end(Ctx* ctx, Scene* sc, int n_obj, const float4* d_obj_a, cons
     return set_error(ctx, "BVH build: out of device memory"), RX_ERR_CAPACITY;
   k_prim_bounds<<<grid_for(ctx, n), 256, 0, st>>>(sc->n_tris, sc->d_v0, sc->d_v1, sc->d_v2, n_obj, d_obj_a, d_obj_b,
                                                    lbvh_keys, pmin.p, pmax.p, cen.p);
-  k_reduce_bounds<<<parts, 256, 0, st>>>(n, cen.p, part_min.p, part_max.p);
-  k_bounds_final<<<1, kBoundsThreads, 0, st>>>(parts, part_min.p, part_max.p, cbox.p);
-  k_morton<<<grid_for(ctx, n), 256, 0, st>>>(n, cen.p, cbox.p, lbvh_keys, codes.p, order.p);
+  launch_chained(st, true, dim3(parts), 256, 0, k_reduce_bounds, n, cen.p, part_min.p, part_max.p);
+  launch_chained(st, true, dim3(1), kBoundsThreads, 0, k_bounds_final, parts, part_min.p, part_max.p, cbox.p);
+  launch_chained(st, true, dim3(grid_for(ctx, n)), 256, 0, k_morton, n, cen.p, cbox.p, lbvh_keys, codes.p, order.p);
   if (int rc = radix_sort(ctx, n, codes.p, order.p, 30)) return rc;
   sc->tmp_codes.swap(codes);
   return RX_OK;
@@ -999,9 +1052,9 @@ int build_reference(Ctx* ctx, Scene* sc, int leaf) {
   }
   k_ref_to_layout<<<grid_for(ctx, n_nodes), 256, 0, st>>>(n_nodes, left.p, right.p, tstart.p, tcount.p, nmin.p,
                                                            nmax.p, sc->d_nodes.p);
-  k_gather_prims<<<grid_for(ctx, n), 256, 0, st>>>(n, order.p, sc->n_tris, sc->d_v0, sc->d_v1, sc->d_v2, sc->d_n0,
-                                                    sc->d_n1, sc->d_n2, sc->d_tri_mat, nullptr, nullptr, nullptr, nullptr,
-                                                    sc->d_prims.p, sc->d_shade.p);
+  launch_chained(st, true, dim3(grid_for(ctx, n)), 256, 0, k_gather_prims, n, order.p, sc->n_tris, sc->d_v0, sc->d_v1,
+                 sc->d_v2, sc->d_n0, sc->d_n1, sc->d_n2, sc->d_tri_mat, nullptr, nullptr, nullptr, nullptr,
+                 sc->d_prims.p, sc->d_shade.p);
   float3 rb[2];
   cudaMemcpyAsync(&rb[0], nmin.p, sizeof(float3), cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(&rb[1], nmax.p, sizeof(float3), cudaMemcpyDeviceToHost, st);
@@ -1050,9 +1103,9 @@ int set_reference_nodes(Ctx* ctx, Scene* sc, int n_nodes, const float* node_min,
   cudaMemcpyAsync(ord.p, order, sizeof(int) * n, cudaMemcpyHostToDevice, st);
   k_ref_to_layout<<<grid_for(ctx, n_nodes), 256, 0, st>>>(n_nodes, l.p, r.p, s.p, c.p, nmin.p, nmax.p,
                                                            sc->d_nodes.p);
-  k_gather_prims<<<grid_for(ctx, n), 256, 0, st>>>(n, ord.p, sc->n_tris, sc->d_v0, sc->d_v1, sc->d_v2, sc->d_n0,
-                                                    sc->d_n1, sc->d_n2, sc->d_tri_mat, nullptr, nullptr, nullptr, nullptr,
-                                                    sc->d_prims.p, sc->d_shade.p);
+  launch_chained(st, true, dim3(grid_for(ctx, n)), 256, 0, k_gather_prims, n, ord.p, sc->n_tris, sc->d_v0, sc->d_v1,
+                 sc->d_v2, sc->d_n0, sc->d_n1, sc->d_n2, sc->d_tri_mat, nullptr, nullptr, nullptr, nullptr,
+                 sc->d_prims.p, sc->d_shade.p);
   sc->ref_left.swap(l);
   sc->ref_right.swap(r);
   sc->ref_start.swap(s);
@@ -1072,7 +1125,7 @@ int set_reference_nodes(Ctx* ctx, Scene* sc, int n_nodes, const float* node_min,
   return RX_OK;
 }
 
-// Mask, ranks and counts for n nodes, the counts cleared on the stream.
+// Mask, ranks and counts for n nodes.
 struct MaskBuf {
   int blocks;
   DevBuf<uint32_t> mask;
@@ -1082,11 +1135,6 @@ struct MaskBuf {
         mask(ctx, (size_t)blocks * kRankWords),
         rank(ctx, (size_t)blocks * kRankWords),
         counts(ctx, blocks) {}
-  cudaError_t clear(cudaStream_t st) {
-    // words beyond the last marked node are never written: they must be zero
-    cudaError_t e = cudaMemsetAsync(mask.p, 0, sizeof(uint32_t) * (size_t)blocks * kRankWords, st);
-    return e != cudaSuccess ? e : cudaMemsetAsync(counts.p, 0, sizeof(int) * (size_t)blocks, st);
-  }
   NodeMask view() const { return {mask.p, rank.p, counts.p}; }
 };
 
@@ -1097,16 +1145,18 @@ static int build_wide(Ctx* ctx, Scene* sc, const int* at_lo) {
   const int nb = sc->n_nodes;
   sc->n_nodes4 = 0;
   if (nb <= 0) return RX_OK;
-  if (!sc->d_nodes4.alloc(ctx, (size_t)8 * nb)) return set_error(ctx, "out of device memory for the 4-wide BVH"), RX_ERR_CAPACITY;
+  if (!sc->d_nodes4.alloc(ctx, (size_t)8 * nb)) return set_error(ctx, "out of device memory for the 4-wide BVH"),
+  RX_ERR_CAPACITY;
   MaskBuf m(ctx, nb);
   DevBuf<int4> kids(ctx, (size_t)2 * nb);
   DevBuf<int> total(ctx, 1);
   if (!all_ok(m.mask, m.rank, m.counts, kids, total)) return set_error(ctx, "out of device memory"), RX_ERR_CAPACITY;
-  CUDA_TRY(ctx, m.clear(st));
-  k_wide_kids<<<(nb + 127) / 128, 128, 0, st>>>(sc->d_nodes.p, nb, at_lo, kids.p, ctx->d_err);
-  k_wide_roots<<<(nb + 255) / 256, 256, 0, st>>>(nb, kids.p, at_lo, m.view());
-  k_rank<<<m.blocks, kRankWords, 0, st>>>(m.view(), total.p);
-  k_wide_write<<<(nb + 127) / 128, 128, 0, st>>>(sc->d_nodes.p, nb, m.view(), sc->d_nodes4.p, ctx->d_err);
+  launch_chained(st, true, dim3((nb + 127) / 128), 128, 0, k_wide_kids, sc->d_nodes.p, nb, at_lo, kids.p, m.counts.p,
+                 m.blocks, ctx->d_err);
+  launch_chained(st, true, dim3((nb + 255) / 256), 256, 0, k_wide_roots, nb, kids.p, at_lo, m.view());
+  launch_chained(st, true, dim3(m.blocks), kRankWords, 0, k_rank, m.view(), nb, total.p);
+  launch_chained(st, true, dim3((nb + 127) / 128), 128, 0, k_wide_write, sc->d_nodes.p, nb, m.view(), sc->d_nodes4.p,
+                 ctx->d_err);
   CUDA_TRY(ctx, cudaGetLastError());
   int n4 = 0;
   CUDA_TRY(ctx, cudaMemcpyAsync(&n4, total.p, sizeof(n4), cudaMemcpyDeviceToHost, st));
@@ -1158,28 +1208,14 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
   if (int rc = front_end(ctx, sc, n_obj, d_oa.p, d_ob.p, 1, pmin, pmax, order)) return rc;
   sc->d_prims.alloc(ctx, (size_t)kPrimQuads * n);
   sc->d_shade.alloc(ctx, (size_t)3 * n);
-  DevBuf<float3> rb(ctx, 2);
-  if (!all_ok(sc->d_prims, sc->d_shade, rb)) {
+  if (!all_ok(sc->d_prims, sc->d_shade)) {
     sc->clear_bvh();
     return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
   }
-  k_gather_prims<<<grid_for(ctx, n), 256, 0, st>>>(n, order.p, sc->n_tris, sc->d_v0, sc->d_v1, sc->d_v2, sc->d_n0,
-                                                    sc->d_n1, sc->d_n2, sc->d_tri_mat, d_oa.p, d_ob.p, d_obj_mat.p,
-                                                    d_obj_slot.p, sc->d_prims.p, sc->d_shade.p);
-  {
-    // root box = union of all primitive boxes (two-stage parallel reduction)
-    int parts = std::min(grid_for(ctx, n), 1024);
-    DevBuf<float3> lo_min(ctx, parts), lo_max(ctx, parts), hi_min(ctx, parts), hi_max(ctx, parts);
-    if (!all_ok(lo_min, lo_max, hi_min, hi_max)) {
-      sc->clear_bvh();
-      return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
-    }
-    k_reduce_bounds<<<parts, 256, 0, st>>>(n, pmin.p, lo_min.p, lo_max.p);
-    k_reduce_bounds<<<parts, 256, 0, st>>>(n, pmax.p, hi_min.p, hi_max.p);
-    k_bounds_final<<<1, kBoundsThreads, 0, st>>>(parts, lo_min.p, hi_max.p, rb.p);
-  }
-  float3 hb[2];
-  cudaMemcpyAsync(hb, rb.p, sizeof(hb), cudaMemcpyDeviceToHost, st);
+  launch_chained(st, true, dim3(grid_for(ctx, n)), 256, 0, k_gather_prims, n, order.p, sc->n_tris, sc->d_v0, sc->d_v1,
+                 sc->d_v2, sc->d_n0, sc->d_n1, sc->d_n2, sc->d_tri_mat, d_oa.p, d_ob.p, d_obj_mat.p, d_obj_slot.p,
+                 sc->d_prims.p, sc->d_shade.p);
+  float4 hb[2];  // the root's box: the union of all primitives'
   int n_int = n - 1;
   DevBuf<int> at_lo;  // first sorted position under each laid-out node
   if (n == 1) {
@@ -1187,7 +1223,9 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
       sc->clear_bvh();
       return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
     }
-    k_single_leaf_root<<<1, 1, 0, st>>>(rb.p, rb.p + 1, 1, sc->d_nodes.p);
+    k_single_leaf_root<<<1, 1, 0, st>>>(pmin.p, pmax.p, 1, sc->d_nodes.p);
+    CUDA_TRY(ctx, cudaMemcpyAsync(&hb[0], pmin.p, sizeof(float3), cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(ctx, cudaMemcpyAsync(&hb[1], pmax.p, sizeof(float3), cudaMemcpyDeviceToHost, st));
     sc->n_nodes = 1;
   } else {
     DevBuf<int4> range(ctx, n_int);
@@ -1201,24 +1239,25 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
       sc->clear_bvh();
       return set_error(ctx, "LBVH: out of device memory"), RX_ERR_CAPACITY;
     }
-    cudaMemsetAsync(par_int.p, 0xff, sizeof(int) * n_int, st);
-    k_karras<<<grid_for(ctx, n_int), 256, 0, st>>>(n, sc->tmp_codes.p, range.p, par_int.p, par_leaf.p);
-    cudaMemsetAsync(flags.p, 0, sizeof(int) * n_int, st);
-    k_lbvh_bottom_up<<<(n + kUpLeaves - 1) / kUpLeaves, kUpLeaves, 0, st>>>(
-        n, order.p, range.p, par_int.p, par_leaf.p, pmin.p, pmax.p, rec.p, flags.p, max_leaf, c_t, c_i);
-    CUDA_TRY(ctx, m.clear(st));
-    k_lbvh_keep<<<(n_int + 255) / 256, 256, 0, st>>>(n_int, range.p, par_int.p, rec.p, max_leaf, m.view(), info.p + 1);
-    k_rank<<<m.blocks, kRankWords, 0, st>>>(m.view(), info.p);
-    k_lbvh_layout<<<grid_for(ctx, n_int), 256, 0, st>>>(n_int, range.p, order.p, pmin.p, pmax.p, rec.p, m.view(),
-                                                         sc->d_nodes.p, at_lo.p);
+    launch_chained(st, true, dim3(grid_for(ctx, n_int)), 256, 0, k_karras, n, sc->tmp_codes.p, range.p, par_int.p,
+                   par_leaf.p, flags.p, m.counts.p, m.blocks);
+    launch_chained(st, true, dim3((n + kUpLeaves - 1) / kUpLeaves), kUpLeaves, 0, k_lbvh_bottom_up, n, order.p, range.p,
+                   par_int.p, par_leaf.p, pmin.p, pmax.p, rec.p, flags.p, max_leaf, c_t, c_i);
+    launch_chained(st, true, dim3((n_int + 255) / 256), 256, 0, k_lbvh_keep, n_int, range.p, par_int.p, rec.p,
+                     max_leaf, m.view(), info.p + 1);
+    launch_chained(st, true, dim3(m.blocks), kRankWords, 0, k_rank, m.view(), n_int, info.p);
+    launch_chained(st, true, dim3(grid_for(ctx, n_int)), 256, 0, k_lbvh_layout, n_int, range.p, order.p, pmin.p, pmax.p,
+                   rec.p, m.view(), sc->d_nodes.p, at_lo.p);
     CUDA_TRY(ctx, cudaGetLastError());
     int h_info[2] = {0, 0};
+    CUDA_TRY(ctx, cudaMemcpyAsync(hb, rec.p, sizeof(hb), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(ctx, cudaMemcpyAsync(h_info, info.p, sizeof(h_info), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(ctx, cudaStreamSynchronize(st));
     sc->n_nodes = h_info[0];
     sc->depth = h_info[1];
     if (sc->n_nodes == 0) {  // the whole tree is one leaf
-      k_single_leaf_root<<<1, 1, 0, st>>>(rb.p, rb.p + 1, n, sc->d_nodes.p);
+      k_single_leaf_root<<<1, 1, 0, st>>>(reinterpret_cast<const float3*>(rec.p),
+                                          reinterpret_cast<const float3*>(rec.p + 1), n, sc->d_nodes.p);
       sc->n_nodes = 1;
     }
   }
@@ -1228,8 +1267,8 @@ int build_lbvh(Ctx* ctx, Scene* sc, int max_leaf, int spheres_in_bvh, float c_t,
     sc->clear_bvh();
     return rc;
   }
-  sc->root_min = hb[0];
-  sc->root_max = hb[1];
+  sc->root_min = f3(hb[0].x, hb[0].y, hb[0].z);
+  sc->root_max = f3(hb[1].x, hb[1].y, hb[1].z);
   sc->n_prims = n;
   sc->n_bvh_spheres = n_obj;
   sc->method = RX_BVH_LBVH_SAH;
