@@ -357,10 +357,11 @@ def run_ours(args):
     shade_dram = measured.get("k_shade")
 
     # k_accumulate: one launch folds the wave's frames; per pixel it reads
-    # each frame's sample radiance and first-hit guides (3 x 16 B) and reads
-    # (3 x 16 B) and writes (4 x 16 B, display included) the running means
+    # each frame's sample radiance (16 B; the 32 B of guides of a sample whose
+    # camera ray hit something are not counted here) and reads (3 x 16 B) and
+    # writes (4 x 16 B, display included) the running means
     acc_ms = kern["accumulate_ms"] / max(args.steps, 1)
-    acc_bytes = W * H * (48.0 * w["spp"] + 112.0)
+    acc_bytes = W * H * (16.0 * w["spp"] + 112.0)
     acc_gbs = acc_bytes / (acc_ms / 1e3) / 1e9 if acc_ms > 0 else 0.0
     atrous = _atrous_roofline(nat, acc, stream, dn_params, W, H, peak, dev)
 
@@ -437,7 +438,7 @@ def run_ours(args):
                                        "dram_bytes_per_ray_small_case": shade_dram},
                              "accumulate": {"achieved": acc_gbs, "frac": acc_gbs / peak, "ms_per_step": acc_ms,
                                             "algorithmic_bytes_per_step": acc_bytes,
-                                            "bytes": "per pixel 48 B x spp sample reads + 112 B running means"},
+                                            "bytes": "per pixel 16 B x spp radiance reads + 112 B running means"},
                              "atrous": atrous,
                              # the rest of a step: generate + accumulate (+ a
                              # separate shadow launch); and the timed step
