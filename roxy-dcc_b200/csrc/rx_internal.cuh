@@ -408,6 +408,19 @@ __device__ __forceinline__ float div_by(float x, float d, float r) {
   return res == 0.0f ? q : __fmaf_rn(res, r, q);
 }
 
+// Rays a warp of k_extend or of a query takes at a time: 32, or fewer while
+// the rays would leave the device with less than eight warps per SM.  A warp's
+// time is its slowest ray's, and fewer rays diverge less; with more warps than
+// that asked for (16 per SM, or all that fit) the closed box's short queues
+// lose 3 % to idle lanes, as they do with k_tail's paths spread.  Query of 100
+// rays 32 -> 15 us, 1,000 56 -> 37, 10,000 95 -> 92; 160x90 view 0.44 ->
+// 0.39 ms, 64x64 closed box 0.404 -> 0.409; from 38 k rays on it is 32.
+__host__ __device__ __forceinline__ int warp_items(long long total) {
+  constexpr long long kWarps = 148 * 8;
+  const long long take = (total + kWarps - 1) / kWarps;
+  return take > 32 ? 32 : take < 1 ? 1 : (int)take;
+}
+
 // A kernel launched with launch_chained may start its blocks while the kernel
 // before it in the stream still runs: everything before chain_wait must leave
 // global memory alone; chain_go lets the next kernel's blocks come (after any

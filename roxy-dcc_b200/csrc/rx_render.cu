@@ -575,13 +575,14 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
   const int total = n + (int)ns;
   int* fetch = &counters[C_FE + (b >= 0 ? b : kMaxBounce - 1)];
   const int lane = threadIdx.x & 31;
+  const int take = warp_items(total);
   int run_job = -1, run_rays = 0;  // batches: rays of this warp's current job, not yet added to its count
   for (;;) {
     int base = 0;
-    if (lane == 0) base = atomicAdd(fetch, 32);
+    if (lane == 0) base = atomicAdd(fetch, take);
     base = __shfl_sync(0xffffffffu, base, 0);
     if (base >= total) break;
-    int i = base + lane;
+    const int i = lane < take ? base + lane : total;
     int job = -1, rays_here = 0;
     if (i < n) {
       float3 o, d;

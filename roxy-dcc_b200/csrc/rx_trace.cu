@@ -10,11 +10,26 @@ namespace rx {
 
 __device__ __forceinline__ float3 ld3f(const float* p, long i) { return f3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
 
+// The rays of a query, `take` consecutive ones per warp and turn.
+struct RayItem {
+  long i;
+  int step;
+  bool idle;
+  __device__ __forceinline__ explicit RayItem(int take) {
+    const int lane = threadIdx.x & 31;
+    i = (blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5)) * take + lane;
+    step = gridDim.x * (blockDim.x >> 5) * take;
+    idle = lane >= take;
+  }
+  __device__ __forceinline__ operator long() const { return idle ? LONG_MAX : i; }
+  __device__ __forceinline__ void next() { i += step; }
+};
+
 template <bool EXACT>
-__global__ void k_trace_closest(DevScene S, long n, const float* __restrict__ ro, const float* __restrict__ rd,
-                                float* __restrict__ out_t, int* __restrict__ out_id, float* __restrict__ out_u,
-                                float* __restrict__ out_v, int* err) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+__global__ void k_trace_closest(DevScene S, long n, int take, const float* __restrict__ ro,
+                                const float* __restrict__ rd, float* __restrict__ out_t, int* __restrict__ out_id,
+                                float* __restrict__ out_u, float* __restrict__ out_v, int* err) {
+  for (RayItem i(take); i < n; i.next()) {
     float3 o = ld3f(ro, i), d = ld3f(rd, i);
     float t = 1e9f, u = 0.0f, v = 0.0f;
     int p = bvh_closest<EXACT, false>(S, o, d, t, u, v, err);
@@ -32,9 +47,9 @@ __global__ void k_trace_closest(DevScene S, long n, const float* __restrict__ ro
 }
 
 template <bool EXACT>
-__global__ void k_trace_any(DevScene S, long n, const float* __restrict__ ro, const float* __restrict__ rd,
+__global__ void k_trace_any(DevScene S, long n, int take, const float* __restrict__ ro, const float* __restrict__ rd,
                             const float* __restrict__ tmax, int* __restrict__ out, int* err) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+  for (RayItem i(take); i < n; i.next()) {
     out[i] = scene_any<EXACT, false, false>(S, ld3f(ro, i), ld3f(rd, i), tmax[i], err) ? 1 : 0;
   }
 }
@@ -62,11 +77,11 @@ __device__ __forceinline__ float3 hit_normal(const DevScene& S, float3 o, float3
 }
 
 template <bool EXACT>
-__global__ void k_scene_query(DevScene S, long n, const float* __restrict__ ro, const float* __restrict__ rd,
+__global__ void k_scene_query(DevScene S, long n, int take, const float* __restrict__ ro, const float* __restrict__ rd,
                               const int* __restrict__ lin_slot, float* __restrict__ out_t, int* __restrict__ out_kind,
                               int* __restrict__ out_id, float* __restrict__ out_u, float* __restrict__ out_v,
                               float* __restrict__ out_n, int* err) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+  for (RayItem i(take); i < n; i.next()) {
     float3 o = ld3f(ro, i), d = ld3f(rd, i);
     SceneHit h = scene_closest<EXACT, false, false>(S, o, d, err);
     int kind = 0, id = -1;
@@ -90,8 +105,8 @@ __global__ void k_scene_query(DevScene S, long n, const float* __restrict__ ro, 
   }
 }
 
-static int grid_for_rays(Ctx* ctx, long n) {
-  long g = (n + 127) / 128;
+static int grid_for_rays(Ctx* ctx, long n, int take) {
+  long g = (n + 4 * take - 1) / (4 * take);
   long cap = (long)ctx->num_sms * 16;
   if (g > cap) g = cap;
   return g < 1 ? 1 : (int)g;
@@ -101,12 +116,13 @@ int trace_closest(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d
                   float* d_u, float* d_v) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
+  const int take = warp_items(n);
   if (S.exact_slab)
-    k_trace_closest<true><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, d_t, d_id, d_u, d_v,
-                                                                          ctx->d_err);
+    k_trace_closest<true><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_t, d_id, d_u,
+                                                                                d_v, ctx->d_err);
   else
-    k_trace_closest<false><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, d_t, d_id, d_u, d_v,
-                                                                           ctx->d_err);
+    k_trace_closest<false><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_t, d_id, d_u,
+                                                                                 d_v, ctx->d_err);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }
@@ -114,10 +130,13 @@ int trace_closest(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d
 int trace_any(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d_rd, const float* d_tmax, int* d_occ) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
+  const int take = warp_items(n);
   if (S.exact_slab)
-    k_trace_any<true><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, d_tmax, d_occ, ctx->d_err);
+    k_trace_any<true><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_tmax, d_occ,
+                                                                            ctx->d_err);
   else
-    k_trace_any<false><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, d_tmax, d_occ, ctx->d_err);
+    k_trace_any<false><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_tmax, d_occ,
+                                                                             ctx->d_err);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
 }
@@ -126,17 +145,18 @@ int scene_query(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d_r
                 int* d_id, float* d_u, float* d_v, float* d_n) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
+  const int take = warp_items(n);
   DevBuf<int> lin(ctx, std::max<size_t>(sc->lin_slot.size(), 1));
   if (!lin.ok()) return set_error(ctx, "scene query: out of device memory"), RX_ERR_CAPACITY;
   if (!sc->lin_slot.empty())
     cudaMemcpyAsync(lin.p, sc->lin_slot.data(), sizeof(int) * sc->lin_slot.size(), cudaMemcpyHostToDevice,
                     ctx->stream);
   if (S.exact_slab)
-    k_scene_query<true><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, lin.p, d_t, d_kind, d_id,
-                                                                        d_u, d_v, d_n, ctx->d_err);
+    k_scene_query<true><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, lin.p, d_t,
+                                                                              d_kind, d_id, d_u, d_v, d_n, ctx->d_err);
   else
-    k_scene_query<false><<<grid_for_rays(ctx, n), 128, 0, ctx->stream>>>(S, n, d_ro, d_rd, lin.p, d_t, d_kind, d_id,
-                                                                         d_u, d_v, d_n, ctx->d_err);
+    k_scene_query<false><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, lin.p, d_t,
+                                                                               d_kind, d_id, d_u, d_v, d_n, ctx->d_err);
   CUDA_TRY(ctx, cudaGetLastError());
   CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return RX_OK;

@@ -212,6 +212,22 @@ def test_benchmark_scene_hit_ids_match_reference_traversal():
     assert r["t_bit_exact"]
 
 
+@pytest.mark.parametrize("n", [1, 33, 1184, 1185, 4000, 37_887, 37_889])
+def test_short_queries_equal_long_ones(n):
+    """Fewer rays per warp below 37,888 of them: every ray's answer is the one
+    it has in a query of 60,000, whatever the number of lanes a warp uses."""
+    v0, v1, v2 = gs.soup_triangles(3000, 11)
+    sc = _scene(v0, v1, v2, nat.RX_BVH_LBVH_SAH, 4)
+    rng = np.random.default_rng(2)
+    ro = rng.normal(size=(60_000, 3)).astype(np.float32) * 2
+    rd = rng.normal(size=(60_000, 3)).astype(np.float32)
+    rd /= np.linalg.norm(rd, axis=1, keepdims=True)
+    tm = rng.uniform(0.1, 4.0, 60_000).astype(np.float32)
+    for a, b in zip(sc.trace_closest(ro, rd), sc.trace_closest(ro[-n:], rd[-n:])):
+        assert np.array_equal(a[-n:].view(np.int32), b.view(np.int32))
+    assert np.array_equal(sc.trace_any(ro, rd, tm)[-n:], sc.trace_any(ro[-n:], rd[-n:], tm[-n:]))
+
+
 @pytest.mark.parametrize("n,scale,offset", [(1, 1.0, 0.0), (2, 0.01, 0.0), (5, 1.0, 50.0), (33, 100.0, 0.0),
                                             (3000, 1.0, 0.0), (3000, 0.05, 20.0), (3000, 100.0, 50.0)])
 def test_wide_nodes_find_what_the_reference_tree_finds(n, scale, offset):
