@@ -72,7 +72,7 @@ __global__ void k_prim_bounds(int n_tris, const float* __restrict__ v0, const fl
 // Two-stage exact min/max reduction of the centroids.
 __global__ void k_reduce_bounds(int n, const float3* __restrict__ p, float3* __restrict__ part_min,
                                 float3* __restrict__ part_max) {
-  chain_wait();
+  chain_wait(p, part_min, part_max);
   chain_go();
   __shared__ float smin[3][256], smax[3][256];
   float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
@@ -107,7 +107,7 @@ constexpr int kBoundsThreads = 1024;
 __global__ void __launch_bounds__(kBoundsThreads) k_bounds_final(int parts, const float3* __restrict__ mins,
                                                                  const float3* __restrict__ maxs,
                                                                  float3* __restrict__ out) {
-  chain_wait();
+  chain_wait(mins, maxs, out);
   chain_go();
   __shared__ float3 slo[kBoundsThreads], shi[kBoundsThreads];
   float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
@@ -149,7 +149,7 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
 // `bounds`: the centroid bounds (k_bounds_final).
 __global__ void k_morton(int n, const float3* __restrict__ cen, const float3* __restrict__ bounds, int cubic,
                          uint32_t* __restrict__ codes, int* __restrict__ idx) {
-  chain_wait();
+  chain_wait(cen, bounds, codes, idx);
   chain_go();
   __shared__ float3 s_lo, s_ext;
   if (threadIdx.x == 0) {
@@ -191,7 +191,7 @@ __host__ __device__ constexpr int sort_tile(int chunks) { return kSortWarps * ch
 
 __global__ void k_sort_hist(int n, const uint32_t* __restrict__ keys, int shift, int tile, uint32_t* __restrict__ hist,
                             int nblocks) {
-  chain_wait();
+  chain_wait(keys, hist);
   chain_go();
   __shared__ uint32_t h[256];
   for (int i = threadIdx.x; i < 256; i += blockDim.x) h[i] = 0;
@@ -232,7 +232,7 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t v, uint32_t* wa
 // took 21 us per pass at 80 blocks; a row each takes 3.)
 __global__ void __launch_bounds__(256) k_sort_rows(uint32_t* __restrict__ hist, uint32_t* __restrict__ totals,
                                                    int nblocks) {
-  chain_wait();
+  chain_wait(hist, totals);
   chain_go();
   __shared__ uint32_t warp_sums[8];
   uint32_t* row = hist + (size_t)blockIdx.x * nblocks;
@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kSortWarps * 32)
     k_sort_scatter(int n, const uint32_t* __restrict__ keys_in, const int* __restrict__ vals_in,
                    uint32_t* __restrict__ keys_out, int* __restrict__ vals_out, int shift,
                    const uint32_t* __restrict__ hist, const uint32_t* __restrict__ totals, int nblocks) {
-  chain_wait();
+  chain_wait(keys_in, vals_in, keys_out, vals_out, hist, totals);
   chain_go();
   static_assert(kSortWarps * 32 == 256, "one thread per digit");
   __shared__ uint32_t wcount[kSortWarps][256];
@@ -476,7 +476,7 @@ __global__ void k_gather_prims(int n, const int* __restrict__ order, int n_tris,
                                const float4* __restrict__ obj_a, const float4* __restrict__ obj_b,
                                const int* __restrict__ obj_mat, const int* __restrict__ obj_slot,
                                float4* __restrict__ prims, float4* __restrict__ shade) {
-  chain_wait();
+  chain_wait(order, v0, v1, v2, n0, n1, n2, tri_mat, obj_a, obj_b, obj_mat, obj_slot, prims, shade);
   chain_go();
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
     int i = order[k];
@@ -525,7 +525,7 @@ __device__ __forceinline__ int right_child(int hi, int gamma) { return hi == gam
 __global__ void k_karras(int n, const uint32_t* __restrict__ codes, int4* __restrict__ range,
                          int* __restrict__ parent_int, int* __restrict__ parent_leaf, int* __restrict__ flags,
                          int* __restrict__ counts, int n_counts) {
-  chain_wait();
+  chain_wait(codes, range, parent_int, parent_leaf, flags, counts);
   chain_go();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
     int d = (lcp(codes, n, i, i + 1) - lcp(codes, n, i, i - 1)) >= 0 ? 1 : -1;
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kUpLeaves)
                      const int* __restrict__ parent_int, const int* __restrict__ parent_leaf,
                      const float3* __restrict__ pmin, const float3* __restrict__ pmax, float4* __restrict__ rec,
                      int* __restrict__ flags, int max_leaf, float c_t, float c_i) {
-  chain_wait();
+  chain_wait(order, range, parent_int, parent_leaf, pmin, pmax, rec, flags);
   chain_go();
   __shared__ float4 s_a[kUpLeaves], s_b[kUpLeaves];  // records of this block's nodes, by node - base
   __shared__ float3 s_lo[kUpLeaves], s_hi[kUpLeaves];
@@ -703,7 +703,7 @@ struct NodeMask {
 
 // One block per kRankWords words; the last one writes *total.
 __global__ void __launch_bounds__(kRankWords) k_rank(NodeMask m, int n, int* __restrict__ total) {
-  chain_wait();
+  chain_wait(m.mask, m.rank, m.counts, total);
   chain_go();
   __shared__ uint32_t warp_sums[8];
   uint32_t before = 0, part = 0, here = 0;
@@ -728,7 +728,7 @@ __device__ __forceinline__ int rec_height(const float4* rec, int node) {
 __global__ void __launch_bounds__(256)
     k_lbvh_keep(int n_int, const int4* __restrict__ range, const int* __restrict__ parent_int,
                 const float4* __restrict__ rec, int max_leaf, NodeMask m, int* __restrict__ levels) {
-  chain_wait();
+  chain_wait(range, parent_int, rec, m.mask, m.rank, m.counts, levels);
   chain_go();
   const int i = blockIdx.x * 256 + threadIdx.x;
   bool keep = i < n_int && rec_height(rec, i) > 0;
@@ -748,7 +748,7 @@ __global__ void k_lbvh_layout(int n_int, const int4* __restrict__ range, const i
                               const float3* __restrict__ pmin, const float3* __restrict__ pmax,
                               const float4* __restrict__ rec, NodeMask m, float4* __restrict__ out,
                               int* __restrict__ at_lo) {
-  chain_wait();
+  chain_wait(range, order, pmin, pmax, rec, m.mask, m.rank, m.counts, out, at_lo);
   chain_go();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_int; i += gridDim.x * blockDim.x) {
     if (!m.has(i)) continue;
@@ -897,7 +897,7 @@ __device__ __forceinline__ void wide_open(WideNode& v, const float4* __restrict_
 __global__ void __launch_bounds__(128) k_wide_kids(const float4* __restrict__ bin, int n_bin,
                                                    const int* __restrict__ at_lo, int4* __restrict__ kids,
                                                    int* __restrict__ counts, int n_counts, int* err) {
-  chain_wait();
+  chain_wait(bin, at_lo, kids, counts);
   chain_go();
   const int b = blockIdx.x * 128 + threadIdx.x;
   if (b >= n_bin) return;
@@ -921,7 +921,7 @@ __global__ void __launch_bounds__(128) k_wide_kids(const float4* __restrict__ bi
 // below it.
 __global__ void __launch_bounds__(256) k_wide_roots(int n_bin, const int4* __restrict__ kids,
                                                     const int* __restrict__ at_lo, NodeMask m) {
-  chain_wait();
+  chain_wait(kids, at_lo, m.mask, m.rank, m.counts);
   chain_go();
   const int b = blockIdx.x * 256 + threadIdx.x;
   int cur = b < n_bin ? 0 : -1;
@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(256) k_wide_roots(int n_bin, const int4* __res
 
 __global__ void __launch_bounds__(128) k_wide_write(const float4* __restrict__ bin, int n_bin, NodeMask m,
                                                     float4* __restrict__ out4, int* err) {
-  chain_wait();
+  chain_wait(bin, m.mask, m.rank, m.counts, out4);
   chain_go();
   const int b = blockIdx.x * 128 + threadIdx.x;
   if (b >= n_bin || !m.has(b)) return;

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, 1)
     }
   };
 
-  chain_wait();
+  chain_wait(x, w);  // bias: read behind the loops below only; through here it costs the epilogue 12 %
   chain_go();
   for (int c = tid; c < BN * 9 * KC; c += 256) {
     const int row = c / (9 * KC), k = c - row * (9 * KC);
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG, ADD)) k_conv_fwd
   // no chain_go: the next kernel's blocks, let in while this one works, took
   // more than they hid (a 1080p inference 1,255 us with it, 1,160 without,
   // 1,225 unchained)
-  chain_wait();
+  chain_wait(w, bias, y, y32, acc_in);
   for (int c = tid; c < NG; c += blockDim.x) sbias[c] = bias ? bias[grp * NG + c] : 0.0f;
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
                  "r"(A.tcols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
-  chain_wait();
+  chain_wait(dw);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -1390,7 +1390,7 @@ __global__ void __cluster_dims__(kBiasCluster, 1, 1) __launch_bounds__(kBiasThre
     k_bias_grad(rx_conv_desc d, const bf16* __restrict__ dy, float* __restrict__ db, int pix_per_block) {
   __shared__ float part[kBiasThreads][9];  // 8 channels, padded against bank conflicts
   __shared__ double sums[kBiasWidth * 8];
-  chain_wait();
+  chain_wait(dy, db);
   chain_go();
   auto cluster = cooperative_groups::this_cluster();
   const long long P = (long long)d.N * d.H * d.W;
@@ -1454,7 +1454,7 @@ __global__ void k_rot_weights(int Cout, int Cin, const bf16* __restrict__ w, bf1
 // scalar form's 64-bit divisions and 2-byte stores took 39 us for the ten
 // layers of a training step, this 31 (a launch each).
 __global__ void k_rot_weights_v8(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
-  chain_wait();
+  chain_wait(w, wr);
   chain_go();
   const unsigned n = (unsigned)(Cout / 8) * 9u * (unsigned)Cin;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1504,7 +1504,7 @@ __global__ void k_relu_mask(long long P, int C, const bf16* __restrict__ yv, int
 // training step 203 -> 89 us.
 __global__ void k_relu_mask_v8(long long P, int C, const bf16* __restrict__ yv, int y_stride, int y_off,
                                bf16* __restrict__ g, int g_stride, int g_off) {
-  chain_wait();
+  chain_wait(yv, g);
   chain_go();
   const int CK = C >> 3;
   const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
@@ -1577,7 +1577,7 @@ __device__ __forceinline__ void chunk_index(long long i, int CK, int W, int H, i
 
 __global__ void k_up2_v8(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                          bf16* __restrict__ y, int y_stride, int y_off) {
-  chain_wait();
+  chain_wait(x, y);
   chain_go();
   const int CK = C >> 3;
   RX_EW_LOOP((long long)N * H * W * CK) {
@@ -1596,7 +1596,7 @@ __global__ void k_up2_v8(int N, int H, int W, int C, const bf16* __restrict__ x,
 
 __global__ void k_pool2_v8(int N, int H, int W, int C, const bf16* __restrict__ x, int x_stride, int x_off,
                            bf16* __restrict__ y, int y_stride, int y_off) {
-  chain_wait();
+  chain_wait(x, y);
   chain_go();
   const int CK = C >> 3, h2 = H / 2, w2 = W / 2;
   RX_EW_LOOP((long long)N * h2 * w2 * CK) {
@@ -1645,7 +1645,7 @@ __global__ void k_pool2_bwd(int N, int H, int W, int C, const bf16* __restrict__
 // 86 -> 15 us, the two upsamples' 52 -> 16.
 __global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
                                bf16* __restrict__ dx, int dx_stride, int dx_off, int accumulate) {
-  chain_wait();
+  chain_wait(dy, dx);
   chain_go();
   const int CK = C >> 3, h2 = H / 2, w2 = W / 2;
   RX_EW_LOOP((long long)N * h2 * w2 * CK) {
@@ -1682,7 +1682,7 @@ __global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restric
 
 __global__ void k_up2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
                              bf16* __restrict__ dx, int dx_stride, int dx_off) {
-  chain_wait();
+  chain_wait(dy, dx);
   chain_go();
   const int CK = C >> 3;
   RX_EW_LOOP((long long)N * H * W * CK) {
@@ -1782,7 +1782,7 @@ __global__ void k_features(long long P, const float* __restrict__ rad, const flo
 __global__ void k_features_v4(long long P4, const float4* __restrict__ rad, const float4* __restrict__ alb,
                               const float4* __restrict__ nrm, const float4* __restrict__ dep, uint4* __restrict__ out,
                               float4* __restrict__ base) {
-  chain_wait();
+  chain_wait(rad, alb, nrm, dep, out, base);
   chain_go();
   RX_EW_LOOP(P4) {
     float4 r[3], a[3], n[3], l[3];
@@ -1815,7 +1815,7 @@ template <bool CHUNKS>
 __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
                           const float* __restrict__ t, float scale, bf16* __restrict__ g, int gs,
                           float* __restrict__ loss) {
-  chain_wait();
+  chain_wait(y32, base, t, g, loss);
   chain_go();
   float s = 0.0f;
   RX_EW_LOOP(P) {
@@ -1845,7 +1845,7 @@ __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stri
 // radiance = max(expm1(y + base), 0) from the head's first three channels
 __global__ void k_output(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
                          float* __restrict__ out) {
-  chain_wait();
+  chain_wait(y32, base, out);
   chain_go();
   RX_EW_LOOP(P) {
 #pragma unroll
@@ -2018,7 +2018,7 @@ static int launch_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
 // Input channels [p * cp, (p + 1) * cp) of weights [Cout][9][Cin] as
 // contiguous [Cout][9][cp], for p = 0, 1 (16-byte chunks).
 __global__ void k_weight_halves(int Cout, int Cin, const uint4* __restrict__ w, uint4* __restrict__ out) {
-  chain_wait();
+  chain_wait(w, out);
   chain_go();
   const int cp8 = Cin / 16, c8 = Cin / 8;  // chunks per half row, per row
   const long long n = (long long)Cout * 9 * c8;

@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kA1Warps * 32, a1_blocks(EXACT, GUIDES))
   };
   // launched while the pass before still runs: wait for its results, then let
   // the next one come
-  chain_wait();
+  chain_wait(in, src, gn, ga, out);
   chain_go();
   // three row buffers in turn, so that no row is moved between registers
   Row r0, r1, r2;

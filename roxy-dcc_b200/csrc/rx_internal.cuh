@@ -425,8 +425,23 @@ __host__ __device__ __forceinline__ int warp_items(long long total) {
 // before it in the stream still runs: everything before chain_wait must leave
 // global memory alone; chain_go lets the next kernel's blocks come (after any
 // allocation of tensor memory, so that a waiting block cannot hold what an
-// unstarted one needs).
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// unstarted one needs).  The pointers that the kernel reads through pass
+// through chain_wait: a load that depends on its result cannot be moved
+// before the wait, as one through a const __restrict__ parameter may be, nor
+// be taken for a load of memory that is constant while the kernel runs.
+template <typename T>
+__device__ __forceinline__ void after_wait(T& q) {
+  // as a global address, so that what follows stays global loads and atomics
+  // (generic ones cost the weight gradient a quarter of its time)
+  size_t g = __cvta_generic_to_global(q);
+  asm volatile("" : "+l"(g)::"memory");
+  q = static_cast<T>(__cvta_global_to_generic(g));
+}
+template <typename... P>
+__device__ __forceinline__ void chain_wait(P&... p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (after_wait(p), ...);
+}
 __device__ __forceinline__ void chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Packed child word: >= 0 internal node index; < 0 leaf with

@@ -3,6 +3,8 @@
 // parity hooks for the reference's bvh_intersect / bvh_occluded /
 // scene_intersect (rendering/taichi/intersect.py:81-309) and a direct
 // traversal benchmark.
+#include <climits>
+
 #include "rx_internal.cuh"
 #include "rx_runtime.h"
 
