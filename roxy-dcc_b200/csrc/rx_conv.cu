@@ -1811,13 +1811,17 @@ __global__ void k_features_v4(long long P4, const float4* __restrict__ rad, cons
 // (bf16, channel stride gs; pad channels 3..gs-1 zero)
 // CHUNKS: gs is a multiple of 8 and g 16-byte aligned, so the pixel's
 // channels are stored 16 bytes at a time (16x128x128, gs 16: 28 -> 18 us).
+// The sum is kept in float64 up to one fp32 atomic per block of 1,024 threads,
+// at most a block per SM: an atomic per warp, 8,192 on one address, left it an
+// order-dependent 1.3e-6 off.
+constexpr int kLossThreads = 1024;
 template <bool CHUNKS>
-__global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
-                          const float* __restrict__ t, float scale, bf16* __restrict__ g, int gs,
-                          float* __restrict__ loss) {
+__global__ void __launch_bounds__(kLossThreads)
+    k_l1_loss(long long P, const float* __restrict__ y32, int y_stride, const float* __restrict__ base,
+              const float* __restrict__ t, float scale, bf16* __restrict__ g, int gs, float* __restrict__ loss) {
   chain_wait(y32, base, t, g, loss);
   chain_go();
-  float s = 0.0f;
+  double s = 0.0;
   RX_EW_LOOP(P) {
     alignas(4) bf16 v[8];
 #pragma unroll
@@ -1825,7 +1829,7 @@ __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stri
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       float dlt = (y32[i * y_stride + k] + (base ? base[3 * i + k] : 0.0f)) - t[3 * i + k];
-      s += fabsf(dlt);
+      s += (double)fabsf(dlt);
       v[k] = __float2bfloat16_rn(dlt > 0.0f ? scale : (dlt < 0.0f ? -scale : 0.0f));
     }
     if (CHUNKS) {
@@ -1838,8 +1842,15 @@ __global__ void k_l1_loss(long long P, const float* __restrict__ y32, int y_stri
       for (int k = 3; k < gs; ++k) g[i * gs + k] = v[7];
     }
   }
+  __shared__ double warp_sum[kLossThreads / 32];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, s);
+  if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double b = 0.0;
+    for (int w = 0; w < kLossThreads / 32; ++w) b += warp_sum[w];
+    atomicAdd(loss, (float)b);
+  }
 }
 
 // radiance = max(expm1(y + base), 0) from the head's first three channels
@@ -2405,7 +2416,8 @@ int dn_l1_loss(Ctx* ctx, long long P, const float* y32, int y_stride, const floa
   if (P <= 0 || !y32 || !target || !grad || !loss || y_stride < 3 || grad_stride < 3)
     return set_error(ctx, "dn_l1_loss: bad arguments"), RX_ERR_ARG;
   auto kern = grad_stride % 8 == 0 && (uintptr_t)grad % 16 == 0 ? k_l1_loss<true> : k_l1_loss<false>;
-  launch_chained(st, true, dim3(ew_blocks(ctx, P)), 256, 0, kern, P, y32, y_stride, base, target, scale,
+  const int blocks = (int)std::min<long long>((P + kLossThreads - 1) / kLossThreads, ctx->num_sms);
+  launch_chained(st, true, dim3(blocks), kLossThreads, 0, kern, P, y32, y_stride, base, target, scale,
                  static_cast<bf16*>(grad), grad_stride, loss);
   CUDA_TRY(ctx, cudaGetLastError());
   return RX_OK;
