@@ -89,8 +89,8 @@ __device__ __forceinline__ float tap_weight(const AtrousArgs& A, float sw, float
 }
 
 // Weight of a pair of pixels as tap_weight's, without branches, so that the
-// pairs of a row interleave; guides that are not in use are zeros (a term of
-// exactly 1, or nothing added to the exponent).
+// pairs of a row interleave; guides that are not in use are zeros with a
+// 2 sigma^2 of 1 (a term of exactly 1, or nothing added to the exponent).
 //
 // EXACT forms div_by's quotient without its range test, which the
 // exponential makes needless for 2 sigma^2 in [2^-30, 2^30]: below 2^-96 any
@@ -451,6 +451,11 @@ static size_t atrous_smem(const AtrousArgs& A) {
 static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, const float4* color, const float4* gn,
                                  const float4* ga, float4* out, float4* s0, float4* s1) {
   const long long P = (long long)A.H * A.W;
+  // k_atrous_r1 evaluates the terms of unused guides on zeros: whatever their
+  // sigma holds (a NaN, too), they must come to exactly 1
+  if (!A.use_n) A.s2n = 1.0f;
+  if (!A.use_a) A.s2a = 1.0f;
+  if (!A.use_d) A.s2d = 1.0f;
   A.r2c = 1.0f / A.s2c, A.r2n = 1.0f / A.s2n, A.r2a = 1.0f / A.s2a, A.r2d = 1.0f / A.s2d;
   A.quot = std::max(std::max(A.s2c, A.s2n), std::max(A.s2a, A.s2d)) <= 0x1p+30f;
   const float4* in = color;

@@ -187,3 +187,23 @@ def test_spheres_and_cubes_in_the_bvh_hit_as_the_linear_scan():
     plane = objs & (linear["id"] == 300)
     assert plane.any() and (objs & ~plane).any()
     assert (in_bvh["kind"][objs & ~plane] == 2).all() and (in_bvh["kind"][plane] == 3).all()
+
+
+@pytest.mark.parametrize("radius", [1, 2])
+@pytest.mark.parametrize("passes", [1, 5])
+@pytest.mark.parametrize("guides", ["", "n", "a", "d", "na", "nd", "ad"])
+@pytest.mark.parametrize("sigma", [float("nan"), float("inf"), 0.0, 1e30])
+def test_atrous_sigma_of_an_unused_guide_is_ignored(radius, passes, guides, sigma):
+    """A guide that is not given has no say, whatever its sigma holds (a caller
+    may fill in only what it uses): the bits of the default sigmas."""
+    rng = np.random.default_rng(3)
+    src = rng.random((37, 53, 3)).astype(np.float32)
+    g = {"n": rng.normal(size=(37, 53, 3)).astype(np.float32), "a": rng.random((37, 53, 3)).astype(np.float32),
+         "d": rng.random((37, 53)).astype(np.float32)}
+    names = {"n": "normal", "a": "albedo", "d": "depth"}
+    kw = {names[k]: g[k] for k in guides}
+    unused = {"sigma_" + names[k]: sigma for k in "nad" if k not in guides}
+    want = edge_aware_denoise(src, radius, 0.08, 0.8, passes=passes, **kw)
+    got = edge_aware_denoise(src, radius, 0.08, 0.8, passes=passes, **kw, **unused)
+    assert np.isfinite(want).all()
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
