@@ -1046,6 +1046,12 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG, ADD)) k_conv_fwd
 // four) at N = 64, three at N = 128; blockIdx.x % G picks its input-channel
 // group, output-channel group and taps.  At the end the strips' sums meet
 // in dw by fp32 atomics (32 consecutive input channels per warp).
+// A width that is no multiple of 16 leaves a row's last step with pixels past
+// the image, where dy is zero fill.  So is x, but for tap column 0, whose
+// first such pixel reads the image's last column, and zero times an infinity
+// or a NaN there would reach a sum that it does not belong to.  That step of
+// that column reads 16 pixels of its own instead, loaded behind the row
+// through a map that ends one column early.
 //   warps 0-3: read the accumulators at the end.  warps 4-5: MMA issuers,
 //   each with half of the block's taps, so that one's waits pass under the
 //   other's MMAs.  warp 6: producer.  Waits are bounded as in k_conv_fwd_ws.
@@ -1062,11 +1068,15 @@ struct WgradArgs {
   int taps, tg;      // taps per group, groups
   int Sx, Sy;        // ring slots of x and dy rows
   int xslot, yslot;  // bytes
+  int xcut;          // offset of the cut step's pixels in an x slot (0: no row has one)
   int tcols;         // tensor-memory columns (a power of two)
 };
 constexpr int kWgThreads = 224, kWgSlots = 6;
 
+// CUT: rows may have a cut step (W not a multiple of 16).
+template <bool CUT>
 __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_constant__ CUtensorMap xmap,
+                                                                 const __grid_constant__ CUtensorMap cutmap,
                                                                  const __grid_constant__ CUtensorMap ymap, WgradArgs A,
                                                                  float* __restrict__ dw, long long per_cta, int* err) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1114,9 +1124,10 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
     // ------------------------------------------------ producer
     if (elect_one()) {
       const uint32_t xbytes = (uint32_t)((A.tw + 2) * 16 * (A.cm / 8)), ybytes = (uint32_t)(A.tw * 16 * (A.nc / 8));
-      auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t bar, uint32_t bytes, int px, int chunk, int row,
-                      int img) {
+      auto expect = [&](uint32_t bar, uint32_t bytes) {
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
+      };
+      auto load = [&](const CUtensorMap* map, uint32_t dst, uint32_t bar, int px, int chunk, int row, int img) {
         asm volatile(
             "cp.async.bulk.tensor.5d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
             "%6}], [%7];\n" ::"r"(dst),
@@ -1129,18 +1140,27 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
         const long long col = u / A.H;
         const int ylo = (int)(u - col * A.H), nrows = (int)min((long long)(A.H - ylo), uend - u);
         const int n = (int)(col / A.tiles), x0 = (int)(col % A.tiles) * A.tw;
+        const int px = min(A.tw, A.W - x0);
+        const bool cut = CUT && px % 16 != 0;  // the row's last step reaches past the image
+        // first pixel of that step for tap column 0; an image of one column
+        // has none to read (past its end: zeros)
+        const int cut_px = A.W > 1 ? x0 - 1 + (px & ~15) : A.W;
         for (int r = -1; r <= nrows && ok; ++r) {
           const int s = kx % A.Sx;
           ok = wait(&xempty[s], (uint32_t)(((kx / A.Sx) & 1) ^ 1));
           if (!ok) break;
-          load(&xmap, sx + (uint32_t)(s * A.xslot), smem_u32(&xfull[s]), xbytes, x0 - 1, ci0 / 8, ylo + r, n);
+          const uint32_t slot = sx + (uint32_t)(s * A.xslot), bar = smem_u32(&xfull[s]);
+          expect(bar, xbytes + (cut ? (uint32_t)(16 * 16 * (A.cm / 8)) : 0u));
+          load(&xmap, slot, bar, x0 - 1, ci0 / 8, ylo + r, n);
+          if (cut) load(&cutmap, slot + (uint32_t)A.xcut, bar, cut_px, ci0 / 8, ylo + r, n);
           ++kx;
           if (r < 1) continue;
           // dy row r - 1 goes with x rows r - 2 .. r
           const int t = ky % A.Sy;
           ok = wait(&yempty[t], (uint32_t)(((ky / A.Sy) & 1) ^ 1));
           if (!ok) break;
-          load(&ymap, sy + (uint32_t)(t * A.yslot), smem_u32(&yfull[t]), ybytes, x0, co0 / 8, ylo + r - 1, n);
+          expect(smem_u32(&yfull[t]), ybytes);
+          load(&ymap, sy + (uint32_t)(t * A.yslot), smem_u32(&yfull[t]), x0, co0 / 8, ylo + r - 1, n);
           ++ky;
         }
         u += nrows;
@@ -1166,6 +1186,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
       // channels) one plane
       const uint64_t a_hi = (uint64_t)((uint32_t)(A.tw + 2) | (1u << 14)) << 32;
       const uint64_t b_hi = (uint64_t)((uint32_t)A.tw | (1u << 14)) << 32;
+      const uint64_t cut_hi = (uint64_t)(16u | (1u << 14)) << 32;  // planes of 16 pixels
       auto mma = [&](uint32_t d, uint64_t ad, uint64_t bd, uint32_t p) {
         asm volatile(
             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -1190,7 +1211,8 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
         const long long col = u / A.H;
         const int ylo = (int)(u - col * A.H), nrows = (int)min((long long)(A.H - ylo), uend - u);
         const int x0 = (int)(col % A.tiles) * A.tw;
-        const int ksteps = (min(A.tw, A.W - x0) + 15) / 16;
+        const int px = min(A.tw, A.W - x0), ksteps = (px + 15) / 16;
+        const bool cut = CUT && px % 16 != 0;
         // x rows yy - 1, yy, yy + 1 of output row yy
         const int sa = xs;
         ok = wait(&xfull[xs], xph);
@@ -1212,13 +1234,18 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_conv_wgrad_ws(const __grid_co
             const int dx = tap < 3 ? tap : tap < 6 ? tap - 3 : tap - 6;
             uint32_t a_lo = (tap < 3 ? r0 : tap < 6 ? r1 : r2) + (uint32_t)dx;
             const uint32_t d = tmem + (uint32_t)(j * A.nc);
+            // the last step's pixels
+            const uint64_t a_last = cut && dx == 0 ? cut_hi | (a_lo + ((uint32_t)A.xcut >> 4))
+                                                   : a_hi | (a_lo + 16 * (uint32_t)(ksteps - 1));
             if (ksteps == 8) {  // compile-time offsets, as in issue_row
 #pragma unroll
-              for (int k = 0; k < 8; ++k) mma(d, a_hi | (a_lo + 16 * k), b_hi | (b_lo + 16 * k), k ? 1u : acc);
+              for (int k = 0; k < 7; ++k) mma(d, a_hi | (a_lo + 16 * k), b_hi | (b_lo + 16 * k), k ? 1u : acc);
+              mma(d, a_last, b_hi | (b_lo + 16 * 7), 1u);
             } else {
 #pragma unroll 1
-              for (int k = 0; k < ksteps; ++k)  // 16 pixels each
+              for (int k = 0; k < ksteps - 1; ++k)  // 16 pixels each
                 mma(d, a_hi | (a_lo + 16 * k), b_hi | (b_lo + 16 * k), k ? 1u : acc);
+              mma(d, a_last, b_hi | (b_lo + 16 * (ksteps - 1)), ksteps > 1 ? 1u : acc);
             }
           }
           acc = 1u;
@@ -1910,9 +1937,11 @@ static int launch_tc(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16*
 
 // An NHWC view (`C` channels at `v`, pixel stride `stride` elements) as the
 // 5-d tensor (8 channels, W, channel chunks, H, N) whose boxes -- `px`
-// pixels x `chunks` chunks of one row -- land as [chunk][pixel x 16 B].
-// False when the driver has no tensor maps or cannot describe the view.
-static bool row_map(int N, int H, int W, int C, int stride, const bf16* v, int px_box, int chunks, CUtensorMap* map) {
+// pixels x `chunks` chunks of one row -- land as [chunk][pixel x 16 B], with
+// zeros from pixel `cols` of a row on (W, or fewer).  False when the driver
+// has no tensor maps or cannot describe the view.
+static bool row_map(int N, int H, int W, int cols, int C, int stride, const bf16* v, int px_box, int chunks,
+                    CUtensorMap* map) {
   using Encode = decltype(&cuTensorMapEncodeTiled);
   static const Encode encode = [] {
     void* fn = nullptr;
@@ -1925,7 +1954,7 @@ static bool row_map(int N, int H, int W, int C, int stride, const bf16* v, int p
   }();
   if (!encode) return false;
   const cuuint64_t px = (cuuint64_t)stride * sizeof(bf16);
-  const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)C / 8, (cuuint64_t)H, (cuuint64_t)N};
+  const cuuint64_t dims[5] = {8, (cuuint64_t)cols, (cuuint64_t)C / 8, (cuuint64_t)H, (cuuint64_t)N};
   const cuuint64_t strides[4] = {px, 16, px * W, px * W * H};
   const cuuint32_t box[5] = {8, (cuuint32_t)px_box, (cuuint32_t)chunks, 1, 1}, step[5] = {1, 1, 1, 1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<bf16*>(v), dims, strides, box, step,
@@ -1955,7 +1984,7 @@ static int launch_ws_ng(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf
     attr_dev = ctx->device;
   }
   CUtensorMap xmap;
-  if (!row_map(d->N, d->H, d->W, d->Cin, d->x_cstride, x + d->x_coff, tc::HALO_W, d->Cin / 8, &xmap)) return 0;
+  if (!row_map(d->N, d->H, d->W, d->W, d->Cin, d->x_cstride, x + d->x_coff, tc::HALO_W, d->Cin / 8, &xmap)) return 0;
   // resident CTAs per SM from shared memory (dynamic + static + the
   // per-block reservation), capped by the registers (ws_min_blocks) and so
   // that every resident CTA gets its tensor memory
@@ -2234,10 +2263,11 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   const int limit = 232448 - 1024;  // opt-in shared memory per block, less the static part
   static int attr_dev = -1;
   if (attr_dev != ctx->device) {
-    if (cudaFuncSetAttribute(k_conv_wgrad_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
+    for (auto kern : {k_conv_wgrad_ws<false>, k_conv_wgrad_ws<true>})
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+      }
     attr_dev = ctx->device;
   }
   WgradArgs A{};
@@ -2280,22 +2310,27 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   while (A.tcols < A.taps * A.nc) A.tcols <<= 1;
   const int plane = (A.tw + 2) * 16;
   A.xslot = (A.cm / 8 * plane + 127) / 128 * 128;
+  if (d->W % 16) {
+    A.xcut = A.xslot;
+    A.xslot += A.cm / 8 * 16 * 16;
+  }
   A.yslot = (A.nc / 8 * A.tw * 16 + 127) / 128 * 128;
   // M = 128 reads sixteen planes from any x slot: room behind the last one
   // (the dy slots count; rows past the group's channels are not stored)
-  const int tail = 16 * plane;
+  const int tail = std::max(16 * plane, A.xcut + 16 * 16 * 16);
   A.Sy = 3, A.Sx = kWgSlots;
   auto bytes = [&] { return std::max(A.Sx * A.xslot + A.Sy * A.yslot, (A.Sx - 1) * A.xslot + tail) + 128; };
   while (bytes() > limit && A.Sx > 4) --A.Sx;
   while (bytes() > limit && A.Sy > 2) --A.Sy;
   if (bytes() > limit) return 0;
-  CUtensorMap xmap, ymap;
-  if (!row_map(d->N, d->H, d->W, d->Cin, d->x_cstride, x + d->x_coff, A.tw + 2, A.cm / 8, &xmap) ||
-      !row_map(d->N, d->H, d->W, d->Cout, d->y_cstride, dy + d->y_coff, A.tw, A.nc / 8, &ymap))
+  CUtensorMap xmap, cutmap, ymap;
+  if (!row_map(d->N, d->H, d->W, d->W, d->Cin, d->x_cstride, x + d->x_coff, A.tw + 2, A.cm / 8, &xmap) ||
+      !row_map(d->N, d->H, d->W, std::max(d->W - 1, 1), d->Cin, d->x_cstride, x + d->x_coff, 16, A.cm / 8, &cutmap) ||
+      !row_map(d->N, d->H, d->W, d->W, d->Cout, d->y_cstride, dy + d->y_coff, A.tw, A.nc / 8, &ymap))
     return 0;
   const int G = A.mg * A.ng * A.tg;
   launch_chained(st, true, dim3((unsigned)(strips * G)), kWgThreads, sole_block_smem(ctx, strips * G, bytes()),
-                 k_conv_wgrad_ws, xmap, ymap, A, dw, per_cta, ctx->d_err);
+                 A.xcut ? k_conv_wgrad_ws<true> : k_conv_wgrad_ws<false>, xmap, cutmap, ymap, A, dw, per_cta, ctx->d_err);
   cudaError_t e = cudaGetLastError();
   *rc = e == cudaSuccess ? RX_OK : (set_error(ctx, "conv_bf16_bwd_weight: %s", cudaGetErrorString(e)), RX_ERR_CUDA);
   return 1;

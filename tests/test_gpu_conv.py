@@ -421,3 +421,36 @@ def test_weight_gradient_tile_edges(N, H, W, Cin, Cout, xs, xo, ys, yo):
         cols = xv[:, tap // 3:tap // 3 + H, tap % 3:tap % 3 + W].reshape(-1, Cin)
         ref, mag = dv.t() @ cols, dv.abs().t() @ cols.abs()
         assert bool(((dw[:, tap].double() - 1.0 - ref).abs() <= (N * H * W + 2) * 2.0 ** -22 * (mag + 1.0)).all()), tap
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo", [
+    (1, 3, 1, 16, 16, 16, 0),       # one column: no product of the left taps at all
+    (1, 4, 17, 32, 32, 48, 16),     # a whole step and one pixel
+    (2, 3, 40, 96, 64, 96, 0),      # half a last step
+    (1, 3, 125, 128, 128, 128, 0),  # eight steps, the last one short
+    (1, 2, 130, 48, 16, 48, 0),     # the second tile's last step
+    (1, 3, 48, 64, 48, 64, 0),      # no short step
+])
+def test_weight_gradient_takes_only_products_of_the_image(N, H, W, Cin, Cout, xs, xo, bad):
+    """A non-finite activation in the last column enters the gradient of the
+    taps that read it for some output pixel and of no other: the left taps
+    (tap column 0) read the column to the left of a pixel, so never the
+    last.  Their gradient is that of the activations without it."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(W)
+    x = torch.randint(-3, 4, (N, H, W, xs), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randint(-3, 4, (N, H, W, Cout), generator=g, device="cuda").to(torch.bfloat16)
+    dws = []
+    for v in (0.0, bad):
+        x[:, :, W - 1, xo:xo + Cin:3] = v
+        dw = torch.zeros((Cout, 9, Cin), device="cuda")
+        d = nat.ConvDesc(N, H, W, Cin, Cout, xs, xo, Cout, 0)
+        ctx.check(nat.lib().rx_conv_bf16_bwd_weight(ctx.h, ctypes.byref(d), _p(dy), _p(x), _p(dw), None, _stream()))
+        ctx.check(nat.lib().rx_ctx_sync(ctx.h))
+        dws.append(dw)
+    for tap in (0, 3, 6):
+        assert torch.equal(dws[0][:, tap], dws[1][:, tap]), tap
+    for tap in (1, 4, 7):
+        hit = torch.isfinite(dws[1][:, tap]).logical_not()
+        assert not hit[:, 1::3].any() and hit[:, 0::3].any()
