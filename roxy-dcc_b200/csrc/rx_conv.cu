@@ -2131,10 +2131,13 @@ static int launch_res_as(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const b
     const long long nx = (d->W + (1 << c) - 1) >> c, ny = (d->H + (128 >> c) - 1) / (128 >> c);
     if (nx * ny < best) best = nx * ny, cl = c, tx = nx, ty = ny;
   }
-  if (best * d->N > 0x3fffffffLL || S::smem(cl) > 232448) return 0;  // opt-in shared memory per block
+  const int limit = 232448;  // opt-in shared memory per block
+  if (best * d->N > 0x3fffffffLL || S::smem(cl) > (size_t)limit) return 0;
   auto kern = k_conv_fwd_res<BN, KS>;
   const int smem = sole_block_smem(ctx, 0, (int)S::smem(cl));
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // the limit, not this launch's size: the attribute is the kernel's, and
+  // another thread's smaller launch would take it from under this one
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;

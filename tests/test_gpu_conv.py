@@ -4,6 +4,7 @@ weight / bias gradients (tolerance 2 % of the reference's largest value,
 the bf16 rounding of the outputs), pool / upsample and their gradients,
 the whole network's loss and weight gradients, and a short training run."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -454,3 +455,41 @@ def test_weight_gradient_takes_only_products_of_the_image(N, H, W, Cin, Cout, xs
     for tap in (1, 4, 7):
         hit = torch.isfinite(dws[1][:, tap]).logical_not()
         assert not hit[:, 1::3].any() and hit[:, 0::3].any()
+
+
+def test_resident_weight_conv_from_several_threads():
+    """Eight threads, each with its own context and stream, on two sizes whose
+    tiles ask for different amounts of shared memory: every call is accepted
+    and gives the bits it gives alone."""
+    cases = [(1, 128, 128, 64, 192), (1, 16, 8, 64, 192)] * 4
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    data = [(rnd(n, h, w, ci), rnd(co, 9, ci), torch.empty((n, h, w, co), dtype=torch.bfloat16, device="cuda"))
+            for n, h, w, ci, co in cases]
+    ctxs = [nat.Context(0) for _ in cases]
+    fails, want = [0] * len(cases), []
+
+    def work(i, times):
+        n, h, w, ci, co = cases[i]
+        d = nat.ConvDesc(n, h, w, ci, co, ci, 0, co, 0)
+        x, wt, y = data[i]
+        args = (ctxs[i].h, ctypes.byref(d), _p(x), _p(wt), None, _p(y), None, 0, ctypes.c_void_p(ctxs[i].stream))
+        for _ in range(times):
+            fails[i] += nat.lib().rx_conv_bf16_fwd(*args) != 0
+
+    torch.cuda.synchronize()
+    for i in range(len(cases)):
+        work(i, 1)
+        ctxs[i].sync()
+        want.append(data[i][2].clone())
+        data[i][2].zero_()
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i, 4000)) for i in range(len(cases))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for c in ctxs:
+        c.sync()
+    assert not any(fails)
+    assert all(torch.equal(data[i][2], want[i]) for i in range(len(cases)))
