@@ -440,6 +440,7 @@ static float two_sigma2(float s) {
 }
 
 // Dynamic shared memory of one tiled block: colour, plus each guide in use.
+constexpr int kAtMaxSmem = (kAtTW + 2 * kAtMaxTiledR) * (kAtTH + 2 * kAtMaxTiledR) * 3 * (int)sizeof(float4);
 static size_t atrous_smem(const AtrousArgs& A) {
   const size_t px = (size_t)(kAtTW + 2 * A.r) * (kAtTH + 2 * A.r);
   return px * sizeof(float4) * (1 + ((A.use_n || A.use_d) ? 1 : 0) + (A.use_a ? 1 : 0));
@@ -499,7 +500,9 @@ static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, cons
       auto kern = A.r == 2 ? (exact ? k_atrous_tiled<true, 2> : k_atrous_tiled<false, 2>)
                            : (exact ? k_atrous_tiled<true, 0> : k_atrous_tiled<false, 0>);
       if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the most a tile takes, not this launch's: the attribute is the
+        // kernel's, and another thread's smaller launch would lower it
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kAtMaxSmem);
         if (e != cudaSuccess) return e;
       }
       kern<<<(unsigned)blocks, kAtThreads, smem, st>>>(A, (int)tiles_x, in, color, gn, ga, o);

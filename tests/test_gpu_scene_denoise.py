@@ -2,6 +2,7 @@
 against golden vectors from the reference's scene_intersect and
 edge_aware_denoise."""
 import os
+import threading
 
 import numpy as np
 import pytest
@@ -207,3 +208,31 @@ def test_atrous_sigma_of_an_unused_guide_is_ignored(radius, passes, guides, sigm
     got = edge_aware_denoise(src, radius, 0.08, 0.8, passes=passes, **kw, **unused)
     assert np.isfinite(want).all()
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+def test_atrous_tiles_from_several_threads():
+    """Eight threads, each with its own context, at two radii whose tiles ask
+    for different amounts of shared memory: every call is accepted and gives
+    what it gives alone."""
+    rng = np.random.default_rng(4)
+    src, alb = (rng.random((24, 40, 3)).astype(np.float32) for _ in range(2))
+    nrm = rng.normal(size=(24, 40, 3)).astype(np.float32)
+    dep = rng.random((24, 40)).astype(np.float32)
+    ctxs = [nat.Context(0) for _ in range(8)]
+    run = lambda i: nat.denoise(src, normal=nrm, albedo=alb, depth=dep, radius=(8, 5)[i % 2], passes=4, ctx=ctxs[i])
+    want = [run(0), run(1)]
+    wrong = [0] * 8
+
+    def work(i):
+        for _ in range(400):
+            try:
+                wrong[i] += not np.array_equal(run(i), want[i % 2])
+            except Exception:
+                wrong[i] += 1
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not any(wrong)
