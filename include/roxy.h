@@ -328,7 +328,10 @@ int rx_scene_device_bytes(rx_scene* scene, long long* bytes);
  * All pointers are device pointers; `stream` NULL means the context's
  * stream.  Activations are viewed through a channel stride and offset (a
  * concatenation is a wider tensor); channel counts are multiples of 16,
- * strides and offsets multiples of 8.  Weights: [Cout][3][3][Cin] bf16. */
+ * strides and offsets multiples of 8.  Weights: [Cout][3][3][Cin] bf16.
+ * What a convolution reads as an activation or as its kernel's weights (x,
+ * dy, w of the forward call, w_rot) starts on a 16-byte boundary, an output
+ * on a 4-byte one; other pointers are refused with RX_ERR_ARG. */
 typedef struct {
   int N, H, W;            /* images, height, width                    */
   int Cin, Cout;          /* input / output channels                  */

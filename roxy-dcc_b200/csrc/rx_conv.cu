@@ -1464,43 +1464,42 @@ __global__ void __cluster_dims__(kBiasCluster, 1, 1) __launch_bounds__(kBiasThre
   }
 }
 
-// w_rot[ci][tap][co] = w[co][8 - tap][ci]: the weights of the input-gradient
-// convolution (a 3x3 convolution of dy with the flipped, transposed kernel)
-__global__ void k_rot_weights(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
-  long long n = (long long)Cout * 9 * Cin;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    int ci = (int)(i % Cin);
-    int tap = (int)((i / Cin) % 9);
-    int co = (int)(i / ((long long)Cin * 9));
-    wr[((long long)ci * 9 + (8 - tap)) * Cout + co] = w[i];
-  }
-}
-
-// The same with eight output channels per item: lanes read eight weights
-// each along ci and write one 16-byte chunk (Cout is a multiple of 16).  The
-// scalar form's 64-bit divisions and 2-byte stores took 39 us for the ten
-// layers of a training step, this 31 (a launch each).
-__global__ void k_rot_weights_v8(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
-  chain_wait(w, wr);
-  chain_go();
-  const unsigned n = (unsigned)(Cout / 8) * 9u * (unsigned)Cin;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const unsigned t = i / (unsigned)Cin, ci = i - t * (unsigned)Cin;
-    const unsigned co8 = t / 9u, tap = t - co8 * 9u;
-    const bf16* s = w + ((size_t)co8 * 72 + (8 - tap)) * Cin + ci;
-    uint4 v;
-    bf16* e = reinterpret_cast<bf16*>(&v);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) e[k] = s[(size_t)k * 9 * Cin];
-    *reinterpret_cast<uint4*>(wr + ((size_t)ci * 9 + tap) * Cout + co8 * 8) = v;
-  }
-}
-
 // ------------------------------------------------------------ element-wise
 // Every element-wise kernel walks (pixel, channel) of an NHWC view
 // (stride, offset) with a grid-stride loop.
 #define RX_EW_LOOP(count) \
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (count); i += (long long)gridDim.x * blockDim.x)
+
+// w_rot[ci][tap][co] = w[co][8 - tap][ci]: the weights of the input-gradient
+// convolution (a 3x3 convolution of dy with the flipped, transposed kernel).
+// Eight output channels per item: lanes read eight weights each along ci and
+// write one 16-byte chunk (Cout is a multiple of 16).  One weight per item,
+// with 64-bit divisions and 2-byte stores, took 39 us for the ten layers of a
+// training step's gradients, this 31 (a launch each).
+__global__ void k_rot_weights_v8(int Cout, int Cin, const bf16* __restrict__ w, bf16* __restrict__ wr) {
+  chain_wait(w, wr);
+  chain_go();
+  RX_EW_LOOP((long long)(Cout / 8) * 9 * Cin) {
+    size_t ci, tap, co8;
+    if (i <= 0xffffffffLL) {  // 32-bit divisions
+      const unsigned t = (unsigned)i / (unsigned)Cin, c = t / 9u;
+      ci = (unsigned)i - t * (unsigned)Cin;
+      tap = t - c * 9u;
+      co8 = c;
+    } else {
+      const long long t = i / Cin;
+      ci = (size_t)(i - t * Cin);
+      co8 = (size_t)(t / 9);
+      tap = (size_t)t - co8 * 9;
+    }
+    const bf16* s = w + (co8 * 72 + (8 - tap)) * Cin + ci;
+    uint4 v;
+    bf16* e = reinterpret_cast<bf16*>(&v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e[k] = s[(size_t)k * 9 * Cin];
+    *reinterpret_cast<uint4*>(wr + (ci * 9 + tap) * Cout + co8 * 8) = v;
+  }
+}
 
 // dst = src (channels [0, C) of each view); accumulate: dst += src
 __global__ void k_copy_ch(long long P, int C, const bf16* __restrict__ src, int s_stride, int s_off,
@@ -1920,6 +1919,8 @@ static bool conv_ok(const rx_conv_desc* d) {
          d->y_coff % 8 == 0 && d->x_coff + d->Cin <= d->x_cstride && d->y_coff + d->Cout <= d->y_cstride;
 }
 
+static bool unaligned(const void* p, size_t bytes) { return (uintptr_t)p % bytes != 0; }
+
 template <int COUT>
 static int launch_tc(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const bf16* w, const float* bias, bf16* y,
                      float* y32, int relu, cudaStream_t st) {
@@ -2178,6 +2179,10 @@ int conv_fwd(Ctx* ctx, const rx_conv_desc* d, const void* x, const void* w, cons
              int relu, cudaStream_t st) {
   if (!conv_ok(d) || !x || !w || !y)
     return set_error(ctx, "conv_bf16_fwd: bad descriptor (channels multiples of 16, strides of 8)"), RX_ERR_ARG;
+  // every kernel copies x and w in 16-byte pieces, the mma.sync ones store
+  // pairs of channels
+  if (unaligned(x, 16) || unaligned(w, 16) || unaligned(y, 4) || unaligned(bias, 4) || unaligned(y32, 4))
+    return set_error(ctx, "conv_bf16_fwd: x and w must be 16-byte aligned, y, y32 and bias 4"), RX_ERR_ARG;
   if (ctx->conv_impl == 0) {
     int rc = RX_OK;
     if (launch_ws(ctx, d, static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias, static_cast<bf16*>(y), y32,
@@ -2185,7 +2190,7 @@ int conv_fwd(Ctx* ctx, const rx_conv_desc* d, const void* x, const void* w, cons
         launch_ws_split(ctx, d, static_cast<const bf16*>(x), static_cast<const bf16*>(w), bias,
                         static_cast<bf16*>(y), y32, relu, st, &rc))
       return rc;
-  } else if (ctx->conv_impl == 2 && d->H <= 65535 && d->N <= 65535) {
+  } else if (ctx->conv_impl == 2 && d->H <= 65535 && d->N <= 65535 && !unaligned(y, 16)) {
     const bf16* xb = static_cast<const bf16*>(x);
     const bf16* wb = static_cast<const bf16*>(w);
     bf16* yb = static_cast<bf16*>(y);
@@ -2230,13 +2235,10 @@ int conv_bwd_data(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* w
                   cudaStream_t st) {
   if (!conv_ok(d) || !dy || !w || !w_rot || !dx) return set_error(ctx, "conv_bf16_bwd_data: bad arguments"), RX_ERR_ARG;
   long long nw = (long long)d->Cout * 9 * d->Cin;
-  // whole 16-byte chunks where the buffer allows them and 32 bits count them
-  if (((uintptr_t)w_rot & 15) == 0 && nw / 8 <= 0x7fffffffLL)
-    launch_chained(st, true, dim3(ew_blocks(ctx, nw / 8)), 256, 0, k_rot_weights_v8,
-                   d->Cout, d->Cin, static_cast<const bf16*>(w), static_cast<bf16*>(w_rot));
-  else
-    k_rot_weights<<<ew_blocks(ctx, nw), 256, 0, st>>>(d->Cout, d->Cin, static_cast<const bf16*>(w),
-                                                     static_cast<bf16*>(w_rot));
+  if (unaligned(dy, 16) || unaligned(w_rot, 16) || unaligned(w, 2) || unaligned(dx, 4))
+    return set_error(ctx, "conv_bf16_bwd_data: dy and w_rot must be 16-byte aligned, dx 4"), RX_ERR_ARG;
+  launch_chained(st, true, dim3(ew_blocks(ctx, nw / 8)), 256, 0, k_rot_weights_v8, d->Cout, d->Cin,
+                 static_cast<const bf16*>(w), static_cast<bf16*>(w_rot));
   CUDA_TRY(ctx, cudaGetLastError());
   // dx = conv(dy, w_rot): input channels Cout (read from the y view), output Cin (the x view)
   rx_conv_desc t = *d;
@@ -2259,10 +2261,9 @@ static int wgrad_chain(Ctx* ctx, const rx_conv_desc* d) {
 }
 
 // Weight gradient on k_conv_wgrad_ws.  Returns 1 if it launched, 0 if the
-// shape or the pointers do not suit it.
+// shape does not suit it.
 static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, const bf16* x, float* dw, cudaStream_t st,
                            int* rc) {
-  if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15)) return 0;
   const int limit = 232448 - 1024;  // opt-in shared memory per block, less the static part
   static int attr_dev = -1;
   if (attr_dev != ctx->device) {
@@ -2342,6 +2343,8 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
 int conv_bwd_weight(Ctx* ctx, const rx_conv_desc* d, const void* dy, const void* x, float* dw, float* db,
                     cudaStream_t st) {
   if (!conv_ok(d) || !dy || !x || !dw) return set_error(ctx, "conv_bf16_bwd_weight: bad arguments"), RX_ERR_ARG;
+  if (unaligned(dy, 16) || unaligned(x, 16) || unaligned(dw, 4) || unaligned(db, 4))
+    return set_error(ctx, "conv_bf16_bwd_weight: dy and x must be 16-byte aligned, dw and dbias 4"), RX_ERR_ARG;
   long long P = (long long)d->N * d->H * d->W;
   int rc = RX_OK;
   const bool ws = ctx->conv_impl == 0 && launch_wgrad_ws(ctx, d, static_cast<const bf16*>(dy),

@@ -493,3 +493,36 @@ def test_resident_weight_conv_from_several_threads():
         c.sync()
     assert not any(fails)
     assert all(torch.equal(data[i][2], want[i]) for i in range(len(cases)))
+
+
+def test_unaligned_buffers_are_refused_or_served(impl):
+    """What the kernels copy in 16-byte pieces is refused where it does not
+    start on such a boundary, before anything is enqueued; an output on a
+    4-byte one is served, with the bits of an aligned one."""
+    ctx, L = _ctx(), nat.lib()
+    N, H, W, ci, co = 1, 5, 33, 64, 32
+    g = torch.Generator(device="cuda").manual_seed(8)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    x, w, dy = rnd(N * H * W * ci + 8), rnd(co * 9 * ci + 8), rnd(N * H * W * co + 8)
+    rot, y = torch.zeros_like(w), torch.zeros_like(dy)
+    dw, db, bias = torch.zeros((co, 9, ci), device="cuda"), torch.zeros(co, device="cuda"), torch.zeros(co, device="cuda")
+    at = lambda t, n: ctypes.c_void_p(t.data_ptr() + n)  # noqa: E731
+    d = ctypes.byref(nat.ConvDesc(N, H, W, ci, co, ci, 0, co, 0))
+    fwd = lambda a, b, c: L.rx_conv_bf16_fwd(ctx.h, d, at(x, a), at(w, b), _p(bias), at(y, c), None, 0, _stream())  # noqa: E731
+    bwd = lambda a, b, c: L.rx_conv_bf16_bwd_data(ctx.h, d, at(dy, a), at(w, 2), at(rot, b), at(x, c), _stream())  # noqa: E731
+    wgt = lambda a, b: L.rx_conv_bf16_bwd_weight(ctx.h, d, at(dy, a), at(x, b), _p(dw), _p(db), _stream())  # noqa: E731
+    keep = x.clone()
+    for k in (2, 4, 8):
+        assert fwd(k, 0, 0) == fwd(0, k, 0) == bwd(k, 0, 0) == bwd(0, k, 0) == wgt(k, 0) == wgt(0, k) == nat.RX_ERR_ARG
+    assert fwd(0, 0, 2) == bwd(0, 0, 2) == nat.RX_ERR_ARG
+    torch.cuda.synchronize()
+    assert not rot.any() and not y.any() and not dw.any() and torch.equal(x, keep)
+    assert fwd(0, 0, 4) == 0
+    torch.cuda.synchronize()
+    off = y[2:2 + N * H * W * co].clone()
+    ctx.check(L.rx_conv_set_impl(ctx.h, 1))
+    assert fwd(0, 0, 0) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(off, y[:N * H * W * co]) and bool(off.any())
+    assert bwd(0, 0, 4) == 0 and wgt(0, 0) == 0
+    ctx.sync()
