@@ -210,7 +210,11 @@ struct ResShape {
   static size_t smem(int cl) { return (size_t)W_BYTES + 2 * (size_t)halo(cl); }
 };
 
-template <int BN, int KS>
+// BIAS: there is one.  Its values sit in registers from the start, as a load
+// behind the wait; 32 -> 96 channels at 16x128x128 and 64 -> 192 at 16x64x64,
+// back to back: 63 and 50 us (59 and 50 without a bias; read in the epilogue
+// through the untied pointer 72 and 57).
+template <int BN, int KS, bool BIAS>
 __global__ void __launch_bounds__(256, 1)
     k_conv_fwd_res(rx_conv_desc d, const bf16* __restrict__ x, const bf16* __restrict__ w,
                    const float* __restrict__ bias, bf16* __restrict__ y, float* __restrict__ y32, int relu, int cl,
@@ -248,8 +252,16 @@ __global__ void __launch_bounds__(256, 1)
     }
   };
 
-  chain_wait(x, w);  // bias: read behind the loops below only; through here it costs the epilogue 12 %
+  chain_wait(x, w, bias);
   chain_go();
+  float bias_of[NT][2] = {};  // this lane's channels
+  if constexpr (BIAS) {
+#pragma unroll
+    for (int ni = 0; ni < NT; ++ni) {
+      const int co = n0 + wn * (BN / 2) + ni * 8 + 2 * (lane & 3);
+      if (co < d.Cout) bias_of[ni][0] = bias[co], bias_of[ni][1] = bias[co + 1];
+    }
+  }
   for (int c = tid; c < BN * 9 * KC; c += 256) {
     const int row = c / (9 * KC), k = c - row * (9 * KC);
     const bool ok = n0 + row < d.Cout;
@@ -322,9 +334,9 @@ __global__ void __launch_bounds__(256, 1)
           const int co = n0 + wn * (BN / 2) + ni * 8 + 2 * q;
           if (co >= d.Cout) continue;
           float v0 = acc[mi][ni][2 * h], v1 = acc[mi][ni][2 * h + 1];
-          if (bias) {
-            v0 += bias[co];
-            v1 += bias[co + 1];
+          if constexpr (BIAS) {
+            v0 += bias_of[ni][0];
+            v1 += bias_of[ni][1];
           }
           if (relu) {
             v0 = fmaxf(v0, 0.0f);
@@ -2134,7 +2146,7 @@ static int launch_res_as(Ctx* ctx, const rx_conv_desc* d, const bf16* x, const b
   }
   const int limit = 232448;  // opt-in shared memory per block
   if (best * d->N > 0x3fffffffLL || S::smem(cl) > (size_t)limit) return 0;
-  auto kern = k_conv_fwd_res<BN, KS>;
+  auto kern = bias ? k_conv_fwd_res<BN, KS, true> : k_conv_fwd_res<BN, KS, false>;
   const int smem = sole_block_smem(ctx, 0, (int)S::smem(cl));
   // the limit, not this launch's size: the attribute is the kernel's, and
   // another thread's smaller launch would take it from under this one

@@ -54,3 +54,32 @@ def test_errors_without_device_are_reported_not_raised(L):
     L.rx_device_count(ctypes.byref(n))
     assert n.value >= 0
     assert L.rx_version() >= 1
+
+
+def _chained_kernels():
+    """(kernel, pointers it only reads, what its chain_wait ties) of every
+    kernel that may come up while the one before it runs."""
+    csrc = os.path.join(os.path.dirname(nat.LIB_PATH), "csrc")
+    for f in sorted(os.listdir(csrc)):
+        if not f.endswith(".cu"):
+            continue
+        src = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        for part in re.split(r"\b__global__\b", src)[1:]:
+            m = re.match(r"[^{;]*?\b(k_\w+)\s*\(((?:[^(){}]|\([^()]*\))*)\)\s*\{", part, re.S)
+            assert m, part[:200]
+            body = part[m.end():]
+            end = re.search(r"^\}", body, re.M)
+            w = re.search(r"\bchain_wait\(([^()]*)\)", body[:end.start()])
+            if w:
+                reads = re.findall(r"\bconst\s+\w+\s*\*\s*(?:__restrict__\s*)?(\w+)", m.group(2))
+                yield m.group(1), reads, [a.strip() for a in w.group(1).split(",")]
+
+
+def test_chained_kernels_tie_what_they_read_to_the_wait():
+    """A load through a const pointer that did not pass through chain_wait may
+    be moved before it, ahead of the kernel that writes the memory."""
+    found = list(_chained_kernels())
+    assert len(found) >= 20
+    assert {"k_conv_fwd_ws", "k_conv_fwd_res", "k_atrous_r1", "k_lbvh_bottom_up"} <= {k for k, _, _ in found}
+    loose = {k: sorted(set(reads) - set(tied)) for k, reads, tied in found}
+    assert not {k: v for k, v in loose.items() if v}
