@@ -18,7 +18,7 @@ LIB_PATH = os.environ.get("ROXY_CUDA_LIB") or os.path.join(HERE, "libroxy_cuda.s
 REPO = os.path.dirname(HERE)
 SOURCES = ["rx_api.cu", "rx_bvh.cu", "rx_extract.cu", "rx_trace.cu", "rx_render.cu", "rx_denoise.cu",
            "rx_serve.cu", "rx_conv.cu", "rx_obj.cu", "rx_hostcopy.cu"]
-HEADERS = ["rx_internal.cuh", "rx_runtime.h"]
+HEADERS = ["rx_internal.cuh", "rx_runtime.h", "rx_wave.h"]
 
 RX_OK, RX_ERR_ARG, RX_ERR_CAPACITY, RX_ERR_CUDA, RX_ERR_STATE, RX_ERR_DEVICE, RX_ERR_TIMEOUT = range(7)
 RX_REQ_QUEUED, RX_REQ_ACTIVE, RX_REQ_DONE, RX_REQ_FAILED = range(4)

@@ -1,7 +1,9 @@
 """The C-ABI library loads and exports every entry point include/roxy.h declares
 (no device needed; nothing here launches a kernel)."""
+import ctypes
 import os
 import re
+import subprocess
 
 import pytest
 
@@ -83,3 +85,44 @@ def test_chained_kernels_tie_what_they_read_to_the_wait():
     assert {"k_conv_fwd_ws", "k_conv_fwd_res", "k_atrous_r1", "k_lbvh_bottom_up"} <= {k for k, _, _ in found}
     loose = {k: sorted(set(reads) - set(tied)) for k, reads, tied in found}
     assert not {k: v for k, v in loose.items() if v}
+
+
+_WAVE_CPP = """
+#include "rx_wave.h"
+extern "C" long long wave(long long frames, long long P, long long cap, long long shadow_cap, long long per_shadow,
+                          long long free_bytes, int* asked) {
+  return rx::default_wave_paths(frames, P, cap, shadow_cap, per_shadow, [&] { ++*asked; return free_bytes; });
+}
+"""
+
+
+def test_free_memory_is_asked_for_only_while_the_buffers_do_not_hold_the_wave(tmp_path):
+    """Images that do and do not divide the largest wave, one call after
+    another: once the buffers hold the wave that a call takes, no later call
+    like it asks (the question can stall for tens of milliseconds)."""
+    (tmp_path / "wave.cpp").write_text(_WAVE_CPP)
+    so = tmp_path / "wave.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I",
+                    os.path.join(os.path.dirname(nat.LIB_PATH), "csrc"), "-o", so, tmp_path / "wave.cpp"], check=True)
+    f = ctypes.CDLL(str(so)).wave
+    f.restype, f.argtypes = ctypes.c_longlong, [ctypes.c_longlong] * 6 + [ctypes.POINTER(ctypes.c_int)]
+    big = 180 << 30
+
+    def call(frames, P, held, per, free):
+        asked = ctypes.c_int(0)
+        target = f(frames, P, held, held * per, per, free, ctypes.byref(asked))
+        return target, max(1, min(frames, target // P)) * P, asked.value
+
+    for P in (64 * 64, 1024 * 1024, 1920 * 1080, 1917 * 1081, 3840 * 2160, 7680 * 4320, 12000 * 12000):
+        for frames in (1, 7, 64, 65, 100, 4096):
+            for per in (1, 5):
+                target, wave, asked = call(frames, P, 0, per, big)
+                assert target == 1 << 27 and asked == (wave > 1 << 25)
+                assert call(frames, P, wave, per, big) == (target, wave, 0), (P, frames)
+                # held for a smaller wave than this call's: asked again
+                if wave > 1 << 25:
+                    assert call(frames, P, wave - 1, per, big)[2] == 1
+    # a quarter of the free memory decides between 32 M and 128 M paths
+    need = lambda paths: 4 * paths * (120 + 48)  # noqa: E731
+    for free, want in ((need(1 << 27), 27), (need(1 << 27) - 4, 26), (need(1 << 26) - 4, 25), (0, 25)):
+        assert call(4096, 1920 * 1080, 0, 1, free)[0] == 1 << want
