@@ -448,9 +448,10 @@ static size_t atrous_smem(const AtrousArgs& A) {
 
 // Enqueues `passes` a-trous passes on `st`: pass i reads `in` (the colour for
 // i = 0) and writes scratch half (i & 1), the last pass writes `out` (and
-// reads `color` again for the blend).  A is filled except step / last.
-static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, const float4* color, const float4* gn,
-                                 const float4* ga, float4* out, float4* s0, float4* s1) {
+// reads `color` again for the blend).  A is filled except step / last; sms: the
+// device's SMs.
+static cudaError_t atrous_passes(cudaStream_t st, int sms, AtrousArgs A, int passes, const float4* color,
+                                 const float4* gn, const float4* ga, float4* out, float4* s0, float4* s1) {
   const long long P = (long long)A.H * A.W;
   // k_atrous_r1 evaluates the terms of unused guides on zeros: whatever their
   // sigma holds (a NaN, too), they must come to exactly 1
@@ -475,7 +476,7 @@ static cudaError_t atrous_passes(cudaStream_t st, AtrousArgs A, int passes, cons
       // cost is waves x (r + 2).  1280x720, later passes, us for all five:
       // 3 rows 113, 4 104, 6 98, 8 111, 12 97, 16 107 by this rule's
       // 20, 18, 16, 20, 14, 18; 640x360: 2 rows 43, 3 35, 4 41.
-      const long long cap = 148LL * kA1Warps * a1_blocks(exact, guides);
+      const long long cap = (long long)sms * kA1Warps * a1_blocks(exact, guides);
       long long rows = 1, best = LLONG_MAX;
       for (long long r = 1; r <= kA1MaxRows && r <= sub_h; ++r) {
         const long long n = per_row * ((sub_h + r - 1) / r), cost = (n + cap - 1) / cap * (r + 2);
@@ -546,7 +547,7 @@ int denoise_device(Ctx* ctx, int h, int w, const float4* d_color, const float4* 
   A.keep = (float)(1.0 - amount);
   A.amount = (float)amount;
   A.to_display = to_display;
-  CUDA_TRY(ctx, atrous_passes(st, A, passes, d_color, d_gn, d_ga, d_out, d_s0, d_s1));
+  CUDA_TRY(ctx, atrous_passes(st, ctx->num_sms, A, passes, d_color, d_gn, d_ga, d_out, d_s0, d_s1));
   return RX_OK;
 }
 
@@ -753,7 +754,11 @@ extern "C" int rx_denoise_noalloc(int height, int width, const float* d_color, c
     A.keep = (float)(1.0 - amount);
     A.amount = (float)amount;
     A.to_display = params->to_display;
-    e = atrous_passes(st, A, params->passes, color, gn, ga, out, scratch, scratch + kNoAllocMaxPixels);
+    int dev = 0, sms = 1;
+    e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+      e = atrous_passes(st, sms, A, params->passes, color, gn, ga, out, scratch, scratch + kNoAllocMaxPixels);
   }
   if (e != cudaSuccess)
     return set_error(nullptr, "rx_denoise_noalloc: launch failed: %s", cudaGetErrorString(e)), RX_ERR_CUDA;

@@ -409,15 +409,15 @@ __device__ __forceinline__ float div_by(float x, float d, float r) {
 }
 
 // Rays a warp of k_extend or of a query takes at a time: 32, or fewer while
-// the rays would leave the device with less than eight warps per SM.  A warp's
-// time is its slowest ray's, and fewer rays diverge less; with more warps than
-// that asked for (16 per SM, or all that fit) the closed box's short queues
-// lose 3 % to idle lanes, as they do with k_tail's paths spread.  Query of 100
-// rays 32 -> 15 us, 1,000 56 -> 37, 10,000 95 -> 92; 160x90 view 0.44 ->
-// 0.39 ms, 64x64 closed box 0.404 -> 0.409; from 38 k rays on it is 32.
-__host__ __device__ __forceinline__ int warp_items(long long total) {
-  constexpr long long kWarps = 148 * 8;
-  const long long take = (total + kWarps - 1) / kWarps;
+// the rays would leave the device (sms SMs) with less than eight warps per
+// SM.  A warp's time is its slowest ray's, and fewer rays diverge less; with
+// more warps than that asked for (16 per SM, or all that fit) the closed box's
+// short queues lose 3 % to idle lanes, as they do with k_tail's paths spread.
+// Query of 100 rays 32 -> 15 us, 1,000 56 -> 37, 10,000 95 -> 92; 160x90 view
+// 0.44 -> 0.39 ms, 64x64 closed box 0.404 -> 0.409; on 148 SMs it is 32 from
+// 36,705 rays on.
+__host__ __device__ __forceinline__ int warp_items(long long total, int sms) {
+  const long long warps = 8LL * sms, take = (total + warps - 1) / warps;
   return take > 32 ? 32 : take < 1 ? 1 : (int)take;
 }
 

@@ -559,7 +559,7 @@ template <bool EXACT, class Src, int BS, bool CAM = false>
 __global__ void __launch_bounds__(BS, 1024 / BS)
     k_extend(Src src, int b, const int* __restrict__ qin, int* counters, const float4* __restrict__ ray,
              float4* __restrict__ hits, int sb, const float4* __restrict__ shadow,
-             float4* __restrict__ rad, long long shadow_cap, int* err) {
+             float4* __restrict__ rad, long long shadow_cap, int sms, int* err) {
   // Items [0, n): closest hit of bounce b's queue.  Items [n, n + ns): the
   // shadow rays bounce sb (the previous one) emitted, traced any-hit here so
   // they share this launch instead of paying for a small one of their own.
@@ -576,7 +576,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
   const int total = n + (int)ns;
   int* fetch = &counters[C_FE + (b >= 0 ? b : kMaxBounce - 1)];
   const int lane = threadIdx.x & 31;
-  const int take = warp_items(total);
+  const int take = warp_items(total, sms);
   int run_job = -1, run_rays = 0;  // batches: rays of this warp's current job, not yet added to its count
   for (;;) {
     int base = 0;
@@ -1476,7 +1476,7 @@ static void launch_extend(Accum* a, const DevScene& S, const RenderK& K, int b, 
   SingleSrc src{S, K, a->frame_base.p, wave_phase(a, K)};
   auto go = [&](auto kernel) {
     kernel<<<a->occ_ext, 128, 0, ctx->stream>>>(src, b, qin, a->counters.p, a->ray.p, a->hits.p, sb,
-                                                 a->shadow.p, a->rad.p, K.shadow_cap, ctx->d_err);
+                                                 a->shadow.p, a->rad.p, K.shadow_cap, ctx->num_sms, ctx->d_err);
   };
   const bool cam = b == 0 && K.camera0;
   if (S.exact_slab) {
@@ -1991,7 +1991,7 @@ template <int BS>
 static void launch_extend_batch(Batch* B, const BatchSrc& src, bool wide, int occ, int b, const int* qin, int sb) {
   auto go = [&](auto kernel, const auto& s) {
     kernel<<<occ, BS, 0, B->ctx->stream>>>(s, b, qin, B->counters.p, B->ray.p, B->hits.p, sb,
-                                           B->shadow.p, B->rad.p, B->shadow_cap, B->ctx->d_err);
+                                           B->shadow.p, B->rad.p, B->shadow_cap, B->ctx->num_sms, B->ctx->d_err);
   };
   if (wide) go(k_extend<false, BatchSrc4, BS>, BatchSrc4{src});
   else go(k_extend<false, BatchSrc, BS>, src);

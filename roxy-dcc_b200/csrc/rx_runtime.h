@@ -18,7 +18,7 @@ namespace rx {
 struct Ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
-  int num_sms = 148;
+  int num_sms = 1;  // rx_ctx_create asks the device
   std::string err;
   std::recursive_mutex mu;
   std::atomic<int> hold_waiters{0};  // threads blocked in rx_ctx_hold (the serving loop lets them go first)

@@ -118,7 +118,7 @@ int trace_closest(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d
                   float* d_u, float* d_v) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
-  const int take = warp_items(n);
+  const int take = warp_items(n, ctx->num_sms);
   if (S.exact_slab)
     k_trace_closest<true><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_t, d_id, d_u,
                                                                                 d_v, ctx->d_err);
@@ -132,7 +132,7 @@ int trace_closest(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d
 int trace_any(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d_rd, const float* d_tmax, int* d_occ) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
-  const int take = warp_items(n);
+  const int take = warp_items(n, ctx->num_sms);
   if (S.exact_slab)
     k_trace_any<true><<<grid_for_rays(ctx, n, take), 128, 0, ctx->stream>>>(S, n, take, d_ro, d_rd, d_tmax, d_occ,
                                                                             ctx->d_err);
@@ -147,7 +147,7 @@ int scene_query(Ctx* ctx, Scene* sc, long n, const float* d_ro, const float* d_r
                 int* d_id, float* d_u, float* d_v, float* d_n) {
   DevScene S = sc->view();
   if (n <= 0) return RX_OK;
-  const int take = warp_items(n);
+  const int take = warp_items(n, ctx->num_sms);
   DevBuf<int> lin(ctx, std::max<size_t>(sc->lin_slot.size(), 1));
   if (!lin.ok()) return set_error(ctx, "scene query: out of device memory"), RX_ERR_CAPACITY;
   if (!sc->lin_slot.empty())

@@ -253,3 +253,23 @@ def test_wide_nodes_find_what_the_reference_tree_finds(n, scale, offset):
     np.testing.assert_array_equal(t0.view(np.uint32), t1.view(np.uint32))
     tmax = rng.uniform(0.0, 3.0 * scale, m).astype(np.float32)
     np.testing.assert_array_equal(wide.trace_any(ro, rd, tmax), ref.trace_any(ro, rd, tmax))
+
+
+@pytest.mark.parametrize("n", [8_001, 20_000, 36_704, 36_705])
+def test_query_lanes_up_to_whole_warps(n):
+    """Odd numbers of rays per warp (7, 17, 31, then 32 from 36,705 rays on
+    148 SMs), the hits with normals among the queries: the answers of a query
+    of 60,000 rays."""
+    v0, v1, v2 = gs.soup_triangles(3000, 11)
+    sc = _scene(v0, v1, v2, nat.RX_BVH_LBVH_SAH, 4)
+    rng = np.random.default_rng(2)
+    ro = rng.normal(size=(60_000, 3)).astype(np.float32) * 2
+    rd = rng.normal(size=(60_000, 3)).astype(np.float32)
+    rd /= np.linalg.norm(rd, axis=1, keepdims=True)
+    tm = rng.uniform(0.1, 4.0, 60_000).astype(np.float32)
+    for a, b in zip(sc.trace_closest(ro, rd), sc.trace_closest(ro[-n:], rd[-n:])):
+        assert np.array_equal(a[-n:].view(np.int32), b.view(np.int32))
+    assert np.array_equal(sc.trace_any(ro, rd, tm)[-n:], sc.trace_any(ro[-n:], rd[-n:], tm[-n:]))
+    whole, part = sc.intersect(ro, rd), sc.intersect(ro[-n:], rd[-n:])
+    for k in whole:
+        assert np.array_equal(whole[k][-n:].view(np.int32), part[k].view(np.int32)), k

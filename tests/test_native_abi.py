@@ -126,3 +126,12 @@ def test_free_memory_is_asked_for_only_while_the_buffers_do_not_hold_the_wave(tm
     need = lambda paths: 4 * paths * (120 + 48)  # noqa: E731
     for free, want in ((need(1 << 27), 27), (need(1 << 27) - 4, 26), (need(1 << 26) - 4, 25), (0, 25)):
         assert call(4096, 1920 * 1080, 0, 1, free)[0] == 1 << want
+
+
+def test_no_device_size_is_written_into_the_code():
+    """The number of SMs comes from the device (Ctx::num_sms), so that rules
+    that fill it hold on a part of one, too."""
+    csrc = os.path.join(os.path.dirname(nat.LIB_PATH), "csrc")
+    for f in sorted(os.listdir(csrc)):
+        code = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(csrc, f)).read(), flags=re.S)
+        assert not re.search(r"\b148(?:LL|u|U)?\b", code), f
