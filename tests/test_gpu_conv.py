@@ -526,3 +526,68 @@ def test_unaligned_buffers_are_refused_or_served(impl):
     assert torch.equal(off, y[:N * H * W * co]) and bool(off.any())
     assert bwd(0, 0, 4) == 0 and wgt(0, 0) == 0
     ctx.sync()
+
+
+@pytest.mark.parametrize("P,Cout,stride,off", [(1, 16, 16, 0), (37, 48, 64, 8), (70001, 16, 96, 64), (263, 2064, 2064, 0),
+                                               (262147, 16, 16, 0), (100003, 48, 48, 0)])
+def test_bias_gradient_is_exact_on_small_integers(P, Cout, stride, off):
+    """Sums of integers below 2^24 are exact in any order, so a pixel that is
+    lost or taken twice -- in a lane, block or cluster, eight of those from
+    229,377 pixels of 16 channels on -- shows."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(P)
+    dy = torch.randint(1, 4, (1, 1, P, stride), generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.zeros((1, 1, P, 16), dtype=torch.bfloat16, device="cuda")
+    dw, db = torch.zeros((Cout, 9, 16), device="cuda"), torch.ones(Cout, device="cuda")
+    d = nat.ConvDesc(1, 1, P, 16, Cout, 16, 0, stride, off)
+    ctx.check(nat.lib().rx_conv_bf16_bwd_weight(ctx.h, ctypes.byref(d), _p(dy), _p(x), _p(dw), _p(db), _stream()))
+    ctx.check(nat.lib().rx_ctx_sync(ctx.h))
+    assert torch.equal(db.double(), _view(dy, off, Cout).double().reshape(P, Cout).sum(0) + 1.0)
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,xs,xo,ys,yo", [
+    (3, 90, 130, 16, 48, 16, 0, 48, 0),       # strips over several blocks and images, a two-pixel second tile
+    (2, 100, 128, 96, 32, 96, 0, 32, 0),      # whole tiles
+    (5, 64, 64, 64, 64, 72, 8, 96, 32),       # several taps' groups
+    (2, 57, 33, 128, 128, 128, 0, 192, 64),
+    (1, 61, 300, 272, 16, 272, 0, 16, 0),     # three input groups
+])
+def test_weight_gradient_is_exact_on_small_integers(N, H, W, Cin, Cout, xs, xo, ys, yo):
+    """The same for the weight gradient: products of integers up to 3, sums
+    below 2^24, so a row, a strip's end or an image border that is lost,
+    taken twice or shifted shows."""
+    assert 9 * N * H * W < 2 ** 24
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(H * 1000 + W)
+    x = torch.randint(-3, 4, (N, H, W, xs), generator=g, device="cuda").to(torch.bfloat16)
+    dy = torch.randint(-3, 4, (N, H, W, ys), generator=g, device="cuda").to(torch.bfloat16)
+    dw = torch.ones((Cout, 9, Cin), device="cuda")
+    d = nat.ConvDesc(N, H, W, Cin, Cout, xs, xo, ys, yo)
+    ctx.check(nat.lib().rx_conv_bf16_bwd_weight(ctx.h, ctypes.byref(d), _p(dy), _p(x), _p(dw), None, _stream()))
+    ctx.check(nat.lib().rx_ctx_sync(ctx.h))
+    xv = F.pad(_view(x, xo, Cin).double(), (0, 0, 1, 1, 1, 1))
+    dv = _view(dy, yo, Cout).double().reshape(-1, Cout)
+    for tap in range(9):
+        cols = xv[:, tap // 3:tap // 3 + H, tap % 3:tap % 3 + W].reshape(-1, Cin)
+        assert torch.equal(dw[:, tap].double(), dv.t() @ cols + 1.0), tap
+
+
+@pytest.mark.parametrize("P", [1, 1023, 1025, 151_553, 262_147])
+@pytest.mark.parametrize("gs,with_base", [(16, True), (12, False)])
+def test_loss_is_exact_on_quarters(P, gs, with_base):
+    """Distances that are multiples of 1/4 with a sum below 2^22: exact in
+    float32, so a pixel or block that the reduction loses shows; up to more
+    pixels than one per thread of a block per SM."""
+    ctx = _ctx()
+    g = torch.Generator(device="cuda").manual_seed(P)
+    quarters = lambda *s: torch.randint(-4, 5, s, generator=g, device="cuda").float() / 4  # noqa: E731
+    y32, base, t = quarters(P, 16), quarters(P, 3) if with_base else None, quarters(P, 3)
+    gr = torch.empty((P, gs), dtype=torch.bfloat16, device="cuda")
+    loss = torch.ones(1, device="cuda")
+    ctx.check(nat.lib().rx_dn_l1_loss(ctx.h, P, _p(y32), 16, _p(base), _p(t), ctypes.c_float(0.5), _p(gr), gs,
+                                      _p(loss), _stream()))
+    torch.cuda.synchronize()
+    dlt = y32[:, :3].double() + (base.double() if with_base else 0.0) - t.double()
+    want = dlt.abs().sum() + 1.0
+    assert want < 2 ** 22 and float(loss) == float(want)
+    assert torch.equal(gr[:, :3].double(), torch.sign(dlt) * 0.5)
