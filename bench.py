@@ -338,13 +338,17 @@ def run_ours(args):
     cam_rays = W * H * w["spp"]
     ext_bytes = 40.0 * max(ext_rays - cam_rays, 0) + 16.0 * min(cam_rays, ext_rays)
     ext_gbs = ext_bytes / (ext_ms / 1e3) / 1e9 if ext_ms > 0 else 0.0
-    # k_shade: 272 B per ray, less the 48 B of ray state a camera ray does
-    # not read at bounce 0.  64 B of it (the hit triangle's normals and
-    # palette index, the material record) come from the scene, which stays
-    # in L2; the rest is path state streamed through HBM.
-    shade_bytes = 272.0 * ext_rays - 48.0 * min(cam_rays, ext_rays)
+    # k_shade, what every ray surely moves through HBM: a camera ray its hit
+    # record in and its radiance out (32 B); a later ray its state written by
+    # the bounce before (ray, throughput, queue entry: 52 B) and read with its
+    # hit record (68 B); a shadow ray its record (48 B).  Guides (32 B of a
+    # camera ray that hits) and radiance updates are not counted.  64 B per
+    # later ray (the hit triangle's normals and palette index, the material
+    # record) come from the scene, which stays in L2.
+    later_rays = max(ext_rays - cam_rays, 0)
+    shade_hbm = 32.0 * min(cam_rays, ext_rays) + 120.0 * later_rays + 48.0 * max(per_step - ext_rays, 0)
+    shade_bytes = shade_hbm + 64.0 * later_rays
     shade_gbs = shade_bytes / (shade_ms / 1e3) / 1e9 if shade_ms > 0 else 0.0
-    shade_hbm = shade_bytes - 64.0 * ext_rays
     shade_hbm_gbs = shade_hbm / (shade_ms / 1e3) / 1e9 if shade_ms > 0 else 0.0
     # DRAM bytes per k_extend launch: ncu's DRAM bytes per closest-hit ray
     # (committed summary: one-pass DRAM counters over the 12 extend launches
@@ -433,7 +437,7 @@ def run_ours(args):
                                        "ms_per_step": shade_ms,
                                        "hbm_streamed": {"achieved": shade_hbm_gbs, "frac": shade_hbm_gbs / peak,
                                                         "bytes_per_ray": shade_hbm / max(ext_rays, 1),
-                                                        "note": "algorithmic bytes less the 64 B per ray read "
+                                                        "note": "algorithmic bytes less the 64 B per later ray read "
                                                                 "from the L2-resident scene"},
                                        "dram_bytes_per_ray_small_case": shade_dram},
                              "accumulate": {"achieved": acc_gbs, "frac": acc_gbs / peak, "ms_per_step": acc_ms,
