@@ -9,9 +9,12 @@
 // weights [Cout][3][3][Cin] bf16 (K = tap * Cin + ci), biases fp32.
 // Channel counts are multiples of 16.
 //
-// Tensor-core path: tiles staged in shared memory by cp.async (16-byte
-// copies, zero-filled outside the image), fragments loaded with ldmatrix
-// and multiplied with mma.sync m16n8k16 bf16 -> f32.
+// Two tensor-core paths.  tcgen05: rows in shared memory by TMA (zero-filled
+// outside the image), one elected thread issuing operations that accumulate in
+// tensor memory (k_conv_fwd_ws, k_conv_wgrad_ws; k_conv_fwd_tc streams its
+// weights).  mma.sync m16n8k16 bf16 -> f32 for the shapes those do not take:
+// tiles by cp.async (16-byte copies, zero-filled outside the image), fragments
+// by ldmatrix (k_conv_fwd_res, k_conv_fwd, k_conv_wgrad).
 #include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -200,8 +203,8 @@ __global__ void __launch_bounds__(128) k_conv_fwd(rx_conv_desc d, const bf16* __
 // products); a tap is an offset of the ldmatrix addresses.  Tiles are
 // 128 pixels of 128 >> cl rows by 1 << cl columns.  Pixel and weight rows are
 // padded to an odd number of 16-byte chunks: no bank conflicts.  121 -> 65 and
-// 97 -> 56 us; mma.sync keeps the tensor pipe 45-53 % busy with the two warps
-// per scheduler that the weights leave room for (its floor is 29 us).
+// 97 -> 56 us; mma.sync keeps the tensor pipe 46-54 % busy (ncu) with the two
+// warps per scheduler that the weights leave room for (its floor is 29 us).
 template <int BN, int KS>
 struct ResShape {
   static constexpr int CIN = 16 * KS, PX = CIN + 8, WROW = 9 * CIN + 8;  // elements
@@ -588,9 +591,10 @@ __global__ void __launch_bounds__(128, 1) k_conv_fwd_tc(rx_conv_desc d, const bf
 // MMAs are waited for (bounded), the device error flag is set.
 // Bound by the MMAs' A-operand reads (40-48 cycles per M=128, K=16 MMA at
 // N <= 64) in the wide layers, by the row hand-overs in the narrow ones.
-// The eleven layers at 1920x1080, back to back: 984 us (2,157 us with one
+// The eleven layers at 1920x1080, back to back: 880-910 us (2,157 us with one
 // lane-0 issuer looping over the steps, one epilogue group and cp.async
-// producers); 96 -> 32 channels 167 us, 686 TFLOP/s (472 us, 243).
+// producers); 96 -> 32 channels 172-191 us, 600-667 TFLOP/s (472 us, 243).
+// ncu: tensor pipe 13 % busy (N = 16) to 41 % (64 -> 64), DRAM 6-48 %.
 namespace tc {
 constexpr int PLANE = HALO_W * 16;  // one 8-channel chunk of one row
 // a row slot, on the 128-byte boundary that a TMA box needs
@@ -731,7 +735,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t (&r)[N], uint32_t addr) {
         : "r"(addr));
 }
 
-// 32 bytes (one sector) to a 32-byte aligned address
 // CW floats from a 32-byte aligned address (not through the read-only path:
 // the kernel before wrote them)
 template <int CW>
@@ -744,6 +747,7 @@ __device__ __forceinline__ void ld_global_floats(float (&v)[CW], const float* p)
                  : "l"(p + k));
 }
 
+// 32 bytes (one sector) to a 32-byte aligned address
 __device__ __forceinline__ void st_global_32B(void* p, const uint32_t* v) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -1070,8 +1074,8 @@ __global__ void __launch_bounds__(kWsThreads, ws_min_blocks(NG, ADD)) k_conv_fwd
 // Bound by the MMAs' operand reads at N <= 32 (72 MMAs of about 40 cycles
 // per 128 pixels), by TMA's 16 B per cycle at N >= 64.  The eleven layers'
 // weight gradients at 16 x 128^2 pixels, back to back: 1,510 us with
-// k_conv_wgrad (a block per tap, each reading x and dy again), 371 us here;
-// 96 -> 32 channels 390 -> 68 us.
+// k_conv_wgrad (a block per tap, each reading x and dy again), 304 us here;
+// 96 -> 32 channels 390 -> 52 us.  ncu: tensor pipe 19-41 % busy, DRAM 4-19 %.
 struct WgradArgs {
   int N, H, W, Cin, Cout;
   int tw, tiles;     // pixels per row tile (a multiple of 16), tiles per row
@@ -1422,7 +1426,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(rx_conv_desc d, const bf16* 
 // 4.9e-7 of the float64 sum at 16 x 128^2 pixels, against 1.2e-7).
 // With a thread per channel walking 4096 pixels in series (64 blocks, 32-64
 // busy threads each, one 2-byte load in flight per thread) the eleven layers
-// of a training step took 3,440 us.
+// of a training step's gradients took 3,440 us.
 constexpr int kBiasThreads = 1024, kBiasCluster = 8, kBiasBlocks = 64;
 constexpr int kBiasWidth = 128;  // channel chunks handled side by side, at most
 __global__ void __cluster_dims__(kBiasCluster, 1, 1) __launch_bounds__(kBiasThreads)
@@ -1539,7 +1543,7 @@ __global__ void k_relu_mask(long long P, int C, const bf16* __restrict__ yv, int
 // The same on 8-channel chunks (views whose channel count, stride and offset
 // are multiples of 8): the gradient is read and written only where some
 // output is not positive.  Bound by memory; the ten masks of a 16x128x128
-// training step 203 -> 89 us.
+// training step's gradients 203 -> 89 us.
 __global__ void k_relu_mask_v8(long long P, int C, const bf16* __restrict__ yv, int y_stride, int y_off,
                                bf16* __restrict__ g, int g_stride, int g_off) {
   chain_wait(yv, g);
@@ -1679,7 +1683,7 @@ __global__ void k_pool2_bwd(int N, int H, int W, int C, const bf16* __restrict__
 // The two gradients on 8-channel chunks, one item per chunk of a pooled
 // (small) pixel: the pool's reads its gradient once for four input pixels,
 // the upsample's sums four; float32 sums in the order of the scalar forms.
-// Bound by memory; in a 16x128x128 training step the two pools' gradients
+// Bound by memory; in a 16x128x128 training batch the two pools' gradients
 // 86 -> 15 us, the two upsamples' 52 -> 16.
 __global__ void k_pool2_bwd_v8(int N, int H, int W, int C, const bf16* __restrict__ dy, int dy_stride, int dy_off,
                                bf16* __restrict__ dx, int dx_stride, int dx_off, int accumulate) {
@@ -1979,7 +1983,7 @@ static bool row_map(int N, int H, int W, int cols, int C, int stride, const bf16
 // that a second block does not fit.  Blocks that come up while the kernel
 // before drains would otherwise pair up on the SMs that are free first and
 // leave others idle (and a pair may want all the tensor memory twice): a
-// 16x256x256 training step took 4,050 instead of 3,100 us.
+// 16x256x256 batch's gradients took 4,050 instead of 3,100 us.
 static int sole_block_smem(Ctx* ctx, long long blocks, int smem) {
   return blocks <= ctx->num_sms ? std::max(smem, 233472 / 2) : smem;
 }
@@ -2297,9 +2301,11 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   // Pixels one accumulator sums before it meets the others in dw: the split
   // k_conv_wgrad makes.  The tensor core truncates as it accumulates, so a
   // sum's distance from the exact one grows with this length (1e-6 of it per
-  // 1,300 pixels); with k_conv_wgrad's split the two kernels agree to a few
-  // 1e-7, where one block per SM (1,772 pixels at 16 x 128^2, against 7,944)
-  // left 96 -> 32 channels 1.7e-5 apart.
+  // 1,300 pixels).  With k_conv_wgrad's split (7,944 pixels at 16 x 128^2) the
+  // two kernels agree to a few 1e-7, both 3-7e-6 from float64.  The length is
+  // for that agreement alone: one block per SM (1,772 pixels) was nearer to
+  // float64 (1.3e-6; at 96 -> 32 channels it left k_conv_wgrad's result by
+  // 1.7e-5) and faster (296 against 371 us, both with M = 128).
   const int chain = wgrad_chain(ctx, d);
   const long long total = (long long)d->N * d->H * A.tiles;
   const long long per_cta = std::max<long long>(1, (long long)chain * A.tiles / d->W);
@@ -2309,7 +2315,7 @@ static int launch_wgrad_ws(Ctx* ctx, const rx_conv_desc* d, const bf16* dy, cons
   // (MMAs: about 40 each up to N = 32, N / 2 above, and 28 and 44 for N = 32
   // and 64 with M = 64, half the channels to read; TMA: 16 B per cycle), the
   // rows of a block and the rounds of blocks.  M = 64 for up to 64 channels
-  // took the eleven layers of a 16x128x128 step from 346 to 296 us.
+  // took the eleven layers of a 16x128x128 batch from 346 to 299 us.
   const int mg_min = (d->Cin + 127) / 128;
   double best = 0.0;
   for (int mg = mg_min; mg <= 4 * mg_min && (mg == mg_min || d->Cin / mg >= 16); ++mg)

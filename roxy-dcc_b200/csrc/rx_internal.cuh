@@ -110,7 +110,7 @@ struct DevScene {
   const float4* nodes4;    // n_nodes4 * 8: the same tree 4-wide (LBVH builds), or null
   int n_nodes4;
   float3 root_min, root_max;
-  const float4* prims;     // n_prims * 3
+  const float4* prims;     // n_prims * kPrimQuads
   const float4* shade;     // n_prims * 3
   int n_prims;
   const float4* mat_a;     // (albedo, type bits)
